@@ -111,9 +111,13 @@ SweepConst make_sweep_const(const FsgProbe* p, const FsgMedium* m, const FsgFreq
 
 static size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 
+// The shortest band of a sweep: the anchor tables hold a row per band.  simus_lane_kernel's largest
+// band is 24 to 52 frequencies, whatever the probe (lane_layout).
+constexpr int kMinBand = 24;
+
 size_t tables_bytes(int E, int U, int F) {
   const int n_src = E * U;
-  const int n_anchor = (F + kAnchor - 1) / kAnchor;
+  const int n_anchor = (F + kMinBand - 1) / kMinBand;
   size_t b = 0;
   b += align256((size_t)n_src * 16);
   b += align256((size_t)E * 8);
@@ -130,7 +134,7 @@ size_t tables_bytes(int E, int U, int F) {
 
 Tables carve_tables(unsigned char* base, int E, int U, int F) {
   const int n_src = E * U;
-  const int n_anchor = (F + kAnchor - 1) / kAnchor;
+  const int n_anchor = (F + kMinBand - 1) / kMinBand;
   Tables t;
   size_t o = 0;
   t.src_pos = reinterpret_cast<float4*>(base + o); o += align256((size_t)n_src * 16);
@@ -147,12 +151,13 @@ Tables carve_tables(unsigned char* base, int E, int U, int F) {
 }
 
 int launch_setup(const FsgProbe* p, const FsgMedium* m, const FsgFreqPlan* plan, const double* delays,
-                 const double* apod, const Tables& t, cudaStream_t stream) {
+                 const double* apod, const Tables& t, int anchor_step, cudaStream_t stream) {
   SetupArgs a;
   a.E = p->n_elements;
   a.U = p->n_sub;
   a.F = plan->n_freq;
-  a.n_anchor = (plan->n_freq + kAnchor - 1) / kAnchor;
+  a.anchor_step = anchor_step;
+  a.n_anchor = (plan->n_freq + anchor_step - 1) / anchor_step;
   a.pitch = p->pitch;
   a.width = p->element_width;
   a.radius = p->radius;
@@ -216,8 +221,10 @@ static int choose_plane_pad(int E, int U, int gn, int st) {
   return best_pad;
 }
 
-// Geometry cache per chunk: sized to stay resident in L2 while every band's CTAs read it.
-constexpr size_t kGeoCacheBudget = size_t(48) << 20;
+// Geometry cache per chunk: sized to stay resident in the 129 MB L2 while every band's CTAs read it
+// (200,000 scatterers x 128 elements: 26.37 ms at 48 MiB, 26.11 at 80, 26.00 at 112: fewer chunks,
+// fewer launches and tails).
+constexpr size_t kGeoCacheBudget = size_t(112) << 20;
 
 // Grid of one simus chunk: every (band, tile) unit is one CTA's work at most.
 static int simus_grid(int n_bands, int64_t chunk_tiles, int num_sms) {
@@ -225,40 +232,53 @@ static int simus_grid(int n_bands, int64_t chunk_tiles, int num_sms) {
   return (int)(units < num_sms ? units : num_sms);
 }
 
-// Simus sweep shape.  The scatterers are processed in chunks of chunk_tiles tiles, so that the
-// chunk's geometry cache (chunk_tiles * geo_bytes) stays below cache_budget.  A chunk's
-// n_bands x chunk_tiles (band, tile) units are split evenly over min(num_sms, units) CTAs in
-// band-major order: every SM gets the same work whatever the band count divides into, and a
-// CTA whose share crosses a band boundary sweeps two bands one after the other.  n_slices
-// bounds the number of CTAs that share a band (the partial-spectrum slots per band) for any
-// chunk size: a band's ct units hold fewer than ceil(grid / n_bands) CTA starts besides its
-// first unit's CTA.
-// simus_stash_kernel shape: the fewest lanes per point (GN) whose element slots cover the probe
-// (16 source slots per lane; one, two or four per element for U = 1, 2, 3-4), with bands of
-// kTxAnchor frequencies, else of kAnchor, such that the shared memory fits.  False when no
-// shape fits (simus_band_kernel takes those probes).
-static bool stash_shape(int E, int U, int ffd, SweepConfig* c) {
+// Shape of the sweep kernel and its bands for a probe; false when no kernel maps it.
+//
+// simus_lane_kernel takes probes of more than 32 elements with up to four sub-elements: the bands
+// are as many as the largest that fits shared memory asks for, of equal length.  A launch of few
+// tiles (`tiles` > 0: all of them) takes the band length, down to kMinBand, that leaves the SMs
+// the least work after rounding to whole (band, tile) units; kBandCost stands for a unit's
+// anchors in frequency steps.
+//
+// simus_stash_kernel: the fewest lanes per point (GN) whose element slots cover the probe
+// (16 source slots per lane; one, two, four or eight per element for U = 1, 2, 3-4, 5-8), with
+// bands of kTxAnchor frequencies, else of kAnchor, such that the shared memory fits.
+constexpr int kBandCost = 6;
+static bool sweep_shape(int E, int U, int F, int64_t tiles_of_points, int num_sms, int ffd, SweepConfig* c) {
   if (U < 1 || U > 8) return false;
+  if (E > 32 && U <= 4) {
+    const int nw = (E + 63) / 64, threads = lane_threads(nw, ffd != 0), groups = threads / (32 * nw);
+    const int fs = 16 / lane_points(U);
+    int top = fs;
+    while (lane_layout(nw, top + fs, threads, ffd != 0).total <= kMaxDynSmem - 1024) top += fs;
+    c->kind = 2;
+    c->nw = nw;
+    c->gn = 0;
+    c->plane_pad = 0;
+    c->st = groups * lane_points(U);
+    const int64_t tiles = (tiles_of_points + c->st - 1) / c->st;
+    auto even = [&](int nb) { return ((F + nb - 1) / nb + fs - 1) / fs * fs; };
+    const int nb0 = (F + top - 1) / top;
+    int best = even(nb0);
+    int64_t best_cost = INT64_MAX;
+    for (int nb = nb0; tiles > 0 && tiles * nb <= 16 * (int64_t)num_sms; ++nb) {
+      const int fb = even(nb);
+      if (nb > nb0 && fb < kMinBand) break;
+      const int64_t per = (tiles * ((F + fb - 1) / fb) + num_sms - 1) / num_sms, cost = per * (fb + kBandCost);
+      if (cost < best_cost) {
+        best_cost = cost;
+        best = fb;
+      }
+    }
+    c->fb = best;
+    if ((F + best - 1) / best > (F + kMinBand - 1) / kMinBand) return false;
+    c->smem = lane_layout(nw, best, threads, ffd != 0).total;
+    const size_t slots = (size_t)groups * U * lane_points(U) * 32 * nw;
+    c->geo_bytes = align16(slots * (ffd ? 48 : 40) + (size_t)c->st * 4);
+    return true;
+  }
   const int spe = U == 1 ? 1 : (U == 2 ? 2 : (U <= 4 ? 4 : 8));
   const int epl = kSrcPerThread / spe;
-  // the warp-specialised kernel: E = 64, 128 (U <= 4) or 256 (U <= 2); 128 transmit threads
-  if ((E == 64 || E == 128 || E == 256) && U <= (E == 256 ? 2 : 4)) {
-    int gn = E * spe / kSrcPerThread;
-    if (gn < 4) gn = 4;
-    const int st = 128 / gn, fb = E > 128 ? 32 : 64;
-    const int pad = choose_plane_pad(E, U, gn, st);
-    const WsLayout L = ws_layout(st, fb, E, U, pad, ffd != 0);
-    if (gn <= 32 && L.total <= kMaxDynSmem - 1024) {
-      c->kind = 2;
-      c->gn = gn;
-      c->st = st;
-      c->fb = fb;
-      c->plane_pad = pad;
-      c->smem = L.total;
-      c->geo_bytes = L.g.geo_bytes;
-      return true;
-    }
-  }
   for (int fb = kTxAnchor; fb >= kAnchor; fb /= 2) {
     for (int gn = 4; gn <= 32; gn *= 2) {
       if (gn * epl < E) continue;
@@ -267,6 +287,7 @@ static bool stash_shape(int E, int U, int ffd, SweepConfig* c) {
       const StashLayout L = stash_layout(st, fb, E, U, pad, ffd != 0);
       if (L.total > kMaxDynSmem - 1024) continue;
       c->kind = 1;
+      c->nw = 0;
       c->gn = gn;
       c->st = st;
       c->fb = fb;
@@ -279,24 +300,25 @@ static bool stash_shape(int E, int U, int ffd, SweepConfig* c) {
   return false;
 }
 
-SweepConfig simus_config(int E, int U, int F, int64_t n_scat, int num_sms, size_t cache_budget, int ffd) {
+// Simus sweep.  The scatterers are processed in chunks of chunk_tiles tiles, so that the
+// chunk's geometry cache (chunk_tiles * geo_bytes) stays below cache_budget.  A chunk's
+// n_bands x chunk_tiles (band, tile) units are split evenly over min(num_sms, units) CTAs in
+// band-major order: every SM gets the same work whatever the band count divides into, and a
+// CTA whose share crosses a band boundary sweeps two bands one after the other.  n_slices
+// bounds the number of CTAs that share a band (the partial-spectrum slots per band) for any
+// chunk size: a band's ct units hold fewer than ceil(grid / n_bands) CTA starts besides its
+// first unit's CTA.
+// short_bands: the lane kernel's bands of kAnchor frequencies, whose slots take the least memory.
+SweepConfig simus_config(int E, int U, int F, int64_t n_scat, int num_sms, size_t cache_budget, int ffd,
+                         bool short_bands = false) {
   SweepConfig c;
-  if (!stash_shape(E, U, ffd, &c)) {
-    const int n_src = E * U;
-    c.kind = 0;
-    c.gn = next_pow2((n_src + kSrcPerThread - 1) / kSrcPerThread);
-    if (c.gn < 4) c.gn = 4;
-    c.st = kThreads / c.gn;
-    int runs = kThreads / E;
-    if (runs > 4) runs = 4;
-    c.fb = kAnchor * runs;
-    c.plane_pad = choose_plane_pad(E, U, c.gn, c.st);
-    const SmemLayout L = smem_layout(c.st, c.fb, E, U, c.plane_pad, true, ffd != 0);
-    c.smem = L.total;
-    c.geo_bytes = L.geo_bytes;
+  memset(&c, 0, sizeof(c));
+  if (!sweep_shape(E, U, F, n_scat, num_sms, ffd, &c)) return c;  // kind 0
+  if (short_bands && c.kind == 2 && c.fb > kAnchor) {
+    c.fb = kAnchor;
+    c.smem = lane_layout(c.nw, c.fb, lane_threads(c.nw, ffd != 0), ffd != 0).total;
   }
   c.n_bands = (F + c.fb - 1) / c.fb;
-  c.per_slice = 0;
   const int64_t tiles = n_scat > 0 ? (n_scat + c.st - 1) / c.st : 1;
   int64_t ct = (int64_t)(cache_budget / c.geo_bytes);
   if (ct < 1) ct = 1;
@@ -309,7 +331,7 @@ SweepConfig simus_config(int E, int U, int F, int64_t n_scat, int num_sms, size_
 
 SweepConfig pfield_config(int E, int U, int F, int64_t n_pts, int num_sms, int ffd) {
   SweepConfig c;
-  c.kind = 0;
+  memset(&c, 0, sizeof(c));
   const int n_src = E * U;
   c.gn = next_pow2((n_src + kSrcPerThread - 1) / kSrcPerThread);
   if (c.gn < 4) c.gn = 4;
@@ -350,24 +372,50 @@ static size_t simus_ws_size(const SweepConfig& c, int E, int U, int F) {
 }
 
 // The default workspace, large enough with or without full-frequency directivity (whose
-// geometry block carries one more array).
+// geometry block carries one more array) and with the slots of the longest bands, so that a
+// workspace sized for few scatterers also holds the fixed part for many.
 static size_t simus_ws_size(const FsgProbe* probe, const FsgFreqPlan* plan, int64_t n_scat, int num_sms) {
   size_t need = 0;
+  const int E = probe->n_elements, U = probe->n_sub, F = plan->n_freq;
   for (int ffd = 0; ffd < 2; ++ffd) {
-    SweepConfig c = simus_config(probe->n_elements, probe->n_sub, plan->n_freq, n_scat, num_sms, kGeoCacheBudget, ffd);
-    const size_t n = simus_ws_size(c, probe->n_elements, probe->n_sub, plan->n_freq);
+    SweepConfig c = simus_config(E, U, F, n_scat, num_sms, kGeoCacheBudget, ffd);
+    const int slots = simus_config(E, U, F, 0, num_sms, 0, ffd).n_slices;
+    if (slots > c.n_slices) c.n_slices = slots;
+    const size_t n = simus_ws_size(c, E, U, F);
     if (n > need) need = n;
   }
   return need;
 }
 
-// The smallest workspace fsg_simus runs in for this request: the fixed part (tables, status
-// word, partial spectra) plus the geometry cache of one tile, i.e. chunks of one tile each.
-// fsg_simus shrinks its chunks to whatever a smaller-than-default workspace holds above this.
+// The sweep of a request within a workspace of `bytes`: the default shape, in smaller chunks of
+// scatterers if its geometry cache does not fit; else bands of kAnchor frequencies; else also
+// fewer CTAs, down to one slot per band beyond the first.  False when nothing fits; c is then the
+// smallest.  *grid_cap: the CTAs that the slots allow.
+static bool simus_fit(int E, int U, int F, int64_t n_scat, int num_sms, int ffd, size_t bytes, SweepConfig* c,
+                      int* grid_cap) {
+  *grid_cap = num_sms;
+  *c = simus_config(E, U, F, n_scat, num_sms, kGeoCacheBudget, ffd);
+  if (c->kind == 0 || simus_ws_size(*c, E, U, F) <= bytes) return true;
+  for (int cut = 0; cut < 2; ++cut) {
+    *c = simus_config(E, U, F, n_scat, num_sms, 0, ffd, cut != 0);
+    const size_t fixed = simus_ws_size(*c, E, U, F) - align256(c->geo_bytes);
+    if (bytes >= fixed + align256(c->geo_bytes)) {
+      *c = simus_config(E, U, F, n_scat, num_sms, (bytes - fixed) & ~size_t(255), ffd, cut != 0);
+      return true;
+    }
+  }
+  while (c->n_slices > 2 && simus_ws_size(*c, E, U, F) > bytes) {
+    --c->n_slices;
+    *grid_cap = (c->n_slices - 1) * c->n_bands;
+  }
+  return simus_ws_size(*c, E, U, F) <= bytes;
+}
+
 size_t fsg::simus_min_workspace(const FsgProbe* probe, const FsgFreqPlan* plan, int64_t n_scat, int ffd, int num_sms) {
-  const int E = probe->n_elements, U = probe->n_sub, F = plan->n_freq;
-  SweepConfig c = simus_config(E, U, F, n_scat, num_sms, 0, ffd);  // a zero budget gives one-tile chunks
-  return simus_ws_size(c, E, U, F);
+  SweepConfig c;
+  int cap = 0;
+  simus_fit(probe->n_elements, probe->n_sub, plan->n_freq, n_scat, num_sms, ffd, 0, &c, &cap);
+  return simus_ws_size(c, probe->n_elements, probe->n_sub, plan->n_freq);
 }
 
 extern "C" size_t fsg_simus_workspace_size(const FsgProbe* probe, const FsgFreqPlan* plan, int64_t n_scat) {
@@ -405,21 +453,17 @@ extern "C" int32_t fsg_simus(const FsgProbe* probe, const FsgMedium* medium, con
   int sms = 0;
   if ((st = device_sm_count(&sms)) != FSG_OK) return st;
   const int E = probe->n_elements, U = probe->n_sub, F = plan->n_freq;
-  // the default chunking, or smaller chunks when the caller's workspace is smaller
-  SweepConfig c = simus_config(E, U, F, n_scat, sms, kGeoCacheBudget, ffd);
-  if (c.kind == 0 && U > 4)
+  SweepConfig c;
+  int grid_cap = 0;
+  const bool fits = simus_fit(E, U, F, n_scat, sms, ffd, workspace ? workspace_bytes : 0, &c, &grid_cap);
+  if (c.kind == 0)
     return set_error(FSG_EUNSUPPORTED,
                      "n_sub = %d > 4 is supported for probes whose 8-slot elements map onto 32 lanes "
                      "(n_elements <= 64); got n_elements = %d",
                      U, E);
-  if (workspace && workspace_bytes < simus_ws_size(c, E, U, F)) {
-    const size_t fixed = simus_ws_size(c, E, U, F) - align256((size_t)c.chunk_tiles * c.geo_bytes);
-    if (workspace_bytes > fixed) c = simus_config(E, U, F, n_scat, sms, workspace_bytes - fixed - 256, ffd);
-  }
-  const size_t need = simus_ws_size(c, E, U, F);
-  if (!workspace || workspace_bytes < need)
+  if (!workspace || !fits)
     return set_error(FSG_EWORKSPACE, "workspace of %zu bytes is smaller than the %zu bytes required", workspace_bytes,
-                     need);
+                     simus_ws_size(c, E, U, F));
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_ptr);
   unsigned char* ws = static_cast<unsigned char*>(workspace);
   Tables t = carve_tables(ws, E, U, F);
@@ -427,7 +471,9 @@ extern "C" int32_t fsg_simus(const FsgProbe* probe, const FsgMedium* medium, con
   float2* partial = reinterpret_cast<float2*>(ws + tables_bytes(E, U, F) + 256);
   unsigned char* geo = reinterpret_cast<unsigned char*>(partial) + align256((size_t)c.n_slices * F * E * 8);
   if ((st = check_cuda(cudaMemsetAsync(status, 0, sizeof(int), s), "status reset")) != FSG_OK) return st;
-  if ((st = launch_setup(probe, medium, plan, delays, apod, t, s)) != FSG_OK) return st;
+  // the stash kernel's bands start at multiples of kAnchor, the lane kernel's at those of its band length
+  const int anchor_step = c.kind == 2 ? c.fb : kAnchor;
+  if ((st = launch_setup(probe, medium, plan, delays, apod, t, anchor_step, s)) != FSG_OK) return st;
   if (n_scat > 0) {
     BandArgs A;
     A.pts = scat_xz;
@@ -439,6 +485,7 @@ extern "C" int32_t fsg_simus(const FsgProbe* probe, const FsgMedium* medium, con
     A.U = U;
     A.n_src = E * U;
     A.gn = c.gn;
+    A.nw = c.nw;
     A.plane_pad = c.plane_pad;
     A.st = c.st;
     A.fb = c.fb;
@@ -459,12 +506,13 @@ extern "C" int32_t fsg_simus(const FsgProbe* probe, const FsgMedium* medium, con
       const int64_t left = tiles - k * c.chunk_tiles;
       const int64_t ct = left < c.chunk_tiles ? left : c.chunk_tiles;
       A.chunk_tiles = ct;
-      A.grid = simus_grid(c.n_bands, ct, sms);
+      A.grid = simus_grid(c.n_bands, ct, grid_cap);
       const int64_t cap = (int64_t)sms * 8;
       const int blocks = (int)(ct < cap ? ct : cap);
-      geometry_kernel<<<blocks, kThreads, 0, s>>>(A, ct);
+      if (c.kind == 2) lane_geometry_kernel<<<blocks, kThreads, 0, s>>>(A, ct);
+      else geometry_kernel<<<blocks, kThreads, 0, s>>>(A, ct);
       if ((st = check_cuda(cudaGetLastError(), "geometry_kernel launch")) != FSG_OK) return st;
-      if ((st = check_cuda(launch_simus_band_any(U, c, A, s), "simus_band_kernel launch")) != FSG_OK) return st;
+      if ((st = check_cuda(launch_simus_any(U, c, A, s), "simus sweep launch")) != FSG_OK) return st;
     }
   }
   const int full = out_layout == FSG_OUT_FULL_CORRECTED;
@@ -472,7 +520,7 @@ extern "C" int32_t fsg_simus(const FsgProbe* probe, const FsgMedium* medium, con
   const int64_t n_out = (int64_t)rows * E;
   simus_reduce<<<(unsigned)((n_out + 255) / 256), 256, 0, s>>>(
       partial, n_scat > 0 ? c.n_slices : 0, F, E, t.probe, full ? (float)plan->correction_factor : 1.0f, full, rows,
-      plan->freq_idx_start, status, c.kind >= 1 ? delays : nullptr, plan->freq_start, plan->freq_step,
+      plan->freq_idx_start, status, delays, plan->freq_start, plan->freq_step,
       static_cast<float2*>(out));
   return check_cuda(cudaGetLastError(), "simus_reduce launch");
 }
@@ -507,7 +555,7 @@ extern "C" int32_t fsg_pfield(const FsgProbe* probe, const FsgMedium* medium, co
   unsigned char* ws = static_cast<unsigned char*>(workspace);
   Tables t = carve_tables(ws, E, U, F);
   float* partial = reinterpret_cast<float*>(ws + tables_bytes(E, U, F));
-  if ((st = launch_setup(probe, medium, plan, delays, apod, t, s)) != FSG_OK) return st;
+  if ((st = launch_setup(probe, medium, plan, delays, apod, t, kAnchor, s)) != FSG_OK) return st;
   SweepConfig c = pfield_config(E, U, F, n_points, sms, ffd);
   BandArgs A;
   A.pts = points;

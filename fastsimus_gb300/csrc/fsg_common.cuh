@@ -118,9 +118,9 @@ __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(
 // in separate pairs (gr, gi) and the steps as (sr, si, sn = -si).  Four packed instructions
 // replace eight scalar ones; each lane rounds exactly like the scalar fmaf/mul sequence.
 __device__ __forceinline__ void cstep2(float2& gr, float2& gi, float2 sr, float2 si, float2 sn) {
-  const float2 tr = __fmul2_rn(gr, sr);
+  const float2 tr = __fmul2_rn(gi, sn);
   const float2 ti = __fmul2_rn(gi, sr);
-  const float2 nr = __ffma2_rn(gi, sn, tr);  // gr sr - gi si
+  const float2 nr = __ffma2_rn(gr, sr, tr);  // gr sr - gi si
   const float2 ni = __ffma2_rn(gr, si, ti);  // gr si + gi sr
   gr = nr;
   gi = ni;

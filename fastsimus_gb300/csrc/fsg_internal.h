@@ -25,6 +25,7 @@ struct Tables {
 
 struct SetupArgs {
   int E, U, F, n_anchor;
+  int anchor_step;     // frequencies between the rows of da / dph
   double pitch, width, radius, c, att, f0, df, seg;
   const double* delays;
   const double* apod;
@@ -41,13 +42,15 @@ struct BandArgs {
   Tables t;
   SweepConst C;
   int E, U, n_src, gn, st, fb, F, n_anchor;
+  int nw;              // simus_lane_kernel: warps per group
   int plane_pad;       // extra words between the sub-element planes of the geometry arrays
   int convex;
   double apex, radius2;
   void* partial;       // simus: float2 [slots][F][E], zeroed, accumulated; pfield: float [bands][n_pts]
   // simus: scatterers are processed in chunks; the geometry of a chunk's tiles is computed
-  // once by geometry_kernel into `geo` (one SmemLayout geometry block of geo_bytes per tile)
-  // and copied into shared memory by each band's CTA with a TMA bulk copy
+  // once into `geo`, geo_bytes per tile: by geometry_kernel as one SmemLayout geometry block that
+  // each band's CTA copies into shared memory with a TMA bulk copy (simus_stash_kernel), or by
+  // lane_geometry_kernel in lane_block order, read straight into registers (simus_lane_kernel)
   unsigned char* geo;
   size_t geo_bytes;
   int64_t chunk_s0;    // first scatterer of the chunk (pts / rc are indexed globally)
@@ -131,30 +134,30 @@ __host__ __device__ inline StashLayout stash_layout(int st, int fb, int E, int U
   return S;
 }
 
-// simus_ws_kernel: the tile's geometry block from offset 0, then two stash buffers
-// [stx][kStashFreqs][ep], two W buffers [stx][kStashFreqs] and the band tables.
-struct WsLayout {
-  SmemLayout g;  // the tile's geometry block, from offset 0
-  int ep;
-  size_t off_stash, off_w, off_pp, off_kb, off_dph, off_dstep, total;
+// simus_lane_kernel: scatterers per group and tile (16 source slots per thread: two elements of
+// lane_points scatterers, all sub-elements; 16 / lane_points frequencies per sub-block), and its
+// shared memory: the groups' running spectra, then the band tables and the hand-over buffers.
+__host__ __device__ constexpr int lane_points(int U) { return U <= 2 ? 4 : 2; }
+__host__ __device__ constexpr int lane_threads(int nw, bool ffd) { return ffd && nw != 3 ? 256 : 384; }
+constexpr int kLaneTrPitch = 18;  // complex per lane row of the transpose buffer (16 values)
+struct LaneLayout {
+  size_t off_pp, off_kb, off_part, off_w, off_tr, total;
 };
-__host__ __device__ inline WsLayout ws_layout(int stx, int fb, int E, int U, int plane_pad, bool ffd) {
-  WsLayout S;
-  S.g = smem_layout(stx, fb, E, U, plane_pad, true, ffd);
-  S.ep = E | 1;
-  size_t o = (S.g.geo_bytes + 127) & ~size_t(127);
-  S.off_stash = o; o = align16(o + 2 * (size_t)stx * kStashFreqs * S.ep * 8);
-  S.off_w = o; o = align16(o + 2 * (size_t)stx * kStashFreqs * 8);
+__host__ __device__ inline LaneLayout lane_layout(int nw, int fb, int threads, bool ffd) {
+  LaneLayout S;
+  size_t o = (size_t)fb * threads * 16;
   S.off_pp = o; o = align16(o + (size_t)fb * 8);
   S.off_kb = o; o = align16(o + (ffd ? (size_t)fb * 4 : 0));
-  S.off_dph = o; o = align16(o + (size_t)E * 8);
-  S.off_dstep = o; o = align16(o + (size_t)E * 8);
+  S.off_part = o; o += nw > 1 ? (size_t)(threads / 32) * 2 * 16 * 8 : 0;
+  S.off_w = o; o += (size_t)(threads / 32) * 2 * 16 * 8;
+  S.off_tr = o; o += (size_t)threads * kLaneTrPitch * 8;
   S.total = o;
   return S;
 }
 
 struct SweepConfig {
-  int kind;            // simus: 0 = simus_band_kernel, 1 = simus_stash_kernel
+  int kind;            // simus: 0 = no kernel maps the probe, 1 = simus_stash_kernel, 2 = simus_lane_kernel
+  int nw;              // simus_lane_kernel: warps per group
   int gn, st, fb, n_bands, plane_pad;
   int n_slices;        // pfield: point slices; simus: partial-spectrum slots per band
   int64_t per_slice;   // pfield: points per slice
@@ -167,9 +170,13 @@ struct SweepConfig {
 __global__ void setup_tables(SetupArgs a);
 // Geometry of every (scatterer, source) of one chunk into A.geo (tile-major SmemLayout blocks).
 __global__ void geometry_kernel(const BandArgs A, int64_t chunk_tiles);
-// Launches simus_band_kernel<U> or simus_stash_kernel<U> (U = n_sub in 1..4), as c.kind says,
-// with c's grid and shared memory.
-cudaError_t launch_simus_band_any(int U, const SweepConfig& c, const BandArgs& A, cudaStream_t s);
+// The same for simus_lane_kernel's blocks.
+__global__ void lane_geometry_kernel(const BandArgs A, int64_t chunk_tiles);
+// Launches simus_lane_kernel<U> or simus_stash_kernel<U>, as c.kind says, with c's grid and
+// shared memory.
+cudaError_t launch_simus_any(int U, const SweepConfig& c, const BandArgs& A, cudaStream_t s);
+cudaError_t launch_simus_lane(int U, const SweepConfig& c, const BandArgs& A, cudaStream_t s);
+cudaError_t launch_simus_lane_ffd(int U, const SweepConfig& c, const BandArgs& A, cudaStream_t s);
 cudaError_t launch_simus_stash(int U, const SweepConfig& c, const BandArgs& A, cudaStream_t s);
 cudaError_t launch_simus_stash_ffd(int U, const SweepConfig& c, const BandArgs& A, cudaStream_t s);
 // Launches pfield_band_kernel<gn> with c's grid and shared memory.

@@ -3,15 +3,13 @@
 // in fsg_sweep_kernels.cuh.
 //
 // simus, per chunk of scatterers:
-//   geometry_kernel    once per (scatterer, source): double-float distance, amplitude
+//   geometry           once per (scatterer, source): double-float distance, amplitude
 //                      (obliquity x centre-frequency sinc / sqrt(r) / n_sub), recurrence step
 //                      (and half_seg sin(theta) with full-frequency directivity), written as
-//                      one shared-memory-layout block per tile into an L2-sized cache;
-//   simus_band_kernel  one CTA per SM, each sweeping an even share of the chunk's (band, tile)
-//                      units; per tile: TMA bulk copy of the tile's block, TX (packed FP32x2
-//                      recurrences, reduce-scatter of the source sums across the point's lanes,
-//                      W[s][f] = rc pulse probe P), RX (thread = element x 32 frequencies,
-//                      Y[e][f] += W[s][f] mean_u G), added into the band's partial slot;
+//                      one block per tile into an L2-sized cache (geometry_kernel here for
+//                      simus_stash_kernel, lane_geometry_kernel for simus_lane_kernel);
+//   sweep              simus_lane_kernel or simus_stash_kernel, one CTA per SM, each sweeping an
+//                      even share of the chunk's (band, tile) units into the band's partial slot;
 // then simus_reduce sums the slots' partial spectra in a fixed order.  Neither the
 // scatterer x element Green's tile nor W ever leaves the SM.
 // pfield: pfield_band_kernel computes its geometry in place (one band for large grids) and
@@ -75,7 +73,7 @@ __global__ void setup_tables(SetupArgs a) {
     double tau = a.delays[e];
     double w = a.apod ? a.apod[e] : 1.0;
     if (isnan(tau)) { tau = 0.0; w = 0.0; }
-    double f = a.f0 + (double)m * kAnchor * a.df;
+    double f = a.f0 + (double)m * a.anchor_step * a.df;
     double s, c;
     sincos(2.0 * kPi * f * tau, &s, &c);
     a.t.da[i] = make_float2((float)(w * c), (float)(w * s));
@@ -159,9 +157,9 @@ __global__ void pfield_reduce(const float* __restrict__ partial, int n_bands, in
   out[i] = sqrtf(acc * corr);
 }
 
-cudaError_t launch_simus_band_any(int U, const SweepConfig& c, const BandArgs& A, cudaStream_t s) {
-  if (c.kind >= 1) return A.C.ffd ? launch_simus_stash_ffd(U, c, A, s) : launch_simus_stash(U, c, A, s);
-  return A.C.ffd ? launch_simus_band_ffd(U, c, A, s) : launch_simus_band_u<false>(U, c, A, s);
+cudaError_t launch_simus_any(int U, const SweepConfig& c, const BandArgs& A, cudaStream_t s) {
+  if (c.kind == 2) return launch_simus_lane(U, c, A, s);
+  return A.C.ffd ? launch_simus_stash_ffd(U, c, A, s) : launch_simus_stash(U, c, A, s);
 }
 
 cudaError_t launch_pfield_band_any(const SweepConfig& c, const BandArgs& A, cudaStream_t s) {

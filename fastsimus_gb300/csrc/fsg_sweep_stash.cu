@@ -4,7 +4,6 @@
 namespace fsg {
 
 cudaError_t launch_simus_stash(int U, const SweepConfig& c, const BandArgs& A, cudaStream_t s) {
-  if (c.kind == 2) return launch_simus_ws_any<false>(U, c, A, s);
   return launch_simus_stash_u<false>(U, c, A, s);
 }
 
