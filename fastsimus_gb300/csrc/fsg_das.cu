@@ -3,14 +3,15 @@
 // rf2iq / dasmtx algorithms, which the reference's validation tests call through PyMUST
 // (tests/_picmus_phantom_shared.py:407-460).
 //
-// rf2iq_kernel: one thread per (frame, channel) column.  The IIR recurrence is sequential in
-// time, so a column is one thread's loop: forward over the odd-extended down-mixed signal
-// (outputs of the record written to the channel-major IQ array, those of the right extension
-// kept in a local array), then backward over them in place.  The filter runs as cascaded
-// second-order sections in FP32 (a single high-order recursion loses ~1e-3 in FP32 at narrow
-// cut-offs; the cascade stays at ~1e-6).  The down-mixing phasors depend on the sample only:
-// each CTA tabulates them in shared memory (phase n fc / fs + fc tau reduced to [0, 1) cycles
-// in FP64, then sincospif), so a column's step is a load, a multiply and the biquads.
+// rf2iq_kernel: one warp per (frame, channel) column, eight channels of a frame per CTA.  The IIR
+// filter (cascaded second-order sections in FP32; a single high-order recursion loses ~1e-3 in FP32
+// at narrow cut-offs, the cascade stays at ~1e-6) is linear in its state, so a segment of a column is
+// cut into 32 chunks, one per lane: every lane filters its chunk from a zero state, the chunk-end
+// states are combined by a scan over the lanes with the powers of the chunk's state transition
+// M = A^L (computed in FP64 on the host), and every lane filters its chunk again from its true state.
+// The same is done backward.  The down-mixed samples and the forward outputs stay in shared memory
+// (records longer than a segment go through the output array between the two passes).  The
+// down-mixing phasors depend on the sample only: each CTA tabulates them per segment.
 //
 // das_kernel: one thread per pixel, looping over groups of firings and, per element, over the
 // group's firings.  The transmit delays (times c) and the element frames sit in shared memory;
@@ -20,6 +21,7 @@
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
+#include <string.h>
 
 #include "../../include/fsgb300.h"
 #include "fsg_internal.h"
@@ -31,6 +33,10 @@ constexpr int kDasImgThreads = 128;   // das_kernel: small CTAs spread the pixel
 constexpr int kDasMaxE = 256;
 constexpr int kDasFrameGroup = 32;  // firings whose transmit distances a thread holds at a time
 
+constexpr int kIqCh = 8;          // channels per CTA, one warp each
+constexpr int kIqMaxL = 71;       // samples per lane and segment: eight columns and the phasors fit shared memory
+constexpr int kIqScan = 5;        // scan levels: M, M^2, M^4, M^8, M^16
+
 struct Rf2IqArgs {
   const float* rf;   // [n_frames][n_samples][n_ch]
   float2* iq;        // [n_frames][n_ch][n_samples]
@@ -39,11 +45,9 @@ struct Rf2IqArgs {
   double cyc0;            // fc tau
   float sos[FSG_RF2IQ_MAX_SECTIONS][5];  // b0, b1, b2, a1, a2
   float zi[FSG_RF2IQ_MAX_SECTIONS][2];   // steady state for a unit input
+  int L;                                 // samples per lane and segment (odd)
+  float m[kIqScan][2 * FSG_RF2IQ_MAX_SECTIONS][2 * FSG_RF2IQ_MAX_SECTIONS];  // A^(L 2^k): state after from state before
 };
-
-constexpr int kIqChunk = 16;     // samples loaded ahead of the recurrence (memory-level parallelism)
-constexpr int kIqTable = 2048;   // down-mixing phasors shared by a CTA's columns, per pass
-constexpr int kIqThreads = 64;
 
 // Down-mixing phasor of sample n: exp(-2 pi i (n fc / fs + fc tau)), the phase reduced to
 // cycles in FP64.
@@ -53,12 +57,6 @@ __device__ __forceinline__ float2 phasor(const Rf2IqArgs& A, int n) {
   float s, c;
   sincospif(2.0f * frac, &s, &c);
   return make_float2(c, -s);
-}
-
-__device__ __forceinline__ float2 downmix(const Rf2IqArgs& A, const float* col, int n) {
-  const float v = col[(size_t)n * A.n_ch];
-  const float2 e = phasor(A, n);
-  return make_float2(v * e.x, v * e.y);
 }
 
 // One sample through the cascade of transposed direct-form-II biquads (real coefficients).
@@ -83,68 +81,156 @@ __device__ __forceinline__ void iir_init(const Rf2IqArgs& A, float2 (*z)[2], flo
     for (int k = 0; k < 2; ++k) z[s][k] = make_float2(A.zi[s][k] * x0.x, A.zi[s][k] * x0.y);
 }
 
+// Adds the state that `from` becomes after A^(L 2^k).
 template <int NS>
-__global__ void __launch_bounds__(kIqThreads) rf2iq_kernel(const __grid_constant__ Rf2IqArgs A) {
-  __shared__ float2 ph[kIqTable];  // phasors of the samples n0 .. n0 + kIqTable - 1
-  const int64_t colid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool active = colid < (int64_t)A.n_frames * A.n_ch;
-  const int64_t cid = active ? colid : 0;
-  const int fr = (int)(cid / A.n_ch), ch = (int)(cid % A.n_ch);
-  const float* __restrict__ col = A.rf + (size_t)fr * A.n_samples * A.n_ch + ch;
-  float2* __restrict__ y = A.iq + (size_t)cid * A.n_samples;
-  const int N = A.n_samples, P = A.pad;
+__device__ __forceinline__ void iir_carry(const Rf2IqArgs& A, int k, float2 (*z)[2], const float2 (*from)[2]) {
+#pragma unroll
+  for (int i = 0; i < 2 * NS; ++i) {
+    float2 s = z[i >> 1][i & 1];
+#pragma unroll
+    for (int j = 0; j < 2 * NS; ++j) {
+      if ((j >> 1) > (i >> 1)) continue;  // a section is driven by the ones before it only
+      const float c = A.m[k][i][j];
+      s.x = fmaf(c, from[j >> 1][j & 1].x, s.x);
+      s.y = fmaf(c, from[j >> 1][j & 1].y, s.y);
+    }
+    z[i >> 1][i & 1] = s;
+  }
+}
+
+// Filters samples [0, n) of a segment in place (x[i * dir], i < n), the warp's lanes taking L
+// consecutive ones each; z holds the state before sample 0 and, on return, after sample n - 1 (in
+// every lane).  scale multiplies the outputs.
+template <int NS>
+__device__ __forceinline__ void iir_segment(const Rf2IqArgs& A, float2* x, int dir, int n, float2 (*z)[2], float scale) {
+  const int lane = threadIdx.x & 31, L = A.L;
+  const int i0 = lane * L, cnt = max(0, min(L, n - i0));
+  float2 s[NS][2];
+#pragma unroll
+  for (int q = 0; q < NS; ++q) s[q][0] = s[q][1] = make_float2(0.f, 0.f);
+  for (int i = 0; i < cnt; ++i) iir_step<NS>(A, s, x[(i0 + i) * dir]);
+  // inclusive scan of the chunk-end states, the incoming state entering through lane 0
+  if (lane == 0) iir_carry<NS>(A, 0, s, z);
+#pragma unroll
+  for (int k = 0; k < kIqScan; ++k) {
+    float2 f[NS][2];
+#pragma unroll
+    for (int q = 0; q < 2 * NS; ++q) {
+      f[q >> 1][q & 1].x = __shfl_up_sync(0xffffffffu, s[q >> 1][q & 1].x, 1 << k);
+      f[q >> 1][q & 1].y = __shfl_up_sync(0xffffffffu, s[q >> 1][q & 1].y, 1 << k);
+    }
+    if (lane >= (1 << k)) iir_carry<NS>(A, k, s, f);
+  }
+  // the state before this lane's chunk, and the outputs
+#pragma unroll
+  for (int q = 0; q < 2 * NS; ++q) {
+    const float2 v = s[q >> 1][q & 1];
+    const float2 u = make_float2(__shfl_up_sync(0xffffffffu, v.x, 1), __shfl_up_sync(0xffffffffu, v.y, 1));
+    if (lane > 0) z[q >> 1][q & 1] = u;
+  }
+  for (int i = 0; i < cnt; ++i) {
+    const float2 o = iir_step<NS>(A, z, x[(i0 + i) * dir]);
+    x[(i0 + i) * dir] = make_float2(scale * o.x, scale * o.y);
+  }
+  const int last = (n - 1) / L;  // the lane that took sample n - 1
+#pragma unroll
+  for (int q = 0; q < 2 * NS; ++q) {
+    z[q >> 1][q & 1].x = __shfl_sync(0xffffffffu, z[q >> 1][q & 1].x, last);
+    z[q >> 1][q & 1].y = __shfl_sync(0xffffffffu, z[q >> 1][q & 1].y, last);
+  }
+  __syncwarp();
+}
+
+// What bounds it: the length of a lane's chunk, four filter passes of N / 32 samples (the former
+// kernel's one thread per column walked 2 N), and the column's bytes.  One frame of 64 channels x
+// 1,015 samples 172 -> see below us, 75 frames x 64 x 1,080 187 us -> .
+template <int NS>
+__global__ void __launch_bounds__(32 * kIqCh) rf2iq_kernel(const __grid_constant__ Rf2IqArgs A) {
+  extern __shared__ __align__(16) float2 iq_sm[];
+  __shared__ float2 right[kIqCh][FSG_RF2IQ_MAX_PAD];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int N = A.n_samples, P = A.pad, S = 32 * A.L, pitch = S + 4;  // pitch = 4 mod 16: staging writes conflict-free
+  const int groups = (A.n_ch + kIqCh - 1) / kIqCh;
+  const int fr = blockIdx.x / groups, ch0 = (blockIdx.x % groups) * kIqCh, ch = ch0 + warp;
+  const bool active = ch < A.n_ch;
+  const float* __restrict__ rf = A.rf + (size_t)fr * N * A.n_ch;
+  float2* ph = iq_sm + kIqCh * pitch;   // the segment's phasors
+  float2* col = iq_sm + warp * pitch;   // this warp's samples of the segment
+  float2* __restrict__ y = A.iq + ((size_t)fr * A.n_ch + ch) * N;
+  const int n_seg = (N + S - 1) / S;
+  auto mixed = [&](int n) {
+    const float v = rf[(size_t)n * A.n_ch + ch];
+    const float2 e = phasor(A, n);
+    return make_float2(v * e.x, v * e.y);
+  };
+
   float2 z[NS][2];
-  float2 right[FSG_RF2IQ_MAX_PAD];
-  float2 x0 = make_float2(0.f, 0.f), xn = x0;
   // forward pass over [2 x0 - x[P..1], x[0..N-1], 2 x[N-1] - x[N-2..N-1-P]]
   if (active) {
-    x0 = downmix(A, col, 0);
-    xn = downmix(A, col, N - 1);
-    const float2 xp = downmix(A, col, P);
-    iir_init<NS>(A, z, P > 0 ? make_float2(2.f * x0.x - xp.x, 2.f * x0.y - xp.y) : x0);
+    const float2 x0 = mixed(0);
+    // lanes hold the left extension, broadcast in turn
+    float2 e = make_float2(0.f, 0.f);
     for (int k = 0; k < P; ++k) {
-      const float2 v = downmix(A, col, P - k);
-      iir_step<NS>(A, z, make_float2(2.f * x0.x - v.x, 2.f * x0.y - v.y));
+      if ((k & 31) == 0) {
+        const float2 v = mixed(max(0, P - k - lane));
+        e = make_float2(2.f * x0.x - v.x, 2.f * x0.y - v.y);
+      }
+      const float2 v = make_float2(__shfl_sync(0xffffffffu, e.x, k & 31), __shfl_sync(0xffffffffu, e.y, k & 31));
+      if (k == 0) iir_init<NS>(A, z, v);
+      iir_step<NS>(A, z, v);
     }
+    if (P == 0) iir_init<NS>(A, z, x0);
   }
-  // the record: the phasors are the same for every column, so the CTA tabulates them; the
-  // recurrence is sequential, the loads are not, so each chunk's samples are requested first
-  for (int n0 = 0; n0 < N; n0 += kIqTable) {
+  for (int g = 0; g < n_seg; ++g) {
+    const int n0 = g * S, n = min(S, N - n0);
     __syncthreads();
-    for (int j = threadIdx.x; j < kIqTable && n0 + j < N; j += blockDim.x) ph[j] = phasor(A, n0 + j);
+    for (int j = threadIdx.x; j < n; j += blockDim.x) ph[j] = phasor(A, n0 + j);
     __syncthreads();
-    if (!active) continue;
-    const int n_end = min(N, n0 + kIqTable);
-    for (int m0 = n0; m0 < n_end; m0 += kIqChunk) {
-      float v[kIqChunk];
-#pragma unroll
-      for (int j = 0; j < kIqChunk; ++j) v[j] = m0 + j < n_end ? col[(size_t)(m0 + j) * A.n_ch] : 0.f;
-#pragma unroll
-      for (int j = 0; j < kIqChunk; ++j)
-        if (m0 + j < n_end) {
-          const float2 e = ph[m0 + j - n0];
-          y[m0 + j] = iir_step<NS>(A, z, make_float2(v[j] * e.x, v[j] * e.y));
+    {
+      const int c = threadIdx.x & (kIqCh - 1);
+      if (ch0 + c < A.n_ch) {
+        const float* src = rf + (size_t)n0 * A.n_ch + ch0 + c;
+#pragma unroll 4
+        for (int j = threadIdx.x / kIqCh; j < n; j += 32) {
+          const float v = src[(size_t)j * A.n_ch];
+          const float2 e = ph[j];
+          iq_sm[c * pitch + j] = make_float2(v * e.x, v * e.y);
         }
+      }
+    }
+    __syncthreads();
+    if (active) {
+      iir_segment<NS>(A, col, 1, n, z, 1.f);
+      if (n_seg > 1)
+        for (int j = lane; j < n; j += 32) y[n0 + j] = col[j];
     }
   }
   if (!active) return;
-  for (int k = 0; k < P; ++k) {
-    const float2 v = downmix(A, col, N - 2 - k);
-    right[k] = iir_step<NS>(A, z, make_float2(2.f * xn.x - v.x, 2.f * xn.y - v.y));
-  }
-  // backward pass, started from the last forward output
-  iir_init<NS>(A, z, P > 0 ? right[P - 1] : y[N - 1]);
-  for (int k = P - 1; k >= 0; --k) iir_step<NS>(A, z, right[k]);
-  for (int n1 = N - 1; n1 >= 0; n1 -= kIqChunk) {
-    float2 w[kIqChunk];
-#pragma unroll
-    for (int j = 0; j < kIqChunk; ++j) w[j] = n1 - j >= 0 ? y[n1 - j] : make_float2(0.f, 0.f);
-#pragma unroll
-    for (int j = 0; j < kIqChunk; ++j)
-      if (n1 - j >= 0) {
-        const float2 o = iir_step<NS>(A, z, w[j]);
-        y[n1 - j] = make_float2(2.f * o.x, 2.f * o.y);
+  {
+    const float2 xn = mixed(N - 1);
+    float2 e = make_float2(0.f, 0.f), o = e;
+    for (int k = 0; k < P; ++k) {
+      if ((k & 31) == 0) {
+        const float2 v = mixed(max(0, N - 2 - k - lane));
+        e = make_float2(2.f * xn.x - v.x, 2.f * xn.y - v.y);
       }
+      o = iir_step<NS>(A, z, make_float2(__shfl_sync(0xffffffffu, e.x, k & 31), __shfl_sync(0xffffffffu, e.y, k & 31)));
+      if (lane == 0) right[warp][k] = o;
+    }
+    __syncwarp();
+    // backward pass, started from the last forward output
+    iir_init<NS>(A, z, P > 0 ? o : col[(N - 1) - (n_seg - 1) * S]);
+    for (int k = P - 1; k >= 0; --k) iir_step<NS>(A, z, right[warp][k]);
+  }
+  for (int g = n_seg - 1; g >= 0; --g) {
+    const int n0 = g * S, n = min(S, N - n0);
+    if (n_seg > 1) {
+      __syncwarp();
+      for (int j = lane; j < n; j += 32) col[j] = y[n0 + j];
+      __syncwarp();
+    }
+    iir_segment<NS>(A, col + n - 1, -1, n, z, 2.f);
+    for (int j = lane; j < n; j += 32) y[n0 + j] = col[j];
   }
 }
 
@@ -387,16 +473,61 @@ extern "C" int32_t fsg_rf2iq(const float* rf, int32_t n_frames, int32_t n_sample
     for (int k = 0; k < 5; ++k) A.sos[sct][k] = on ? (float)sos[6 * sct + take[k]] : 0.f;
     for (int k = 0; k < 2; ++k) A.zi[sct][k] = on ? (float)zi[2 * sct + k] : 0.f;
   }
-  const int64_t cols = (int64_t)n_frames * n_channels;
-  const unsigned grid = (unsigned)((cols + kIqThreads - 1) / kIqThreads);
-  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  switch (n_sections) {
-    case 1: rf2iq_kernel<1><<<grid, kIqThreads, 0, s>>>(A); break;
-    case 2: rf2iq_kernel<2><<<grid, kIqThreads, 0, s>>>(A); break;
-    case 3: rf2iq_kernel<3><<<grid, kIqThreads, 0, s>>>(A); break;
-    default: rf2iq_kernel<4><<<grid, kIqThreads, 0, s>>>(A); break;
+  // segments of at most 32 kIqMaxL samples, the chunk length odd (the lanes' strided shared-memory
+  // accesses then use every bank)
+  const int n_seg = (n_samples + 32 * kIqMaxL - 1) / (32 * kIqMaxL);
+  A.L = ((n_samples + 32 * n_seg - 1) / (32 * n_seg)) | 1;
+  {
+    // state transition of the cascade over L samples of zero input, and its squares, in FP64
+    double m[2 * FSG_RF2IQ_MAX_SECTIONS][2 * FSG_RF2IQ_MAX_SECTIONS], sq[2 * FSG_RF2IQ_MAX_SECTIONS][2 * FSG_RF2IQ_MAX_SECTIONS];
+    const int ns2 = 2 * n_sections;
+    for (int j = 0; j < ns2; ++j) {
+      double z[FSG_RF2IQ_MAX_SECTIONS][2] = {};
+      z[j / 2][j % 2] = 1.0;
+      for (int n = 0; n < A.L; ++n) {
+        double x = 0.0;
+        for (int q = 0; q < n_sections; ++q) {
+          const float* c = A.sos[q];
+          const double o = c[0] * x + z[q][0];
+          z[q][0] = c[1] * x - c[3] * o + z[q][1];
+          z[q][1] = c[2] * x - c[4] * o;
+          x = o;
+        }
+      }
+      for (int i = 0; i < ns2; ++i) m[i][j] = z[i / 2][i % 2];
+    }
+    memset(A.m, 0, sizeof(A.m));
+    for (int k = 0; k < kIqScan; ++k) {
+      for (int i = 0; i < ns2; ++i)
+        for (int j = 0; j < ns2; ++j) A.m[k][i][j] = (float)m[i][j];
+      for (int i = 0; i < ns2; ++i)
+        for (int j = 0; j < ns2; ++j) {
+          double s = 0.0;
+          for (int q = 0; q < ns2; ++q) s += m[i][q] * m[q][j];
+          sq[i][j] = s;
+        }
+      memcpy(m, sq, sizeof(m));
+    }
   }
-  return check_cuda(cudaGetLastError(), "rf2iq_kernel launch");
+  const int64_t grid64 = (int64_t)n_frames * ((n_channels + kIqCh - 1) / kIqCh);
+  if (grid64 > INT32_MAX) return set_error(FSG_EUNSUPPORTED, "%lld channel groups exceed the grid", (long long)grid64);
+  const unsigned grid = (unsigned)grid64;
+  const size_t smem = ((size_t)kIqCh * (32 * A.L + 4) + 32 * A.L) * sizeof(float2);
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  auto launch = [&](auto kernel) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    kernel<<<grid, 32 * kIqCh, smem, s>>>(A);
+    return cudaGetLastError();
+  };
+  cudaError_t e;
+  switch (n_sections) {
+    case 1: e = launch(rf2iq_kernel<1>); break;
+    case 2: e = launch(rf2iq_kernel<2>); break;
+    case 3: e = launch(rf2iq_kernel<3>); break;
+    default: e = launch(rf2iq_kernel<4>); break;
+  }
+  return check_cuda(e, "rf2iq_kernel launch");
 }
 
 static int das_args(const FsgProbe* probe, const FsgDasParams* p, int n_frames, int n_samples, const double* txd,
