@@ -1,0 +1,48 @@
+"""Edges of the spectrum -> RF transform and of the I/Q demodulation: element and sample remainders of
+the 64 x 64 tile, one-chunk and many-chunk bands (frequency splits over a cluster of 1 to 8 CTAs),
+twiddle tables beyond shared memory; channel remainders, records of one lane's chunk up to several
+segments, narrow filters.  Tolerances: FP32 sums of up to 2,000 terms, relative L2 <= 2e-6; the FP32
+filter cascade <= 2e-5, both as in the tests of the plain sizes."""
+
+import numpy as np
+import pytest
+
+from oracle import das_fp64 as D
+from tests import _golden as G
+from tests._gpu import np64, require_gpu, torch
+
+pytestmark = pytest.mark.gpu
+
+
+class _Plan:
+    def __init__(self, n_fft):
+        self.n_fft = n_fft
+
+
+@pytest.mark.parametrize("n_fft,k0,kc,E,nb", [(130, 3, 1, 1, 1), (258, 10, 64, 65, 2), (1023, 100, 129, 64, 1),
+                                              (2030, 200, 257, 130, 1), (2030, 200, 700, 64, 9), (14001, 900, 1100, 5, 1)])
+def test_irfft_tiles_and_splits(n_fft, k0, kc, E, nb):
+    require_gpu()
+    from fastsimus_gb300.simus import irfft_and_threshold
+
+    rng = np.random.default_rng(n_fft + E)
+    s = np.zeros((nb, n_fft // 2 + 1, E), dtype=np.complex64)
+    s[:, k0:k0 + kc] = rng.standard_normal((nb, kc, E)) + 1j * rng.standard_normal((nb, kc, E))
+    got = np64(irfft_and_threshold(torch.as_tensor(s, device="cuda"), _Plan(n_fft), k_first=k0, k_count=kc, gate=False))
+    ref = np.fft.irfft(np.conj(s.astype(np.complex128)), n=n_fft, axis=1)[:, : (n_fft + 1) // 2]
+    assert got.shape == ref.shape
+    assert G.rel_l2(got, ref) < 2e-6
+
+
+@pytest.mark.parametrize("ns,nc,nf,bw", [(19, 1, 1, None), (32, 7, 1, None), (33, 8, 2, None), (1015, 9, 1, None),
+                                         (2272, 3, 1, None), (2273, 8, 1, None), (5003, 2, 2, 1.5e6)])
+def test_rf2iq_chunks_and_segments(ns, nc, nf, bw):
+    require_gpu()
+    from fastsimus_gb300.beamform import rf2iq
+
+    rng = np.random.default_rng(ns)
+    rf = rng.standard_normal((nf, ns, nc)).astype(np.float32)
+    got = np64(rf2iq(torch.as_tensor(rf, device="cuda"), 20e6, 5e6, bw))
+    ref = np.stack([D.rf2iq(x.astype(np.float64), 20e6, 5e6, bw) for x in rf])
+    assert got.shape == ref.shape
+    assert G.rel_l2(got, ref) < 2e-5
