@@ -10,8 +10,8 @@ The field oscillates at the wavelength in space and at 1/delay in frequency, and
 plane wave of the firing it carries the waves that start at the two ends of the aperture and,
 at the pitch of these arrays (about one wavelength), the first grating lobes.  The head
 therefore predicts the complex amplitudes a_j of five analytic carriers c_j -- the ideal plane
-wave, the two edge waves and the grating lobes m = -1, +1, whose phases are computed exactly
-(FP64) from the geometry -- and the field is  p = scale * sum_j a_j c_j.  What is left to learn
+wave, the two edge waves and the grating lobes m = -1, +1, whose phases are computed in double-float
+arithmetic from the geometry -- and the field is  p = scale * sum_j a_j c_j.  What is left to learn
 is a set of slowly varying amplitudes.
 
 Training runs entirely in libfsgb300's tcgen05 kernels (fsg_mlp_train_*): a step gathers its
