@@ -15,7 +15,8 @@
 //              formed once per item, and the reduction multiplies it by pulse x probe.
 //
 // Each real GEMM is A_hi B_hi + A_hi B_lo + A_lo B_hi (three tcgen05.mma kind::f16 per K step).
-// TX operands are K-major; RX operands are written MN-major so that no thread transposes data.
+// The Green's tile is stored once; the TX product reads it K-major (rows s), the RX product MN-major
+// (rows e), so that no thread transposes data.
 // Every wait on an mbarrier is bounded: on timeout the CTA records FSG_ETIMEOUT in the status
 // word, skips the remaining work, frees its TMEM and exits.
 
@@ -108,48 +109,50 @@ __device__ __forceinline__ float2 tc_anchor(float rc, float amp, float2 k0, floa
 __device__ __forceinline__ int tc_sg(int tid) { return (tid >> 5) * 8 + (tid & 7); }
 __device__ __forceinline__ int tc_eg(int tid) { return (tid >> 3) & 3; }
 
-// SMEM layout (bytes).
-constexpr uint32_t kOffAtxHi = 0;                 // K-major  128 x 64 bf16
-constexpr uint32_t kOffAtxLo = 16384;
-constexpr uint32_t kOffArxHi = 32768;             // MN-major 128 x 64 bf16
-constexpr uint32_t kOffArxLo = 49152;
-constexpr int kXPitch = 33;
-// The rest depends on the transmit chunks nc (N = 64 nc): B_rx MN-major N (n) x 64 (k), hi
-// then lo; the exchange buffer, 2 x 64 rows x 33 floats (padded: conflict-free); per band
-// frequency B_tx K-major N x 64, hi then lo.
-struct TcSmem {
-  uint32_t brx_hi, brx_lo, x, btx, btx_bytes;
-};
-__host__ __device__ inline TcSmem tc_smem(int nc) {
-  TcSmem L;
-  L.brx_hi = 65536;
-  L.brx_lo = 65536 + 8192u * nc;
-  L.x = 65536 + 16384u * nc;
-  L.btx = ((L.x + 2u * 64u * kXPitch * 4u + 1023u) / 1024u) * 1024u;
-  L.btx_bytes = 16384u * nc;
-  return L;
-}
+// Shared memory (bytes).  The Green's tile A of a frequency, 32 KB (BF16 hi, then lo), serves both
+// products: core matrices of 8 scatterers x 8 elements (16-byte rows of elements) at
+// (s / 8) 2048 + c 1024 + (e / 8) 128, c = re, im.  Read K-major (rows s, K = e) it has M stride 1024
+// and K stride 128, its M rows in the order (s / 8, c, s % 8); read MN-major (rows (c, e), K = s) M
+// stride 128 and K stride 2048.  Two tiles alternate.  Then B_rx MN-major N (n) x 64 (k), hi and lo;
+// then per band frequency B_tx K-major N x 64, hi and lo.
+constexpr uint32_t kATile = 32768, kALo = 16384;
+constexpr uint32_t kOffBrx = 2 * kATile;
+constexpr int kXPitch = 33;  // exchange buffer of the final combination (2 x 64 rows), over the A tiles
+__host__ __device__ constexpr uint32_t tc_off_btx(int nc) { return kOffBrx + 16384u * nc; }
+__host__ __device__ constexpr uint32_t tc_btx_bytes(int nc) { return 16384u * nc; }
 __host__ __device__ inline uint32_t tc_smem_bytes(int fb, int nc) {
-  const TcSmem L = tc_smem(nc);
-  return L.btx + (uint32_t)fb * L.btx_bytes + 1024;
+  return tc_off_btx(nc) + (uint32_t)fb * tc_btx_bytes(nc) + 1024;
+}
+__device__ __forceinline__ uint32_t a_off(int s, int c, int e) {
+  return ((uint32_t)(s >> 3) << 11) + ((uint32_t)c << 10) + ((uint32_t)(e >> 3) << 7) + ((uint32_t)(s & 7) << 4);
 }
 
-// kSplitTx: the TX product is formed in passes of two chunks (three chunks, N = 192); else in
-// one pass of all nc chunks.
-template <int U, bool kSplitTx>
+// One step per (tile, band frequency), pipelined over the steps of an item:
+//   values of step i + 1 (recurrence, BF16 split) in registers, while RX(i - 1) and TX(i) run
+//   wait RX(i - 1); store them into the A tile that it has read
+//   wait TX(i); TMEM -> P (the rows of re and im of a scatterer are eight lanes apart: one shuffle
+//   per value) -> B_rx
+//   one barrier; then RX(i) and TX(i + 1) are issued back to back, by two warps
+// With three transmit chunks (N = 192) the TX product has a second pass: its MMAs run while the first
+// pass's P is formed, behind one more barrier.
+//
+// What bounds it: the CUDA cores' part of a step (32 recurrences, the split and its stores and the
+// epilogue per thread, about 1,000 issue cycles), with the tensor pipe (768 cycles of MMAs at N = 64)
+// under it.  The kernel before this one kept the Green's tile twice (once per product), exchanged P
+// through shared memory and met at seven barriers per step: 5,800 cycles a step at 31 firings.
+template <int U, int NC>
 __global__ void __launch_bounds__(kThreads, 1) tc_kernel(const __grid_constant__ TcArgs A) {
+  constexpr int NT = kTcTxChunk * NC, N = 2 * NT;
+  constexpr int TXK = NC < 2 ? NC : 2, TXC = 64 * TXK;  // chunks per TX pass, TX TMEM columns
+  constexpr bool kTwoPass = NC > 2;
   extern __shared__ __align__(1024) unsigned char sm[];
   __shared__ uint64_t mbar_tx, mbar_rx;
   __shared__ uint32_t tmem_holder;
   __shared__ int s_item, s_fail;
-  __shared__ float rcs[kTcT];
+  __shared__ float rcs[2][kTcT];
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int fb = A.fb, E = A.E, T = A.n_tx;
-  const int NC = A.nc, NT = kTcTxChunk * NC, N = 2 * NT;
-  const int TXK = kSplitTx ? 2 : NC, TXC = 64 * TXK;  // chunks per TX pass, TX TMEM columns
-  const int n_pass = kSplitTx ? (NC + 1) / 2 : 1;
-  const TcSmem SL = tc_smem(NC);
   if (tid == 0) {
     tc::mbar_init(&mbar_tx, 1);
     tc::mbar_init(&mbar_rx, 1);
@@ -161,26 +164,59 @@ __global__ void __launch_bounds__(kThreads, 1) tc_kernel(const __grid_constant__
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = tmem_holder;
-  // mbarrier phases and the pending-RX flag are only used by thread 0
-  uint32_t ph_tx = 0, ph_rx = 0;
-  bool rx_pending = false;
+  uint32_t ph_tx = 0, ph_rx = 0;  // every thread waits for every phase
 
   const uint32_t sbase = tc::smem_u32(sm);
-  const uint32_t id_tx = tc::idesc_bf16(128, TXC, 0, 0);  // A K-major, B K-major (a full pass)
-  const uint32_t id_rx = tc::idesc_bf16(128, N, 1, 1);  // A MN-major, B MN-major
-  float* X = reinterpret_cast<float*>(sm + SL.x);
+  constexpr uint32_t id_rx = tc::idesc_bf16(128, N, 1, 1);  // A MN-major, B MN-major
+  unsigned char* brx = sm + kOffBrx;
+  unsigned char* btx0 = sm + tc_off_btx(NC);
 
   const int s_g = tc_sg(tid), eg = tc_eg(tid);
-  // TMEM read mapping: lane quarter q (rows 32q..32q+31), column half h
+  // TMEM rows of this thread: lane quarter q; half h of each chunk's transmits; and, in the TX
+  // product, scatterer s_p and part c_p (0 re, 1 im)
   const int q = warp & 3, h = warp >> 2;
+  const int s_p = (2 * q + (lane >> 4)) * 8 + (lane & 7), c_p = (lane >> 3) & 1;
+  const uint32_t trow = tmem + ((uint32_t)(32 * q) << 16);
 
-  // thread 0 waits on an mbarrier (bounded); the result reaches every thread through s_fail
-  // after the next __syncthreads, so all threads take the same branches.
-  auto wait0 = [&](uint64_t* mb, uint32_t& ph) {
-    if (tid == 0) {
-      if (!tc::mbar_wait_bounded(mb, ph, kWaitTries)) s_fail = 1;
-      ph ^= 1u;
+  auto wait = [&](uint64_t* mb, uint32_t& ph) {
+    if (!tc::mbar_test(mb, ph) && !s_fail && !tc::mbar_wait_bounded(mb, ph, kWaitTries)) s_fail = 1;
+    ph ^= 1u;
+    __syncwarp();
+  };
+  auto meet = [&]() {
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+  };
+  // A_hi B_hi + A_hi B_lo + A_lo B_hi over K = 64
+  auto issue_tx = [&](int par, int f, int pass) {
+    const uint32_t bt = sbase + tc_off_btx(NC) + f * tc_btx_bytes(NC) + 8192u * TXK * pass;  // 64 rows per chunk
+    const uint32_t at = sbase + par * kATile;
+    const uint32_t id = tc::idesc_bf16(128, kTwoPass && pass ? 64 * (NC - TXK) : TXC, 0, 0);  // both K-major
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks) {
+      const uint64_t ah = tc::sdesc(at + ks * 256, 128, 1024), al = tc::sdesc(at + kALo + ks * 256, 128, 1024);
+      const uint64_t bh = tc::sdesc(bt + ks * 256, 128, 1024);
+      const uint64_t bl = tc::sdesc(bt + tc_btx_bytes(NC) / 2 + ks * 256, 128, 1024);
+      tc::mma_bf16(tmem, ah, bh, id, ks > 0);
+      tc::mma_bf16(tmem, ah, bl, id, 1);
+      tc::mma_bf16(tmem, al, bh, id, 1);
     }
+    tc::commit(&mbar_tx);
+  };
+  auto issue_rx = [&](int par, int f, bool first) {
+    const uint32_t d = tmem + TXC + N * f, at = sbase + par * kATile, bt = sbase + kOffBrx;
+    constexpr uint32_t lbo = 16u * N;  // N / 8 core matrices of 128 bytes per K group
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks) {
+      const uint64_t ah = tc::sdesc(at + ks * 4096, 2048, 128), al = tc::sdesc(at + kALo + ks * 4096, 2048, 128);
+      const uint64_t bh = tc::sdesc(bt + ks * 2 * lbo, lbo, 128);
+      const uint64_t bl = tc::sdesc(bt + 8192 * NC + ks * 2 * lbo, lbo, 128);
+      tc::mma_bf16(d, ah, bh, id_rx, (first && ks == 0) ? 0u : 1u);
+      tc::mma_bf16(d, ah, bl, id_rx, 1);
+      tc::mma_bf16(d, al, bh, id_rx, 1);
+    }
+    tc::commit(&mbar_rx);
   };
 
   for (;;) {
@@ -198,18 +234,14 @@ __global__ void __launch_bounds__(kThreads, 1) tc_kernel(const __grid_constant__
     const int nf = min(fb, P.n_freq - f0);
     const int64_t s_begin = (int64_t)chunk * A.chunk;
     const int64_t s_end = min(P.n_scat, s_begin + A.chunk);
-    SweepConst C = A.C;
-    C.dk = P.dk;
-    C.dalpha = P.dalpha;
 
-    // ---- B_tx for the band: K-major rows n', K = e; value D_c'(e, t).  With split TX passes
+    // ---- B_tx for the band: K-major rows n', K = e; value D_c'(e, t).  With two TX passes
     //      the rows are (chunk, c', t mod 32), so that each chunk of 32 transmits is 64
     //      contiguous rows; else (c', t). ----
     for (int i = tid; i < fb * N * 64; i += kThreads) {
       const int f = i / (N * 64), n = (i >> 6) % N, e = i & 63;
-      // chunk-major rows when the TX product is formed in passes; else (c', t) order
-      const int c = kSplitTx ? (n >> 5) & 1 : n / NT;
-      const int t = kSplitTx ? kTcTxChunk * (n >> 6) + (n & 31) : n % NT;
+      const int c = kTwoPass ? (n >> 5) & 1 : n / NT;
+      const int t = kTwoPass ? kTcTxChunk * (n >> 6) + (n & 31) : n % NT;
       float v = 0.f;
       if (f < nf && e < E && t < T) {
         const float w = A.apod[t * E + e];
@@ -228,427 +260,169 @@ __global__ void __launch_bounds__(kThreads, 1) tc_kernel(const __grid_constant__
       }
       __nv_bfloat16 hi, lo;
       tc::split_bf16(v, hi, lo);
-      unsigned char* bt = sm + SL.btx + f * SL.btx_bytes;
+      unsigned char* bt = btx0 + f * tc_btx_bytes(NC);
       const uint32_t off = tc::kmajor_off(n, e, 8);
       *reinterpret_cast<__nv_bfloat16*>(bt + off) = hi;
-      *reinterpret_cast<__nv_bfloat16*>(bt + SL.btx_bytes / 2 + off) = lo;
+      *reinterpret_cast<__nv_bfloat16*>(bt + tc_btx_bytes(NC) / 2 + off) = lo;
     }
     const float2 k0 = P.kf[f0];
     const float a0 = P.af[f0];
-    bool first_tile = true;
+    const int64_t tiles = (s_end - s_begin + kTcT - 1) / kTcT, steps = tiles * nf;
 
-    if constexpr (!kSplitTx) {
-      // Software-pipelined tile loop (one pass of the transmit product): the Green's values of
-      // frequency f + 1 are formed while the receive MMAs of f run, written to the transmit A
-      // operand as soon as the transmit MMAs of f are done, and to the receive A operand once
-      // the receive MMAs of f are; the transmit MMAs of f + 1 queue right behind the receive
-      // MMAs of f.  Order per frequency: wait TX(f) | epilogue(f) -> B_rx | issue RX(f) |
-      // values(f + 1) -> A_tx | issue TX(f + 1) | wait RX(f) | values(f + 1) -> A_rx.
-      for (int64_t t0 = s_begin; t0 < s_end; t0 += kTcT) {
+    float2 G[16 * U], S[16 * U];
+    // the tile's reflectivities and cached geometry -> anchors at the band's first frequency
+    auto start_tile = [&](int64_t tile) {
+      const int64_t t0 = s_begin + tile * kTcT;
+      if (eg == 0) {
         const int64_t s = t0 + s_g;
-        const bool sval = s < s_end;
-        if (eg == 0) {
-          float w = 0.f;
-          if (sval) {
-            const double x = P.scat[2 * s], z = P.scat[2 * s + 1];
-            bool out = z < 0.0;
-            if (A.convex) out = out || (x * x + (z + A.apex) * (z + A.apex) <= A.radius2);
-            w = out ? 0.f : (float)P.rc[s];
-          }
-          rcs[s_g] = w;
+        float w = 0.f;
+        if (s < s_end) {
+          const double x = P.scat[2 * s], z = P.scat[2 * s + 1];
+          bool out = z < 0.0;
+          if (A.convex) out = out || (x * x + (z + A.apex) * (z + A.apex) <= A.radius2);
+          w = out ? 0.f : (float)P.rc[s];
         }
-        float2 G[16 * U], S[16 * U];
-        {
-          const float4* gp = A.geo + ((P.tile0 + t0 / kTcT) * (16 * U)) * kThreads + tid;
-#pragma unroll
-          for (int i = 0; i < 16 * U; ++i) {
-            const float4 v = gp[(size_t)i * kThreads];
-            G[i] = tc_anchor(v.x, v.y, k0, a0);
-            S[i] = make_float2(v.z, v.w);
-          }
-        }
-        // the BF16 hi/lo words of this thread's 16 Green's values at the current frequency
-        // (both halves of 8 elements: re hi, re lo, im hi, im lo), then one recurrence step
-        uint4 wv[2][4];
-        auto gen_values = [&]() {
-#pragma unroll
-          for (int half = 0; half < 2; ++half) {
-            float gr[8], gi[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const int jj = half * 8 + j;
-              float2 acc = G[jj * U];
-#pragma unroll
-              for (int u = 1; u < U; ++u) acc = cadd(acc, G[jj * U + u]);
-              gr[j] = acc.x;
-              gi[j] = acc.y;
-#pragma unroll
-              for (int u = 0; u < U; ++u) G[jj * U + u] = cmul(G[jj * U + u], S[jj * U + u]);
-            }
-            tc::split8(gr, wv[half][0], wv[half][1]);
-            tc::split8(gi, wv[half][2], wv[half][3]);
-          }
-        };
-        auto store_tx = [&]() {
-#pragma unroll
-          for (int half = 0; half < 2; ++half) {
-            const int e0 = eg * 16 + half * 8;
-            const uint32_t o_re = tc::kmajor_off(s_g, e0, 8), o_im = tc::kmajor_off(64 + s_g, e0, 8);
-            *reinterpret_cast<uint4*>(sm + kOffAtxHi + o_re) = wv[half][0];
-            *reinterpret_cast<uint4*>(sm + kOffAtxLo + o_re) = wv[half][1];
-            *reinterpret_cast<uint4*>(sm + kOffAtxHi + o_im) = wv[half][2];
-            *reinterpret_cast<uint4*>(sm + kOffAtxLo + o_im) = wv[half][3];
-          }
-        };
-        auto store_rx = [&]() {
-#pragma unroll
-          for (int half = 0; half < 2; ++half) {
-            const int e0 = eg * 16 + half * 8;
-            const uint32_t q_re = tc::mnmajor_off(e0, s_g, 16), q_im = tc::mnmajor_off(64 + e0, s_g, 16);
-            *reinterpret_cast<uint4*>(sm + kOffArxHi + q_re) = wv[half][0];
-            *reinterpret_cast<uint4*>(sm + kOffArxLo + q_re) = wv[half][1];
-            *reinterpret_cast<uint4*>(sm + kOffArxHi + q_im) = wv[half][2];
-            *reinterpret_cast<uint4*>(sm + kOffArxLo + q_im) = wv[half][3];
-          }
-        };
-        auto issue_tx = [&](int f) {  // thread 0
-          const uint32_t bt = sbase + SL.btx + f * SL.btx_bytes;
-#pragma unroll
-          for (int ks = 0; ks < 4; ++ks) {
-            const uint64_t ah = tc::sdesc(sbase + kOffAtxHi + ks * 256, 128, 1024);
-            const uint64_t al = tc::sdesc(sbase + kOffAtxLo + ks * 256, 128, 1024);
-            const uint64_t bh = tc::sdesc(bt + ks * 256, 128, 1024);
-            const uint64_t bl = tc::sdesc(bt + SL.btx_bytes / 2 + ks * 256, 128, 1024);
-            tc::mma_bf16(tmem, ah, bh, id_tx, ks > 0);
-            tc::mma_bf16(tmem, ah, bl, id_tx, 1);
-            tc::mma_bf16(tmem, al, bh, id_tx, 1);
-          }
-          tc::commit(&mbar_tx);
-        };
-        gen_values();
-        // the previous receive MMAs read A_rx and B_rx: wait for them before the prologue writes
-        if (tid == 0 && rx_pending) {
-          wait0(&mbar_rx, ph_rx);
-          rx_pending = false;
-        }
-        tc::fence_before_sync();
-        __syncthreads();  // rcs visible, the previous receive product done
-        tc::fence_after_sync();
-        if (s_fail) break;
-        store_tx();
-        store_rx();
-        tc::fence_proxy_async_smem();
-        tc::fence_before_sync();
-        __syncthreads();
-        tc::fence_after_sync();
-        if (tid == 0) issue_tx(0);
-        for (int f = 0; f < nf; ++f) {
-          if (tid == 0) wait0(&mbar_tx, ph_tx);
-          tc::fence_before_sync();
-          __syncthreads();
-          tc::fence_after_sync();
-          if (s_fail) break;
-          // ---- P = combine(D_tx); write B_rx (MN-major rows n' = (c', t), K = s), one chunk
-          //      of 32 transmits at a time ----
-          const int row = 32 * q + lane;  // (c, s) with c = row / 64
-          for (int k = 0; k < NC; ++k) {
-            float v[32];
-            tc::tmem_ld32(tmem + ((uint32_t)(32 * q) << 16) + h * NT + 32 * k, v);
-            if (row >= 64) {
-#pragma unroll
-              for (int t = 0; t < 32; ++t) X[(h * 64 + (row - 64)) * kXPitch + t] = v[t];
-            }
-            __syncthreads();
-            if (row < 64) {
-              const float* x = X + ((1 - h) * 64 + row) * kXPitch;
-              const float rw = rcs[row];
-#pragma unroll
-              for (int t = 0; t < 32; ++t) v[t] = rw * (h ? v[t] + x[t] : v[t] - x[t]);
-#pragma unroll
-              for (int c8 = 0; c8 < 4; ++c8) {
-                uint4 hh, ll;
-                tc::split8(v + 8 * c8, hh, ll);
-                const uint32_t o = tc::mnmajor_off(h * NT + 32 * k + 8 * c8, row, N / 8);
-                *reinterpret_cast<uint4*>(sm + SL.brx_hi + o) = hh;
-                *reinterpret_cast<uint4*>(sm + SL.brx_lo + o) = ll;
-              }
-            }
-            if (k + 1 < NC) __syncthreads();  // X is reused by the next chunk
-          }
-          tc::fence_proxy_async_smem();
-          tc::fence_before_sync();
-          __syncthreads();
-          tc::fence_after_sync();
-          // ---- RX MMAs into this frequency's accumulator ----
-          if (tid == 0) {
-            const uint32_t d = tmem + TXC + N * f;
-#pragma unroll
-            for (int ks = 0; ks < 4; ++ks) {
-              const uint64_t ah = tc::sdesc(sbase + kOffArxHi + ks * 2 * 2048, 2048, 128);
-              const uint64_t al = tc::sdesc(sbase + kOffArxLo + ks * 2 * 2048, 2048, 128);
-              const uint32_t lbo = 16u * N;  // N / 8 core matrices of 128 bytes per K group
-              const uint64_t bh = tc::sdesc(sbase + SL.brx_hi + ks * 2 * lbo, lbo, 128);
-              const uint64_t bl = tc::sdesc(sbase + SL.brx_lo + ks * 2 * lbo, lbo, 128);
-              tc::mma_bf16(d, ah, bh, id_rx, (first_tile && ks == 0) ? 0u : 1u);
-              tc::mma_bf16(d, ah, bl, id_rx, 1);
-              tc::mma_bf16(d, al, bh, id_rx, 1);
-            }
-            tc::commit(&mbar_rx);
-            rx_pending = true;
-          }
-          if (f + 1 < nf) {
-            gen_values();
-            store_tx();  // the transmit MMAs of f are done (waited above)
-            tc::fence_proxy_async_smem();
-            tc::fence_before_sync();
-            __syncthreads();
-            tc::fence_after_sync();
-            if (tid == 0) {
-              issue_tx(f + 1);
-              wait0(&mbar_rx, ph_rx);
-              rx_pending = false;
-            }
-            tc::fence_before_sync();
-            __syncthreads();  // the receive MMAs of f are done: A_rx may be overwritten
-            tc::fence_after_sync();
-            if (s_fail) break;
-            store_rx();
-            tc::fence_proxy_async_smem();  // published by the barrier that opens the next frequency
-          }
-        }
-        first_tile = false;
-        if (s_fail) break;
+        rcs[tile & 1][s_g] = w;
       }
-    } else {
-      for (int64_t t0 = s_begin; t0 < s_end; t0 += kTcT) {
-        const int64_t s = t0 + s_g;
-        const bool sval = s < s_end;
-        if (eg == 0) {
-          float w = 0.f;
-          if (sval) {
-            const double x = P.scat[2 * s], z = P.scat[2 * s + 1];
-            bool out = z < 0.0;
-            if (A.convex) out = out || (x * x + (z + A.apex) * (z + A.apex) <= A.radius2);
-            w = out ? 0.f : (float)P.rc[s];
-          }
-          rcs[s_g] = w;
+      const float4* gp = A.geo + ((P.tile0 + t0 / kTcT) * (16 * U)) * kThreads + tid;
+#pragma unroll
+      for (int i = 0; i < 16 * U; ++i) {
+        const float4 v = gp[(size_t)i * kThreads];
+        G[i] = tc_anchor(v.x, v.y, k0, a0);
+        S[i] = make_float2(v.z, v.w);
+      }
+    };
+    // the BF16 hi/lo words of this thread's 16 Green's values at the current frequency (both halves
+    // of 8 elements: re hi, re lo, im hi, im lo), then one recurrence step
+    uint4 wv[2][4];
+    auto values = [&]() {
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        float gr[8], gi[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int jj = half * 8 + j;
+          float2 acc = G[jj * U];
+#pragma unroll
+          for (int u = 1; u < U; ++u) acc = cadd(acc, G[jj * U + u]);
+          gr[j] = acc.x;
+          gi[j] = acc.y;
+#pragma unroll
+          for (int u = 0; u < U; ++u) G[jj * U + u] = cmul(G[jj * U + u], S[jj * U + u]);
         }
-        // ---- the tile's cached geometry (16 elements x U sub-elements per thread) -> anchors ----
-        float2 G[16 * U], S[16 * U];
-        {
-          const float4* gp = A.geo + ((P.tile0 + t0 / kTcT) * (16 * U)) * kThreads + tid;
-  #pragma unroll
-          for (int i = 0; i < 16 * U; ++i) {
-            const float4 v = gp[(size_t)i * kThreads];
-            G[i] = tc_anchor(v.x, v.y, k0, a0);
-            S[i] = make_float2(v.z, v.w);
-          }
-        }
-        __syncthreads();  // rcs visible
+        tc::split8(gr, wv[half][0], wv[half][1]);
+        tc::split8(gi, wv[half][2], wv[half][3]);
+      }
+    };
+    auto store = [&](int par) {
+      unsigned char* at = sm + par * kATile;
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const uint32_t o_re = a_off(s_g, 0, eg * 16 + half * 8), o_im = a_off(s_g, 1, eg * 16 + half * 8);
+        *reinterpret_cast<uint4*>(at + o_re) = wv[half][0];
+        *reinterpret_cast<uint4*>(at + kALo + o_re) = wv[half][1];
+        *reinterpret_cast<uint4*>(at + o_im) = wv[half][2];
+        *reinterpret_cast<uint4*>(at + kALo + o_im) = wv[half][3];
+      }
+    };
+    // this thread's 16 transmits of chunk k: columns c' = 0 and c' = 1 of its row
+    auto load_chunk = [&](int k, float* d0, float* d1) {
+      const int kk = kTwoPass ? k % TXK : k;
+      const uint32_t col0 = kTwoPass ? 64 * kk : 32 * kk, col1 = kTwoPass ? col0 + 32 : NT + 32 * kk;
+      tc::tmem_ld16x2(trow + col0 + 16 * h, trow + col1 + 16 * h, d0, d1);
+    };
+    // P = (D[re][re] - D[im][im]) + i (D[re][im] + D[im][re]), times rc: the re lane forms the real
+    // part, the im lane the imaginary part; then its words of B_rx (rows n' = (c', t), K = s)
+    auto form = [&](int k, const float* d0, const float* d1, float rw) {
+      float v[16];
+#pragma unroll
+      for (int t = 0; t < 16; ++t) {
+        const float x = __shfl_xor_sync(0xffffffffu, d1[t], 8);
+        v[t] = rw * (c_p ? x + d0[t] : d0[t] - x);
+      }
+#pragma unroll
+      for (int c8 = 0; c8 < 2; ++c8) {
+        uint4 hh, ll;
+        tc::split8(v + 8 * c8, hh, ll);
+        const uint32_t o = tc::mnmajor_off(c_p * NT + 32 * k + 16 * h + 8 * c8, s_p, N / 8);
+        *reinterpret_cast<uint4*>(brx + o) = hh;
+        *reinterpret_cast<uint4*>(brx + 8192 * NC + o) = ll;
+      }
+    };
 
-        for (int f = 0; f < nf; ++f) {
-          // previous RX MMAs read A_rx / B_rx: wait before overwriting
-          if (tid == 0 && rx_pending) {
-            wait0(&mbar_rx, ph_rx);
-            rx_pending = false;
-          }
-          tc::fence_before_sync();
-          __syncthreads();
-          tc::fence_after_sync();
-          if (s_fail) break;
-          // ---- Green's values at f; write A_tx (K-major rows (c, s), K = e) and
-          //      A_rx (MN-major rows (c, e), K = s) in halves of 8 elements.  Both operands hold
-          //      the same BF16 hi/lo words: eight consecutive elements of one scatterer are one
-          //      16-byte core-matrix row in either layout.  The receive weights rc (real) go into
-          //      B_rx and pulse x probe (one complex factor per frequency) into the reduction. ----
-  #pragma unroll
-          for (int half = 0; half < 2; ++half) {
-            float gr[8], gi[8];
-  #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const int jj = half * 8 + j;
-              float2 acc = G[jj * U];
-  #pragma unroll
-              for (int u = 1; u < U; ++u) acc = cadd(acc, G[jj * U + u]);
-              gr[j] = acc.x;
-              gi[j] = acc.y;
-  #pragma unroll
-              for (int u = 0; u < U; ++u) G[jj * U + u] = cmul(G[jj * U + u], S[jj * U + u]);
-            }
-            const int e0 = eg * 16 + half * 8;
-            uint4 hr, lr, hi_, li_;
-            tc::split8(gr, hr, lr);
-            tc::split8(gi, hi_, li_);
-            const uint32_t o_re = tc::kmajor_off(s_g, e0, 8), o_im = tc::kmajor_off(64 + s_g, e0, 8);
-            *reinterpret_cast<uint4*>(sm + kOffAtxHi + o_re) = hr;
-            *reinterpret_cast<uint4*>(sm + kOffAtxLo + o_re) = lr;
-            *reinterpret_cast<uint4*>(sm + kOffAtxHi + o_im) = hi_;
-            *reinterpret_cast<uint4*>(sm + kOffAtxLo + o_im) = li_;
-            const uint32_t q_re = tc::mnmajor_off(e0, s_g, 16), q_im = tc::mnmajor_off(64 + e0, s_g, 16);
-            *reinterpret_cast<uint4*>(sm + kOffArxHi + q_re) = hr;
-            *reinterpret_cast<uint4*>(sm + kOffArxLo + q_re) = lr;
-            *reinterpret_cast<uint4*>(sm + kOffArxHi + q_im) = hi_;
-            *reinterpret_cast<uint4*>(sm + kOffArxLo + q_im) = li_;
-          }
-          tc::fence_proxy_async_smem();
-          tc::fence_before_sync();
-          __syncthreads();
-          tc::fence_after_sync();
-          if constexpr (!kSplitTx) {
-            // ---- TX MMAs (one pass, N columns) ----
-            if (tid == 0) {
-              const uint32_t bt = sbase + SL.btx + f * SL.btx_bytes;
-  #pragma unroll
-              for (int ks = 0; ks < 4; ++ks) {
-                const uint64_t ah = tc::sdesc(sbase + kOffAtxHi + ks * 256, 128, 1024);
-                const uint64_t al = tc::sdesc(sbase + kOffAtxLo + ks * 256, 128, 1024);
-                const uint64_t bh = tc::sdesc(bt + ks * 256, 128, 1024);
-                const uint64_t bl = tc::sdesc(bt + SL.btx_bytes / 2 + ks * 256, 128, 1024);
-                tc::mma_bf16(tmem, ah, bh, id_tx, ks > 0);
-                tc::mma_bf16(tmem, ah, bl, id_tx, 1);
-                tc::mma_bf16(tmem, al, bh, id_tx, 1);
-              }
-              tc::commit(&mbar_tx);
-              wait0(&mbar_tx, ph_tx);
-            }
-            tc::fence_before_sync();
-            __syncthreads();
-            tc::fence_after_sync();
-            if (s_fail) break;
-            // ---- P = combine(D_tx); write B_rx (MN-major rows n' = (c', t), K = s), one chunk
-            //      of 32 transmits at a time ----
-            const int row = 32 * q + lane;  // (c, s) with c = row / 64
-            for (int k = 0; k < NC; ++k) {
-              float v[32];
-              tc::tmem_ld32(tmem + ((uint32_t)(32 * q) << 16) + h * NT + 32 * k, v);
-              if (row >= 64) {
-  #pragma unroll
-                for (int t = 0; t < 32; ++t) X[(h * 64 + (row - 64)) * kXPitch + t] = v[t];
-              }
-              __syncthreads();
-              if (row < 64) {
-                // h = 0: Pr = D[0,s][0,t] - D[1,s][1,t];  h = 1: Pi = D[0,s][1,t] + D[1,s][0,t];
-                // times the scatterer's reflectivity
-                const float* x = X + ((1 - h) * 64 + row) * kXPitch;
-                const float rw = rcs[row];
-  #pragma unroll
-                for (int t = 0; t < 32; ++t) v[t] = rw * (h ? v[t] + x[t] : v[t] - x[t]);
-  #pragma unroll
-                for (int c8 = 0; c8 < 4; ++c8) {
-                  uint4 hh, ll;
-                  tc::split8(v + 8 * c8, hh, ll);
-                  const uint32_t o = tc::mnmajor_off(h * NT + 32 * k + 8 * c8, row, N / 8);
-                  *reinterpret_cast<uint4*>(sm + SL.brx_hi + o) = hh;
-                  *reinterpret_cast<uint4*>(sm + SL.brx_lo + o) = ll;
-                }
-              }
-              if (k + 1 < NC) __syncthreads();  // X is reused by the next chunk
-            }
-          } else {
-            // ---- TX MMAs, at most two chunks of 32 transmits per pass (columns [0, 64 chunks)),
-            //      then P = combine(D_tx) -> B_rx (MN-major rows n' = (c', t), K = s) chunk by
-            //      chunk ----
-            const int row = 32 * q + lane;  // (c, s) with c = row / 64
-            for (int pz = 0; pz < n_pass; ++pz) {
-              const int k0 = pz * TXK, k1 = kSplitTx ? min(NC, k0 + 2) : NC;
-              if (kSplitTx && pz > 0) {  // the previous pass's TMEM reads and exchange are done
-                tc::fence_before_sync();
-                __syncthreads();
-                tc::fence_after_sync();
-              }
-              if (tid == 0) {
-                const uint32_t bt = sbase + SL.btx + f * SL.btx_bytes + 8192u * k0;  // 64 rows per chunk
-                const uint32_t idp = (!kSplitTx || k1 - k0 == TXK) ? id_tx : tc::idesc_bf16(128, 64 * (k1 - k0), 0, 0);
-  #pragma unroll
-                for (int ks = 0; ks < 4; ++ks) {
-                  const uint64_t ah = tc::sdesc(sbase + kOffAtxHi + ks * 256, 128, 1024);
-                  const uint64_t al = tc::sdesc(sbase + kOffAtxLo + ks * 256, 128, 1024);
-                  const uint64_t bh = tc::sdesc(bt + ks * 256, 128, 1024);
-                  const uint64_t bl = tc::sdesc(bt + SL.btx_bytes / 2 + ks * 256, 128, 1024);
-                  tc::mma_bf16(tmem, ah, bh, idp, ks > 0);
-                  tc::mma_bf16(tmem, ah, bl, idp, 1);
-                  tc::mma_bf16(tmem, al, bh, idp, 1);
-                }
-                tc::commit(&mbar_tx);
-                wait0(&mbar_tx, ph_tx);
-              }
-              tc::fence_before_sync();
-              __syncthreads();
-              tc::fence_after_sync();
-              if (s_fail) break;
-              for (int k = k0; k < k1; ++k) {
-                float v[32];
-                // split passes: chunk k occupies TX columns 64 (k - k0) + 32 c'; one pass: c' NT + 32 k
-                const int col = kSplitTx ? 64 * (k - k0) + 32 * h : h * NT + 32 * k;
-                tc::tmem_ld32(tmem + ((uint32_t)(32 * q) << 16) + col, v);
-                if (row >= 64) {
-  #pragma unroll
-                  for (int t = 0; t < 32; ++t) X[(h * 64 + (row - 64)) * kXPitch + t] = v[t];
-                }
-                __syncthreads();
-                if (row < 64) {
-                  // h = 0: Pr = D[0,s][0,t] - D[1,s][1,t];  h = 1: Pi = D[0,s][1,t] + D[1,s][0,t];
-                  // times the scatterer's reflectivity
-                  const float* x = X + ((1 - h) * 64 + row) * kXPitch;
-                  const float rw = rcs[row];
-  #pragma unroll
-                  for (int t = 0; t < 32; ++t) v[t] = rw * (h ? v[t] + x[t] : v[t] - x[t]);
-  #pragma unroll
-                  for (int c8 = 0; c8 < 4; ++c8) {
-                    uint4 hh, ll;
-                    tc::split8(v + 8 * c8, hh, ll);
-                    const uint32_t o = tc::mnmajor_off(h * NT + 32 * k + 8 * c8, row, N / 8);
-                    *reinterpret_cast<uint4*>(sm + SL.brx_hi + o) = hh;
-                    *reinterpret_cast<uint4*>(sm + SL.brx_lo + o) = ll;
-                  }
-                }
-                if (k + 1 < k1) __syncthreads();  // X is reused by the next chunk
-              }
-            }
-          }
-          if (s_fail) break;
-          tc::fence_proxy_async_smem();
-          tc::fence_before_sync();
-          __syncthreads();
-          tc::fence_after_sync();
-          // ---- RX MMAs into this frequency's accumulator ----
-          if (tid == 0) {
-            const uint32_t d = tmem + TXC + N * f;
-  #pragma unroll
-            for (int ks = 0; ks < 4; ++ks) {
-              const uint64_t ah = tc::sdesc(sbase + kOffArxHi + ks * 2 * 2048, 2048, 128);
-              const uint64_t al = tc::sdesc(sbase + kOffArxLo + ks * 2 * 2048, 2048, 128);
-              const uint32_t lbo = 16u * N;  // N / 8 core matrices of 128 bytes per K group
-              const uint64_t bh = tc::sdesc(sbase + SL.brx_hi + ks * 2 * lbo, lbo, 128);
-              const uint64_t bl = tc::sdesc(sbase + SL.brx_lo + ks * 2 * lbo, lbo, 128);
-              tc::mma_bf16(d, ah, bh, id_rx, (first_tile && ks == 0) ? 0u : 1u);
-              tc::mma_bf16(d, ah, bl, id_rx, 1);
-              tc::mma_bf16(d, al, bh, id_rx, 1);
-            }
-            tc::commit(&mbar_rx);
-            rx_pending = true;
-          }
-        }
-        first_tile = false;
-        __syncthreads();
-        if (s_fail) break;
+    bool fail = false, rx_out = false;
+    int64_t tile = 0;
+    int f = 0;
+    if (steps > 0) {
+      start_tile(0);
+      values();
+      store(0);
+      tc::fence_proxy_async_smem();
+      meet();
+      if (tid == 32) issue_tx(0, 0, 0);
+    }
+    for (int64_t i = 0; i < steps; ++i) {
+      const int par = (int)(i & 1);
+      const bool more = i + 1 < steps;
+      const int f_next = f + 1 < nf ? f + 1 : 0;
+      if (more) {
+        if (f_next == 0) start_tile(tile + 1);
+        values();
       }
+      if (rx_out) wait(&mbar_rx, ph_rx);  // RX(i - 1) has read its A tile and B_rx
+      if (more) store(par ^ 1);
+      const float rw = rcs[tile & 1][s_p];
+      wait(&mbar_tx, ph_tx);
+      tc::fence_after_sync();
+      if constexpr (kTwoPass) {
+        float d0[TXK][16], d1[TXK][16];
+#pragma unroll
+        for (int k = 0; k < TXK; ++k) load_chunk(k, d0[k], d1[k]);
+        meet();  // every warp has read the first pass
+        if (tid == 32 && !s_fail) issue_tx(par, f, 1);
+#pragma unroll
+        for (int k = 0; k < TXK; ++k) form(k, d0[k], d1[k], rw);
+        if (s_fail) {  // nothing was issued: all threads leave together
+          fail = true;
+          rx_out = false;
+          break;
+        }
+        wait(&mbar_tx, ph_tx);
+        tc::fence_after_sync();
+        load_chunk(TXK, d0[0], d1[0]);
+        form(TXK, d0[0], d1[0], rw);
+      } else {
+#pragma unroll
+        for (int k = 0; k < NC; ++k) {
+          float d0[16], d1[16];
+          load_chunk(k, d0, d1);
+          form(k, d0, d1, rw);
+        }
+      }
+      tc::fence_proxy_async_smem();
+      meet();
+      if (s_fail) {
+        fail = true;
+        rx_out = false;
+        break;
+      }
+      if (tid == 0) issue_rx(par, f, tile == 0);
+      if (tid == 32 && more) issue_tx(par ^ 1, f_next, 0);
+      rx_out = true;
+      if (f_next == 0) ++tile;
+      f = f_next;
     }
     // ---- drain, then Y = combine(D_rx[f]) -> partial[item][f][t][e] ----
-    if (tid == 0 && rx_pending) {
-      wait0(&mbar_rx, ph_rx);
-      rx_pending = false;
-    }
-    tc::fence_before_sync();
-    __syncthreads();
-    tc::fence_after_sync();
-    const bool fail = s_fail != 0;
+    if (rx_out) wait(&mbar_rx, ph_rx);
+    meet();
+    fail = s_fail != 0;
+    float* X = reinterpret_cast<float*>(sm);
     float2* out = A.partial + (size_t)item * fb * NT * kTcE;
-    for (int f = 0; f < fb; ++f) {
+    for (int fo = 0; fo < fb; ++fo) {
       for (int k = 0; k < NC; ++k) {
         float v[32];
-        const bool have = !first_tile && f < nf && !fail;
-        if (have) tc::tmem_ld32(tmem + ((uint32_t)(32 * q) << 16) + TXC + N * f + h * NT + 32 * k, v);
+        const bool have = steps > 0 && fo < nf && !fail;
+        if (have) tc::tmem_ld32(trow + TXC + N * fo + h * NT + 32 * k, v);
         const int row = 32 * q + lane;  // (c, e)
         if (row >= 64) {
 #pragma unroll
@@ -660,7 +434,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_kernel(const __grid_constant__
 #pragma unroll
           for (int t = 0; t < 32; ++t) {
             const float val = have ? (h ? v[t] + x[t] : v[t] - x[t]) : 0.f;
-            float* o = reinterpret_cast<float*>(out + ((size_t)f * NT + 32 * k + t) * kTcE + row);
+            float* o = reinterpret_cast<float*>(out + ((size_t)fo * NT + 32 * k + t) * kTcE + row);
             o[h] = val;  // h = 0 real part, h = 1 imaginary part
           }
         }
@@ -668,10 +442,15 @@ __global__ void __launch_bounds__(kThreads, 1) tc_kernel(const __grid_constant__
       }
     }
   }
-  // ---- release TMEM ----
+  // ---- release TMEM (after a wait that gave up: once what is still in flight has had its bounded time) ----
   tc::fence_before_sync();
   __syncthreads();
-  if (s_fail && tid == 0) atomicExch(A.status, FSG_ETIMEOUT);
+  if (s_fail && tid == 0) {
+    tc::mbar_wait_bounded(&mbar_tx, ph_tx, kWaitTries);
+    tc::mbar_wait_bounded(&mbar_rx, ph_rx, kWaitTries);
+    atomicExch(A.status, FSG_ETIMEOUT);
+  }
+  __syncthreads();
   if (warp == 0) tc::tmem_dealloc(tmem, kTmemCols);
 }
 
@@ -784,19 +563,25 @@ cudaError_t launch_tc_geometry(int U, int max_tiles, int sms, const TcArgs& A, c
   return cudaGetLastError();
 }
 
-template <int U, bool kSplitTx>
+template <int U, int NC>
 static cudaError_t launch_tc_t(int grid, const TcArgs& A, cudaStream_t s) {
-  const uint32_t smem = tc_smem_bytes(A.fb, A.nc);
-  cudaError_t e = cudaFuncSetAttribute(tc_kernel<U, kSplitTx>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const uint32_t smem = tc_smem_bytes(A.fb, NC);
+  cudaError_t e = cudaFuncSetAttribute(tc_kernel<U, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  tc_kernel<U, kSplitTx><<<grid, kThreads, smem, s>>>(A);
+  tc_kernel<U, NC><<<grid, kThreads, smem, s>>>(A);
   return cudaGetLastError();
 }
 
 cudaError_t launch_tc(int U, int grid, const TcArgs& A, cudaStream_t s) {
-  const bool split = tc_tx_chunks(A.nc) < A.nc;
-  if (U == 1) return split ? launch_tc_t<1, true>(grid, A, s) : launch_tc_t<1, false>(grid, A, s);
-  return split ? launch_tc_t<2, true>(grid, A, s) : launch_tc_t<2, false>(grid, A, s);
+  switch (10 * U + A.nc) {
+    case 11: return launch_tc_t<1, 1>(grid, A, s);
+    case 12: return launch_tc_t<1, 2>(grid, A, s);
+    case 13: return launch_tc_t<1, 3>(grid, A, s);
+    case 21: return launch_tc_t<2, 1>(grid, A, s);
+    case 22: return launch_tc_t<2, 2>(grid, A, s);
+    case 23: return launch_tc_t<2, 3>(grid, A, s);
+    default: return cudaErrorInvalidValue;
+  }
 }
 
 }  // namespace fsg
