@@ -2,14 +2,25 @@
 //
 // Network: 64 random Fourier features [sin(2 pi B u), cos(2 pi B u)] of the normalised
 // inputs, four hidden layers of 256 with SiLU, a linear head of n_out <= 10 outputs (the same
-// network that the training kernels of fsg_mlp_train.cu train, with the same SiLU).  A persistent CTA takes 128 queries at a time and keeps everything on
-// chip:
+// network that the training kernels of fsg_mlp_train.cu train, with the same SiLU).  A persistent CTA
+// takes 128 queries at a time and keeps everything on chip:
 //   features -> A (shared memory, BF16 hi + lo, K-major core matrices)
 //   per hidden layer: D (TMEM, 128 x 256 FP32) = A_hi W^T + A_lo W^T, two tcgen05.mma
-//   kind::f16 per K step of 16, the layer's BF16 weights streamed through two 32 KB
-//   shared-memory buffers by TMA bulk copies (64 input columns per copy);
+//   kind::f16 per K step of 16, the layer's BF16 weights streamed through four 16 KB
+//   shared-memory buffers by TMA bulk copies (32 input columns per copy);
 //   epilogue: D + bias -> SiLU -> next layer's A (hi + lo), or, after the last hidden layer,
 //   the 256 -> n_out head on the CUDA cores.
+// Sixteen worker warps run the features and epilogues, 64 columns at a time; one more streams the weights
+// and one issues the MMAs of a layer's 64 input columns as soon as the workers have written them, so the
+// products run under the epilogue that feeds them (D alternates between two halves of TMEM).  The
+// next tile's features are formed before the last layer's epilogue, for the same reason.
+//
+// What bounds it: per layer and tile 4,200 cycles of MMAs (131 each at N = 256) and, before them, the
+// first 64 columns' epilogue; the 32,768 SiLUs of a layer (two MUFU operations each, 4,096 cycles) run
+// beside.  1,048,576 queries: 1,680 us with products and epilogues in turn on 8 warps, 1,312 with the
+// products under the epilogues, 1,290 with 16 worker warps, 1,191 with four 16 KB weight buffers and
+// their own warp instead of two of 32 KB.
+//
 // The weights are BF16 (as in training) and multiply exactly; splitting the activations into
 // hi + lo BF16 keeps them at FP32-class precision (~1e-5 relative), as in the training forward
 // pass.  Every mbarrier wait is bounded: on timeout the CTA
@@ -29,16 +40,18 @@ namespace fsg {
 constexpr int kMlpRows = 128;      // queries per tile (MMA M)
 constexpr int kMlpWidth = 256;     // hidden width (MMA N)
 constexpr int kMlpFeat = 128;      // 2 x 64 Fourier features
-constexpr int kMlpChunkK = 64;     // input columns per weight copy
+constexpr int kMlpChunkK = 64;     // input columns per packed chunk, and per step of the epilogue
 constexpr uint32_t kMlpChunkBytes = kMlpWidth * kMlpChunkK * 2;  // 32 KB
 constexpr uint32_t kMlpKGroups = kMlpWidth / 8;                 // A operand: 32 core matrices along K
 constexpr uint32_t kMlpABytes = kMlpRows * kMlpWidth * 2;       // 64 KB per hi / lo
 constexpr uint32_t kOffAHi = 0;
 constexpr uint32_t kOffALo = kMlpABytes;
-constexpr uint32_t kOffB0 = 2 * kMlpABytes;
-constexpr uint32_t kOffB1 = kOffB0 + kMlpChunkBytes;
-constexpr uint32_t kMlpSmem = kOffB1 + kMlpChunkBytes + 1024;
+constexpr uint32_t kOffB = 2 * kMlpABytes;
+constexpr int kMlpPieceK = 32, kMlpBufs = 4;         // weights are streamed in half chunks of 32 input columns
+constexpr uint32_t kMlpPieceBytes = kMlpWidth * kMlpPieceK * 2;  // 16 KB
+constexpr uint32_t kMlpSmem = kOffB + kMlpBufs * kMlpPieceBytes;
 constexpr uint32_t kMlpWaitTries = 1u << 26;
+constexpr uint64_t kMlpDrainNs = 1000000;  // a copy or a layer's products take microseconds
 constexpr int kMlpMaxOut = 10;
 
 // SiLU z * sigmoid(z) with the fast exponential and reciprocal, evaluated exactly as the
@@ -55,193 +68,207 @@ __device__ __forceinline__ void store_a8(unsigned char* sm, int r, int k, const 
   *reinterpret_cast<uint4*>(sm + kOffALo + off) = lo;
 }
 
-__global__ void __launch_bounds__(256, 1) mlp_tc_forward_kernel(const __grid_constant__ FsgMlpWeights W,
-                                                                 const float* __restrict__ u, int64_t n,
-                                                                 float* __restrict__ out, int* status) {
+constexpr int kMlpWorkers = 512, kMlpBlock = kMlpWorkers + 64;
+constexpr int kMlpPiecesPerTile = (kMlpFeat + 3 * kMlpWidth) / kMlpPieceK;
+
+__global__ void __launch_bounds__(kMlpBlock, 1) mlp_tc_forward_kernel(const __grid_constant__ FsgMlpWeights W,
+                                                                       const float* __restrict__ u, int64_t n,
+                                                                       float* __restrict__ out, int* status) {
   extern __shared__ __align__(1024) unsigned char sm[];
-  __shared__ uint64_t mbar_full[2], mbar_free[2], mbar_layer;
+  __shared__ uint64_t mbar_full[kMlpBufs], mbar_free[kMlpBufs];  // weight buffers: copied in, released by their MMAs
+  __shared__ uint64_t mbar_a[4];                   // 64 columns of A written, one arrival per worker warp
+  __shared__ uint64_t mbar_layer;                  // a layer's products done
   __shared__ uint32_t tmem_holder;
   __shared__ int s_fail;
   __shared__ float bmat[64 * 4];
   __shared__ float whead[kMlpMaxOut][kMlpWidth];
   __shared__ float bias_s[4][kMlpWidth];
-  __shared__ float hsum[kMlpRows][kMlpMaxOut];
+  __shared__ float hsum[3][kMlpRows][kMlpMaxOut];
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = tc::warp_uniform(tid >> 5), lane = tid & 31;
   const int nout = W.n_out;
   for (int i = tid; i < 64 * 4; i += blockDim.x) bmat[i] = W.bmat[i];
   for (int i = tid; i < kMlpMaxOut * kMlpWidth; i += blockDim.x)
     whead[i / kMlpWidth][i % kMlpWidth] = (i / kMlpWidth < nout) ? W.w_head[i] : 0.f;
   for (int i = tid; i < 4 * kMlpWidth; i += blockDim.x) bias_s[i / kMlpWidth][i % kMlpWidth] = W.bias[i / kMlpWidth][i % kMlpWidth];
   if (tid == 0) {
-    for (int b = 0; b < 2; ++b) {
+    for (int b = 0; b < kMlpBufs; ++b) {
       tc::mbar_init(&mbar_full[b], 1);
       tc::mbar_init(&mbar_free[b], 1);
     }
+    for (int c = 0; c < 4; ++c) tc::mbar_init(&mbar_a[c], kMlpWorkers / 32);
     tc::mbar_init(&mbar_layer, 1);
     tc::fence_mbar_init();
     s_fail = 0;
   }
-  if (warp == 0) tc::tmem_alloc(&tmem_holder, kMlpWidth);
+  if (warp == 0) tc::tmem_alloc(&tmem_holder, 2 * kMlpWidth);
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = tmem_holder;
   const uint32_t sbase = tc::smem_u32(sm);
-  const uint32_t idesc = tc::idesc_bf16(kMlpRows, kMlpWidth, 0, 0);
-  // Thread 0 streams the weights as one sequence of 32 KB chunks over all layers and tiles
-  // (kChunksPerTile per tile), keeping up to two in flight; chunk g goes to buffer g & 1.
-  constexpr int kChunksPerTile = kMlpFeat / kMlpChunkK + 3 * (kMlpWidth / kMlpChunkK);
-  uint32_t ph_full[2] = {0u, 0u}, ph_free[2] = {0u, 0u}, ph_layer = 0u;
-  int64_t next_load = 0;  // next chunk to copy
-  const int64_t my_tiles = ((n + kMlpRows - 1) / kMlpRows - blockIdx.x + gridDim.x - 1) / gridDim.x;
-  const int64_t total_chunks = my_tiles * kChunksPerTile;
-  // issue the copy of chunk g; before reusing a buffer, wait for the MMAs of chunk g - 2
-  auto load = [&](int64_t g) -> bool {
-    const int b = (int)(g & 1);
-    if (g >= 2) {
-      if (!tc::mbar_wait_bounded(&mbar_free[b], ph_free[b], kMlpWaitTries)) return false;
-      ph_free[b] ^= 1u;
-    }
-    const int j = (int)(g % kChunksPerTile);
-    const int layer = j < 2 ? 0 : 1 + (j - 2) / 4, c = j < 2 ? j : (j - 2) % 4;
-    tc::mbar_arrive_expect_tx(&mbar_full[b], kMlpChunkBytes);
-    tc::bulk_g2s(sm + (b ? kOffB1 : kOffB0),
-                 static_cast<const unsigned char*>(W.packed[layer]) + (size_t)c * kMlpChunkBytes, kMlpChunkBytes,
-                 &mbar_full[b]);
-    return true;
-  };
-  int64_t tile_iter = 0;
-
-  // TMEM read mapping: row = 32 (warp % 4) + lane, columns [128 (warp / 4), +128)
-  const int row = 32 * (warp & 3) + lane, chalf = warp >> 2;
   const int64_t n_tiles = (n + kMlpRows - 1) / kMlpRows;
+  const int my_tiles = (int)((n_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x);
+  // a bounded wait of a whole warp; after one has given up nothing waits any more
+  auto wait = [&](uint64_t* mb, uint32_t parity) {
+    if (!tc::mbar_test(mb, parity) && !s_fail && !tc::mbar_wait_bounded(mb, parity, kMlpWaitTries)) s_fail = 1;
+    __syncwarp();
+  };
 
-  for (int64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-    // ---- features of the tile's queries -> A (K = 128) ----
-    {
-      const int r = tid & (kMlpRows - 1), half = tid >> 7;
-      const int64_t q = tile * kMlpRows + r;
-      float4 uv = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (q < n) uv = make_float4(u[4 * q], u[4 * q + 1], u[4 * q + 2], u[4 * q + 3]);
+  const int total = my_tiles * kMlpPiecesPerTile;  // the weights of a tile are one sequence of 16 KB pieces
+  if (warp == kMlpWorkers / 32 + 1) {
+    // =============================== weights ===============================
+    const bool leader = tc::elect_one();
+    int j = 0;
+    for (int g = 0; g < total && !tc::warp_uniform(s_fail); ++g) {
+      const int b = g % kMlpBufs;
+      if (g >= kMlpBufs) wait(&mbar_free[b], (g / kMlpBufs - 1) & 1);  // the MMAs of piece g - kMlpBufs
+      constexpr int kP0 = kMlpFeat / kMlpPieceK, kP1 = kMlpWidth / kMlpPieceK;
+      const int layer = j < kP0 ? 0 : 1 + (j - kP0) / kP1, c = j < kP0 ? j : (j - kP0) % kP1;
+      if (leader) {
+        tc::mbar_arrive_expect_tx(&mbar_full[b], kMlpPieceBytes);
+        tc::bulk_g2s(sm + kOffB + b * kMlpPieceBytes,
+                     static_cast<const unsigned char*>(W.packed[layer]) + (size_t)c * kMlpPieceBytes, kMlpPieceBytes,
+                     &mbar_full[b]);
+      }
+      j = j + 1 == kMlpPiecesPerTile ? 0 : j + 1;
+    }
+  } else if (warp == kMlpWorkers / 32) {
+    // =============================== MMAs ===============================
+    constexpr uint32_t idesc = tc::idesc_bf16(kMlpRows, kMlpWidth, 0, 0);
+    const bool leader = tc::elect_one();
+    uint32_t ph_a = 0;  // bit c: parity of mbar_a[c]
+    int g = 0;
+    for (int tile = 0; tile < my_tiles; ++tile) {
+      for (int layer = 0; layer < 4; ++layer) {
+        const int np = (layer == 0 ? kMlpFeat : kMlpWidth) / kMlpPieceK;
+        const uint32_t d = tmem + (layer & 1) * kMlpWidth;
+        for (int c = 0; c < np; ++c, ++g) {
+          const int b = g % kMlpBufs;
+          if ((c & 1) == 0) {
+            wait(&mbar_a[c >> 1], (ph_a >> (c >> 1)) & 1);
+            ph_a ^= 1u << (c >> 1);
+          }
+          wait(&mbar_full[b], (g / kMlpBufs) & 1);
+          tc::fence_after_sync();
+          if (leader && !s_fail) {
+            const uint32_t bb = sbase + kOffB + b * kMlpPieceBytes;
 #pragma unroll
-      for (int blk = 0; blk < 4; ++blk) {
+            for (int ks = 0; ks < kMlpPieceK / 16; ++ks) {
+              const int kk = c * (kMlpPieceK / 16) + ks;  // K step of 16 within the layer
+              const uint64_t ah = tc::sdesc(sbase + kOffAHi + kk * 256, 128, kMlpKGroups * 128);
+              const uint64_t al = tc::sdesc(sbase + kOffALo + kk * 256, 128, kMlpKGroups * 128);
+              // k-group-major packed piece: K stride 4096 bytes, N stride 128
+              const uint64_t bd = tc::sdesc(bb + ks * 2 * 4096, 4096, 128);
+              tc::mma_bf16(d, ah, bd, idesc, kk > 0);
+              tc::mma_bf16(d, al, bd, idesc, 1);
+            }
+            tc::commit(&mbar_free[b]);
+            if (c == np - 1) tc::commit(&mbar_layer);
+          }
+        }
+      }
+    }
+  } else {
+    // =============================== workers ===============================
+    // TMEM row of this thread, and its 16 columns of each 64
+    const int row = 32 * (warp & 3) + lane, part = warp >> 2;
+    const uint32_t trow = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+    auto ready = [&](int c) {  // this warp's part of A columns [64 c, 64 c + 64) is written, its D reads done
+      tc::fence_proxy_async_smem();
+      tc::fence_before_sync();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&mbar_a[c]);
+    };
+    // features of a tile's queries -> A (K = 128): sines, then cosines
+    auto features = [&](int64_t tile) {
+      const int64_t q = tile * kMlpRows + row;
+      float4 uv = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (q < n) uv = *reinterpret_cast<const float4*>(u + 4 * q);
+#pragma unroll
+      for (int blk = 0; blk < 2; ++blk) {
+        const int j0 = 16 * part + 8 * blk;
         float sv[8], cv[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          const int j = 32 * half + 8 * blk + i;
-          const float t = bmat[4 * j] * uv.x + bmat[4 * j + 1] * uv.y + bmat[4 * j + 2] * uv.z + bmat[4 * j + 3] * uv.w;
+          const float* b = bmat + 4 * (j0 + i);
+          const float t = b[0] * uv.x + b[1] * uv.y + b[2] * uv.z + b[3] * uv.w;
           sincospif(2.0f * t, &sv[i], &cv[i]);
         }
-        store_a8(sm, r, 32 * half + 8 * blk, sv);
-        store_a8(sm, r, 64 + 32 * half + 8 * blk, cv);
+        store_a8(sm, row, j0, sv);
+        store_a8(sm, row, 64 + j0, cv);
       }
-    }
-    tc::fence_proxy_async_smem();
-    tc::fence_before_sync();
-    __syncthreads();
-    tc::fence_after_sync();
-
-    float head[kMlpMaxOut];
+      ready(0);
+      ready(1);
+    };
+    uint32_t ph_layer = 0;
+    if (my_tiles > 0) features(blockIdx.x);
+    for (int it = 0; it < my_tiles; ++it) {
+      const int64_t tile = blockIdx.x + (int64_t)it * gridDim.x;
+      float head[kMlpMaxOut];
 #pragma unroll
-    for (int j = 0; j < kMlpMaxOut; ++j) head[j] = 0.f;
-    int64_t chunk0 = tile_iter * kChunksPerTile;  // global index of this layer's first chunk
-    for (int layer = 0; layer < 4; ++layer) {
-      const int K = layer == 0 ? kMlpFeat : kMlpWidth;
-      const int nch = K / kMlpChunkK;
-      // ---- MMAs: thread 0 keeps two weight chunks in flight and issues the products ----
-      if (tid == 0 && !s_fail) {
-        bool ok = true;
-        for (int c = 0; c < nch && ok; ++c) {
-          const int64_t g = chunk0 + c;
-          const int b = (int)(g & 1);
-          // the look-ahead copy (chunk g + 1) reuses chunk g - 1's buffer: issue it only if that
-          // chunk's MMAs are done, so that the MMAs of consecutive chunks stay queued back to back
-          while (ok && next_load < g + 2 && next_load < total_chunks) {
-            if (next_load > g && next_load >= 2 &&
-                !tc::mbar_test(&mbar_free[next_load & 1], ph_free[next_load & 1]))
-              break;
-            ok = load(next_load++);
-          }
-          if (!ok) break;
-          if (!tc::mbar_wait_bounded(&mbar_full[b], ph_full[b], kMlpWaitTries)) { ok = false; break; }
-          ph_full[b] ^= 1u;
-          tc::fence_after_sync();
-          const uint32_t bb = sbase + (b ? kOffB1 : kOffB0);
-#pragma unroll
-          for (int ks = 0; ks < kMlpChunkK / 16; ++ks) {
-            const int kk = c * (kMlpChunkK / 16) + ks;  // K step of 16 within the layer
-            const uint64_t ah = tc::sdesc(sbase + kOffAHi + kk * 256, 128, kMlpKGroups * 128);
-            const uint64_t al = tc::sdesc(sbase + kOffALo + kk * 256, 128, kMlpKGroups * 128);
-            // k-group-major packed chunk: K stride 4096 bytes, N stride 128
-            const uint64_t bd = tc::sdesc(bb + ks * 2 * 4096, 4096, 128);
-            tc::mma_bf16(tmem, ah, bd, idesc, kk > 0);
-            tc::mma_bf16(tmem, al, bd, idesc, 1);
-          }
-          tc::commit(&mbar_free[b]);
-        }
-        if (ok) {
-          tc::commit(&mbar_layer);
-          ok = tc::mbar_wait_bounded(&mbar_layer, ph_layer, kMlpWaitTries);
-          ph_layer ^= 1u;
-        }
-        // the layer's products are done and both buffers are free: start the next two
-        // copies now, so that they land while the epilogue runs
-        while (ok && next_load < chunk0 + nch + 2 && next_load < total_chunks) ok = load(next_load++);
-        if (!ok) s_fail = 1;
-      }
-      chunk0 += nch;
-      tc::fence_before_sync();
-      __syncthreads();
-      tc::fence_after_sync();
-      if (s_fail) break;
-      // ---- epilogue: bias + SiLU -> next A, or the head ----
-      const float* bias = bias_s[layer];
+      for (int j = 0; j < kMlpMaxOut; ++j) head[j] = 0.f;
+      for (int layer = 0; layer < 4; ++layer) {
+        wait(&mbar_layer, ph_layer);
+        ph_layer ^= 1u;
+        tc::fence_after_sync();
+        if (layer == 3 && it + 1 < my_tiles) features(tile + gridDim.x);
+        const float* bias = bias_s[layer];
+        const uint32_t d = trow + (layer & 1) * kMlpWidth + 16 * part;
+        uint32_t next[16];
+        tc::tmem_ld16_async(d, next);
 #pragma unroll 1
-      for (int cb = 0; cb < 4; ++cb) {
-        const int col0 = 128 * chalf + 32 * cb;
-        float v[32];
-        tc::tmem_ld32(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + col0, v);
+        for (int c = 0; c < 4; ++c) {
+          const int col0 = 64 * c + 16 * part;
+          float v[16];
+          tc::tmem_wait_ld16(next);
 #pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] = mlp_silu(v[i] + bias[col0 + i]);
-        if (layer < 3) {
+          for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(next[i]);
+          if (c < 3) tc::tmem_ld16_async(d + 64 * (c + 1), next);  // lands under this chunk's SiLUs
 #pragma unroll
-          for (int g8 = 0; g8 < 4; ++g8) store_a8(sm, row, col0 + 8 * g8, v + 8 * g8);
-        } else {
+          for (int i = 0; i < 16; ++i) v[i] = mlp_silu(v[i] + bias[col0 + i]);
+          if (layer < 3) {
 #pragma unroll
-          for (int j = 0; j < kMlpMaxOut; ++j) {
-            float acc = head[j];
+            for (int g8 = 0; g8 < 2; ++g8) store_a8(sm, row, col0 + 8 * g8, v + 8 * g8);
+            ready(c);
+          } else {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) acc = fmaf(v[i], whead[j][col0 + i], acc);
-            head[j] = acc;
+            for (int j = 0; j < kMlpMaxOut; ++j) {
+              float acc = head[j];
+#pragma unroll
+              for (int i = 0; i < 16; ++i) acc = fmaf(v[i], whead[j][col0 + i], acc);
+              head[j] = acc;
+            }
           }
         }
       }
-      tc::fence_proxy_async_smem();
+      // ---- head: combine the four column sets of each row ----
       tc::fence_before_sync();
-      __syncthreads();
-      tc::fence_after_sync();
-    }
-    if (s_fail) break;
-    // ---- head: combine the two column halves of each row ----
-    if (chalf == 1) {
+      if (part > 0) {
 #pragma unroll
-      for (int j = 0; j < kMlpMaxOut; ++j) hsum[row][j] = head[j];
-    }
-    __syncthreads();
-    if (chalf == 0) {
-      const int64_t q = tile * kMlpRows + row;
-      if (q < n) {
-        for (int j = 0; j < nout; ++j) out[q * nout + j] = head[j] + hsum[row][j] + W.b_head[j];
+        for (int j = 0; j < kMlpMaxOut; ++j) hsum[part - 1][row][j] = head[j];
       }
+      tc::bar_sync(1, kMlpWorkers);
+      if (part == 0) {
+        const int64_t q = tile * kMlpRows + row;
+        if (q < n && !s_fail) {
+          for (int j = 0; j < nout; ++j)
+            out[q * nout + j] = head[j] + hsum[0][row][j] + hsum[1][row][j] + hsum[2][row][j] + W.b_head[j];
+        }
+      }
+      tc::bar_sync(1, kMlpWorkers);
     }
-    __syncthreads();
-    ++tile_iter;
   }
   tc::fence_before_sync();
   __syncthreads();
-  if (s_fail && tid == 0) atomicExch(status, FSG_ETIMEOUT);
-  if (warp == 0) tc::tmem_dealloc(tmem, kMlpWidth);
+  if (s_fail && tid == 0) {
+    // a wait gave up: what is still in flight gets its bounded time before the memory goes away
+    const uint64_t t0 = tc::global_ns();
+    while (tc::global_ns() - t0 < kMlpDrainNs) __nanosleep(1000);
+    atomicExch(status, FSG_ETIMEOUT);
+  }
+  __syncthreads();
+  if (warp == 0) tc::tmem_dealloc(tmem, 2 * kMlpWidth);
 }
 
 // Packs a row-major [256][K] BF16 weight matrix into K/64 chunks of the K-major no-swizzle
@@ -293,7 +320,7 @@ extern "C" int32_t fsg_mlp_tc_forward(const FsgMlpWeights* weights, const float*
   if (e != cudaSuccess) return check_cuda(e, "cudaFuncSetAttribute(mlp_tc_forward_kernel)");
   const int64_t tiles = (n + kMlpRows - 1) / kMlpRows;
   const int grid = (int)(tiles < sms ? tiles : sms);
-  mlp_tc_forward_kernel<<<grid, 256, kMlpSmem, reinterpret_cast<cudaStream_t>(stream_ptr)>>>(*weights, u, n, out,
+  mlp_tc_forward_kernel<<<grid, kMlpBlock, kMlpSmem, reinterpret_cast<cudaStream_t>(stream_ptr)>>>(*weights, u, n, out,
                                                                                                status);
   return check_cuda(cudaGetLastError(), "mlp_tc_forward_kernel launch");
 }

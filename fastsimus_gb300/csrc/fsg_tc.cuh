@@ -17,6 +17,21 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// True in one lane of a converged warp.  tcgen05.mma takes its descriptors from uniform registers: issued
+// by an elected lane in a branch that the whole warp takes, with operands that do not depend on the lane,
+// 96 MMAs of 128 x 256 x 16 take 131 cycles each (the pipe's rate); in a loop under `threadIdx.x == 0`
+// they took 187, of moving the operands over.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred P;\n\t.reg .b32 r;\n\telect.sync r|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}\n"
+      : "=r"(p));
+  return p != 0;
+}
+
+// The value of lane 0, uniform over the warp for the compiler too.
+__device__ __forceinline__ int warp_uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
+
 // Matrix descriptor, no swizzle, descriptor version 1.
 __device__ __forceinline__ uint64_t sdesc(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
   uint64_t d = 0;
@@ -62,6 +77,11 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* mbar, uint32_t parity) {
   return ok != 0;
 }
 
+// Arrives once on `mbar` (release).
+__device__ __forceinline__ void mbar_arrive(uint64_t* mbar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(mbar)) : "memory");
+}
+
 // Non-blocking test of the phase with the given parity.
 __device__ __forceinline__ bool mbar_test(uint64_t* mbar, uint32_t parity) {
   uint32_t ok;
@@ -85,10 +105,14 @@ constexpr uint64_t kMaxWaitNs = 2000000000ull;  // a wait gives up after 2 s, wh
 // Bounded wait: returns false if the phase did not complete within `max_tries` polls or
 // kMaxWaitNs nanoseconds of the global timer, whichever comes first.
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* mbar, uint32_t parity, uint32_t max_tries) {
-  const uint64_t t0 = global_ns();
+  uint64_t t0 = 0;  // read after the first 256 polls: a wait in step with its producer never reads the timer
   for (uint32_t i = 0; i < max_tries; ++i) {
     if (mbar_try_wait(mbar, parity)) return true;
-    if ((i & 255u) == 255u && global_ns() - t0 > kMaxWaitNs) return false;
+    if ((i & 255u) == 255u) {
+      const uint64_t now = global_ns();
+      if (t0 == 0) t0 = now;
+      else if (now - t0 > kMaxWaitNs) return false;
+    }
   }
   return false;
 }
@@ -132,6 +156,27 @@ __device__ __forceinline__ void tmem_alloc(uint32_t* holder, uint32_t ncols) {
 
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+
+// 16 consecutive FP32 columns of this thread's TMEM lane, without waiting: r may be read after
+// tmem_wait_ld16 on it.
+__device__ __forceinline__ void tmem_ld16_async(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+      "%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+}
+
+// Waits for this thread's TMEM loads; the registers of the one being waited for pass through, so that
+// no use of them moves above the wait.
+__device__ __forceinline__ void tmem_wait_ld16(uint32_t (&r)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                 "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+               :
+               : "memory");
 }
 
 // 32 consecutive FP32 columns of this thread's TMEM lane.
