@@ -232,9 +232,13 @@ def das(iq, x, z, delays, param, method: str = "linear") -> torch.Tensor:
         raise ValueError(f"delays must be ({nf}, {nc}), got {d.shape}")
     txd = torch.as_tensor(np.ascontiguousarray(d), device=device)
     probe, p = _das_call(param, method, is_iq)
-    pix, shape = _pixels(x, z, device)
+    xa, za = np.asarray(x, dtype=np.float64), np.asarray(z, dtype=np.float64)
+    if xa.shape != za.shape:
+        raise ValueError(f"x and z must have the same shape, got {xa.shape} and {za.shape}")
+    # pixels in the grids' own order: neighbours of a row read neighbouring samples
+    pix = torch.stack([torch.as_tensor(np.ascontiguousarray(a).reshape(-1), device=device) for a in (xa, za)], dim=1)
     out = torch.empty(pix.shape[0], dtype=torch.complex64, device=device)
     _native.check(_native.load().fsg_das(ctypes.byref(probe), ctypes.byref(p), cm.data_ptr(), nf, ns, txd.data_ptr(),
                                          pix.data_ptr(), pix.shape[0], out.data_ptr(),
                                          _device.stream_handle(device)))
-    return _from_fortran(out, shape)
+    return out.reshape(xa.shape)

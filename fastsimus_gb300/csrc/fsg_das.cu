@@ -15,8 +15,8 @@
 //
 // das_kernel: one thread per pixel, looping over groups of firings and, per element, over the
 // group's firings.  The transmit delays (times c) and the element frames sit in shared memory;
-// the I/Q samples are read channel-major, so the threads of a warp (consecutive pixels down an
-// image column) read nearby samples of the same element.
+// the I/Q samples are read channel-major, so the threads of a warp (consecutive pixels of an
+// image row) read nearby samples of the same element.
 
 #include <cuda_runtime.h>
 #include <math.h>
@@ -31,7 +31,8 @@ namespace fsg {
 constexpr int kDasThreads = 256;      // dasmtx_kernel
 constexpr int kDasImgThreads = 128;   // das_kernel: small CTAs spread the pixels evenly over the SMs
 constexpr int kDasMaxE = 256;
-constexpr int kDasFrameGroup = 32;  // firings whose transmit distances a thread holds at a time
+constexpr int kDasGroup = 8;          // firings whose transmit distances a thread holds at a time
+constexpr int kDasImgBlocks = 7;      // das_kernel CTAs per SM the registers are cut for
 
 constexpr int kIqCh = 8;          // channels per CTA, one warp each
 constexpr int kIqMaxL = 71;       // samples per lane and segment: eight columns and the phasors fit shared memory
@@ -316,42 +317,81 @@ __device__ __forceinline__ bool das_tap(const DasArgs& A, const DasShared& S, in
   return true;
 }
 
+// floorf(s) and the integer.  Records of up to kDasShort samples do without the conversion unit (a
+// quarter of the rate of the others): exact for |s| < 2^22, and beyond that a value that is out of the
+// record as s is (NaN stays NaN).
+constexpr int kDasShort = 1 << 22;
+template <bool kLong>
+__device__ __forceinline__ float das_floor(float s, int* i) {
+  if constexpr (kLong) {
+    const float fi = floorf(s);
+    *i = fi >= 0.f && fi < 2147483648.0f ? (int)fi : 0;
+    return fi;
+  }
+  const float t = s + 12582912.0f;  // 1.5 * 2^23: rounds to the nearest integer
+  const float r = t - 12582912.0f;
+  const int down = r > s ? 1 : 0;
+  *i = __float_as_int(t) - 0x4B400000 - down;
+  return r - (float)down;
+}
+
 // Matrix-free compounded delay-and-sum.  The I/Q rotation exp(2 pi i fc (d_tx + d_rx) / c)
 // factors into a transmit part per (pixel, firing) and a receive part per (pixel, element), so
 // a thread first computes, for a group of firings, the transmit distance and rotation (kept in
-// registers / local memory), then per element the receive distance, aperture test and rotation
+// registers), then per element the receive distance, aperture test and rotation
 // once, and per firing only the sample gather, the interpolation and one complex multiply-add.
-// The group's transmit delays (times c) sit in dynamic shared memory, [firing][element].
-__global__ void __launch_bounds__(kDasImgThreads, 4) das_kernel(const __grid_constant__ DasArgs A, int group) {
+// The group's transmit delays (times c) sit in dynamic shared memory, [element][firing].
+//
+// What bounds it: instruction issue, about 30 per tap, and the gathers (two 8-byte loads per tap; the
+// host passes neighbouring pixels of a row, whose samples share one or two lines).  The call of 75
+// firings x 64 elements x 131,072 pixels, signal copies and launches included: 1,927 us with the
+// firings' values in local memory, a distance per (element, firing) in the transmit search and floor on
+// the conversion unit; 1,324 us now (12 firings 919 -> 404, one firing 759 -> 259).  Groups of 8 keep
+// the kernel within 72 registers, seven CTAs per SM: groups of 16 (five CTAs) took 350 us more, of 12
+// (five CTAs) 530 us.
+template <int G, bool kLinear, bool kLong = false>
+__global__ void __launch_bounds__(kDasImgThreads, kDasImgBlocks) das_kernel(const __grid_constant__ DasArgs A) {
   __shared__ DasShared S;
-  extern __shared__ float ctx_g[];  // [group][E]
+  extern __shared__ __align__(16) float ctx_g[];  // [E][G]
   das_load_elements(A, S);
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const bool valid = p < A.n_pix;
   const float px = valid ? (float)A.pix[2 * p] : 0.f, pz = valid ? (float)A.pix[2 * p + 1] : 0.f;
   const float k_cyc = 0.5f * A.two_fc * A.inv_c;  // cycles per metre of path, fc / c
-  float dtx[kDasFrameGroup];
-  float2 rtx[kDasFrameGroup];
+  const size_t fstride = (size_t)A.E * A.n_s;
+  const float top = (float)(A.n_s - (kLinear ? 2 : 1));  // the last first sample of a tap
   float2 acc = make_float2(0.f, 0.f);
-  for (int g0 = 0; g0 < A.n_frames; g0 += group) {
-    const int ng = min(group, A.n_frames - g0);
+  for (int g0 = 0; g0 < A.n_frames; g0 += G) {
+    const int ng = min(G, A.n_frames - g0);
     __syncthreads();
-    for (int i = threadIdx.x; i < ng * A.E; i += blockDim.x) {
-      const double v = A.txd[(size_t)g0 * A.E + i];
+    for (int i = threadIdx.x; i < G * A.E; i += blockDim.x) {
+      const int e = i / G, j = i % G;
+      const double v = j < ng ? A.txd[(size_t)(g0 + j) * A.E + e] : NAN;
       ctx_g[i] = isnan(v) ? INFINITY : (float)(A.c * v);
     }
     __syncthreads();
     if (!valid) continue;
-    for (int j = 0; j < ng; ++j) {
-      const float* cj = ctx_g + j * A.E;
-      float d = INFINITY;
-      for (int e = 0; e < A.E; ++e) {
-        const float dx = px - S.ex[e], dz = pz - S.ez[e];
-        d = fminf(d, cj[e] + sqrtf(fmaf(dx, dx, dz * dz)));
+    float dtx[G];
+#pragma unroll
+    for (int j = 0; j < G; ++j) dtx[j] = INFINITY;
+    for (int e = 0; e < A.E; ++e) {
+      const float dx = px - S.ex[e], dz = pz - S.ez[e];
+      const float d = sqrtf(fmaf(dx, dx, dz * dz));
+      const float4* cj = reinterpret_cast<const float4*>(ctx_g + e * G);
+#pragma unroll
+      for (int j = 0; j < G / 4; ++j) {
+        const float4 c = cj[j];
+        dtx[4 * j] = fminf(dtx[4 * j], c.x + d);
+        dtx[4 * j + 1] = fminf(dtx[4 * j + 1], c.y + d);
+        dtx[4 * j + 2] = fminf(dtx[4 * j + 2], c.z + d);
+        dtx[4 * j + 3] = fminf(dtx[4 * j + 3], c.w + d);
       }
-      dtx[j] = d;
+    }
+    float2 rtx[G];
+#pragma unroll
+    for (int j = 0; j < G; ++j) {
       float sn = 0.f, cs = 1.f;
-      if (A.iq_rot && d < INFINITY) sincospif(2.f * k_cyc * d, &sn, &cs);
+      if (A.iq_rot && dtx[j] < INFINITY) sincospif(2.f * k_cyc * dtx[j], &sn, &cs);
       rtx[j] = make_float2(cs, sn);
     }
     for (int e = 0; e < A.E; ++e) {
@@ -364,35 +404,24 @@ __global__ void __launch_bounds__(kDasImgThreads, 4) das_kernel(const __grid_con
       const float dr = sqrtf(fmaf(dx, dx, dz * dz));
       float2 ae = make_float2(0.f, 0.f);
       const float2* ce = A.iq + ((size_t)g0 * A.E + e) * A.n_s;
-      const size_t fstride = (size_t)A.E * A.n_s;
-      const float last = (float)(A.n_s - 1);
-      // branch-free taps (a tap outside the record reads sample 0 with weight 0), unrolled so
-      // that the gathers of several firings are in flight together
-      if (A.method == FSG_DAS_LINEAR) {
-#pragma unroll 4
-        for (int j = 0; j < ng; ++j) {
-          const float s = ((dtx[j] + dr) * A.inv_c - A.t0) * A.fs;
-          const float fi = floorf(s);
-          const bool ok = fi >= 0.f && fi + 1.f <= last;
-          const int i0 = ok ? (int)fi : 0;
+      // branch-free taps (a tap outside the record reads sample 0 with weight 0; the firings past the
+      // last one have no finite delay), unrolled so that the gathers of several firings are in flight
+#pragma unroll
+      for (int j = 0; j < G; ++j) {
+        const float s = ((dtx[j] + dr) * A.inv_c - A.t0) * A.fs;
+        int i;
+        const float fi = das_floor<kLong>(kLinear ? s : s + 0.5f, &i);
+        const bool ok = fi >= 0.f && fi <= top;
+        const float2* cj = ce + (j < ng ? j : 0) * fstride + (ok ? i : 0);
+        float2 v = cj[0];
+        if constexpr (kLinear) {
+          const float2 b = cj[1];
           const float w = s - fi;
-          const float2* cj = ce + j * fstride;
-          const float2 a = cj[i0], b = cj[i0 + 1];
-          const float2 v = ok ? make_float2(fmaf(w, b.x - a.x, a.x), fmaf(w, b.y - a.y, a.y)) : make_float2(0.f, 0.f);
-          ae.x = fmaf(v.x, rtx[j].x, fmaf(-v.y, rtx[j].y, ae.x));
-          ae.y = fmaf(v.x, rtx[j].y, fmaf(v.y, rtx[j].x, ae.y));
+          v = make_float2(fmaf(w, b.x - v.x, v.x), fmaf(w, b.y - v.y, v.y));
         }
-      } else {
-#pragma unroll 4
-        for (int j = 0; j < ng; ++j) {
-          const float s = ((dtx[j] + dr) * A.inv_c - A.t0) * A.fs;
-          const float fi = floorf(s + 0.5f);
-          const bool ok = fi >= 0.f && fi <= last;
-          const float2 c = ce[j * fstride + (ok ? (int)fi : 0)];
-          const float2 v = ok ? c : make_float2(0.f, 0.f);
-          ae.x = fmaf(v.x, rtx[j].x, fmaf(-v.y, rtx[j].y, ae.x));
-          ae.y = fmaf(v.x, rtx[j].y, fmaf(v.y, rtx[j].x, ae.y));
-        }
+        v = ok ? v : make_float2(0.f, 0.f);
+        ae.x = fmaf(v.x, rtx[j].x, fmaf(-v.y, rtx[j].y, ae.x));
+        ae.y = fmaf(v.x, rtx[j].y, fmaf(v.y, rtx[j].x, ae.y));
       }
       float sn = 0.f, cs = 1.f;
       if (A.iq_rot) sincospif(2.f * k_cyc * dr, &sn, &cs);
@@ -573,9 +602,23 @@ extern "C" int32_t fsg_das(const FsgProbe* probe, const FsgDasParams* params, co
   if (n_pixels == 0) return FSG_OK;
   A.iq = static_cast<const float2*>(iq);
   A.out = static_cast<float2*>(image_out);
-  const int group = n_frames < kDasFrameGroup ? n_frames : kDasFrameGroup;
-  das_kernel<<<(unsigned)((n_pixels + kDasImgThreads - 1) / kDasImgThreads), kDasImgThreads,
-               (size_t)group * A.E * sizeof(float), reinterpret_cast<cudaStream_t>(stream)>>>(A, group);
+  const unsigned grid = (unsigned)((n_pixels + kDasImgThreads - 1) / kDasImgThreads);
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  // up to four firings in one group of four: 259 us against 299 for one firing, 268 against 313 for four
+  // (131,072 pixels, 64 elements); at five and more the groups of eight are as fast or faster (311 / 312,
+  // twelve firings 404 / 410 with and without this rule)
+  const bool linear = A.method == FSG_DAS_LINEAR, lng = n_samples > kDasShort, few = n_frames <= 4 || lng;
+  const size_t smem = (size_t)(few ? 4 : kDasGroup) * A.E * sizeof(float);
+  if (lng) {
+    if (linear) das_kernel<4, true, true><<<grid, kDasImgThreads, smem, s>>>(A);
+    else das_kernel<4, false, true><<<grid, kDasImgThreads, smem, s>>>(A);
+  } else if (few) {
+    if (linear) das_kernel<4, true><<<grid, kDasImgThreads, smem, s>>>(A);
+    else das_kernel<4, false><<<grid, kDasImgThreads, smem, s>>>(A);
+  } else {
+    if (linear) das_kernel<kDasGroup, true><<<grid, kDasImgThreads, smem, s>>>(A);
+    else das_kernel<kDasGroup, false><<<grid, kDasImgThreads, smem, s>>>(A);
+  }
   return check_cuda(cudaGetLastError(), "das_kernel launch");
 }
 

@@ -46,3 +46,31 @@ def test_rf2iq_chunks_and_segments(ns, nc, nf, bw):
     ref = np.stack([D.rf2iq(x.astype(np.float64), 20e6, 5e6, bw) for x in rf])
     assert got.shape == ref.shape
     assert G.rel_l2(got, ref) < 2e-5
+
+
+@pytest.mark.parametrize("nf,n_pix,n_s", [(1, 1, 300), (4, 127, 300), (5, 128, 300), (8, 129, 300), (9, 300, 300),
+                                          (17, 33, 300), (2, 40, (1 << 22) + 1)])
+@pytest.mark.parametrize("method", ["linear", "nearest"])
+def test_das_firing_groups(nf, n_pix, n_s, method):
+    """Firing groups (up to four firings, full groups of eight, tails), pixels around a CTA's 128 and a
+    record beyond the short-record floor.  FP32 phases at ~100 wavelengths of path: relative L2 <= 1e-3;
+    the signal varies slowly, so that a nearest tap that rounds the other way stays within it."""
+    require_gpu()
+    from fastsimus_gb300.beamform import DasParam, das
+
+    rng = np.random.default_rng(nf * 1000 + n_pix)
+    E, pitch, fs, c, fc = 12, 0.3e-3, 20e6, 1540.0, 5e6
+    xe = D.element_frame(E, pitch, np.inf)[0]
+    iq = np.zeros((nf, n_s, E), dtype=np.complex64)
+    t = np.arange(300)[None, :, None] / 300.0
+    iq[:, :300] = np.exp(0.3j * np.pi * (t + rng.uniform(0, 2, (nf, 1, E)))) * rng.uniform(0.5, 1.5, (nf, 1, E))
+    delays = np.stack([xe * np.sin(a) / c for a in np.linspace(-0.1, 0.1, nf)])
+    delays -= delays.min(axis=1, keepdims=True)
+    delays[nf // 2, 5] = np.nan
+    x, z = rng.uniform(-2e-3, 2e-3, (n_pix, 1)), rng.uniform(3e-3, 9e-3, (n_pix, 1))
+    param = DasParam(fc=fc, pitch=pitch, Nelements=E, width=0.25e-3, c=c, fs=fs, fnumber=1.0)
+    got = np64(das(torch.as_tensor(iq, device="cuda"), x, z, delays, param, method))
+    ref = D.das(iq[:, :300].astype(np.complex128), x, z, delays, n_elements=E, pitch=pitch, radius=np.inf, c=c, fs=fs,
+                fc=fc, fnumber=1.0, method=method)
+    assert got.shape == x.shape
+    assert G.rel_l2(got, ref) < 1e-3
