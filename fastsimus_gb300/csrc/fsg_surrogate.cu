@@ -31,11 +31,10 @@ struct TxFieldArgs {
   const double* samples;  // [n][4]: x, z, f (Hz), theta (rad)
   int64_t n;
   float2* out;            // [n] complex transmit pressure
-  const float4* src_pos;  // [E*U]
-  const float2* rot_e;    // [E]
+  const float4* src_pos;  // [E*U], z = 0
   float pitch;            // element x = (e - (E-1)/2) * pitch in float32 (utils/geometry.py:33-37)
   int E, U;
-  double fc, inv_c, cyc_fc;  // centre frequency, 1 / c, tx_n_wavelengths / fc (cycles of the pulse per Hz)
+  dfl fc, inv_c, cyc_fc;  // centre frequency, 1 / c, tx_n_wavelengths / fc (cycles of the pulse per Hz)
   float alpha_hz;         // attenuation, Np/m per Hz
   float inv_sigma, shape; // probe response sqrt(exp(-(|f - fc| inv_sigma)^shape))
   SweepConst C;           // geometry constants (dk/dalpha unused)
@@ -51,6 +50,16 @@ __device__ __forceinline__ dfl df_scale(float a, dfl b) {
   return fast_two_sum(p, fmaf(a, b.lo, fmaf(a, b.hi, -p)));
 }
 
+__device__ __forceinline__ dfl df_mul(dfl a, dfl b) {
+  const float p = __fmul_rn(a.hi, b.hi);
+  float e = fmaf(a.hi, b.hi, -p);
+  e = fmaf(a.hi, b.lo, e);
+  e = fmaf(a.lo, b.hi, e);
+  return fast_two_sum(p, e);
+}
+
+__device__ __forceinline__ dfl df_neg(dfl a) { return {-a.hi, -a.lo}; }
+
 // exp(2 pi i k path), k in cycles per metre, both double-float: the whole cycles drop out exactly.
 __device__ __forceinline__ float2 df_cis_cycles(dfl k, dfl path) {
   const float p = __fmul_rn(k.hi, path.hi);
@@ -64,46 +73,94 @@ __device__ __forceinline__ float2 df_cis_cycles(dfl k, dfl path) {
 }
 
 // sin(pi x) / (pi x), the rounding of x to FP32 corrected to first order.
-__device__ __forceinline__ float sinc_pi(double x) {
-  if (x == 0.0) return 1.0f;
-  const float hi = (float)x, lo = (float)kPi * (float)(x - (double)hi);
+__device__ __forceinline__ float sinc_pi(dfl x) {
+  if (x.hi == 0.0f) return 1.0f;
+  const dfl px = df_mul(split_double(kPi), x);
   float s, c;
-  sincospif(hi, &s, &c);
-  return __fdiv_rn(fmaf(lo, c, s), (float)(kPi * x));
+  sincospif(x.hi, &s, &c);
+  return __fdiv_rn(fmaf((float)kPi * x.lo, c, s), px.hi);
 }
 
-// One thread per sample.  The path of a source, r + x_e sin(theta) - min_e(...), and its phase are
-// double-float, the amplitudes FP32; FP64 is left to sin(theta) and a few products per sample (the
-// part runs it at 1/64 of the FP32 rate: with the delays, phases and spectra in FP64 the kernel took
-// 3.2 ms for 1,048,576 samples of the 64-element probe, all of it FP64).
+// 1 / sqrt(x) for normal x (2 ulp)
+__device__ __forceinline__ float rsqrt_normal(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// One thread per sample, one loop over the sources.  The array is linear, so a source differs by its x
+// alone and sin and cos of the angle are dx / r and z / r.  Paths and phases are double-float: the
+// distance is s = r^2 y, y = rsqrt(r^2), plus the residual (r^2 - s^2) y / 2, the delay's phase
+// x_e k sin(theta) is reduced to a fraction of a cycle per element and the distance's per source (their
+// sum is exact: both are multiples of 2^-20 or so below one), and the amplitudes are FP32 from y after
+// one Newton step.  FP64 is left to sin(theta) and the splits of the sample.
+//
+// What bounds it: issue, about 90 instructions per source (a third of them sincospi).  1,048,576 samples
+// of the 64-element probe (two sources per element): 3.2 ms with delays, phases and spectra in FP64,
+// which the part runs at 1/64 of the FP32 rate; 883 us with the sweeps' double-float geometry per
+// source (two correctly rounded divisions, two square roots); 491 us now.
+template <int kBaffle>
 __global__ void __launch_bounds__(128) txfield_kernel(const __grid_constant__ TxFieldArgs a) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.n) return;
-  const double x = a.samples[4 * i], z = a.samples[4 * i + 1], f = a.samples[4 * i + 2], th = a.samples[4 * i + 3];
+  const dfl xs = split_double(a.samples[4 * i]), zs = split_double(a.samples[4 * i + 1]);
+  const dfl fs = split_double(a.samples[4 * i + 2]);
+  const dfl st = split_double(sin(a.samples[4 * i + 3]));
   // pulse (times -i) * probe at f (spectrum.py:24-107)
-  const float pulse_im = sinc_pi(a.cyc_fc * (f - a.fc)) - sinc_pi(a.cyc_fc * (f + a.fc));
-  const float probe = expf(-0.5f * powf((float)fabs(f - a.fc) * a.inv_sigma, a.shape));
-  // plane-wave delays: c tau_e = x_e sin(theta) - min_e
-  const double st = sin(th);
-  const float x_end = element_x(a.E - 1, a.E, a.pitch), x_0 = element_x(0, a.E, a.pitch);
-  const dfl std_ = split_double(st), first = split_double(-fmin((double)x_0 * st, (double)x_end * st));
-  const dfl xs = split_double(x), zs = split_double(z), kc = split_double(f * a.inv_c);
-  const float alpha = a.alpha_hz * (float)f;
+  const dfl df = df_add(fs, df_neg(a.fc));
+  const float pulse_im = sinc_pi(df_mul(a.cyc_fc, df)) - sinc_pi(df_mul(a.cyc_fc, df_add(fs, a.fc)));
+  const float probe = expf(-0.5f * powf(fabsf(df.hi) * a.inv_sigma, a.shape));
+  const dfl kc = df_mul(fs, a.inv_c);  // cycles per metre
+  // cycles of the plane-wave delays, x_e k sin(theta) - min_e(...) (the minimum is at an end)
+  const dfl ks = df_mul(kc, st);
+  const dfl first = df_scale(element_x(a.E - 1, a.E, a.pitch), ks.hi < 0.f ? df_neg(ks) : ks);
+  const float first_r = __fsub_rn(first.hi, rintf(first.hi));
+  const dfl z2 = df_sqr(zs);
+  const float alpha = a.alpha_hz * fs.hi;
+  const float half = (float)((a.E - 1) * 0.5);
   float2 acc = make_float2(0.f, 0.f);
   for (int e = 0; e < a.E; ++e) {
-    const dfl lead = df_add(df_scale(element_x(e, a.E, a.pitch), std_), first);
-    const float2 rot = a.rot_e[e];
+    const float xe = __fmul_rn(__fsub_rn((float)e, half), a.pitch);
+    const float p = __fmul_rn(xe, ks.hi);
+    const float lead_lo = fmaf(xe, ks.lo, fmaf(xe, ks.hi, -p)) + first.lo;
+    const float lead_r = __fadd_rn(__fsub_rn(p, rintf(p)), first_r);
     for (int u = 0; u < a.U; ++u) {
-      const SrcGeo geo = source_geometry(xs, zs, a.src_pos[e * a.U + u], rot, a.C);
-      const float2 cis = df_cis_cycles(kc, df_add(dfl{geo.r_hi, geo.r_lo}, lead));
-      const float m = alpha != 0.f ? geo.amp * expf(-alpha * geo.r_hi) : geo.amp;
-      acc.x = fmaf(m, cis.x, acc.x);
-      acc.y = fmaf(m, cis.y, acc.y);
+      const float2 sp = *reinterpret_cast<const float2*>(a.src_pos + e * a.U + u);
+      dfl dx = two_sum(xs.hi, -sp.x);
+      dx.lo = __fadd_rn(dx.lo, __fsub_rn(xs.lo, sp.y));
+      const float d2 = __fmul_rn(dx.hi, dx.hi);
+      const float d2_lo = fmaf(2.0f * dx.hi, dx.lo, fmaf(dx.hi, dx.hi, -d2));
+      dfl r2 = two_sum(d2, z2.hi);
+      r2.lo = __fadd_rn(r2.lo, __fadd_rn(d2_lo, z2.lo));
+      const bool apart = r2.hi > 0.f && r2.hi <= 3.402823466e38f;
+      float y = rsqrt_normal(fmaxf(r2.hi, 1.17549435e-38f));
+      float s = __fmul_rn(r2.hi, y);
+      float lo = __fmul_rn(0.5f * y, __fadd_rn(fmaf(-s, s, r2.hi), r2.lo));
+      y = fmaf(0.5f * y, fmaf(-s, y, 1.0f), y);
+      // a point on the source (or no number) is seen under 90 degrees
+      const float sth = apart ? dx.hi * y : 1.0f, cth = apart ? zs.hi * y : 0.0f;
+      if (!(s > a.C.min_dist.x || (s == a.C.min_dist.x && lo >= a.C.min_dist.y))) {
+        s = a.C.min_dist.x;
+        lo = a.C.min_dist.y;
+      }
+      const float r = __fadd_rn(s, lo);
+      float m = kBaffle == 0 ? cth : (kBaffle == 1 ? 1.0f : __fdiv_rn(cth, cth + a.C.baffle_val));
+      if (cth <= 0.0f) m = 1e-16f;
+      m *= sinc_rad(a.C.dir_coef * sth) * rsqrt_normal(r);
+      if (alpha != 0.f) m *= expf(-alpha * r);
+      const float q = __fmul_rn(kc.hi, s);
+      const float q_lo = fmaf(kc.lo, s, fmaf(kc.hi, lo, fmaf(kc.hi, s, -q)));
+      float c = __fadd_rn(__fsub_rn(q, rintf(q)), lead_r);
+      c = __fadd_rn(__fsub_rn(c, rintf(c)), __fadd_rn(q_lo, lead_lo));
+      float sn, cs;
+      sincospif(2.0f * c, &sn, &cs);
+      acc.x = fmaf(m, cs, acc.x);
+      acc.y = fmaf(m, sn, acc.y);
     }
   }
-  // times pulse (= i * pulse_im) * probe
-  const float s = pulse_im * probe;
-  const bool out_field = z < 0.0;
+  // times pulse (= i * pulse_im) * probe, mean over the sub-elements
+  const float s = pulse_im * probe * a.C.inv_nsub;
+  const bool out_field = zs.hi < 0.f;
   a.out[i] = out_field ? make_float2(0.f, 0.f) : make_float2(-acc.y * s, acc.x * s);
 }
 
@@ -121,51 +178,59 @@ struct Carriers {
 struct DomainArgs {
   FsgSurrogateDomain d;
   double mul[4], add[4];  // u_k = mul_k sample_k + add_k
-  double inv_c, c_over_pitch;
+  dfl inv_c, c_over_pitch;  // cycles per metre and Hz, lambda / pitch times Hz
+  dfl x_end, x_edge;        // x of the last element and of its outer edge
 };
 
-// sqrt((x - xe)^2 + z^2) in double-float.
-__device__ __forceinline__ dfl df_distance(dfl x, dfl z, double xe) {
-  const dfl dx = df_add(x, split_double(-xe));
-  return df_sqrt(df_add(df_sqr(dx), df_sqr(z)));
+// sqrt(a) for a > 0 and 0 else, from y = rsqrt(a): s = a y plus the residual (a - s^2) y / 2.
+__device__ __forceinline__ dfl df_sqrt_fast(dfl a) {
+  const float y = rsqrt_normal(fmaxf(a.hi, 1.17549435e-38f));
+  const float s = __fmul_rn(a.hi, y);
+  const dfl r = fast_two_sum(s, __fmul_rn(0.5f * y, __fadd_rn(fmaf(-s, s, a.hi), a.lo)));
+  return a.hi > 0.f ? r : dfl{0.f, 0.f};
 }
 
-__device__ __forceinline__ dfl df_mul(dfl a, dfl b) {
-  const float p = __fmul_rn(a.hi, b.hi);
-  float e = fmaf(a.hi, b.hi, -p);
-  e = fmaf(a.hi, b.lo, e);
-  e = fmaf(a.lo, b.hi, e);
-  return fast_two_sum(p, e);
+// sqrt((x - xe)^2 + z2)
+__device__ __forceinline__ dfl df_distance(dfl x, dfl z2, dfl xe) {
+  return df_sqrt_fast(df_add(df_sqr(df_add(x, df_neg(xe))), z2));
+}
+
+// a / b
+__device__ __forceinline__ dfl df_div(dfl a, dfl b) {
+  const float q = __fdividef(a.hi, b.hi);
+  const float e = fmaf(-q, b.lo, __fadd_rn(fmaf(-q, b.hi, a.hi), a.lo));
+  return fast_two_sum(q, __fdividef(e, b.hi));
 }
 
 // c_0: the plane wave exp(i k (x sin th + z cos th - xmin)); c_1, c_2: the waves from the two
 // ends of the aperture, exp(i k (r_edge + x_edge sin th - xmin)); c_3, c_4: the grating lobes
 // m = -1, +1 of the pitch, exp(i k (x sin th_m + z cos th_m - xmin)) with
-// sin th_m = sin th + m lambda / pitch, zero where |sin th_m| >= 1 (evanescent).  Paths and phases are
-// double-float; FP64 is left to sin and cos of theta and lambda / pitch (1,048,576 samples of the
-// combine kernel: 628 us with all of it in FP64).
+// sin th_m = sin th + m lambda / pitch, zero where |sin th_m| >= 1 (evanescent).  Everything but sin and
+// cos of theta is double-float: 1,048,576 samples of the combine kernel took 628 us with all of it in
+// FP64, 225 us with the edges, lambda / pitch and sin th_m in FP64, 108 us now.
 __device__ __forceinline__ Carriers surrogate_carriers(const DomainArgs& D, double x, double z, double f, double th) {
   const FsgSurrogateDomain& d = D.d;
   double st, ct;
   sincos(th, &st, &ct);
-  const double x0 = -0.5 * (d.n_elements - 1) * d.pitch, x1 = -x0;
-  const dfl first = split_double(-fmin(x0 * st, x1 * st));
-  const dfl kc = split_double(f * D.inv_c);  // cycles per metre
-  const double lp = D.c_over_pitch / f;      // lambda / pitch
-  const dfl xs = split_double(x), zs = split_double(z), sd = split_double(st);
+  const dfl xs = split_double(x), zs = split_double(z), fs = split_double(f), sd = split_double(st);
+  const dfl kc = df_mul(fs, D.inv_c);  // cycles per metre
+  const dfl lp = df_div(D.c_over_pitch, fs);
+  const dfl z2 = df_sqr(zs);
+  // -xmin: the delays' minimum is at an end of the array
+  const dfl xe_s = df_mul(D.x_end, sd), first = xe_s.hi < 0.f ? df_neg(xe_s) : xe_s;
+  const dfl edge_s = df_mul(D.x_edge, sd);
   dfl path[kMaxCarriers];
   bool on[kMaxCarriers];
   path[0] = df_add(df_mul(xs, sd), df_mul(zs, split_double(ct)));
-  const double xl = x0 - 0.5 * d.pitch, xr = x1 + 0.5 * d.pitch;
-  path[1] = df_add(df_distance(xs, zs, xl), df_mul(split_double(xl), sd));
-  path[2] = df_add(df_distance(xs, zs, xr), df_mul(split_double(xr), sd));
+  path[1] = df_add(df_distance(xs, z2, df_neg(D.x_edge)), df_neg(edge_s));
+  path[2] = df_add(df_distance(xs, z2, D.x_edge), edge_s);
   on[0] = on[1] = on[2] = true;
 #pragma unroll
   for (int m = 0; m < 2; ++m) {
-    const double sm = st + (m ? lp : -lp);
-    on[3 + m] = fabs(sm) < 1.0;
-    const dfl smd = split_double(sm), cm = df_sqrt(split_double(fmax(0.0, 1.0 - sm * sm)));
-    path[3 + m] = df_add(df_mul(xs, smd), df_mul(zs, cm));
+    const dfl sm = df_add(sd, m ? lp : df_neg(lp));
+    const dfl c2 = df_add(dfl{1.f, 0.f}, df_neg(df_sqr(sm)));
+    on[3 + m] = c2.hi > 0.f;
+    path[3 + m] = df_add(df_mul(xs, sm), df_mul(zs, df_sqrt_fast(c2)));
   }
   Carriers out;
 #pragma unroll
@@ -231,8 +296,10 @@ static DomainArgs domain_args(const FsgSurrogateDomain& d) {
     D.mul[k] = 2.0 / (hi[k] - lo[k]);
     D.add[k] = -(lo[k] + hi[k]) / (hi[k] - lo[k]);
   }
-  D.inv_c = 1.0 / d.speed_of_sound;
-  D.c_over_pitch = d.speed_of_sound / d.pitch;
+  D.inv_c = split_double(1.0 / d.speed_of_sound);
+  D.c_over_pitch = split_double(d.speed_of_sound / d.pitch);
+  D.x_end = split_double(0.5 * (d.n_elements - 1) * d.pitch);
+  D.x_edge = split_double(0.5 * d.n_elements * d.pitch);
   return D;
 }
 
@@ -272,13 +339,12 @@ extern "C" int32_t fsg_txfield(const FsgProbe* probe, const FsgMedium* medium, d
   a.n = n;
   a.out = static_cast<float2*>(out);
   a.src_pos = sa.t.src_pos;
-  a.rot_e = sa.t.rot_e;
   a.pitch = (float)probe->pitch;
   a.E = E;
   a.U = U;
-  a.fc = probe->freq_center;
-  a.inv_c = 1.0 / medium->speed_of_sound;
-  a.cyc_fc = tx_n_wavelengths / probe->freq_center;
+  a.fc = split_double(probe->freq_center);
+  a.inv_c = split_double(1.0 / medium->speed_of_sound);
+  a.cyc_fc = split_double(tx_n_wavelengths / probe->freq_center);
   a.alpha_hz = (float)(medium->attenuation / 8.685889638065035 / 1e6 * 1e2);
   {
     // spectrum.py:53-107, in Hz
@@ -291,7 +357,10 @@ extern "C" int32_t fsg_txfield(const FsgProbe* probe, const FsgMedium* medium, d
   memset(&dummy, 0, sizeof(dummy));
   dummy.seg_length = probe->element_width / U;
   a.C = make_sweep_const(probe, medium, &dummy, 0);
-  txfield_kernel<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(a);
+  const unsigned grid = (unsigned)((n + 127) / 128);
+  if (a.C.baffle == 0) txfield_kernel<0><<<grid, 128, 0, s>>>(a);
+  else if (a.C.baffle == 1) txfield_kernel<1><<<grid, 128, 0, s>>>(a);
+  else txfield_kernel<2><<<grid, 128, 0, s>>>(a);
   return check_cuda(cudaGetLastError(), "txfield_kernel launch");
 }
 

@@ -74,3 +74,30 @@ def test_das_firing_groups(nf, n_pix, n_s, method):
                 fc=fc, fnumber=1.0, method=method)
     assert got.shape == x.shape
     assert G.rel_l2(got, ref) < 1e-3
+
+
+@pytest.mark.parametrize("baffle", ["soft", "rigid", 1.75])
+@pytest.mark.parametrize("E,width,att", [(1, 0.2e-3, 0.0), (33, 0.9e-3, 0.7), (192, 0.27e-3, 0.5)])
+def test_txfield_samples(E, width, att, baffle):
+    """The exact transmit field for every baffle, with and without attenuation, one and more sub-elements,
+    the smallest and a large array; points on a source, on the array's plane, within the clipped distance,
+    behind the array and far off axis.  FP32 amplitudes and phases of up to 10^4 sources: rel-L2 < 1e-5."""
+    require_gpu()
+    from fastsimus_gb300 import MediumParams, TransducerParams
+    from fastsimus_gb300.surrogate import TxFieldSurrogate, cfg5_box
+    import oracle.fastsimus_fp64 as O
+
+    p = TransducerParams(freq_center=5e6, pitch=1.1 * width, n_elements=E, width=width, bandwidth=0.65, baffle=baffle)
+    m = MediumParams(speed_of_sound=1540.0, attenuation=att)
+    sur = TxFieldSurrogate(p, m, cfg5_box(p))
+    rng = np.random.default_rng(E)
+    half = 0.5 * E * p.pitch
+    s = np.stack([rng.uniform(-1.2 * half, 1.2 * half, 140), rng.uniform(1e-3, 40e-3, 140),
+                  5e6 * rng.uniform(0.6, 1.4, 140), rng.uniform(-0.4, 0.4, 140)], axis=-1)
+    s[:4, :2] = [[0.0, 0.0], [3 * half, 0.0], [1e-5, 2e-5], [0.0, -1e-3]]
+    s[4, 2:] = [5e6, 0.0]  # the pulse's centre frequency, no steering
+    got, ref = np64(sur.exact(torch.as_tensor(s))), O.tx_field_samples(s, p, m)
+    assert got.shape == ref.shape and got[3] == 0
+    # on the array's plane a rigid source is on or off by the sign of a 1e-16 in FP64: off here
+    k = slice(2 if baffle == "rigid" else 0, None)
+    assert np.all(np.abs(got[:2]) < 1e-6) and G.rel_l2(got[k], ref[k]) < 1e-5
