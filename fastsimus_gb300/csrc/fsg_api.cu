@@ -97,6 +97,8 @@ SweepConst make_sweep_const(const FsgProbe* p, const FsgMedium* m, const FsgFreq
   const double c = m->speed_of_sound;
   dfl dk = split_double(2.0 * kPi * plan->freq_step / c);
   C.dk = make_float2(dk.hi, dk.lo);
+  const dfl dkc = split_double(plan->freq_step / c);
+  C.dkc = make_float2(dkc.hi, dkc.lo);
   C.dalpha = (float)(m->attenuation / 8.685889638065035 * plan->freq_step / 1e6 * 1e2);
   C.inv_nsub = (float)(1.0 / p->n_sub);
   dfl md = split_double(c / p->freq_center / 2.0);
@@ -352,8 +354,7 @@ SweepConfig pfield_config(int E, int U, int F, int64_t n_pts, int num_sms, int f
   const int64_t tps = (tiles + slices - 1) / slices;
   c.per_slice = tps * c.st;
   c.n_slices = (int)((tiles + tps - 1) / tps);
-  c.plane_pad = choose_plane_pad(E, U, c.gn, c.st);
-  c.smem = smem_layout(c.st, c.fb, E, U, c.plane_pad, false, ffd != 0).total;
+  c.smem = pfield_layout(c.fb, E, ffd != 0).total;
   return c;
 }
 
@@ -568,7 +569,6 @@ extern "C" int32_t fsg_pfield(const FsgProbe* probe, const FsgMedium* medium, co
   A.U = U;
   A.n_src = E * U;
   A.gn = c.gn;
-  A.plane_pad = c.plane_pad;
   A.st = c.st;
   A.fb = c.fb;
   A.F = F;

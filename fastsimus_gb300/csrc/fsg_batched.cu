@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(NTH, MINB) batched_kernel(const __grid_constan
     const float a0 = P.af[f0];
     const float kb0 = k0.x, kb1 = (f0 + 1 < P.n_freq) ? P.kf[f0 + 1].x : 0.f;  // FP32 k_f for the directivity
     SweepConst C = A.C;  // probe constants; the recurrence step belongs to this phantom's plan
-    C.dk = P.dk;
+    C.dkc = P.dkc;
     C.dalpha = P.dalpha;
 
     float2 Y[FB][kRows][5];
@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(kThreads) batched_geometry_kernel(const __grid
   const int n_src = A.E * A.U;
   const int spb = n_src >= kThreads ? 1 : kThreads / n_src;
   SweepConst C = A.C;
-  C.dk = P.dk;
+  C.dkc = P.dkc;
   C.dalpha = P.dalpha;
   for (int64_t s0 = (int64_t)blockIdx.x * spb; s0 < P.n_scat; s0 += (int64_t)gridDim.x * spb) {
     __syncthreads();
@@ -603,7 +603,7 @@ static int32_t simus_batched_impl(const FsgProbe* probe, const FsgMedium* medium
     b.corr = (float)q.plan.correction_factor;
     {
       const SweepConst cp = make_sweep_const(probe, medium, &q.plan, 0);
-      b.dk = cp.dk;
+      b.dkc = cp.dkc;
       b.dalpha = cp.dalpha;
     }
     b.pulse_src = q.plan.pulse_spectrum;

@@ -23,6 +23,7 @@ struct BatchPhantom {
   float corr;
   float dalpha;             // per-step attenuation of this phantom's plan (Np/m)
   float2 dk;                // per-step wavenumber of this phantom's plan (double-float)
+  float2 dkc;               // the same in cycles per metre
   const double* pulse_src;  // plan pulse spectrum, complex128 [n_freq]
   const double* probe_src;  // plan probe spectrum, float64 [n_freq]
   float2* kf;               // workspace: k_f double-float

@@ -74,15 +74,14 @@ struct SmemLayout {
   // (consecutive elements) conflict-free; plane_pad spreads the transmit accesses (lanes =
   // sources g + GN i of one or more points) over the banks.
   int pitch, plane;
-  size_t off_rhi, off_rlo, off_amp, off_step, off_dir, off_w, off_pp, off_kb, off_ka, off_aa, off_da, off_y, total;
+  size_t off_rhi, off_rlo, off_amp, off_step, off_dir;
   size_t geo_bytes;    // the geometry arrays, contiguous from offset 0
 };
 
 __host__ __device__ inline size_t align16(size_t v) { return (v + 15) & ~size_t(15); }
 
 // With ffd, a fifth geometry array holds half_seg * sin(theta) per (source, point).
-__host__ __device__ inline SmemLayout smem_layout(int st, int fb, int E, int U, int plane_pad, bool with_w,
-                                                  bool ffd = false) {
+__host__ __device__ inline SmemLayout smem_layout(int st, int E, int U, int plane_pad, bool ffd) {
   SmemLayout L;
   L.pitch = st + 1;
   L.plane = E * L.pitch + plane_pad;
@@ -94,15 +93,28 @@ __host__ __device__ inline SmemLayout smem_layout(int st, int fb, int E, int U, 
   L.off_step = o; o = align16(o + n * 8);
   L.off_dir = o; o = align16(o + (ffd ? n * 4 : 0));
   L.geo_bytes = o;
-  L.off_w = o; o = align16(o + (with_w ? (size_t)fb * st * 8 : 0));
+  return L;
+}
+
+// pfield_band_kernel: every thread's own geometry, one entry per pair of sources and thread, then the
+// band tables.
+struct PfieldLayout {
+  size_t off_r, off_step, off_amp, off_dir, off_pp, off_kb, off_ka, off_aa, off_da, total;
+};
+__host__ __device__ inline PfieldLayout pfield_layout(int fb, int E, bool ffd) {
+  PfieldLayout L;
+  const size_t n = (size_t)(kSrcPerThread / 2) * kThreads;
+  const int na = fb / kAnchor;
+  size_t o = 0;
+  L.off_r = o; o += n * 16;
+  L.off_step = o; o += n * 16;
+  L.off_amp = o; o += n * 8;
+  L.off_dir = o; o += ffd ? n * 8 : 0;
   L.off_pp = o; o = align16(o + (size_t)fb * 8);
   L.off_kb = o; o = align16(o + (size_t)fb * 4);  // FP32 wavenumber of each band frequency
-  int na = fb / kAnchor;
   L.off_ka = o; o = align16(o + (size_t)na * 8);
   L.off_aa = o; o = align16(o + (size_t)na * 4);
   L.off_da = o; o = align16(o + (size_t)na * E * 8);
-  // simus: each thread's running receive spectrum Y[kAnchor], laid out [j][thread]
-  L.off_y = o; o = align16(o + (with_w ? (size_t)kAnchor * kThreads * 8 : 0));
   L.total = o;
   return L;
 }
@@ -120,7 +132,7 @@ struct StashLayout {
 };
 __host__ __device__ inline StashLayout stash_layout(int st, int fb, int E, int U, int plane_pad, bool ffd) {
   StashLayout S;
-  S.g = smem_layout(st, fb, E, U, plane_pad, true, ffd);
+  S.g = smem_layout(st, E, U, plane_pad, ffd);
   S.ep = E | 1;
   const size_t stash = (size_t)st * kStashFreqs * S.ep * 8;
   size_t o = align16(S.g.geo_bytes > stash ? S.g.geo_bytes : stash);

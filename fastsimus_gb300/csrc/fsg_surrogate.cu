@@ -81,13 +81,6 @@ __device__ __forceinline__ float sinc_pi(dfl x) {
   return __fdiv_rn(fmaf((float)kPi * x.lo, c, s), px.hi);
 }
 
-// 1 / sqrt(x) for normal x (2 ulp)
-__device__ __forceinline__ float rsqrt_normal(float x) {
-  float y;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
 // One thread per sample, one loop over the sources.  The array is linear, so a source differs by its x
 // alone and sin and cos of the angle are dx / r and z / r.  Paths and phases are double-float: the
 // distance is s = r^2 y, y = rsqrt(r^2), plus the residual (r^2 - s^2) y / 2, the delay's phase

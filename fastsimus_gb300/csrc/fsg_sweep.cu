@@ -93,7 +93,7 @@ __global__ void setup_tables(SetupArgs a) {
 // scatterer list repeat the tile's first point (their rc is 0 in the band kernel).
 __global__ void __launch_bounds__(kThreads) geometry_kernel(const BandArgs A, int64_t chunk_tiles) {
   __shared__ float4 xz[kThreads];  // st <= 64 points of the tile
-  const SmemLayout L = smem_layout(A.st, A.fb, A.E, A.U, A.plane_pad, true, A.C.ffd != 0);
+  const SmemLayout L = smem_layout(A.st, A.E, A.U, A.plane_pad, A.C.ffd != 0);
   const int items = A.n_src * A.st;
   for (int64_t tile = blockIdx.x; tile < chunk_tiles; tile += gridDim.x) {
     __syncthreads();

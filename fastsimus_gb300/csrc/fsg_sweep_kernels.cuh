@@ -20,7 +20,7 @@ __device__ __forceinline__ dfl load_coord(const double* p) {
 }
 
 // Loads the band's per-frequency tables into shared memory.
-__device__ __forceinline__ void load_band_tables(const BandArgs& A, const SmemLayout& L, unsigned char* sm, int f_b0) {
+__device__ __forceinline__ void load_band_tables(const BandArgs& A, const PfieldLayout& L, unsigned char* sm, int f_b0) {
   float2* pp = reinterpret_cast<float2*>(sm + L.off_pp);
   float2* ka = reinterpret_cast<float2*>(sm + L.off_ka);
   float* aa = reinterpret_cast<float*>(sm + L.off_aa);
@@ -58,77 +58,87 @@ __device__ __forceinline__ void store_geometry(float* rhi, float* rlo, float* am
 }
 
 // TX over one band for one tile, with the tile's geometry computed here first.
-// Each thread owns point `sl` of the tile and sources g + GN i (i < 16); the GN threads of a
-// point are GN adjacent lanes of one warp.  Frequencies are processed in blocks of GN steps:
-// every lane keeps its partial source sums of the block, then a reduce-scatter across the GN
-// lanes (log2 GN shuffle levels, halving the exchanged values each level) leaves lane g with
+// Each thread owns point `sl` of the tile and eight pairs of sources 2 (g + GN p), 2 (g + GN p) + 1;
+// the GN threads of a point are GN adjacent lanes of one warp.  Frequencies are processed in blocks
+// of GN steps: every lane keeps its partial source sums of the block, then a reduce-scatter across
+// the GN lanes (log2 GN shuffle levels, halving the exchanged values each level) leaves lane g with
 // the full sum of frequency block + g.  `sink(f_local, psum)` is therefore called by every
 // lane, once per block, each for its own frequency.  With FFD every term is weighted by its
 // directivity at the step's frequency, sinc(k_f half_seg sin(theta)), folded into the packed
 // source sum as a fused multiply-add.
+//
+// What bounds it: the FP32 pipe and its register read ports (a source step is four packed instructions
+// per pair, its sum two).  A thread reads back only the geometry it wrote, so that the arrays are laid
+// out by thread and read as 16-byte words; with arrays shared by the tile, their bank padding searched
+// on the host and a division by U per source and anchor, the call took 2,978 us for 131,072 points
+// and 128 elements x 2 sources, now 2,163, and 283 us (190 of them on the host) for 8,181 points and
+// 64 elements, now 87.
 template <int GN, bool FFD, class Sink>
-__device__ __forceinline__ void tx_tile(const BandArgs& A, const SmemLayout& L, unsigned char* sm, int64_t p_idx,
-                                        int sl, int g, Sink& sink) {
-  float* b_rhi = reinterpret_cast<float*>(sm + L.off_rhi);
-  float* b_rlo = reinterpret_cast<float*>(sm + L.off_rlo);
-  float* b_amp = reinterpret_cast<float*>(sm + L.off_amp);
-  float2* b_st = reinterpret_cast<float2*>(sm + L.off_step);
+__device__ __forceinline__ void tx_tile(const BandArgs& A, const PfieldLayout& L, unsigned char* sm, int64_t p_idx,
+                                        int g, Sink& sink) {
+  constexpr int kPairs = kSrcPerThread / 2;
+  float4* b_r = reinterpret_cast<float4*>(sm + L.off_r) + threadIdx.x;        // r_hi, r_hi, r_lo, r_lo
+  float4* b_st = reinterpret_cast<float4*>(sm + L.off_step) + threadIdx.x;    // step re, re, im, im
+  float2* b_amp = reinterpret_cast<float2*>(sm + L.off_amp) + threadIdx.x;
+  float2* b_dir = reinterpret_cast<float2*>(sm + L.off_dir) + threadIdx.x;
   const float2* ka = reinterpret_cast<const float2*>(sm + L.off_ka);
   const float* aa = reinterpret_cast<const float*>(sm + L.off_aa);
   const float2* da = reinterpret_cast<const float2*>(sm + L.off_da);
-  float* b_dir = reinterpret_cast<float*>(sm + L.off_dir);
   const float* kb = reinterpret_cast<const float*>(sm + L.off_kb);
+  // src / U = src * mag >> 20, exact for src and U up to 512
+  const unsigned mag = ((1u << 20) + A.U - 1) / A.U;
 
   // 1. geometry of my sources, parked in shared memory (rolled loop: one copy of the code)
   {
     const dfl xs = load_coord(A.pts + 2 * p_idx);
     const dfl zs = load_coord(A.pts + 2 * p_idx + 1);
 #pragma unroll 1
-    for (int i = 0; i < kSrcPerThread; ++i) {
-      const int src = g + GN * i;
-      if (src < A.n_src) {
-        const int e = src / A.U, u = src - e * A.U;
-        store_geometry(b_rhi, b_rlo, b_amp, b_st, FFD ? b_dir : nullptr, u * L.plane + e * L.pitch + sl, xs, zs, A,
-                       src);
+    for (int p = 0; p < kPairs; ++p) {
+      SrcGeo q[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int src = 2 * (g + GN * p) + h;
+        q[h] = SrcGeo{0.f, 0.f, 0.f, make_float2(0.f, 0.f), 0.f};
+        if (src < A.n_src) {
+          const int e = (int)((src * mag) >> 20);
+          q[h] = source_geometry(xs, zs, A.t.src_pos[src], A.t.rot_e[e], A.C);
+          q[h].step = cmul(q[h].step, A.t.dstep[e]);
+        }
       }
+      b_r[p * kThreads] = make_float4(q[0].r_hi, q[1].r_hi, q[0].r_lo, q[1].r_lo);
+      b_st[p * kThreads] = make_float4(q[0].step.x, q[1].step.x, q[0].step.y, q[1].step.y);
+      b_amp[p * kThreads] = make_float2(q[0].amp, q[1].amp);
+      if (FFD) b_dir[p * kThreads] = make_float2(A.C.half_seg * q[0].sth, A.C.half_seg * q[1].sth);
     }
   }
-  // 2. transmit sweep: exact anchor every kTxAnchor steps, FP32 recurrence in between.
-  // The thread's sources i = 2p and 2p+1 share one packed FP32x2 lane pair (real and
-  // imaginary parts in separate pairs), so a step costs four packed instructions per two
-  // sources and the source sum two packed adds.
-  constexpr int kPairs = kSrcPerThread / 2;
+  // 2. transmit sweep: exact anchor every kTxAnchor steps, FP32 recurrence in between.  The two
+  // sources of a pair share one packed FP32x2 lane pair (real and imaginary parts in separate pairs).
   float2 Gr[kPairs], Gi[kPairs], Sr[kPairs], Si[kPairs], Sn[kPairs];
   float2 Dh[FFD ? kPairs : 1];  // FFD: half_seg sin(theta) of the pair's two sources
+#pragma unroll
+  for (int p = 0; p < kPairs; ++p) {
+    const float4 s = b_st[p * kThreads];
+    Sr[p] = make_float2(s.x, s.y);
+    Si[p] = make_float2(s.z, s.w);
+    Sn[p] = make_float2(-s.z, -s.w);
+    if constexpr (FFD) Dh[p] = b_dir[p * kThreads];
+  }
   const int n_tx_anchor = (A.fb + kTxAnchor - 1) / kTxAnchor;
   for (int m = 0; m < n_tx_anchor; ++m) {
     const int am = m * (kTxAnchor / kAnchor);  // index into the band's kAnchor-spaced tables
+    const float2 k0 = ka[am];
+    const float a0 = aa[am];
+    const float2* d0 = da + am * A.E;
 #pragma unroll
     for (int p = 0; p < kPairs; ++p) {
-      float2 gv[2], sv[2];
-      float dv[2];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int src = g + GN * (2 * p + h);
-        gv[h] = make_float2(0.f, 0.f);
-        sv[h] = make_float2(0.f, 0.f);
-        dv[h] = 0.f;
-        if (src < A.n_src) {
-          const int e = src / A.U, u = src - e * A.U;
-          const int idx = u * L.plane + e * L.pitch + sl;
-          gv[h] = cmul(anchor_value(b_rhi[idx], b_rlo[idx], b_amp[idx], ka[am], aa[am]), da[am * A.E + e]);
-          if (m == 0) sv[h] = cmul(b_st[idx], A.t.dstep[e]);
-          if (FFD) dv[h] = b_dir[idx];
-        }
-      }
-      if constexpr (FFD) Dh[p] = make_float2(dv[0], dv[1]);
-      Gr[p] = make_float2(gv[0].x, gv[1].x);
-      Gi[p] = make_float2(gv[0].y, gv[1].y);
-      if (m == 0) {
-        Sr[p] = make_float2(sv[0].x, sv[1].x);
-        Si[p] = make_float2(sv[0].y, sv[1].y);
-        Sn[p] = make_float2(-sv[0].y, -sv[1].y);
-      }
+      const int src = 2 * (g + GN * p);
+      const int e0 = min((int)((src * mag) >> 20), A.E - 1), e1 = min((int)(((src + 1) * mag) >> 20), A.E - 1);
+      const float4 r = b_r[p * kThreads];
+      const float2 am2 = b_amp[p * kThreads];
+      const float2 g0 = cmul(anchor_value(r.x, r.z, am2.x, k0, a0), d0[e0]);
+      const float2 g1 = cmul(anchor_value(r.y, r.w, am2.y, k0, a0), d0[e1]);
+      Gr[p] = make_float2(g0.x, g1.x);
+      Gi[p] = make_float2(g0.y, g1.y);
     }
     const int n_steps = min(kTxAnchor, A.fb - m * kTxAnchor);  // a multiple of kAnchor, so of GN
 #pragma unroll 1
@@ -193,7 +203,7 @@ struct PfieldSink {
 template <int GN, bool FFD>
 __global__ void __launch_bounds__(kThreads, (GN >= 32 || FFD) ? 1 : 2) pfield_band_kernel(const BandArgs A) {
   extern __shared__ __align__(16) unsigned char sm[];
-  const SmemLayout L = smem_layout(A.st, A.fb, A.E, A.U, A.plane_pad, false, FFD);
+  const PfieldLayout L = pfield_layout(A.fb, A.E, FFD);
   const int tid = threadIdx.x;
   const int f_b0 = blockIdx.x * A.fb;
   const int64_t p_begin = (int64_t)blockIdx.y * A.per_slice;
@@ -209,7 +219,7 @@ __global__ void __launch_bounds__(kThreads, (GN >= 32 || FFD) ? 1 : 2) pfield_ba
     bool valid = p < p_end;
     int64_t pi = valid ? p : t0;
     PfieldSink sink{pp, 0.f, min(A.fb, A.F - f_b0)};
-    tx_tile<GN, FFD>(A, L, sm, pi, sl, g, sink);
+    tx_tile<GN, FFD>(A, L, sm, pi, g, sink);
     // each lane holds the band's |p|^2 over its own frequencies: sum the GN lanes in a fixed tree
     float acc = sink.acc;
 #pragma unroll
