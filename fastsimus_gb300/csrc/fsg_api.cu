@@ -55,6 +55,12 @@ static int next_pow2(int v) {
   return p;
 }
 
+// The largest directivity argument of a plan, k_f seg / 2 at its highest frequency.
+static double ffd_x_max(const FsgMedium* medium, const FsgFreqPlan* plan) {
+  const double f_max = plan->freq_start + (plan->n_freq - 1) * plan->freq_step;
+  return 2.0 * kPi * f_max / medium->speed_of_sound * plan->seg_length / 2.0;
+}
+
 int validate_common(const FsgProbe* probe, const FsgMedium* medium, const FsgFreqPlan* plan, int ffd) {
   if (!probe || !medium || !plan) return set_error(FSG_EINVAL, "probe, medium and plan must be non-NULL");
   if (probe->n_elements < 1) return set_error(FSG_EINVAL, "n_elements must be >= 1 (got %d)", probe->n_elements);
@@ -81,8 +87,7 @@ int validate_common(const FsgProbe* probe, const FsgMedium* medium, const FsgFre
     // the per-frequency directivity is evaluated as a polynomial valid for |k_f seg / 2| <= 2 pi,
     // i.e. sub-elements up to two wavelengths of the highest selected frequency wide (the
     // automatic sub-element count keeps them within about one)
-    const double f_max = plan->freq_start + (plan->n_freq - 1) * plan->freq_step;
-    const double x_max = 2.0 * kPi * f_max / medium->speed_of_sound * plan->seg_length / 2.0;
+    const double x_max = ffd_x_max(medium, plan);
     if (x_max > 2.0 * kPi)
       return set_error(FSG_EUNSUPPORTED,
                        "full_frequency_directivity with sub-elements wider than two wavelengths "
@@ -106,7 +111,7 @@ SweepConst make_sweep_const(const FsgProbe* p, const FsgMedium* m, const FsgFreq
   C.dir_coef = (float)(2.0 * kPi * p->freq_center / c * plan->seg_length / 2.0);
   C.baffle_val = (float)p->baffle_impedance;
   C.baffle = p->baffle;
-  C.ffd = ffd;
+  C.ffd = !ffd ? 0 : (ffd_x_max(m, plan) <= kSincShortMax ? kSincShort : kSincTerms);
   C.half_seg = (float)(plan->seg_length / 2.0);
   return C;
 }
@@ -173,10 +178,7 @@ int launch_setup(const FsgProbe* p, const FsgMedium* m, const FsgFreqPlan* plan,
   a.pulse = plan->pulse_spectrum;
   a.probe = plan->probe_spectrum;
   a.t = t;
-  int n = a.E * a.U;
-  if (a.F > n) n = a.F;
-  if (a.n_anchor * a.E > n) n = a.n_anchor * a.E;
-  setup_tables<<<(n + 127) / 128, 128, 0, stream>>>(a);
+  setup_tables<<<(setup_threads(a) + 127) / 128, 128, 0, stream>>>(a);
   return check_cuda(cudaGetLastError(), "setup_tables launch");
 }
 
@@ -510,8 +512,15 @@ extern "C" int32_t fsg_simus(const FsgProbe* probe, const FsgMedium* medium, con
       A.grid = simus_grid(c.n_bands, ct, grid_cap);
       const int64_t cap = (int64_t)sms * 8;
       const int blocks = (int)(ct < cap ? ct : cap);
-      if (c.kind == 2) lane_geometry_kernel<<<blocks, kThreads, 0, s>>>(A, ct);
-      else geometry_kernel<<<blocks, kThreads, 0, s>>>(A, ct);
+      if (c.kind == 2) {
+        // few tiles: several CTAs each, down to 256 slots (42 tiles, 2,000 scatterers x 128
+        // sources: 18.9 us with one CTA each, 7.1 with eight)
+        const int per = (c.st * U * 32 * c.nw + kThreads - 1) / kThreads;
+        const int split = blocks < 2 * sms ? (2 * sms + blocks - 1) / blocks : 1;
+        lane_geometry_kernel<<<dim3(blocks, split < per ? split : per), kThreads, 0, s>>>(A, ct);
+      } else {
+        geometry_kernel<<<blocks, kThreads, 0, s>>>(A, ct);
+      }
       if ((st = check_cuda(cudaGetLastError(), "geometry_kernel launch")) != FSG_OK) return st;
       if ((st = check_cuda(launch_simus_any(U, c, A, s), "simus sweep launch")) != FSG_OK) return st;
     }

@@ -34,6 +34,13 @@ struct SetupArgs {
   Tables t;
 };
 
+// setup_tables' threads: the sources, the frequencies, the anchors and the elements' steps, each from a
+// whole warp on, so that a warp takes one of the FP64 paths and not all of them in turn.
+__host__ __device__ inline int setup_round(int n) { return (n + 31) & ~31; }
+__host__ __device__ inline int setup_threads(const SetupArgs& a) {
+  return setup_round(a.E * a.U) + setup_round(a.F) + setup_round(a.n_anchor * a.E) + (a.n_anchor > 0 ? a.E : 0);
+}
+
 struct BandArgs {
   const double* pts;   // [n_pts*2]
   const double* rc;    // [n_pts] (simus) or NULL (pfield)

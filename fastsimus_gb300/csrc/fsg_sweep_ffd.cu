@@ -9,7 +9,7 @@
 namespace fsg {
 
 cudaError_t launch_pfield_band_ffd(const SweepConfig& c, const BandArgs& A, cudaStream_t s) {
-  return launch_pfield_band_gn<true>(c, A, s);
+  return A.C.ffd == kSincShort ? launch_pfield_band_gn<kSincShort>(c, A, s) : launch_pfield_band_gn<kSincTerms>(c, A, s);
 }
 
 }  // namespace fsg

@@ -30,7 +30,8 @@ __device__ __forceinline__ void load_band_tables(const BandArgs& A, const Pfield
   for (int i = threadIdx.x; i < A.fb; i += blockDim.x) {
     int f = f_b0 + i;
     pp[i] = (f < A.F) ? A.t.pp[f] : make_float2(0.f, 0.f);
-    kb[i] = A.t.kf[min(f, A.F - 1)].x;
+    const float k = A.t.kf[min(f, A.F - 1)].x;
+    kb[i] = k * k;
   }
   for (int m = threadIdx.x; m < na; m += blockDim.x) {
     int f = min(f_b0 + m * kAnchor, A.F - 1);
@@ -63,9 +64,9 @@ __device__ __forceinline__ void store_geometry(float* rhi, float* rlo, float* am
 // of GN steps: every lane keeps its partial source sums of the block, then a reduce-scatter across
 // the GN lanes (log2 GN shuffle levels, halving the exchanged values each level) leaves lane g with
 // the full sum of frequency block + g.  `sink(f_local, psum)` is therefore called by every
-// lane, once per block, each for its own frequency.  With FFD every term is weighted by its
-// directivity at the step's frequency, sinc(k_f half_seg sin(theta)), folded into the packed
-// source sum as a fused multiply-add.
+// lane, once per block, each for its own frequency.  With DT > 0 every term is weighted by its
+// directivity at the step's frequency, sinc(k_f half_seg sin(theta)) (a polynomial of DT terms), folded
+// into the packed source sum as a fused multiply-add.
 //
 // What bounds it: the FP32 pipe and its register read ports (a source step is four packed instructions
 // per pair, its sum two).  A thread reads back only the geometry it wrote, so that the arrays are laid
@@ -73,10 +74,11 @@ __device__ __forceinline__ void store_geometry(float* rhi, float* rlo, float* am
 // on the host and a division by U per source and anchor, the call took 2,978 us for 131,072 points
 // and 128 elements x 2 sources, now 2,163, and 283 us (190 of them on the host) for 8,181 points and
 // 64 elements, now 87.
-template <int GN, bool FFD, class Sink>
+template <int GN, int DT, class Sink>
 __device__ __forceinline__ void tx_tile(const BandArgs& A, const PfieldLayout& L, unsigned char* sm, int64_t p_idx,
                                         int g, Sink& sink) {
   constexpr int kPairs = kSrcPerThread / 2;
+  constexpr bool FFD = DT > 0;
   float4* b_r = reinterpret_cast<float4*>(sm + L.off_r) + threadIdx.x;        // r_hi, r_hi, r_lo, r_lo
   float4* b_st = reinterpret_cast<float4*>(sm + L.off_step) + threadIdx.x;    // step re, re, im, im
   float2* b_amp = reinterpret_cast<float2*>(sm + L.off_amp) + threadIdx.x;
@@ -108,13 +110,13 @@ __device__ __forceinline__ void tx_tile(const BandArgs& A, const PfieldLayout& L
       b_r[p * kThreads] = make_float4(q[0].r_hi, q[1].r_hi, q[0].r_lo, q[1].r_lo);
       b_st[p * kThreads] = make_float4(q[0].step.x, q[1].step.x, q[0].step.y, q[1].step.y);
       b_amp[p * kThreads] = make_float2(q[0].amp, q[1].amp);
-      if (FFD) b_dir[p * kThreads] = make_float2(A.C.half_seg * q[0].sth, A.C.half_seg * q[1].sth);
+      if (FFD) b_dir[p * kThreads] = sqr2(make_float2(A.C.half_seg * q[0].sth, A.C.half_seg * q[1].sth));
     }
   }
   // 2. transmit sweep: exact anchor every kTxAnchor steps, FP32 recurrence in between.  The two
   // sources of a pair share one packed FP32x2 lane pair (real and imaginary parts in separate pairs).
   float2 Gr[kPairs], Gi[kPairs], Sr[kPairs], Si[kPairs], Sn[kPairs];
-  float2 Dh[FFD ? kPairs : 1];  // FFD: half_seg sin(theta) of the pair's two sources
+  float2 Dh[FFD ? kPairs : 1];  // FFD: (half_seg sin(theta))^2 of the pair's two sources
 #pragma unroll
   for (int p = 0; p < kPairs; ++p) {
     const float4 s = b_st[p * kThreads];
@@ -152,7 +154,7 @@ __device__ __forceinline__ void tx_tile(const BandArgs& A, const PfieldLayout& L
           const float2 kk = make_float2(k, k);
 #pragma unroll
           for (int p = 0; p < kPairs; ++p) {
-            const float2 d = sinc_poly2(__fmul2_rn(Dh[p], kk));
+            const float2 d = sinc_poly2<DT>(__fmul2_rn(Dh[p], kk));
             ar = p ? __ffma2_rn(Gr[p], d, ar) : __fmul2_rn(Gr[p], d);
             ai = p ? __ffma2_rn(Gi[p], d, ai) : __fmul2_rn(Gi[p], d);
             cstep2(Gr[p], Gi[p], Sr[p], Si[p], Sn[p]);
@@ -200,10 +202,10 @@ struct PfieldSink {
   }
 };
 
-template <int GN, bool FFD>
-__global__ void __launch_bounds__(kThreads, (GN >= 32 || FFD) ? 1 : 2) pfield_band_kernel(const BandArgs A) {
+template <int GN, int DT>
+__global__ void __launch_bounds__(kThreads, (GN >= 32 || DT) ? 1 : 2) pfield_band_kernel(const BandArgs A) {
   extern __shared__ __align__(16) unsigned char sm[];
-  const PfieldLayout L = pfield_layout(A.fb, A.E, FFD);
+  const PfieldLayout L = pfield_layout(A.fb, A.E, DT > 0);
   const int tid = threadIdx.x;
   const int f_b0 = blockIdx.x * A.fb;
   const int64_t p_begin = (int64_t)blockIdx.y * A.per_slice;
@@ -219,7 +221,7 @@ __global__ void __launch_bounds__(kThreads, (GN >= 32 || FFD) ? 1 : 2) pfield_ba
     bool valid = p < p_end;
     int64_t pi = valid ? p : t0;
     PfieldSink sink{pp, 0.f, min(A.fb, A.F - f_b0)};
-    tx_tile<GN, FFD>(A, L, sm, pi, g, sink);
+    tx_tile<GN, DT>(A, L, sm, pi, g, sink);
     // each lane holds the band's |p|^2 over its own frequencies: sum the GN lanes in a fixed tree
     float acc = sink.acc;
 #pragma unroll
@@ -233,22 +235,22 @@ __global__ void __launch_bounds__(kThreads, (GN >= 32 || FFD) ? 1 : 2) pfield_ba
   }
 }
 
-template <int GN, bool FFD>
+template <int GN, int DT>
 static cudaError_t launch_pfield_band(const SweepConfig& c, const BandArgs& A, cudaStream_t s) {
   cudaError_t e =
-      cudaFuncSetAttribute(pfield_band_kernel<GN, FFD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem);
+      cudaFuncSetAttribute(pfield_band_kernel<GN, DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem);
   if (e != cudaSuccess) return e;
-  pfield_band_kernel<GN, FFD><<<dim3(c.n_bands, c.n_slices), kThreads, c.smem, s>>>(A);
+  pfield_band_kernel<GN, DT><<<dim3(c.n_bands, c.n_slices), kThreads, c.smem, s>>>(A);
   return cudaGetLastError();
 }
 
-template <bool FFD>
+template <int DT>
 static cudaError_t launch_pfield_band_gn(const SweepConfig& c, const BandArgs& A, cudaStream_t s) {
   switch (c.gn) {
-    case 4: return launch_pfield_band<4, FFD>(c, A, s);
-    case 8: return launch_pfield_band<8, FFD>(c, A, s);
-    case 16: return launch_pfield_band<16, FFD>(c, A, s);
-    case 32: return launch_pfield_band<32, FFD>(c, A, s);
+    case 4: return launch_pfield_band<4, DT>(c, A, s);
+    case 8: return launch_pfield_band<8, DT>(c, A, s);
+    case 16: return launch_pfield_band<16, DT>(c, A, s);
+    case 32: return launch_pfield_band<32, DT>(c, A, s);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -27,12 +27,13 @@
 // between transmit and receive: 16 bytes of shared traffic per term and a CTA-wide hand-over per 8
 // frequencies.  Here a term never leaves its thread.  40,000 scatterers, one firing (spectrum
 // call): 64 elements x 2 sub-elements 1,583 -> 1,353 us, 64 x 1 2,453 -> 1,081 us, 128 x 2 5,367 ->
-// 5,207 us, 128 x 2 with full-frequency directivity 11,850 -> 10,100 us; 192 x 2, 8,000
+// 5,207 us, 128 x 2 with full-frequency directivity 11,850 -> 10,100 us with 14 directivity terms (8 terms:
+// 4,570 -> 3,526 us for the convex probe below); 192 x 2, 8,000
 // scatterers, 3,547 -> 2,120 us.
 //
 // Block size: 384 threads (168 registers, three warps per scheduler) beat 256 (232 registers) by
-// 0 to 9% without full-frequency directivity; with it the extra state spills, and 256 win by 10%
-// (4,640 against 5,260 us for a 128-element convex probe).  Groups of three warps (129 to 192
+// 0 to 9% without full-frequency directivity; with it the extra state spills, and 256 win by 19%
+// (3,526 against 4,326 us for a 128-element convex probe, 15,001 scatterers).  Groups of three warps (129 to 192
 // elements) take 384 in either case, which they divide.
 //
 // The receive sums carry the transmit delay phase exp(i 2 pi f tau_e) of every term; simus_reduce
@@ -44,13 +45,13 @@
 namespace fsg {
 
 // Geometry block of a tile, from geo + tile * geo_bytes: per group, pair p = u PPT + s and thread,
-// the two elements' (r_hi, r_lo), (amp, step re), step im and with FFD half_seg sin(theta); then
+// the two elements' (r_hi, r_lo), (amp, step re), step im and with FFD (half_seg sin(theta))^2; then
 // the tile's reflectivities (0 for padding and out of field).
 struct LaneBlock {
   float4* a;   // r_hi0, r_hi1, r_lo0, r_lo1
   float4* b;   // amp0, amp1, step.x0, step.x1
   float2* c;   // step.y0, step.y1
-  float2* d;   // dir0, dir1 (FFD)
+  float2* d;   // dir0^2, dir1^2 (FFD)
   float* w;    // [tile points]
 };
 
@@ -65,10 +66,12 @@ __host__ __device__ inline LaneBlock lane_block(unsigned char* base, int slots, 
   return B;
 }
 
+// DT: terms of the directivity polynomial with full-frequency directivity (FFD), else 0.
 // MAXT: the block's threads, a multiple of the group's 32 NW.
-template <int U, bool FFD, int MAXT>
+template <int U, int DT, int MAXT>
 __global__ void __launch_bounds__(MAXT, 1) simus_lane_kernel(const BandArgs A) {
   constexpr int PPT = lane_points(U), FS = 16 / PPT, NP = U * PPT;
+  constexpr bool FFD = DT > 0;
   extern __shared__ __align__(16) unsigned char sm[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int NW = A.nw, T = 32 * NW, FB = A.fb;
@@ -103,7 +106,10 @@ __global__ void __launch_bounds__(MAXT, 1) simus_lane_kernel(const BandArgs A) {
     for (int i = tid; i < FB; i += MAXT) {
       const int f = f_b0 + i;
       pp[i] = (f < A.F) ? A.t.pp[f] : make_float2(0.f, 0.f);
-      if (FFD) kb[i] = A.t.kf[min(f, A.F - 1)].x;
+      if (FFD) {
+        const float k = A.t.kf[min(f, A.F - 1)].x;
+        kb[i] = k * k;
+      }
     }
     for (int f = 0; f < FB; ++f) Y[f * T] = make_float4(0.f, 0.f, 0.f, 0.f);
     __syncthreads();
@@ -147,12 +153,12 @@ __global__ void __launch_bounds__(MAXT, 1) simus_lane_kernel(const BandArgs A) {
           for (int s = 0; s < PPT; ++s) {
             float2 r, q;
             if constexpr (FFD) {
-              const float2 d = sinc_poly2(__fmul2_rn(Dh[s], kk));
+              const float2 d = sinc_poly2<DT>(__fmul2_rn(Dh[s], kk));
               r = __fmul2_rn(Gr[s], d);
               q = __fmul2_rn(Gi[s], d);
 #pragma unroll
               for (int u = 1; u < U; ++u) {
-                const float2 du = sinc_poly2(__fmul2_rn(Dh[u * PPT + s], kk));
+                const float2 du = sinc_poly2<DT>(__fmul2_rn(Dh[u * PPT + s], kk));
                 r = __ffma2_rn(Gr[u * PPT + s], du, r);
                 q = __ffma2_rn(Gi[u * PPT + s], du, q);
               }
@@ -255,32 +261,32 @@ __global__ void __launch_bounds__(MAXT, 1) simus_lane_kernel(const BandArgs A) {
   }
 }
 
-template <int U, bool FFD, int MAXT>
+template <int U, int DT, int MAXT>
 static cudaError_t launch_lane_t(const SweepConfig& c, const BandArgs& A, cudaStream_t s) {
-  cudaError_t e = cudaFuncSetAttribute(simus_lane_kernel<U, FFD, MAXT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  cudaError_t e = cudaFuncSetAttribute(simus_lane_kernel<U, DT, MAXT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)c.smem);
   if (e != cudaSuccess) return e;
-  simus_lane_kernel<U, FFD, MAXT><<<A.grid, MAXT, c.smem, s>>>(A);
+  simus_lane_kernel<U, DT, MAXT><<<A.grid, MAXT, c.smem, s>>>(A);
   return cudaGetLastError();
 }
 
-template <bool FFD>
+template <int DT>
 static cudaError_t launch_lane_any(int U, const SweepConfig& c, const BandArgs& A, cudaStream_t s) {
-  if constexpr (FFD) {
+  if constexpr (DT > 0) {
     if (c.nw != 3) switch (U) {
-        case 1: return launch_lane_t<1, FFD, 256>(c, A, s);
-        case 2: return launch_lane_t<2, FFD, 256>(c, A, s);
-        case 3: return launch_lane_t<3, FFD, 256>(c, A, s);
-        case 4: return launch_lane_t<4, FFD, 256>(c, A, s);
+        case 1: return launch_lane_t<1, DT, 256>(c, A, s);
+        case 2: return launch_lane_t<2, DT, 256>(c, A, s);
+        case 3: return launch_lane_t<3, DT, 256>(c, A, s);
+        case 4: return launch_lane_t<4, DT, 256>(c, A, s);
         default: return cudaErrorInvalidValue;
       }
   }
   switch (U) {
-    case 1: return launch_lane_t<1, FFD, 384>(c, A, s);
-    case 2: return launch_lane_t<2, FFD, 384>(c, A, s);
-    case 3: return launch_lane_t<3, FFD, 384>(c, A, s);
+    case 1: return launch_lane_t<1, DT, 384>(c, A, s);
+    case 2: return launch_lane_t<2, DT, 384>(c, A, s);
+    case 3: return launch_lane_t<3, DT, 384>(c, A, s);
     case 4:
-      if constexpr (!FFD) return launch_lane_t<4, FFD, 384>(c, A, s);  // 129 or more elements hold at most three
+      if constexpr (DT == 0) return launch_lane_t<4, DT, 384>(c, A, s);  // 129 or more elements hold at most three
     default: return cudaErrorInvalidValue;
   }
 }

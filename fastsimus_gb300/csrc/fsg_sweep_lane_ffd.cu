@@ -4,7 +4,7 @@
 namespace fsg {
 
 cudaError_t launch_simus_lane_ffd(int U, const SweepConfig& c, const BandArgs& A, cudaStream_t s) {
-  return launch_lane_any<true>(U, c, A, s);
+  return A.C.ffd == kSincShort ? launch_lane_any<kSincShort>(U, c, A, s) : launch_lane_any<kSincTerms>(U, c, A, s);
 }
 
 }  // namespace fsg

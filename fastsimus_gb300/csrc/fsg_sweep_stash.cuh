@@ -103,14 +103,14 @@ __device__ __forceinline__ void stash_transmit(float2 (&Gr)[kSrcPerThread / 2], 
       if constexpr (U == 1) {
         const int p = k >> 1;
         if constexpr (FFD) {
-          const float2 d = sinc_poly2(__fmul2_rn(Dh[p], kk));
+          const float2 d = sinc_poly2<kSincTerms>(sqr2(__fmul2_rn(Dh[p], kk)));
           m = (k & 1) ? make_float2(Gr[p].y * d.y, Gi[p].y * d.y) : make_float2(Gr[p].x * d.x, Gi[p].x * d.x);
         } else {
           m = (k & 1) ? make_float2(Gr[p].y, Gi[p].y) : make_float2(Gr[p].x, Gi[p].x);
         }
       } else if constexpr (U == 2) {
         if constexpr (FFD) {
-          const float2 d = sinc_poly2(__fmul2_rn(Dh[k], kk));
+          const float2 d = sinc_poly2<kSincTerms>(sqr2(__fmul2_rn(Dh[k], kk)));
           const float2 tr = __fmul2_rn(Gr[k], d), ti = __fmul2_rn(Gi[k], d);
           m = make_float2(tr.x + tr.y, ti.x + ti.y);
         } else {
@@ -121,12 +121,12 @@ __device__ __forceinline__ void stash_transmit(float2 (&Gr)[kSrcPerThread / 2], 
         constexpr int PPE = SPE / 2;
         float2 tr, ti;
         if constexpr (FFD) {
-          const float2 d0 = sinc_poly2(__fmul2_rn(Dh[PPE * k], kk));
+          const float2 d0 = sinc_poly2<kSincTerms>(sqr2(__fmul2_rn(Dh[PPE * k], kk)));
           tr = __fmul2_rn(Gr[PPE * k], d0);
           ti = __fmul2_rn(Gi[PPE * k], d0);
 #pragma unroll
           for (int q = 1; q < PPE; ++q) {
-            const float2 d = sinc_poly2(__fmul2_rn(Dh[PPE * k + q], kk));
+            const float2 d = sinc_poly2<kSincTerms>(sqr2(__fmul2_rn(Dh[PPE * k + q], kk)));
             tr = __ffma2_rn(Gr[PPE * k + q], d, tr);
             ti = __ffma2_rn(Gi[PPE * k + q], d, ti);
           }

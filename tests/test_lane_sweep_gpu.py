@@ -77,3 +77,35 @@ def test_small_workspaces(E, U, ffd):
         ran += 1
         assert G.rel_l2(np64(out), ref) < PLAIN_TOL
     assert ran >= 3
+
+
+@pytest.mark.parametrize("U", [1, 3])
+@pytest.mark.parametrize("x_max", [1.0, 3.99, 4.01, 6.2])
+def test_directivity_polynomials(x_max, U):
+    """Full-frequency directivity on both sides of the argument where its polynomial changes and near the
+    largest one accepted, in the sweep of the RF spectrum and in the field (an odd number of sources)."""
+    import fastsimus_gb300 as F
+
+    E, n = 67, 21
+    rng = np.random.default_rng(int(100 * x_max) + U)
+    m = F.MediumParams(attenuation=0.4)
+    s = np.stack([rng.uniform(-12e-3, 12e-3, n), rng.uniform(3e-3, 25e-3, n)], axis=-1)
+    r, d = rng.standard_normal(n), np.linspace(0.0, 1e-6, E)
+
+    def probe(width):
+        return F.TransducerParams(freq_center=4e6, pitch=1.05 * width, n_elements=E, width=width, bandwidth=0.6)
+
+    width = 3e-4
+    for _ in range(3):  # the plan's highest frequency hardly depends on the width
+        plan = F.simus_precompute(s, r, d, probe(width), m, element_splitting=U)
+        width = x_max * U * m.speed_of_sound / (np.pi * float(plan.selected_freqs[-1]))
+    p = probe(width)
+    plan = F.simus_precompute(s, r, d, p, m, element_splitting=U)
+    got = np64(F.simus_compute(s, r, d, plan, p, m, full_frequency_directivity=True).spectrum)
+    ref = O.simus_compute(s, r, d, plan, p, m, full_frequency_directivity=True).spectrum
+    assert G.rel_l2(got, ref) < PLAIN_TOL
+    fplan = F.pfield_precompute(s, d, p, m, element_splitting=U)
+    got = np64(F.pfield_compute(s, d, fplan, p, m, full_frequency_directivity=True))
+    assert G.rel_l2(got, O.pfield_compute(s, d, fplan, p, m, full_frequency_directivity=True)) < PLAIN_TOL
+    got = np64(F.pfield_compute(s, d, fplan, p, m))
+    assert G.rel_l2(got, O.pfield_compute(s, d, fplan, p, m)) < PLAIN_TOL
