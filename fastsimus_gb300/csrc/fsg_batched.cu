@@ -30,6 +30,7 @@
 #include "fsg_batched.h"
 #include "fsg_common.cuh"
 #include "fsg_internal.h"
+#include "fsg_tc.cuh"
 
 namespace fsg {
 
@@ -68,13 +69,46 @@ __device__ __forceinline__ float2 pk_cfma(float2 a, float4 b, float2 acc) {
   return __ffma2_rn(make_float2(a.y, a.y), make_float2(b.z, b.w), acc);
 }
 
+// Threads that only generate Green's terms, beside the NTH of the products: with two frequencies per
+// item there are two Green's tiles, and while the products of one run the other is filled with the
+// next tile's terms.  Generating in the product threads between barriers left the FP32 pipe idle for
+// the latency of the geometry loads (two phantoms of 30,000 scatterers x 75 firings: 67.8 ms, now
+// 57.4, and 55.7 with more, smaller items).  What bounds it now: the register reads of the products'
+// scalar FMAs, which a 4 x 5 complex tile sustains at 0.73 of the lane peak (52 ms).  One frequency per
+// item has one tile, and its product threads generate.
+__host__ __device__ constexpr int batched_gen_threads(int fb) { return fb == 2 ? 128 : 0; }
+
+// mean_u G(s, e, u, f) of N scatterers `stride` records apart (the first `n` of them; 0 for the
+// others), from the cached geometry; the loads of a source are issued together.
+template <int N>
+__device__ __forceinline__ void batched_green(const BatchArgs& A, int64_t rec, int64_t stride, int n, float2 k, float a,
+                                              float2 (&g)[N]) {
+#pragma unroll
+  for (int q = 0; q < N; ++q) g[q] = make_float2(0.f, 0.f);
+  for (int u = 0; u < A.U; ++u) {
+    float4 ga[N];
+#pragma unroll
+    for (int q = 0; q < N; ++q) ga[q] = q < n ? A.geo[rec + q * stride + u] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int q = 0; q < N; ++q) {
+      const float2 v = anchor_value(ga[q].x, ga[q].y, ga[q].z, k, a);
+      if (A.C.ffd) {
+        const float d = sinc_poly(k.x * ga[q].w);
+        g[q] = make_float2(fmaf(v.x, d, g[q].x), fmaf(v.y, d, g[q].y));
+      } else {
+        g[q] = cadd(g[q], v);
+      }
+    }
+  }
+}
+
 // FB frequencies per item, EB padded elements, BT scatterers per tile, NTH threads (256 or 512:
 // 4 or 8 row groups of warps x 2 column groups); the transmit register tile is
 // BT / (4 NTH / 64) scatterer rows x 5 transmits per thread, the receive tile EB / (4 NTH / 64)
 // element rows x 5 transmits.  PK: the complex MACs on the FP32x2 pipe with (b, conj-swapped
 // b) operands in shared memory.  MINB: CTAs per SM the register budget is cut for.
 template <int FB, int EB, int BT, bool PK, int MINB, int NTH>
-__global__ void __launch_bounds__(NTH, MINB) batched_kernel(const __grid_constant__ BatchArgs A) {
+__global__ void __launch_bounds__(NTH + batched_gen_threads(FB), MINB) batched_kernel(const __grid_constant__ BatchArgs A) {
   extern __shared__ __align__(16) unsigned char sm[];
   constexpr int kGmPitch = gm_pitch(EB);
   constexpr int NWM = NTH / 64;                                      // row groups of warps
@@ -84,7 +118,9 @@ __global__ void __launch_bounds__(NTH, MINB) batched_kernel(const __grid_constan
   float2* Gm = reinterpret_cast<float2*>(sm);                       // [FB][BT][kGmPitch]
   BOp* D = reinterpret_cast<BOp*>(Gm + FB * BT * kGmPitch);          // [FB][EB][kWPitch]
   BOp* W = D + FB * EB * kWPitch;                                    // [BT][kWPitch]
-  float* rcs = reinterpret_cast<float*>(W + BT * kWPitch);           // [BT]
+  float* rcs = reinterpret_cast<float*>(W + BT * kWPitch);           // [2][BT], a tile's and the next one's
+  constexpr int kGen = batched_gen_threads(FB);
+  constexpr int kBarFull = 2, kBarEmpty = 4;  // named barriers: Green's tile f filled, read
   __shared__ int s_item;
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -109,6 +145,52 @@ __global__ void __launch_bounds__(NTH, MINB) batched_kernel(const __grid_constan
     const int64_t s_begin = (int64_t)chunk * A.chunk;
     const int64_t s_end = min(P.n_scat, s_begin + A.chunk);
 
+    // the reflectivities (0 out of field) of the tile at t0, by `n` threads from `i` on
+    auto load_rc = [&](int64_t t0, int i, float* dst) {
+      if (i >= BT) return;
+      const int64_t s = t0 + i;
+      float w = 0.f;
+      if (s < s_end) {
+        const double x = P.scat[2 * s], z = P.scat[2 * s + 1];
+        bool out = z < 0.0;
+        if (A.convex) out = out || (x * x + (z + A.apex) * (z + A.apex) <= A.radius2);
+        w = out ? 0.f : (float)P.rc[s];
+      }
+      dst[i] = w;
+    };
+    // Green's matrix Gm[f][s][e] of the tile at t0 by NT threads: thread (e, group of scatterers)
+    auto generate = [&](auto nt, int64_t t0, int f, int i) {
+      constexpr int NT = decltype(nt)::value, kSpg = BT * EB / NT, N = kSpg < 8 ? kSpg : 8;
+      const int e = i % EB, sg = i / EB, fi = min(f0 + f, P.n_freq - 1);
+      const float2 k = P.kf[fi];
+      const float al = P.af[fi];
+      const int64_t stride = (int64_t)E * U;
+      float2* G = Gm + f * BT * kGmPitch;
+      for (int q = 0; q < kSpg; q += N) {
+        const int sl = sg * kSpg + q;
+        const int64_t left = s_end - (t0 + sl);
+        const int n = e < E ? (int)max((int64_t)0, min(left, (int64_t)N)) : 0;
+        float2 g[N];
+        batched_green<N>(A, (P.geo0 + t0 + sl) * stride + (int64_t)e * U, stride, n, k, al, g);
+#pragma unroll
+        for (int j = 0; j < N; ++j) G[(sl + j) * kGmPitch + e] = g[j];
+      }
+    };
+    if constexpr (kGen > 0) {
+      if (tid >= NTH) {
+        int par = 0;
+        for (int64_t t0 = s_begin; t0 < s_end; t0 += BT, par ^= 1) {
+          load_rc(t0, tid - NTH, rcs + par * BT);
+          for (int f = 0; f < FB; ++f) {
+            if (t0 > s_begin) tc::bar_sync(kBarEmpty + f, NTH + kGen);
+            generate(std::integral_constant<int, kGen>{}, t0, f, tid - NTH);
+            tc::bar_arrive(kBarFull + f, NTH + kGen);
+          }
+        }
+        continue;
+      }
+    }
+
     // --- transmit matrices D[f][e][t] for the band (exact, per item) ---
     for (int i = tid; i < FB * EB * kBTX; i += NTH) {
       const int f = i / (EB * kBTX), r = i % (EB * kBTX), e = r / kBTX, t = r % kBTX;
@@ -129,13 +211,6 @@ __global__ void __launch_bounds__(NTH, MINB) batched_kernel(const __grid_constan
     float2 pp[FB];
 #pragma unroll
     for (int f = 0; f < FB; ++f) pp[f] = (f < nf) ? P.pp[f0 + f] : make_float2(0.f, 0.f);
-    const float2 k0 = P.kf[f0];
-    const float a0 = P.af[f0];
-    const float kb0 = k0.x, kb1 = (f0 + 1 < P.n_freq) ? P.kf[f0 + 1].x : 0.f;  // FP32 k_f for the directivity
-    SweepConst C = A.C;  // probe constants; the recurrence step belongs to this phantom's plan
-    C.dkc = P.dkc;
-    C.dalpha = P.dalpha;
-
     float2 Y[FB][kRows][5];
 #pragma unroll
     for (int f = 0; f < FB; ++f)
@@ -145,56 +220,17 @@ __global__ void __launch_bounds__(NTH, MINB) batched_kernel(const __grid_constan
         for (int j = 0; j < 5; ++j) Y[f][i][j] = make_float2(0.f, 0.f);
 
     for (int64_t t0 = s_begin; t0 < s_end; t0 += BT) {
-      // --- the tile's reflectivities (0 out of field) ---
-      if (tid < BT) {
-        const int64_t s = t0 + tid;
-        float w = 0.f;
-        if (s < s_end) {
-          const double x = P.scat[2 * s], z = P.scat[2 * s + 1];
-          bool out = z < 0.0;
-          if (A.convex) out = out || (x * x + (z + A.apex) * (z + A.apex) <= A.radius2);
-          w = out ? 0.f : (float)P.rc[s];
-        }
-        rcs[tid] = w;
+      const float* rct = rcs;
+      if constexpr (kGen > 0) {
+        rct += ((t0 - s_begin) / BT & 1) * BT;
+      } else {
+        load_rc(t0, tid, rcs);
+        for (int f = 0; f < FB; ++f) generate(std::integral_constant<int, NTH>{}, t0, f, tid);
+        __syncthreads();
       }
-      __syncthreads();
-      // --- Green's matrix Gm[f][s][e] for the tile: thread (e, s-group of BT * EB / 256) ---
-      {
-        constexpr int kSpg = BT * EB / NTH;
-        const int e = tid % EB;
-        const int sg = tid / EB;
-        for (int k = 0; k < kSpg; ++k) {
-          const int sl = sg * kSpg + k;
-          const int64_t s = t0 + sl;
-          float2 g0 = make_float2(0.f, 0.f), g1 = make_float2(0.f, 0.f);
-          if (e < E && s < s_end) {
-            // cached geometry of (s, e, u): the U records of a thread are contiguous
-            const int64_t rec = (P.geo0 + s) * (int64_t)(E * U) + e * U;
-            for (int u = 0; u < U; ++u) {
-              const float4 ga = A.geo_a[rec + u];
-              const float2 a = anchor_value(ga.x, ga.y, ga.z, k0, a0);
-              if (A.geo_c) {
-                const float x = A.geo_c[rec + u];
-                const float d0 = sinc_poly(kb0 * x);
-                g0 = make_float2(fmaf(a.x, d0, g0.x), fmaf(a.y, d0, g0.y));
-                if (FB > 1) {
-                  const float2 a1 = cmul(a, make_float2(ga.w, A.geo_b[rec + u]));
-                  const float d1 = sinc_poly(kb1 * x);
-                  g1 = make_float2(fmaf(a1.x, d1, g1.x), fmaf(a1.y, d1, g1.y));
-                }
-              } else {
-                g0 = cadd(g0, a);
-                if (FB > 1) g1 = cadd(g1, cmul(a, make_float2(ga.w, A.geo_b[rec + u])));
-              }
-            }
-          }
-          Gm[sl * kGmPitch + e] = g0;
-          if (FB > 1) Gm[(BT + sl) * kGmPitch + e] = g1;
-        }
-      }
-      __syncthreads();
 #pragma unroll
       for (int f = 0; f < FB; ++f) {
+        if constexpr (kGen > 0) tc::bar_sync(kBarFull + f, NTH + kGen);
         const float2* G = Gm + f * BT * kGmPitch;
         if (A.tx_in) {
           // transmit field supplied by the caller (already includes pulse * probe): W = rc * p
@@ -204,7 +240,7 @@ __global__ void __launch_bounds__(NTH, MINB) batched_kernel(const __grid_constan
             float2 v = make_float2(0.f, 0.f);
             if (sg < s_end && t < T && f < nf) {
               const float2 pv = A.tx_in[((size_t)sg * P.n_freq + (f0 + f)) * T + t];
-              v = make_float2(rcs[sl] * pv.x, rcs[sl] * pv.y);
+              v = make_float2(rct[sl] * pv.x, rct[sl] * pv.y);
             }
             if constexpr (PK) W[sl * kWPitch + t] = pk_operand(v);
             else W[sl * kWPitch + t] = v;
@@ -238,7 +274,7 @@ __global__ void __launch_bounds__(NTH, MINB) batched_kernel(const __grid_constan
   #pragma unroll
           for (int i = 0; i < kTRows; ++i) {
             const int s = wm * (BT / NWM) + lm + 4 * i;
-            const float w = rcs[s];
+            const float w = rct[s];
             const float2 sc = make_float2(w * pp[f].x, w * pp[f].y);
   #pragma unroll
             for (int j = 0; j < 5; ++j) {
@@ -248,7 +284,7 @@ __global__ void __launch_bounds__(NTH, MINB) batched_kernel(const __grid_constan
             }
           }
         }
-        __syncthreads();
+        tc::bar_sync(1, NTH);
         // --- RX: Y[e][t] += sum_s G[s][e] W[s][t]; thread rows e = wm*(EB/4) + lm + 4i
 #pragma unroll 4
         for (int s = 0; s < BT; ++s) {
@@ -266,7 +302,12 @@ __global__ void __launch_bounds__(NTH, MINB) batched_kernel(const __grid_constan
               else Y[f][i][j] = cfma(a[i], b[j], Y[f][i][j]);
             }
         }
-        __syncthreads();
+        // the next products wait for every thread here (kBarFull) before W is written again
+        if constexpr (kGen > 0) {
+          if (t0 + BT < s_end) tc::bar_arrive(kBarEmpty + f, NTH + kGen);
+        } else {
+          __syncthreads();
+        }
       }
     }
     // --- partial spectrum of this item: [item][f][t][e] ---
@@ -338,8 +379,8 @@ __global__ void batched_reduce(const __grid_constant__ BatchReduceArgs a) {
 }
 
 // Geometry of every (scatterer, source) of every phantom, once per sweep (the FP32 path keeps
-// the plain kernels' double-float distance and accurate step, so the cache carries r as a
-// double-float pair).  A CTA takes `spb` scatterers at a time: their coordinates are split
+// the plain kernels' double-float distance, so the cache carries r as a double-float pair; a term at
+// any frequency is exact from it).  A CTA takes `spb` scatterers at a time: their coordinates are split
 // once into shared memory, then consecutive threads write consecutive sources.
 __global__ void __launch_bounds__(kThreads) batched_geometry_kernel(const __grid_constant__ BatchArgs A) {
   __shared__ float4 xz[kThreads];
@@ -364,9 +405,7 @@ __global__ void __launch_bounds__(kThreads) batched_geometry_kernel(const __grid
       const float4 c = xz[sl];
       const SrcGeo g = source_geometry(dfl{c.x, c.y}, dfl{c.z, c.w}, A.src_pos[src], A.rot_e[src / A.U], C);
       const int64_t rec = (P.geo0 + s) * (int64_t)n_src + src;
-      A.geo_a[rec] = make_float4(g.r_hi, g.r_lo, g.amp, g.step.x);
-      A.geo_b[rec] = g.step.y;
-      if (A.geo_c) A.geo_c[rec] = C.half_seg * g.sth;
+      A.geo[rec] = make_float4(g.r_hi, g.r_lo, g.amp, C.half_seg * g.sth);
     }
   }
 }
@@ -374,7 +413,7 @@ __global__ void __launch_bounds__(kThreads) batched_geometry_kernel(const __grid
 size_t batched_smem_bytes(int fb, int eb, int bt, int pk) {
   const size_t bop = pk ? sizeof(float4) : sizeof(float2);
   return (size_t)fb * bt * gm_pitch(eb) * sizeof(float2) + ((size_t)fb * eb * kWPitch + (size_t)bt * kWPitch) * bop +
-         bt * sizeof(float);
+         2 * bt * sizeof(float);
 }
 
 int batched_pad_elements(int n_elements) { return n_elements <= 64 ? 64 : 128; }
@@ -385,7 +424,7 @@ static cudaError_t launch_batched_t(int grid, const BatchArgs& A, cudaStream_t s
   auto k = batched_kernel<FB, EB, BT, PK, MINB, NTH>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  k<<<grid, NTH, smem, s>>>(A);
+  k<<<grid, NTH + batched_gen_threads(FB), smem, s>>>(A);
   return cudaGetLastError();
 }
 
@@ -431,12 +470,13 @@ struct BatchPlanLayout {
   int fb, eb, bt, pk, minb, nth, chunk, n_items;
   int n_bands[kMaxPhantoms], n_chunks[kMaxPhantoms], item0[kMaxPhantoms];
   int64_t geo0[kMaxPhantoms], max_scat;
-  size_t off_src, off_rot, off_tau, off_apod, off_queue, off_tab[kMaxPhantoms], off_partial, off_geo_a, off_geo_b,
-      off_geo_c, total;
+  size_t off_src, off_rot, off_tau, off_apod, off_queue, off_tab[kMaxPhantoms], off_partial, off_geo, total;
 };
 
+constexpr int64_t kItemsTarget = 16 * 152, kMinChunk = 2048;
+
 int plan_layout(const FsgProbe* probe, const FsgPhantom* ph, int n_ph, int n_tx, const FsgBatchTuning* tu,
-                BatchPlanLayout* L, int ffd = 0) {
+                BatchPlanLayout* L) {
   L->eb = batched_pad_elements(probe->n_elements);
   // two frequencies per item only fit the 64-element tile's shared memory
   L->fb = (L->eb > 64 || (tu && tu->freqs_per_item == 1)) ? 1 : 2;
@@ -445,6 +485,16 @@ int plan_layout(const FsgProbe* probe, const FsgPhantom* ph, int n_ph, int n_tx,
   L->nth = (tu && tu->threads_per_cta > 0) ? tu->threads_per_cta : 256;
   L->minb = (tu && tu->ctas_per_sm == 2 && batched_shape_supported(L->fb, L->eb, L->bt, L->pk, 2, L->nth)) ? 2 : 1;
   int64_t chunk = (tu && tu->chunk_scatterers > 0) ? tu->chunk_scatterers : 32768;
+  // at most that many scatterers per item, and as many items as keep the SMs evenly loaded to the end:
+  // sixteen per SM, of not less than kMinChunk scatterers (an item sets up its transmit matrices and
+  // writes a partial spectrum of 80 x 64 complex per frequency)
+  {
+    int64_t work = 0;
+    for (int p = 0; p < n_ph; ++p) work += (int64_t)((ph[p].plan.n_freq + L->fb - 1) / L->fb) * ph[p].n_scat;
+    const int64_t even = (work + kItemsTarget - 1) / kItemsTarget;
+    const int64_t least = even < kMinChunk ? kMinChunk : even;
+    if (chunk > least) chunk = least;
+  }
   chunk = ((chunk + L->bt - 1) / L->bt) * L->bt;
   L->chunk = (int)chunk;
   const int E = probe->n_elements, U = probe->n_sub;
@@ -472,12 +522,8 @@ int plan_layout(const FsgProbe* probe, const FsgPhantom* ph, int n_ph, int n_tx,
   L->n_items = items;
   L->off_partial = o;
   o += a256((size_t)items * L->fb * kBTX * L->eb * 8);
-  L->off_geo_a = o;
+  L->off_geo = o;
   o += a256((size_t)scat * E * U * 16);
-  L->off_geo_b = o;
-  o += a256((size_t)scat * E * U * 4);
-  L->off_geo_c = o;
-  if (ffd) o += a256((size_t)scat * E * U * 4);
   L->total = o;
   return FSG_OK;
 }
@@ -514,7 +560,7 @@ extern "C" size_t fsg_simus_batched_workspace_size(const FsgProbe* probe, const 
                                                    const FsgBatchTuning* tuning) {
   if (!probe || !phantoms || n_phantoms < 1 || n_phantoms > kMaxPhantoms || n_tx < 1) return 0;
   BatchPlanLayout L;
-  plan_layout(probe, phantoms, n_phantoms, n_tx, tuning, &L, full_frequency_directivity ? 1 : 0);
+  plan_layout(probe, phantoms, n_phantoms, n_tx, tuning, &L);
   return L.total;
 }
 
@@ -526,7 +572,7 @@ static int32_t simus_batched_impl(const FsgProbe* probe, const FsgMedium* medium
   if (st != FSG_OK) return st;
   {
     BatchPlanLayout T;
-    plan_layout(probe, phantoms, n_phantoms, n_tx, tuning, &T, ffd);
+    plan_layout(probe, phantoms, n_phantoms, n_tx, tuning, &T);
     if (!batched_shape_supported(T.fb, T.eb, T.bt, T.pk, T.minb, T.nth))
       return set_error(FSG_EUNSUPPORTED,
                        "batched tile shape (freqs_per_item %d, elements tile %d, tile_scatterers %d, packed %d, "
@@ -548,7 +594,7 @@ static int32_t simus_batched_impl(const FsgProbe* probe, const FsgMedium* medium
     }
   }
   BatchPlanLayout L;
-  plan_layout(probe, phantoms, n_phantoms, n_tx, tuning, &L, ffd);
+  plan_layout(probe, phantoms, n_phantoms, n_tx, tuning, &L);
   if (!workspace || workspace_bytes < L.total)
     return set_error(FSG_EWORKSPACE, "workspace of %zu bytes is smaller than the %zu bytes required", workspace_bytes,
                      L.total);
@@ -658,9 +704,7 @@ static int32_t simus_batched_impl(const FsgProbe* probe, const FsgMedium* medium
     A.queue = queue;
     A.partial = partial;
     A.tx_in = tx_in;
-    A.geo_a = reinterpret_cast<float4*>(ws + L.off_geo_a);
-    A.geo_b = reinterpret_cast<float*>(ws + L.off_geo_b);
-    A.geo_c = ffd ? reinterpret_cast<float*>(ws + L.off_geo_c) : nullptr;
+    A.geo = reinterpret_cast<float4*>(ws + L.off_geo);
     if (L.max_scat > 0) {
       const int spb = E * U >= kThreads ? 1 : kThreads / (E * U);
       const int64_t want = (L.max_scat + spb - 1) / spb, cap = (int64_t)sms * 8;

@@ -48,12 +48,8 @@ struct BatchArgs {
   float2* partial;          // [n_items][fb][80][64]
   const float2* tx_in;      // optional [n_scat][n_freq][n_tx] transmit field (phantom 0); NULL = compute
   // geometry of every (scatterer, source), computed once per sweep by batched_geometry_kernel:
-  // record (geo0 + s) * E * U + e * U + u holds (r_hi, r_lo, amp, step.x) and step.y
-  float4* geo_a;
-  float* geo_b;
-  // full-frequency directivity: half_seg * sin(theta) per record (NULL: the centre-frequency
-  // directivity is folded into the amplitude)
-  float* geo_c;
+  // record (geo0 + s) * E * U + e * U + u holds (r_hi, r_lo, amp, half_seg * sin(theta))
+  float4* geo;
 };
 
 struct BatchSetupArgs {

@@ -275,3 +275,26 @@ def test_batched_rejects_uncompiled_tile_shape():
     s, r = W.cfg1_scatterers(100)
     with pytest.raises(NotImplementedError):  # the packed register tile takes one frequency per item
         BatchedSimus([(s, r)], W.plane_wave_delays(p, m, [0.0]), p, m, tuning=BatchTuning(2, 8192, 1, 64, 1)).run()
+
+
+@pytest.mark.parametrize("fb,nth", [(2, 256), (2, 512), (1, 256)])
+@pytest.mark.parametrize("ffd", [False, True])
+def test_tiles_chunks_and_bands(fb, nth, ffd):
+    """No, one, 64 and 65 scatterers and several work items per band, an odd number of frequencies at
+    two per item, few elements: the Green's tiles are filled and read in turn across tiles and items."""
+    from fastsimus_gb300 import MediumParams, TransducerParams
+    from fastsimus_gb300.batched import BatchedSimus, BatchTuning
+
+    p = TransducerParams(freq_center=3e6, pitch=3e-4, n_elements=5, width=2.6e-4, bandwidth=0.4)
+    m = MediumParams(attenuation=0.6)
+    rng = np.random.default_rng(3)
+    ns = (1, 64, 65, 4200)
+    phantoms = [(np.stack([rng.uniform(-6e-3, 6e-3, n), rng.uniform(2e-3, 12e-3, n)], axis=-1),
+                 rng.standard_normal(n)) for n in ns]
+    delays = np.stack([np.linspace(0, 4e-7, 5), np.zeros(5)])
+    b = BatchedSimus(phantoms, delays, p, m, tuning=BatchTuning(fb, 2048, 1, threads_per_cta=nth),
+                     full_frequency_directivity=ffd)
+    for (s, r), plan, out in zip(phantoms, b.plans, b.run()):
+        for t in range(2):
+            ref = O.simus_compute(s, r, delays[t], plan, p, m, full_frequency_directivity=ffd)
+            assert G.rel_l2(np64(out.spectrum)[..., t], ref.spectrum) < PLAIN_TOL
