@@ -23,7 +23,10 @@
 #include <stdint.h>
 #include <string.h>
 
+#include <type_traits>
+
 #include "../../include/fsgb300.h"
+#include "fsg_common.cuh"
 #include "fsg_internal.h"
 
 namespace fsg {
@@ -31,6 +34,7 @@ namespace fsg {
 constexpr int kDasThreads = 256;      // dasmtx_kernel
 constexpr int kDasImgThreads = 128;   // das_kernel: small CTAs spread the pixels evenly over the SMs
 constexpr int kDasMaxE = 256;
+constexpr int kDasStage = 4;          // groups whose delays sit in shared memory at a time
 constexpr int kDasGroup = 8;          // firings whose transmit distances a thread holds at a time
 constexpr int kDasImgBlocks = 7;      // das_kernel CTAs per SM the registers are cut for
 
@@ -318,14 +322,14 @@ __device__ __forceinline__ bool das_tap(const DasArgs& A, const DasShared& S, in
 }
 
 // floorf(s) and the integer.  Records of up to kDasShort samples do without the conversion unit (a
-// quarter of the rate of the others): exact for |s| < 2^22, and beyond that a value that is out of the
-// record as s is (NaN stays NaN).
+// quarter of the rate of the others): exact for |s| < 2^22; beyond that, and for infinities and NaN, *i
+// is no sample of such a record.
 constexpr int kDasShort = 1 << 22;
 template <bool kLong>
 __device__ __forceinline__ float das_floor(float s, int* i) {
   if constexpr (kLong) {
     const float fi = floorf(s);
-    *i = fi >= 0.f && fi < 2147483648.0f ? (int)fi : 0;
+    *i = fi >= 0.f && fi < 2147483648.0f ? (int)fi : -1;
     return fi;
   }
   const float t = s + 12582912.0f;  // 1.5 * 2^23: rounds to the nearest integer
@@ -335,6 +339,13 @@ __device__ __forceinline__ float das_floor(float s, int* i) {
   return r - (float)down;
 }
 
+// sqrt(d2) from one reciprocal root: s = d2 y plus the residual (d2 - s^2) y / 2, within an ulp (the
+// correctly rounded root takes three times the instructions).
+__device__ __forceinline__ float das_sqrt(float d2) {
+  const float y = rsqrt_normal(fmaxf(d2, 1.17549435e-38f)), s = d2 * y;
+  return fmaf(0.5f * y, fmaf(-s, s, d2), s);
+}
+
 // Matrix-free compounded delay-and-sum.  The I/Q rotation exp(2 pi i fc (d_tx + d_rx) / c)
 // factors into a transmit part per (pixel, firing) and a receive part per (pixel, element), so
 // a thread first computes, for a group of firings, the transmit distance and rotation (kept in
@@ -342,41 +353,48 @@ __device__ __forceinline__ float das_floor(float s, int* i) {
 // once, and per firing only the sample gather, the interpolation and one complex multiply-add.
 // The group's transmit delays (times c) sit in dynamic shared memory, [element][firing].
 //
-// What bounds it: instruction issue, about 30 per tap, and the gathers (two 8-byte loads per tap; the
-// host passes neighbouring pixels of a row, whose samples share one or two lines).  The call of 75
-// firings x 64 elements x 131,072 pixels, signal copies and launches included: 1,927 us with the
+// What bounds it: instruction issue (60% of the cycles) and the latency of the gathers, two 8-byte loads
+// per tap (the host passes neighbouring pixels of a row, whose samples share one or two lines).  The call
+// of 75 firings x 64 elements x 131,072 pixels, signal copies and launches included: 1,927 us with the
 // firings' values in local memory, a distance per (element, firing) in the transmit search and floor on
-// the conversion unit; 1,324 us now (12 firings 919 -> 404, one firing 759 -> 259).  Groups of 8 keep
-// the kernel within 72 registers, seven CTAs per SM: groups of 16 (five CTAs) took 350 us more, of 12
-// (five CTAs) 530 us.
+// the conversion unit; 1,324 us with groups in registers; 1,124 us with one unsigned test per tap, 32-bit
+// offsets, das_sqrt and the delays of four groups staged at a time (barriers per group were 11% of the
+// stalls).  Twelve firings 919 -> 373, one 759 -> 254.  Groups of 8 keep the kernel within 72 registers,
+// seven CTAs per SM: six took 150 us more, eight 50; groups of 16 (five CTAs) 350, of 12 (five CTAs) 530.
 template <int G, bool kLinear, bool kLong = false>
 __global__ void __launch_bounds__(kDasImgThreads, kDasImgBlocks) das_kernel(const __grid_constant__ DasArgs A) {
   __shared__ DasShared S;
-  extern __shared__ __align__(16) float ctx_g[];  // [E][G]
+  extern __shared__ __align__(16) float ctx_s[];  // [kDasStage][E][G]
   das_load_elements(A, S);
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const bool valid = p < A.n_pix;
   const float px = valid ? (float)A.pix[2 * p] : 0.f, pz = valid ? (float)A.pix[2 * p + 1] : 0.f;
   const float k_cyc = 0.5f * A.two_fc * A.inv_c;  // cycles per metre of path, fc / c
-  const size_t fstride = (size_t)A.E * A.n_s;
-  const float top = (float)(A.n_s - (kLinear ? 2 : 1));  // the last first sample of a tap
+  const unsigned top = (unsigned)(A.n_s - (kLinear ? 2 : 1));  // the last first sample of a tap
+  // linear taps: one rounding for the sample's position instead of three
+  const float per_m = A.inv_c * A.fs, s0 = -A.t0 * A.fs;
+  using Index = typename std::conditional<kLong, int64_t, unsigned>::type;  // of a sample in the call's I/Q data
   float2 acc = make_float2(0.f, 0.f);
   for (int g0 = 0; g0 < A.n_frames; g0 += G) {
-    const int ng = min(G, A.n_frames - g0);
-    __syncthreads();
-    for (int i = threadIdx.x; i < G * A.E; i += blockDim.x) {
-      const int e = i / G, j = i % G;
-      const double v = j < ng ? A.txd[(size_t)(g0 + j) * A.E + e] : NAN;
-      ctx_g[i] = isnan(v) ? INFINITY : (float)(A.c * v);
+    const int ng = min(G, A.n_frames - g0), stage = g0 / G % kDasStage;
+    if (stage == 0) {
+      const int left = min(kDasStage * G, A.n_frames - g0);
+      __syncthreads();
+      for (int i = threadIdx.x; i < kDasStage * G * A.E; i += blockDim.x) {
+        const int j = i / (G * A.E) * G + i % G, e = i / G % A.E;
+        const double v = j < left ? A.txd[(size_t)(g0 + j) * A.E + e] : NAN;
+        ctx_s[i] = isnan(v) ? INFINITY : (float)(A.c * v);
+      }
+      __syncthreads();
     }
-    __syncthreads();
     if (!valid) continue;
+    const float* ctx_g = ctx_s + stage * G * A.E;
     float dtx[G];
 #pragma unroll
     for (int j = 0; j < G; ++j) dtx[j] = INFINITY;
     for (int e = 0; e < A.E; ++e) {
       const float dx = px - S.ex[e], dz = pz - S.ez[e];
-      const float d = sqrtf(fmaf(dx, dx, dz * dz));
+      const float d = das_sqrt(fmaf(dx, dx, dz * dz));
       const float4* cj = reinterpret_cast<const float4*>(ctx_g + e * G);
 #pragma unroll
       for (int j = 0; j < G / 4; ++j) {
@@ -401,18 +419,19 @@ __global__ void __launch_bounds__(kDasImgThreads, kDasImgBlocks) das_kernel(cons
         const float lat = fmaf(dx, S.ec[e], -dz * S.es[e]);
         if (!(ax > 0.f) || fabsf(lat) > ax * A.aperture) continue;
       }
-      const float dr = sqrtf(fmaf(dx, dx, dz * dz));
+      const float dr = das_sqrt(fmaf(dx, dx, dz * dz));
       float2 ae = make_float2(0.f, 0.f);
-      const float2* ce = A.iq + ((size_t)g0 * A.E + e) * A.n_s;
       // branch-free taps (a tap outside the record reads sample 0 with weight 0; the firings past the
       // last one have no finite delay), unrolled so that the gathers of several firings are in flight
 #pragma unroll
       for (int j = 0; j < G; ++j) {
-        const float s = ((dtx[j] + dr) * A.inv_c - A.t0) * A.fs;
+        const float d = dtx[j] + dr;
+        const float s = kLinear ? fmaf(d, per_m, s0) : (d * A.inv_c - A.t0) * A.fs;
         int i;
         const float fi = das_floor<kLong>(kLinear ? s : s + 0.5f, &i);
-        const bool ok = fi >= 0.f && fi <= top;
-        const float2* cj = ce + (j < ng ? j : 0) * fstride + (ok ? i : 0);
+        const bool ok = (unsigned)i <= top;
+        const Index col = ((Index)(g0 + (j < ng ? j : 0)) * A.E + e) * A.n_s;
+        const float2* cj = A.iq + (Index)(col + (ok ? i : 0));
         float2 v = cj[0];
         if constexpr (kLinear) {
           const float2 b = cj[1];
@@ -605,10 +624,12 @@ extern "C" int32_t fsg_das(const FsgProbe* probe, const FsgDasParams* params, co
   const unsigned grid = (unsigned)((n_pixels + kDasImgThreads - 1) / kDasImgThreads);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   // up to four firings in one group of four: 259 us against 299 for one firing, 268 against 313 for four
-  // (131,072 pixels, 64 elements); at five and more the groups of eight are as fast or faster (311 / 312,
-  // twelve firings 404 / 410 with and without this rule)
-  const bool linear = A.method == FSG_DAS_LINEAR, lng = n_samples > kDasShort, few = n_frames <= 4 || lng;
-  const size_t smem = (size_t)(few ? 4 : kDasGroup) * A.E * sizeof(float);
+  // (131,072 pixels, 64 elements); at five and more the groups of eight are as fast (311 / 312).  Records
+  // or calls beyond 32-bit offsets take 64-bit ones.
+  const bool linear = A.method == FSG_DAS_LINEAR, 
+             lng = n_samples > kDasShort || (int64_t)n_frames * probe->n_elements * n_samples > INT32_MAX,
+             few = n_frames <= 4 || lng;
+  const size_t smem = (size_t)(few ? 4 : kDasGroup) * kDasStage * A.E * sizeof(float);
   if (lng) {
     if (linear) das_kernel<4, true, true><<<grid, kDasImgThreads, smem, s>>>(A);
     else das_kernel<4, false, true><<<grid, kDasImgThreads, smem, s>>>(A);
