@@ -56,7 +56,7 @@ constexpr int kMlpMaxOut = 10;
 
 // SiLU z * sigmoid(z) with the fast exponential and reciprocal, evaluated exactly as the
 // training kernels evaluate it.
-__device__ __forceinline__ float mlp_silu(float z) { return z * __fdividef(1.0f, 1.0f + __expf(-z)); }
+__device__ __forceinline__ float mlp_silu(float z) { return z * tc::sigmoid_fast(z); }
 
 // Writes 8 consecutive activations (row r, columns k..k+7) as hi and lo BF16 into the K-major
 // A operand.

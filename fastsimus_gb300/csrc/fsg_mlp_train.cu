@@ -132,8 +132,6 @@ __device__ __forceinline__ uint64_t mix64(uint64_t x) {  // splitmix64 finaliser
   return x ^ (x >> 31);
 }
 
-__device__ __forceinline__ float sigmoid_f(float z) { return __fdividef(1.0f, 1.0f + __expf(-z)); }
-
 // 8 floats -> 8 BF16 in one 16-byte vector (element 0 at the lowest address).
 __device__ __forceinline__ uint4 pack8(const float* x) {
   uint32_t h[4];
@@ -186,7 +184,7 @@ __global__ void __launch_bounds__(256, 1) mlp_train_fb_kernel(const __grid_const
   __shared__ float s_aux[kRows][kAux];
   __shared__ float s_red[4][kPart];
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = tc::warp_uniform(tid >> 5), lane = tid & 31;
   const int nout = a.net.n_out;
   for (int i = tid; i < 256; i += blockDim.x) s_bmat[i] = a.net.bmat[i];
   for (int i = tid; i < 4 * kW; i += blockDim.x) s_bias[i / kW][i % kW] = a.net.bias[i / kW][i % kW];
@@ -223,15 +221,18 @@ __global__ void __launch_bounds__(256, 1) mlp_train_fb_kernel(const __grid_const
   // Copies piece g into buffer g % kBufs.  The buffer's previous piece (g - kBufs) must be
   // released by its MMAs: with `block` the call waits for that (bounded); without, it returns
   // false at once (nothing issued) if the release has not happened yet.
+  // Warp 0 issues copies and MMAs as a whole, one elected lane executing them: issued by `tid == 0`,
+  // with operands the compiler could not see to be uniform, an MMA took 187 cycles instead of 131.
+  const bool leader = tc::elect_one();
   auto load = [&](int64_t g, bool block, bool& failed) -> bool {
     const int b = (int)(g % kBufs);
     if (g >= kBufs) {
       if (block) {
-        if (!tc::mbar_wait_bounded(&mbar_free[b], ph_free[b], kWaitTries)) {
+        if (!__all_sync(0xffffffffu, tc::mbar_wait_bounded(&mbar_free[b], ph_free[b], kWaitTries))) {
           failed = true;
           return false;
         }
-      } else if (!tc::mbar_test(&mbar_free[b], ph_free[b])) {
+      } else if (!__all_sync(0xffffffffu, tc::mbar_test(&mbar_free[b], ph_free[b]))) {
         return false;
       }
       ph_free[b] ^= 1u;
@@ -252,8 +253,10 @@ __global__ void __launch_bounds__(256, 1) mlp_train_fb_kernel(const __grid_const
       const int q = j - kHeadPiece - 2;
       src = static_cast<const unsigned char*>(a.net.wb[3 - q / kP1]) + (size_t)(q % kP1) * kPieceBytes;
     }
-    tc::mbar_arrive_expect_tx(&mbar_full[b], bytes);
-    tc::bulk_g2s(sm + kOffB + b * kPieceBytes, src, bytes, &mbar_full[b]);
+    if (leader) {
+      tc::mbar_arrive_expect_tx(&mbar_full[b], bytes);
+      tc::bulk_g2s(sm + kOffB + b * kPieceBytes, src, bytes, &mbar_full[b]);
+    }
     return true;
   };
   // Wait for piece g (loading ahead up to kBufs pieces); returns its buffer's shared address.
@@ -269,7 +272,7 @@ __global__ void __launch_bounds__(256, 1) mlp_train_fb_kernel(const __grid_const
       ++next_load;
     }
     const int b = (int)(g % kBufs);
-    if (!tc::mbar_wait_bounded(&mbar_full[b], ph_full[b], kWaitTries)) return false;
+    if (!__all_sync(0xffffffffu, tc::mbar_wait_bounded(&mbar_full[b], ph_full[b], kWaitTries))) return false;
     ph_full[b] ^= 1u;
     ++consumed;
     tc::fence_after_sync();
@@ -277,32 +280,34 @@ __global__ void __launch_bounds__(256, 1) mlp_train_fb_kernel(const __grid_const
     return true;
   };
   auto finish = [&]() -> bool {  // wait for all issued MMAs
-    tc::commit(&mbar_mma);
-    if (!tc::mbar_wait_bounded(&mbar_mma, ph_mma, kWaitTries)) return false;
+    if (leader) tc::commit(&mbar_mma);
+    if (!__all_sync(0xffffffffu, tc::mbar_wait_bounded(&mbar_mma, ph_mma, kWaitTries))) return false;
     ph_mma ^= 1u;
     return true;
   };
-  // One GEMM of the tile on the tensor cores (thread 0): np pieces of 2 K-steps of 16.
+  // One GEMM of the tile on the tensor cores (warp 0): np pieces of 2 K-steps of 16.
   // Forward: D = A_hi W^T + A_lo W^T; backward: D = dZ W (dZ in the A_hi region).
   auto gemm = [&](int64_t piece0, int np, bool bwd) -> bool {
     for (int c = 0; c < np; ++c) {
       const int64_t g = piece0 + c;
       uint32_t bb;
       if (!acquire(g, bb)) return false;
+      if (leader) {
 #pragma unroll
-      for (int ks = 0; ks < kPieceK / 16; ++ks) {
-        const int kk = c * (kPieceK / 16) + ks;
-        const uint64_t ah = tc::sdesc(sbase + kOffAHi + kk * 256, 128, 32 * 128);
-        const uint64_t bd = tc::sdesc(bb + ks * 2 * 4096, 4096, 128);  // both packings: K stride 4096, N stride 128
-        if (!bwd) {
-          const uint64_t al = tc::sdesc(sbase + kOffALo + kk * 256, 128, 32 * 128);
-          tc::mma_bf16(tmem, ah, bd, id_fwd, kk > 0);
-          tc::mma_bf16(tmem, al, bd, id_fwd, 1);
-        } else {
-          tc::mma_bf16(tmem, ah, bd, id_bwd, kk > 0);
+        for (int ks = 0; ks < kPieceK / 16; ++ks) {
+          const int kk = c * (kPieceK / 16) + ks;
+          const uint64_t ah = tc::sdesc(sbase + kOffAHi + kk * 256, 128, 32 * 128);
+          const uint64_t bd = tc::sdesc(bb + ks * 2 * 4096, 4096, 128);  // both packings: K stride 4096, N stride 128
+          if (!bwd) {
+            const uint64_t al = tc::sdesc(sbase + kOffALo + kk * 256, 128, 32 * 128);
+            tc::mma_bf16(tmem, ah, bd, id_fwd, kk > 0);
+            tc::mma_bf16(tmem, al, bd, id_fwd, 1);
+          } else {
+            tc::mma_bf16(tmem, ah, bd, id_bwd, kk > 0);
+          }
         }
+        tc::commit(&mbar_free[(int)(g % kBufs)]);
       }
-      tc::commit(&mbar_free[(int)(g % kBufs)]);
     }
     if (!finish()) return false;
     // every buffer is free now: start the next pieces so they land during the epilogue
@@ -313,22 +318,24 @@ __global__ void __launch_bounds__(256, 1) mlp_train_fb_kernel(const __grid_const
     }
     return true;
   };
-  // The head's forward MMA (thread 0): O = A_4 W_h^T in TMEM columns [256, 272), three products
+  // The head's forward MMA (warp 0): O = A_4 W_h^T in TMEM columns [256, 272), three products
   // A_hi W_hi + A_lo W_hi + A_hi W_lo over K = 256.
   auto head_fwd = [&](int64_t g) -> bool {
     uint32_t hb;
     if (!acquire(g, hb)) return false;
+    if (leader) {
 #pragma unroll
-    for (int kk = 0; kk < kW / 16; ++kk) {
-      const uint64_t ah = tc::sdesc(sbase + kOffAHi + kk * 256, 128, 32 * 128);
-      const uint64_t al = tc::sdesc(sbase + kOffALo + kk * 256, 128, 32 * 128);
-      const uint64_t bh = tc::sdesc(hb + kHeadHi + kk * 256, 128, 32 * 128);
-      const uint64_t bl = tc::sdesc(hb + kHeadLo + kk * 256, 128, 32 * 128);
-      tc::mma_bf16(tmem + kW, ah, bh, id_head, kk > 0);
-      tc::mma_bf16(tmem + kW, al, bh, id_head, 1);
-      tc::mma_bf16(tmem + kW, ah, bl, id_head, 1);
+      for (int kk = 0; kk < kW / 16; ++kk) {
+        const uint64_t ah = tc::sdesc(sbase + kOffAHi + kk * 256, 128, 32 * 128);
+        const uint64_t al = tc::sdesc(sbase + kOffALo + kk * 256, 128, 32 * 128);
+        const uint64_t bh = tc::sdesc(hb + kHeadHi + kk * 256, 128, 32 * 128);
+        const uint64_t bl = tc::sdesc(hb + kHeadLo + kk * 256, 128, 32 * 128);
+        tc::mma_bf16(tmem + kW, ah, bh, id_head, kk > 0);
+        tc::mma_bf16(tmem + kW, al, bh, id_head, 1);
+        tc::mma_bf16(tmem + kW, ah, bl, id_head, 1);
+      }
+      tc::commit(&mbar_free[(int)(g % kBufs)]);
     }
-    tc::commit(&mbar_free[(int)(g % kBufs)]);
     return finish();
   };
   // dA_4 = dOut W_h (K = 16; dOut as BF16 in the A_lo region, K-major [128][16]) into TMEM
@@ -338,8 +345,10 @@ __global__ void __launch_bounds__(256, 1) mlp_train_fb_kernel(const __grid_const
     if (!acquire(g, hb)) return false;
     const uint64_t ad = tc::sdesc(sbase + kOffALo, 128, 2 * 128);
     const uint64_t bd = tc::sdesc(hb, 32 * 128, 128);
-    tc::mma_bf16(tmem + kW, ad, bd, id_bwd, 0u);
-    tc::commit(&mbar_free[(int)(g % kBufs)]);
+    if (leader) {
+      tc::mma_bf16(tmem + kW, ad, bd, id_bwd, 0u);
+      tc::commit(&mbar_free[(int)(g % kBufs)]);
+    }
     return finish();
   };
   auto sync_all = [&]() {
@@ -404,7 +413,7 @@ __global__ void __launch_bounds__(256, 1) mlp_train_fb_kernel(const __grid_const
     int64_t ch = chunk_base;
     for (int l = 0; l < 4; ++l) {
       const int np = l == 0 ? kP0 : kP1;
-      if (tid == 0 && !s_fail)
+      if (warp == 0 && !s_fail)
         if (!gemm(ch, np, false)) s_fail = 1;
       ch += np;
       sync_all();
@@ -419,7 +428,7 @@ __global__ void __launch_bounds__(256, 1) mlp_train_fb_kernel(const __grid_const
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
           const float z = v[i] + s_bias[l][col0 + i];
-          const float s = sigmoid_f(z);
+          const float s = tc::sigmoid_fast(z);
           v[i] = z * s;
           gt[i] = s * fmaf(z, 1.0f - s, 1.0f);
         }
@@ -445,7 +454,7 @@ __global__ void __launch_bounds__(256, 1) mlp_train_fb_kernel(const __grid_const
     if (s_fail) break;
 
     // ---- head on the tensor cores, loss and the head's output gradient ----
-    if (tid == 0 && !s_fail)
+    if (warp == 0 && !s_fail)
       if (!head_fwd(ch)) s_fail = 1;
     ch += 1;
     sync_all();
@@ -506,7 +515,7 @@ __global__ void __launch_bounds__(256, 1) mlp_train_fb_kernel(const __grid_const
     }
     tc::fence_proxy_async_smem();
     sync_all();
-    if (tid == 0 && !s_fail)
+    if (warp == 0 && !s_fail)
       if (!head_bwd(ch)) s_fail = 1;
     ch += 1;
     if (tid < kPart) a.tile_part[(size_t)tile * kPart + tid] = s_red[0][tid] + s_red[1][tid] + s_red[2][tid] + s_red[3][tid];
@@ -525,7 +534,7 @@ __global__ void __launch_bounds__(256, 1) mlp_train_fb_kernel(const __grid_const
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
           const float z = v[i] + s_bias[3][col0 + i];
-          const float s = sigmoid_f(z);
+          const float s = tc::sigmoid_fast(z);
           v[i] = da[i] * s * fmaf(z, 1.0f - s, 1.0f);
         }
 #pragma unroll
@@ -551,7 +560,7 @@ __global__ void __launch_bounds__(256, 1) mlp_train_fb_kernel(const __grid_const
 #pragma unroll
         for (int g8 = 0; g8 < 4; ++g8) graw[4 * cb + g8] = gp[g8];
       }
-      if (tid == 0 && !s_fail)
+      if (warp == 0 && !s_fail)
         if (!gemm(ch, kP1, true)) s_fail = 1;
       ch += kP1;
       sync_all();
@@ -914,33 +923,45 @@ __global__ void __launch_bounds__(256) mlp_train_adam_kernel(const __grid_consta
   }
 }
 
-// Writes the packed BF16 copies of hidden layer l from its FP32 master weights.
-// Writes the packed head chunk: entry (region r, output j, feature k) of W_h, zero for j >= n_out.
-__global__ void mlp_train_pack_head_kernel(const float* __restrict__ wh, int n_out, void* packed) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 3 * kHO * kW) return;
-  const int r = t / (kHO * kW), j = (t / kW) % kHO, k = t % kW;
+struct PackArgs {
+  const float* w[4];
+  const float* wh;
+  void* wf[4];
+  void* wb[4];
+  void* head;
+  int n_out;
+};
+
+// Writes the packed copies of all layers from their FP32 master weights in one launch (five launches,
+// one per layer and the head, took 15 us and their gaps): the hidden layers' elements in order, then the
+// head chunk's, entry (region r, output j, feature k) of W_h, zero for j >= n_out.
+constexpr int kPackTotal = kW * kFeat + 3 * kW * kW + 3 * kHO * kW;
+__global__ void __launch_bounds__(256) mlp_train_pack_kernel(const __grid_constant__ PackArgs a) {
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= kPackTotal) return;
+  if (i < kW * kFeat + 3 * kW * kW) {
+    const int layer = i < kW * kFeat ? 0 : 1 + (i - kW * kFeat) / (kW * kW);
+    if (layer > 0) i = (i - kW * kFeat) % (kW * kW);
+    const int K = layer == 0 ? kFeat : kW, m = i / K, n = i % K;
+    const __nv_bfloat16 hb = __float2bfloat16_rn(a.w[layer][i]);
+    static_cast<__nv_bfloat16*>(a.wf[layer])[(size_t)(n / kChunkK) * (kChunkBytes / 2) + wpack_off(m, n % kChunkK) / 2] =
+        hb;
+    if (layer > 0)
+      static_cast<__nv_bfloat16*>(
+          a.wb[layer])[(size_t)(m / kChunkK) * (kChunkBytes / 2) + tc::mnmajor_off(n, m % kChunkK, 32) / 2] = hb;
+    return;
+  }
+  i -= kW * kFeat + 3 * kW * kW;
+  const int r = i / (kHO * kW), j = (i / kW) % kHO, k = i % kW;
   float v = 0.f;
-  if (j < n_out) {
-    const float w = wh[j * kW + k];
+  if (j < a.n_out) {
+    const float w = a.wh[j * kW + k];
     const __nv_bfloat16 hi = __float2bfloat16_rn(w);
     v = r == 1 ? w - __bfloat162float(hi) : w;
   }
-  __nv_bfloat16* o = static_cast<__nv_bfloat16*>(packed);
+  __nv_bfloat16* o = static_cast<__nv_bfloat16*>(a.head);
   const uint32_t off = r == 2 ? kHeadBwd + tc::mnmajor_off(k, j, kW / 8) : (r ? kHeadLo : kHeadHi) + tc::kmajor_off(j, k, kW / 8);
   o[off / 2] = __float2bfloat16_rn(v);
-}
-
-__global__ void mlp_train_pack_kernel(const float* __restrict__ w, int layer, void* wf, void* wb) {
-  const int K = layer == 0 ? kFeat : kW;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= kW * K) return;
-  const int m = i / K, n = i % K;
-  const __nv_bfloat16 hb = __float2bfloat16_rn(w[i]);
-  static_cast<__nv_bfloat16*>(wf)[(size_t)(n / kChunkK) * (kChunkBytes / 2) + wpack_off(m, n % kChunkK) / 2] = hb;
-  if (layer > 0 && wb)
-    static_cast<__nv_bfloat16*>(wb)[(size_t)(m / kChunkK) * (kChunkBytes / 2) + tc::mnmajor_off(n, m % kChunkK, 32) / 2] =
-        hb;
 }
 
 }  // namespace mlpt
@@ -1120,13 +1141,17 @@ extern "C" int32_t fsg_mlp_train_init(const FsgMlpTrain* t, void* stream) {
   int st = validate_train(t);
   if (st != FSG_OK) return st;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  PackArgs a;
   for (int l = 0; l < 4; ++l) {
-    const int K = l == 0 ? kFeat : kW;
-    mlp_train_pack_kernel<<<(kW * K + 255) / 256, 256, 0, s>>>(t->w[l], l, t->packed_fwd[l], t->packed_bwd[l]);
-    if ((st = check_cuda(cudaGetLastError(), "mlp_train_pack_kernel launch")) != FSG_OK) return st;
+    a.w[l] = t->w[l];
+    a.wf[l] = t->packed_fwd[l];
+    a.wb[l] = t->packed_bwd[l];
   }
-  mlp_train_pack_head_kernel<<<(3 * kHO * kW + 255) / 256, 256, 0, s>>>(t->w_head, t->n_out, t->packed_head);
-  if ((st = check_cuda(cudaGetLastError(), "mlp_train_pack_head_kernel launch")) != FSG_OK) return st;
+  a.wh = t->w_head;
+  a.head = t->packed_head;
+  a.n_out = t->n_out;
+  mlp_train_pack_kernel<<<(kPackTotal + 255) / 256, 256, 0, s>>>(a);
+  if ((st = check_cuda(cudaGetLastError(), "mlp_train_pack_kernel launch")) != FSG_OK) return st;
   unsigned char* ws = static_cast<unsigned char*>(t->workspace);
   unsigned char* done = ws + fsg_mlp_train_workspace_size(t->n_tiles, t->n_split) - 256;
   return check_cuda(cudaMemsetAsync(done, 0, 256, s), "training counter reset");

@@ -239,6 +239,14 @@ __device__ __forceinline__ void split8(const float* x, uint4& hi, uint4& lo) {
   lo = make_uint4(l[0], l[1], l[2], l[3]);
 }
 
+// sigmoid(z) with the fast exponential and reciprocal.  1 + exp(-z) >= 1 needs none of the scaling for
+// subnormal divisors that __fdividef carries (beyond 2^126 both give 0).
+__device__ __forceinline__ float sigmoid_fast(float z) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + __expf(-z)));
+  return r;
+}
+
 // Byte offset of element (row, k) in a K-major no-swizzle tile whose core matrices are laid
 // out row-group-major: core (row/8, k/8) at ((row/8) * kgroups + k/8) * 128.
 __device__ __forceinline__ uint32_t kmajor_off(int row, int k, int kgroups) {
