@@ -13,13 +13,15 @@
 // Sixteen worker warps run the features and epilogues, 64 columns at a time; one more streams the weights
 // and one issues the MMAs of a layer's 64 input columns as soon as the workers have written them, so the
 // products run under the epilogue that feeds them (D alternates between two halves of TMEM).  The
-// next tile's features are formed before the last layer's epilogue, for the same reason.
+// next tile's features are formed while the last layer's products run.
 //
-// What bounds it: per layer and tile 4,200 cycles of MMAs (131 each at N = 256) and, before them, the
-// first 64 columns' epilogue; the 32,768 SiLUs of a layer (two MUFU operations each, 4,096 cycles) run
-// beside.  1,048,576 queries: 1,680 us with products and epilogues in turn on 8 warps, 1,312 with the
-// products under the epilogues, 1,290 with 16 worker warps, 1,191 with four 16 KB weight buffers and
-// their own warp instead of two of 32 KB.
+// What bounds it: the chain of a tile, epilogue after epilogue, each waiting for the tail of its products
+// (issue 53%, tensor pipe 33% and MUFU 32% of the cycles before the last two steps below).  A layer takes
+// 4,200 cycles of MMAs (131 each at N = 256) and the issue of 32,768 SiLUs.  1,048,576 queries: 1,680 us
+// with products and epilogues in turn on 8 warps, 1,312 with the products under the epilogues, 1,290 with
+// 16 worker warps, 1,191 with four 16 KB weight buffers and their own warp instead of two of 32 KB, 1,130
+// with a layer's last inputs multiplied in two halves of the outputs (the epilogue starts on the first),
+// 1,016 with the features formed while waiting and packed FP32x2 arithmetic.
 //
 // The weights are BF16 (as in training) and multiply exactly; splitting the activations into
 // hi + lo BF16 keeps them at FP32-class precision (~1e-5 relative), as in the training forward
@@ -54,9 +56,9 @@ constexpr uint32_t kMlpWaitTries = 1u << 26;
 constexpr uint64_t kMlpDrainNs = 1000000;  // a copy or a layer's products take microseconds
 constexpr int kMlpMaxOut = 10;
 
-// SiLU z * sigmoid(z) with the fast exponential and reciprocal, evaluated exactly as the
+// SiLU z * sigmoid(z) of two values with the fast exponential and reciprocal, evaluated exactly as the
 // training kernels evaluate it.
-__device__ __forceinline__ float mlp_silu(float z) { return z * tc::sigmoid_fast(z); }
+__device__ __forceinline__ float2 mlp_silu2(float2 z) { return __fmul2_rn(z, tc::sigmoid2(z)); }
 
 // Writes 8 consecutive activations (row r, columns k..k+7) as hi and lo BF16 into the K-major
 // A operand.
@@ -77,12 +79,12 @@ __global__ void __launch_bounds__(kMlpBlock, 1) mlp_tc_forward_kernel(const __gr
   extern __shared__ __align__(1024) unsigned char sm[];
   __shared__ uint64_t mbar_full[kMlpBufs], mbar_free[kMlpBufs];  // weight buffers: copied in, released by their MMAs
   __shared__ uint64_t mbar_a[4];                   // 64 columns of A written, one arrival per worker warp
-  __shared__ uint64_t mbar_layer;                  // a layer's products done
+  __shared__ uint64_t mbar_half[2];                // a layer's products done, columns [128 h, 128 h + 128)
   __shared__ uint32_t tmem_holder;
   __shared__ int s_fail;
   __shared__ float bmat[64 * 4];
-  __shared__ float whead[kMlpMaxOut][kMlpWidth];
-  __shared__ float bias_s[4][kMlpWidth];
+  __shared__ __align__(16) float whead[kMlpMaxOut][kMlpWidth];
+  __shared__ __align__(16) float bias_s[4][kMlpWidth];
   __shared__ float hsum[3][kMlpRows][kMlpMaxOut];
 
   const int tid = threadIdx.x, warp = tc::warp_uniform(tid >> 5), lane = tid & 31;
@@ -97,7 +99,7 @@ __global__ void __launch_bounds__(kMlpBlock, 1) mlp_tc_forward_kernel(const __gr
       tc::mbar_init(&mbar_free[b], 1);
     }
     for (int c = 0; c < 4; ++c) tc::mbar_init(&mbar_a[c], kMlpWorkers / 32);
-    tc::mbar_init(&mbar_layer, 1);
+    for (int h = 0; h < 2; ++h) tc::mbar_init(&mbar_half[h], 1);
     tc::fence_mbar_init();
     s_fail = 0;
   }
@@ -135,7 +137,8 @@ __global__ void __launch_bounds__(kMlpBlock, 1) mlp_tc_forward_kernel(const __gr
     }
   } else if (warp == kMlpWorkers / 32) {
     // =============================== MMAs ===============================
-    constexpr uint32_t idesc = tc::idesc_bf16(kMlpRows, kMlpWidth, 0, 0);
+    constexpr uint32_t id_full = tc::idesc_bf16(kMlpRows, kMlpWidth, 0, 0);
+    constexpr uint32_t id_half = tc::idesc_bf16(kMlpRows, kMlpWidth / 2, 0, 0);
     const bool leader = tc::elect_one();
     uint32_t ph_a = 0;  // bit c: parity of mbar_a[c]
     int g = 0;
@@ -143,28 +146,51 @@ __global__ void __launch_bounds__(kMlpBlock, 1) mlp_tc_forward_kernel(const __gr
       for (int layer = 0; layer < 4; ++layer) {
         const int np = (layer == 0 ? kMlpFeat : kMlpWidth) / kMlpPieceK;
         const uint32_t d = tmem + (layer & 1) * kMlpWidth;
-        for (int c = 0; c < np; ++c, ++g) {
-          const int b = g % kMlpBufs;
-          if ((c & 1) == 0) {
-            wait(&mbar_a[c >> 1], (ph_a >> (c >> 1)) & 1);
-            ph_a ^= 1u << (c >> 1);
-          }
-          wait(&mbar_full[b], (g / kMlpBufs) & 1);
-          tc::fence_after_sync();
-          if (leader && !s_fail) {
-            const uint32_t bb = sbase + kOffB + b * kMlpPieceBytes;
+        // piece g (input columns [32 c, 32 c + 32)) times columns [n0, n0 + the descriptor's N) of the weights
+        auto products = [&](int c, int b, uint32_t n0, uint32_t idesc) {
+          const uint32_t bb = sbase + kOffB + b * kMlpPieceBytes + (n0 >> 3) * 128;
 #pragma unroll
-            for (int ks = 0; ks < kMlpPieceK / 16; ++ks) {
-              const int kk = c * (kMlpPieceK / 16) + ks;  // K step of 16 within the layer
-              const uint64_t ah = tc::sdesc(sbase + kOffAHi + kk * 256, 128, kMlpKGroups * 128);
-              const uint64_t al = tc::sdesc(sbase + kOffALo + kk * 256, 128, kMlpKGroups * 128);
-              // k-group-major packed piece: K stride 4096 bytes, N stride 128
-              const uint64_t bd = tc::sdesc(bb + ks * 2 * 4096, 4096, 128);
-              tc::mma_bf16(d, ah, bd, idesc, kk > 0);
-              tc::mma_bf16(d, al, bd, idesc, 1);
+          for (int ks = 0; ks < kMlpPieceK / 16; ++ks) {
+            const int kk = c * (kMlpPieceK / 16) + ks;  // K step of 16 within the layer
+            const uint64_t ah = tc::sdesc(sbase + kOffAHi + kk * 256, 128, kMlpKGroups * 128);
+            const uint64_t al = tc::sdesc(sbase + kOffALo + kk * 256, 128, kMlpKGroups * 128);
+            // k-group-major packed piece: K stride 4096 bytes, N stride 128
+            const uint64_t bd = tc::sdesc(bb + ks * 2 * 4096, 4096, 128);
+            tc::mma_bf16(d + n0, ah, bd, idesc, kk > 0);
+            tc::mma_bf16(d + n0, al, bd, idesc, 1);
+          }
+        };
+        for (int c = 0; c < np; c += 2, g += 2) {
+          const int b0 = g % kMlpBufs, b1 = (g + 1) % kMlpBufs;
+          wait(&mbar_a[c >> 1], (ph_a >> (c >> 1)) & 1);
+          ph_a ^= 1u << (c >> 1);
+          wait(&mbar_full[b0], (g / kMlpBufs) & 1);
+          tc::fence_after_sync();
+          if (c + 2 < np) {
+            if (leader && !s_fail) {
+              products(c, b0, 0, id_full);
+              tc::commit(&mbar_free[b0]);
             }
-            tc::commit(&mbar_free[b]);
-            if (c == np - 1) tc::commit(&mbar_layer);
+            wait(&mbar_full[b1], ((g + 1) / kMlpBufs) & 1);
+            tc::fence_after_sync();
+            if (leader && !s_fail) {
+              products(c + 1, b1, 0, id_full);
+              tc::commit(&mbar_free[b1]);
+            }
+          } else {
+            // the last inputs in two halves of the outputs: the epilogue starts on the first
+            wait(&mbar_full[b1], ((g + 1) / kMlpBufs) & 1);
+            tc::fence_after_sync();
+            if (leader && !s_fail) {
+#pragma unroll
+              for (uint32_t h = 0; h < 2; ++h) {
+                products(c, b0, 128 * h, id_half);
+                if (h == 1) tc::commit(&mbar_free[b0]);
+                products(c + 1, b1, 128 * h, id_half);
+                if (h == 1) tc::commit(&mbar_free[b1]);
+                tc::commit(&mbar_half[h]);
+              }
+            }
           }
         }
       }
@@ -180,39 +206,58 @@ __global__ void __launch_bounds__(kMlpBlock, 1) mlp_tc_forward_kernel(const __gr
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&mbar_a[c]);
     };
-    // features of a tile's queries -> A (K = 128): sines, then cosines
-    auto features = [&](int64_t tile) {
+    // this thread's 16 features of a tile's queries, eight at a time, as hi and lo BF16: sines, cosines
+    uint4 f_hi[2][2], f_lo[2][2];
+    auto features = [&](int64_t tile, int blk) {
       const int64_t q = tile * kMlpRows + row;
       float4 uv = make_float4(0.f, 0.f, 0.f, 0.f);
       if (q < n) uv = *reinterpret_cast<const float4*>(u + 4 * q);
+      float sv[8], cv[8];
 #pragma unroll
-      for (int blk = 0; blk < 2; ++blk) {
-        const int j0 = 16 * part + 8 * blk;
-        float sv[8], cv[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const float* b = bmat + 4 * (j0 + i);
-          const float t = b[0] * uv.x + b[1] * uv.y + b[2] * uv.z + b[3] * uv.w;
-          sincospif(2.0f * t, &sv[i], &cv[i]);
-        }
-        store_a8(sm, row, j0, sv);
-        store_a8(sm, row, 64 + j0, cv);
+      for (int i = 0; i < 8; ++i) {
+        const float* b = bmat + 4 * (16 * part + 8 * blk + i);
+        const float t = b[0] * uv.x + b[1] * uv.y + b[2] * uv.z + b[3] * uv.w;
+        sincospif(2.0f * t, &sv[i], &cv[i]);
       }
-      ready(0);
-      ready(1);
+      tc::split8(sv, f_hi[blk][0], f_lo[blk][0]);
+      tc::split8(cv, f_hi[blk][1], f_lo[blk][1]);
+    };
+    auto store_features = [&]() {  // -> A (K = 128): sines, then cosines
+#pragma unroll
+      for (int blk = 0; blk < 2; ++blk)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const uint32_t o = tc::kmajor_off(row, 64 * h + 16 * part + 8 * blk, kMlpKGroups);
+          *reinterpret_cast<uint4*>(sm + kOffAHi + o) = f_hi[blk][h];
+          *reinterpret_cast<uint4*>(sm + kOffALo + o) = f_lo[blk][h];
+        }
     };
     uint32_t ph_layer = 0;
-    if (my_tiles > 0) features(blockIdx.x);
+    if (my_tiles > 0) {
+      features(blockIdx.x, 0);
+      features(blockIdx.x, 1);
+      store_features();
+      ready(0);
+      ready(1);
+    }
     for (int it = 0; it < my_tiles; ++it) {
       const int64_t tile = blockIdx.x + (int64_t)it * gridDim.x;
       float head[kMlpMaxOut];
 #pragma unroll
       for (int j = 0; j < kMlpMaxOut; ++j) head[j] = 0.f;
       for (int layer = 0; layer < 4; ++layer) {
-        wait(&mbar_layer, ph_layer);
-        ph_layer ^= 1u;
+        // the next tile's features are formed while the last layer's products run
+        const bool more = it + 1 < my_tiles;
+        if (more && layer == 3) {
+          features(tile + gridDim.x, 0);
+          features(tile + gridDim.x, 1);
+        }
+        wait(&mbar_half[0], ph_layer);
         tc::fence_after_sync();
-        if (layer == 3 && it + 1 < my_tiles) features(tile + gridDim.x);
+        if (more && layer == 3) {
+          store_features();
+          ready(0);
+        }
         const float* bias = bias_s[layer];
         const uint32_t d = trow + (layer & 1) * kMlpWidth + 16 * part;
         uint32_t next[16];
@@ -221,12 +266,23 @@ __global__ void __launch_bounds__(kMlpBlock, 1) mlp_tc_forward_kernel(const __gr
         for (int c = 0; c < 4; ++c) {
           const int col0 = 64 * c + 16 * part;
           float v[16];
+          if (c == 1) {  // before the second half is read, and before A columns its products read are written
+            wait(&mbar_half[1], ph_layer);
+            tc::fence_after_sync();
+            // only now may the next tile's first layer finish, which completes mbar_half[1] again
+            if (more && layer == 3) ready(1);
+          }
           tc::tmem_wait_ld16(next);
 #pragma unroll
           for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(next[i]);
           if (c < 3) tc::tmem_ld16_async(d + 64 * (c + 1), next);  // lands under this chunk's SiLUs
 #pragma unroll
-          for (int i = 0; i < 16; ++i) v[i] = mlp_silu(v[i] + bias[col0 + i]);
+          for (int i = 0; i < 16; i += 2) {
+            const float2 z = __fadd2_rn(make_float2(v[i], v[i + 1]), *reinterpret_cast<const float2*>(bias + col0 + i));
+            const float2 y = mlp_silu2(z);
+            v[i] = y.x;
+            v[i + 1] = y.y;
+          }
           if (layer < 3) {
 #pragma unroll
             for (int g8 = 0; g8 < 2; ++g8) store_a8(sm, row, col0 + 8 * g8, v + 8 * g8);
@@ -241,6 +297,7 @@ __global__ void __launch_bounds__(kMlpBlock, 1) mlp_tc_forward_kernel(const __gr
             }
           }
         }
+        ph_layer ^= 1u;
       }
       // ---- head: combine the four column sets of each row ----
       tc::fence_before_sync();

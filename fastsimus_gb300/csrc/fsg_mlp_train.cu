@@ -132,6 +132,12 @@ __device__ __forceinline__ uint64_t mix64(uint64_t x) {  // splitmix64 finaliser
   return x ^ (x >> 31);
 }
 
+// SiLU'(z) = s (1 + z (1 - s)), s = sigmoid(z), of two values
+__device__ __forceinline__ float2 silu_slope2(float2 z, float2 s) {
+  const float2 one = make_float2(1.0f, 1.0f);
+  return __fmul2_rn(s, __ffma2_rn(z, __ffma2_rn(s, make_float2(-1.0f, -1.0f), one), one));
+}
+
 // 8 floats -> 8 BF16 in one 16-byte vector (element 0 at the lowest address).
 __device__ __forceinline__ uint4 pack8(const float* x) {
   uint32_t h[4];
@@ -178,7 +184,7 @@ __global__ void __launch_bounds__(256, 1) mlp_train_fb_kernel(const __grid_const
   __shared__ int s_fail;
   __shared__ int s_step;
   __shared__ float s_bmat[256];
-  __shared__ float s_bias[4][kW];
+  __shared__ __align__(16) float s_bias[4][kW];
   __shared__ float s_bh[kMaxOut];
   __shared__ float4 s_u[kRows];
   __shared__ float s_aux[kRows][kAux];
@@ -426,11 +432,13 @@ __global__ void __launch_bounds__(256, 1) mlp_train_fb_kernel(const __grid_const
         float v[32], gt[32];
         tc::tmem_ld32(trow + col0, v);
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const float z = v[i] + s_bias[l][col0 + i];
-          const float s = tc::sigmoid_fast(z);
-          v[i] = z * s;
-          gt[i] = s * fmaf(z, 1.0f - s, 1.0f);
+        for (int i = 0; i < 32; i += 2) {
+          const float2 z = __fadd2_rn(make_float2(v[i], v[i + 1]), *reinterpret_cast<const float2*>(&s_bias[l][col0 + i]));
+          const float2 s = tc::sigmoid2(z), y = __fmul2_rn(z, s), g = silu_slope2(z, s);
+          v[i] = y.x;
+          v[i + 1] = y.y;
+          gt[i] = g.x;
+          gt[i + 1] = g.y;
         }
 #pragma unroll
         for (int g8 = 0; g8 < 4; ++g8) {
@@ -532,10 +540,11 @@ __global__ void __launch_bounds__(256, 1) mlp_train_fb_kernel(const __grid_const
         tc::tmem_ld32(trow + col0, v);
         tc::tmem_ld32(trow + kW + col0, da);
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const float z = v[i] + s_bias[3][col0 + i];
-          const float s = tc::sigmoid_fast(z);
-          v[i] = da[i] * s * fmaf(z, 1.0f - s, 1.0f);
+        for (int i = 0; i < 32; i += 2) {
+          const float2 z = __fadd2_rn(make_float2(v[i], v[i + 1]), *reinterpret_cast<const float2*>(&s_bias[3][col0 + i]));
+          const float2 y = __fmul2_rn(make_float2(da[i], da[i + 1]), silu_slope2(z, tc::sigmoid2(z)));
+          v[i] = y.x;
+          v[i + 1] = y.y;
         }
 #pragma unroll
         for (int g8 = 0; g8 < 4; ++g8) {

@@ -230,8 +230,9 @@ __device__ __forceinline__ void split8(const float* x, uint4& hi, uint4& lo) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const __nv_bfloat162 hb = __floats2bfloat162_rn(x[2 * i], x[2 * i + 1]);
-    const float2 back = __bfloat1622float2(hb);
-    const __nv_bfloat162 lb = __floats2bfloat162_rn(x[2 * i] - back.x, x[2 * i + 1] - back.y);
+    // x - hi, exact
+    const float2 d = __ffma2_rn(__bfloat1622float2(hb), make_float2(-1.0f, -1.0f), make_float2(x[2 * i], x[2 * i + 1]));
+    const __nv_bfloat162 lb = __floats2bfloat162_rn(d.x, d.y);
     h[i] = *reinterpret_cast<const uint32_t*>(&hb);
     l[i] = *reinterpret_cast<const uint32_t*>(&lb);
   }
@@ -239,11 +240,18 @@ __device__ __forceinline__ void split8(const float* x, uint4& hi, uint4& lo) {
   lo = make_uint4(l[0], l[1], l[2], l[3]);
 }
 
-// sigmoid(z) with the fast exponential and reciprocal.  1 + exp(-z) >= 1 needs none of the scaling for
-// subnormal divisors that __fdividef carries (beyond 2^126 both give 0).
-__device__ __forceinline__ float sigmoid_fast(float z) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + __expf(-z)));
+// sigmoid(z) of two values with the fast exponential and reciprocal, the products and sums on the packed
+// FP32x2 pipe (one issue slot for two).  1 + exp(-z) >= 1 needs none of the scaling for subnormal
+// divisors that __fdividef carries (beyond 2^126 both give 0).
+__device__ __forceinline__ float2 sigmoid2(float2 z) {
+  const float kMinusLog2e = -1.4426950408889634f;
+  const float2 t = __fmul2_rn(z, make_float2(kMinusLog2e, kMinusLog2e));
+  float2 e, r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.x) : "f"(t.x));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.y) : "f"(t.y));
+  e = __fadd2_rn(e, make_float2(1.0f, 1.0f));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(e.x));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(e.y));
   return r;
 }
 

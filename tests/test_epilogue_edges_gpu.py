@@ -101,3 +101,23 @@ def test_txfield_samples(E, width, att, baffle):
     # on the array's plane a rigid source is on or off by the sign of a 1e-16 in FP64: off here
     k = slice(2 if baffle == "rigid" else 0, None)
     assert np.all(np.abs(got[:2]) < 1e-6) and G.rel_l2(got[k], ref[k]) < 1e-5
+
+
+def test_surrogate_forward_of_many_tiles():
+    """Several tiles per CTA: the next tile's features and first products run under the last layer's
+    epilogue.  Repeated calls give the same bits; every tile matches the FP64 network within the tolerance
+    of the single-tile test (BF16 weights, hi + lo activations: 1e-4)."""
+    require_gpu()
+    import oracle.mlp_fp64 as M
+    from fastsimus_gb300 import workloads as W
+    from fastsimus_gb300.surrogate import TxFieldSurrogate, cfg5_box
+
+    p = W.cfg1_probe()
+    sur = TxFieldSurrogate(p, W.cfg1_medium(), cfg5_box(p), seed=2)
+    u, _ = sur.inputs(sur.sample_domain(4 * 152 * 128 + 77, seed=3), with_aux=False)
+    got = sur.forward_tc(u)
+    for _ in range(20):
+        assert torch.equal(sur.forward_tc(u), got)
+    assert sur.tc_status() == 0
+    ref, _, _ = M.forward(u.double().cpu().numpy(), *sur.oracle_params())
+    assert G.rel_l2(np64(got), ref) < 1e-4
