@@ -207,18 +207,22 @@ __global__ void __launch_bounds__(MAXT, 1) simus_lane_kernel(const BandArgs A) {
         }
         {
           const float2 pv = cmul(pp[sb + my_f], P);
-          if (lane < 16) Wb[par * 16 + idx] = make_float2(w * pv.x, w * pv.y);
+          if (lane < 16) Wb[par * 16 + (FFD ? idx : my_f * PPT + my_s)] = make_float2(w * pv.x, w * pv.y);
         }
         __syncwarp();
         // ---- receive ----
+        // two W per read without FFD (200,000 scatterers x 128 elements 24.42 -> 24.05 ms); with it the
+        // registers are short, and single reads win (3,527 against 3,580 us)
         const float2* wb = Wb + par * 16;
+        const float4* wb2 = reinterpret_cast<const float4*>(wb);  // [frequency][scatterer], without FFD
 #pragma unroll
         for (int j = 0; j < FS; ++j) {
           float2 yr = make_float2(0.f, 0.f), yi = yr;
 #pragma unroll
           for (int s = 0; s < PPT; ++s) {
             const int i = s * FS + j;
-            const float2 q = wb[i];
+            const float4 w2 = wb2[(j * PPT + s) / 2];
+            const float2 q = FFD ? wb[i] : (s & 1 ? make_float2(w2.z, w2.w) : make_float2(w2.x, w2.y));
             yr.x = fmaf(mr[i].x, q.x, yr.x);
             yr.y = fmaf(mr[i].y, q.x, yr.y);
             yi.x = fmaf(mi[i].x, q.x, yi.x);
