@@ -34,8 +34,10 @@
 
 namespace fsg {
 
-constexpr int kBTX = 80;       // padded transmits
-constexpr int kWPitch = 81;    // complex per W / D row
+// Padded transmits: the columns of the products, one or two groups of 40 (8 lanes x 5).  Up to 40 firings
+// take one: with 80 columns the products' second half is padding (two phantoms of 20,000 scatterers, 31
+// firings 36.9 ms with 80 columns and 24.6 with 40, 2 firings 36.5 and 24.2; 41 firings 37.1).
+__host__ __device__ constexpr int batched_pad_tx(int n_tx) { return n_tx <= 40 ? 40 : 80; }
 // Elements are padded to EB = 64 or 128 (a template parameter); a Gm row holds EB + 1 complex
 // values (the pad keeps column reads conflict-free).
 __host__ __device__ constexpr int gm_pitch(int eb) { return eb + 1; }
@@ -103,15 +105,16 @@ __device__ __forceinline__ void batched_green(const BatchArgs& A, int64_t rec, i
 }
 
 // FB frequencies per item, EB padded elements, BT scatterers per tile, NTH threads (256 or 512:
-// 4 or 8 row groups of warps x 2 column groups); the transmit register tile is
-// BT / (4 NTH / 64) scatterer rows x 5 transmits per thread, the receive tile EB / (4 NTH / 64)
-// element rows x 5 transmits.  PK: the complex MACs on the FP32x2 pipe with (b, conj-swapped
+// row groups of warps x BTX / 40 column groups); the transmit register tile is
+// BT / (4 NWM) scatterer rows x 5 transmits per thread, the receive tile EB / (4 NWM)
+// element rows x 5 transmits (NWM row groups).  PK: the complex MACs on the FP32x2 pipe with (b, conj-swapped
 // b) operands in shared memory.  MINB: CTAs per SM the register budget is cut for.
-template <int FB, int EB, int BT, bool PK, int MINB, int NTH>
+template <int FB, int EB, int BT, bool PK, int MINB, int NTH, int BTX>
 __global__ void __launch_bounds__(NTH + batched_gen_threads(FB), MINB) batched_kernel(const __grid_constant__ BatchArgs A) {
   extern __shared__ __align__(16) unsigned char sm[];
   constexpr int kGmPitch = gm_pitch(EB);
-  constexpr int NWM = NTH / 64;                                      // row groups of warps
+  constexpr int NWM = NTH / 32 / (BTX / 40);                         // row groups of warps
+  constexpr int kBTX = BTX, kWPitch = BTX + 1;                       // columns, complex per W / D row
   constexpr int kRows = EB / (4 * NWM);                              // receive rows per thread
   constexpr int kTRows = BT / (4 * NWM);                             // transmit rows per thread
   using BOp = typename std::conditional<PK, float4, float2>::type;  // a B-operand entry
@@ -410,7 +413,8 @@ __global__ void __launch_bounds__(kThreads) batched_geometry_kernel(const __grid
   }
 }
 
-size_t batched_smem_bytes(int fb, int eb, int bt, int pk) {
+size_t batched_smem_bytes(int fb, int eb, int bt, int pk, int tx_pad) {
+  const int kWPitch = tx_pad + 1;
   const size_t bop = pk ? sizeof(float4) : sizeof(float2);
   return (size_t)fb * bt * gm_pitch(eb) * sizeof(float2) + ((size_t)fb * eb * kWPitch + (size_t)bt * kWPitch) * bop +
          2 * bt * sizeof(float);
@@ -418,10 +422,10 @@ size_t batched_smem_bytes(int fb, int eb, int bt, int pk) {
 
 int batched_pad_elements(int n_elements) { return n_elements <= 64 ? 64 : 128; }
 
-template <int FB, int EB, int BT, bool PK, int MINB, int NTH>
+template <int FB, int EB, int BT, bool PK, int MINB, int NTH, int BTX>
 static cudaError_t launch_batched_t(int grid, const BatchArgs& A, cudaStream_t s) {
-  const size_t smem = batched_smem_bytes(FB, EB, BT, PK);
-  auto k = batched_kernel<FB, EB, BT, PK, MINB, NTH>;
+  const size_t smem = batched_smem_bytes(FB, EB, BT, PK, BTX);
+  auto k = batched_kernel<FB, EB, BT, PK, MINB, NTH, BTX>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   k<<<grid, NTH + batched_gen_threads(FB), smem, s>>>(A);
@@ -448,7 +452,8 @@ cudaError_t launch_batched(int fb, int eb, int bt, int pk, int minb, int nth, in
                            cudaStream_t s) {
 #define FSG_X(FB, EB, BT, PK, MINB, NTH)                                                  \
   if (fb == FB && eb == EB && bt == BT && pk == (int)PK && minb == MINB && nth == NTH) \
-    return launch_batched_t<FB, EB, BT, PK, MINB, NTH>(grid, A, s);
+    return batched_pad_tx(A.n_tx) == 40 ? launch_batched_t<FB, EB, BT, PK, MINB, NTH, 40>(grid, A, s)           \
+                                        : launch_batched_t<FB, EB, BT, PK, MINB, NTH, 80>(grid, A, s);
   FSG_BATCHED_SHAPES(FSG_X)
 #undef FSG_X
   return cudaErrorInvalidValue;
@@ -521,7 +526,7 @@ int plan_layout(const FsgProbe* probe, const FsgPhantom* ph, int n_ph, int n_tx,
   }
   L->n_items = items;
   L->off_partial = o;
-  o += a256((size_t)items * L->fb * kBTX * L->eb * 8);
+  o += a256((size_t)items * L->fb * batched_pad_tx(n_tx) * L->eb * 8);
   L->off_geo = o;
   o += a256((size_t)scat * E * U * 16);
   L->total = o;
@@ -725,7 +730,7 @@ static int32_t simus_batched_impl(const FsgProbe* probe, const FsgMedium* medium
     a.n_tx = n_tx;
     a.E = E;
     a.fb = L.fb;
-    a.tx_pad = kBTX;
+    a.tx_pad = batched_pad_tx(n_tx);
     a.e_pad = L.eb;
     a.apply_pp = 0;
     a.partial = partial;

@@ -45,7 +45,7 @@ struct BatchArgs {
   SweepConst C;
   double apex, radius2;
   int* queue;
-  float2* partial;          // [n_items][fb][80][64]
+  float2* partial;          // [n_items][fb][padded transmits][padded elements]
   const float2* tx_in;      // optional [n_scat][n_freq][n_tx] transmit field (phantom 0); NULL = compute
   // geometry of every (scatterer, source), computed once per sweep by batched_geometry_kernel:
   // record (geo0 + s) * E * U + e * U + u holds (r_hi, r_lo, amp, half_seg * sin(theta))
@@ -70,7 +70,7 @@ struct BatchReduceArgs {
   const float2* partial;
 };
 
-size_t batched_smem_bytes(int fb, int eb, int bt, int pk);
+size_t batched_smem_bytes(int fb, int eb, int bt, int pk, int tx_pad);
 // Padded element count of the FP32 batched kernel's tiles (64 or 128).
 int batched_pad_elements(int n_elements);
 __global__ void batched_geometry_kernel(const __grid_constant__ BatchArgs A);

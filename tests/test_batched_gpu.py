@@ -298,3 +298,23 @@ def test_tiles_chunks_and_bands(fb, nth, ffd):
         for t in range(2):
             ref = O.simus_compute(s, r, delays[t], plan, p, m, full_frequency_directivity=ffd)
             assert G.rel_l2(np64(out.spectrum)[..., t], ref.spectrum) < PLAIN_TOL
+
+
+@pytest.mark.parametrize("fb", [1, 2])
+@pytest.mark.parametrize("n_tx", [40, 41, 80])
+def test_firing_columns(n_tx, fb):
+    """Around the firings at which the products take one or two groups of 40 columns, and the most."""
+    from fastsimus_gb300 import MediumParams, TransducerParams
+    from fastsimus_gb300.batched import BatchedSimus, BatchTuning
+
+    p = TransducerParams(freq_center=3e6, pitch=3e-4, n_elements=9, width=2.6e-4, bandwidth=0.4)
+    m = MediumParams(attenuation=0.3)
+    rng = np.random.default_rng(n_tx)
+    s = np.stack([rng.uniform(-6e-3, 6e-3, 100), rng.uniform(2e-3, 12e-3, 100)], axis=-1)
+    r = rng.standard_normal(100)
+    delays = rng.uniform(0, 5e-7, (n_tx, 9))
+    b = BatchedSimus([(s, r)], delays, p, m, tuning=BatchTuning(fb, 2048, 1))
+    got = np64(b.run()[0].spectrum)
+    for t in (0, 39, n_tx - 1):
+        ref = O.simus_compute(s, r, delays[t], b.plans[0], p, m)
+        assert G.rel_l2(got[..., t], ref.spectrum) < PLAIN_TOL
