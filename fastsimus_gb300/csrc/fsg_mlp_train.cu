@@ -49,20 +49,25 @@ constexpr int kAux = 12;                              // per row: carriers c_0..
 constexpr int kHO = 16;                               // head width padded for the weight-gradient MMA
 constexpr int kPart = kHO + 1;                        // per-tile partials: head-bias gradients, loss
 // Packed weights (global): chunks of 64 inputs (forward, K-major) or 64 outputs (backward,
-// MN-major), 32 KB each, core matrices k-group-major so that each half chunk of 32 K columns is
-// a contiguous 16 KB piece.  The kernels stream 16 KB pieces through kBufs buffers.
+// MN-major), 32 KB each, core matrices k-group-major so that any 32 or 64 of their K columns are
+// contiguous.  The kernels stream pieces of kPieceK columns through kBufs buffers.
 constexpr int kChunkK = 64;                           // K columns per packed chunk
 constexpr uint32_t kChunkBytes = kW * kChunkK * 2;    // 32 KB
 constexpr int kPieceK = 64;                           // K columns per streamed piece (32 or 64)
-constexpr uint32_t kPieceBytes = kW * kPieceK * 2;    // 16 KB
+constexpr uint32_t kPieceBytes = kW * kPieceK * 2;    // 32 KB
 constexpr int kBufs = kPieceK == 32 ? 5 : 2;          // streamed pieces in shared memory
 constexpr uint32_t kABytes = kRows * kW * 2;          // one BF16 copy of a 128 x 256 operand
 constexpr uint32_t kOffAHi = 0, kOffALo = kABytes, kOffB = 2 * kABytes;
 constexpr uint32_t kFbSmem = kOffB + kBufs * kPieceBytes;
 // The head's packed weights: W_h hi and lo (K-major, 16 rows x 256, row-group-major cores; the
-// forward MMA N = 16), one 16 KB piece, then W_h as the MN-major B operand of dA_4 = dOut W_h
-// (K = 16), an 8 KB piece.
+// forward MMA N = 16), one copy of 16 KB, then W_h as the MN-major B operand of dA_4 = dOut W_h
+// (K = 16), one of 8 KB.
 constexpr uint32_t kHeadHi = 0, kHeadLo = 8192, kHeadBwd = 16384, kHeadBytes = 24576;
+// The two copies of it end where it ends: its buffer is kHeadBytes long (a whole piece from kHeadHi on
+// would read past it).
+constexpr uint32_t kHeadFwdBytes = kHeadBwd - kHeadHi, kHeadBwdBytes = kHeadBytes - kHeadBwd;
+static_assert(kHeadFwdBytes == 2 * kHO * kW * 2 && kHeadBwdBytes == kHO * kW * 2, "head copies cover the packed head");
+static_assert(kHeadFwdBytes <= kPieceBytes && kHeadBwdBytes <= kPieceBytes, "head copies fit a weight buffer");
 // Pieces of one tile: forward (layer 0: P0, layers 1..3: P1 each), the head's two, backward
 // (P1 per layer).
 constexpr int kP0 = kFeat / kPieceK, kP1 = kW / kPieceK;
@@ -251,10 +256,11 @@ __global__ void __launch_bounds__(256, 1) mlp_train_fb_kernel(const __grid_const
     } else if (j < kHeadPiece) {
       src = static_cast<const unsigned char*>(a.net.wf[1 + (j - kP0) / kP1]) + (size_t)((j - kP0) % kP1) * kPieceBytes;
     } else if (j == kHeadPiece) {
-      src = static_cast<const unsigned char*>(a.net.whead) + kHeadHi;  // hi and lo, 16 KB
+      src = static_cast<const unsigned char*>(a.net.whead) + kHeadHi;  // hi and lo
+      bytes = kHeadFwdBytes;
     } else if (j == kHeadPiece + 1) {
       src = static_cast<const unsigned char*>(a.net.whead) + kHeadBwd;
-      bytes = kHeadBytes - kHeadBwd;
+      bytes = kHeadBwdBytes;
     } else {
       const int q = j - kHeadPiece - 2;
       src = static_cast<const unsigned char*>(a.net.wb[3 - q / kP1]) + (size_t)(q % kP1) * kPieceBytes;
