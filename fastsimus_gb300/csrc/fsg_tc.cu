@@ -310,8 +310,8 @@ __global__ void __launch_bounds__(kThreads, 1) tc_kernel(const __grid_constant__
 #pragma unroll
           for (int u = 0; u < U; ++u) G[jj * U + u] = cmul(G[jj * U + u], S[jj * U + u]);
         }
-        tc::split8(gr, wv[half][0], wv[half][1]);
-        tc::split8(gi, wv[half][2], wv[half][3]);
+        tc::split8<false>(gr, wv[half][0], wv[half][1]);
+        tc::split8<false>(gi, wv[half][2], wv[half][3]);
       }
     };
     auto store = [&](int par) {
@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_kernel(const __grid_constant__
 #pragma unroll
       for (int c8 = 0; c8 < 2; ++c8) {
         uint4 hh, ll;
-        tc::split8(v + 8 * c8, hh, ll);
+        tc::split8<false>(v + 8 * c8, hh, ll);
         const uint32_t o = tc::mnmajor_off(c_p * NT + 32 * k + 16 * h + 8 * c8, s_p, N / 8);
         *reinterpret_cast<uint4*>(brx + o) = hh;
         *reinterpret_cast<uint4*>(brx + 8192 * NC + o) = ll;

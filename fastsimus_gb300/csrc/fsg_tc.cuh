@@ -225,13 +225,17 @@ __device__ __forceinline__ void split_bf16(float x, __nv_bfloat16& hi, __nv_bflo
 
 // Pack 8 floats into hi and lo 16-byte vectors (element 0 at the lowest address), two values
 // per conversion.
+// kPacked: the differences x - hi on the packed FP32x2 pipe (the same values, fewer issue slots: the network
+// kernels gain; the tensor-core sweep, at its register limit, loses: 34.2 against 33.5 ms for 31 firings).
+template <bool kPacked = true>
 __device__ __forceinline__ void split8(const float* x, uint4& hi, uint4& lo) {
   uint32_t h[4], l[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const __nv_bfloat162 hb = __floats2bfloat162_rn(x[2 * i], x[2 * i + 1]);
-    // x - hi, exact
-    const float2 d = __ffma2_rn(__bfloat1622float2(hb), make_float2(-1.0f, -1.0f), make_float2(x[2 * i], x[2 * i + 1]));
+    const float2 back = __bfloat1622float2(hb);
+    const float2 d = kPacked ? __ffma2_rn(back, make_float2(-1.0f, -1.0f), make_float2(x[2 * i], x[2 * i + 1]))
+                             : make_float2(x[2 * i] - back.x, x[2 * i + 1] - back.y);
     const __nv_bfloat162 lb = __floats2bfloat162_rn(d.x, d.y);
     h[i] = *reinterpret_cast<const uint32_t*>(&hb);
     l[i] = *reinterpret_cast<const uint32_t*>(&lb);
