@@ -34,7 +34,8 @@ _DEFAULT_MEDIUM = MediumParams()
 @dataclass(frozen=True)
 class BatchTuning:
     """Tile shapes of the batched sweep: frequencies per work item (1 or 2; probes of more
-    than 64 elements always use 1), scatterers per work item, persistent CTAs per SM, and for
+    than 64 elements always use 1), most scatterers per work item (the FP32 path cuts further until
+    there are sixteen items per SM), persistent CTAs per SM, and for
     the FP32 kernel the scatterers per tile (32, 64, 128) and the FP32x2-packed register tile.
     ``FP32_SHAPES`` lists the compiled (freqs_per_item, elements tile, tile_scatterers,
     packed, ctas_per_sm) combinations."""

@@ -7,15 +7,15 @@
 // complex GEMMs over a tile of 64 scatterers:
 //     TX:  P[s][t]  = sum_e Gm[s][e] * D[e][t]      (D = apod * exp(i 2 pi f tau_t,e))
 //     RX:  Y[e][t] += sum_s Gm[s][e] * W[s][t]      (W = rc_s * pulse * probe * P)
-// with Gm = mean_u G(s, e, u, f) generated in shared memory from the exact double-float
-// anchor of each band.  With full-frequency directivity every term is weighted at its own
-// frequency by sinc(k_f half_seg sin(theta)) (_simus_strategies.py:59-62), from half_seg
-// sin(theta) cached per (scatterer, source) beside the rest of the geometry.  Y for the CTA's band (1 or 2 frequencies) stays in registers across
-// all scatterer tiles of the work item.
+// with Gm = mean_u G(s, e, u, f) generated in shared memory, exact (double-float phase) at every
+// frequency.  With full-frequency directivity every term is weighted at its own frequency by
+// sinc(k_f half_seg sin(theta)) (_simus_strategies.py:59-62), from half_seg sin(theta) cached per
+// (scatterer, source) beside the rest of the geometry.  Y for the CTA's band (1 or 2 frequencies) stays
+// in registers across all scatterer tiles of the work item.
 //
 // Persistent launch: one CTA per SM (x blocks_per_sm) pulls work items
-// (phantom, band, scatterer chunk) from an atomic counter until the queue is empty -- there is
-// no waiting anywhere, a CTA simply exits when the counter passes the item count.  Each item
+// (phantom, band, scatterer chunk) from an atomic counter until the queue is empty -- no CTA waits
+// for another, each simply exits when the counter passes the item count.  Each item
 // writes its partial spectrum; batched_reduce sums the chunks of a (phantom, band) in fixed
 // order, so results are deterministic.
 

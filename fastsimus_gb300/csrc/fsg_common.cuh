@@ -172,11 +172,11 @@ __device__ __forceinline__ float sinc_poly(float x) {
 
 // sin(x)/x of both lanes as a polynomial of T terms in u = x^2, on the packed FP32x2 pipe.  T = kSincTerms
 // is the series above.  T = kSincShort is for |x| <= kSincShortMax, where a sweep's time goes into this
-// polynomial (14 terms: 21 of the 27 packed instructions per pair of sources and step; 8: 14): a least-squares fit in u on
-// [0, 16], its coefficients fixed one after the other from the lowest order, each rounded to FP32 before
-// the rest is fitted again.  Truncation 2e-9; evaluated in FP32 its largest error is 1.51e-7 and its rms
-// error 2.6e-8 on |x| <= 4 (the series: 1.55e-7 and 2.8e-8).  The automatic sub-element count gives
-// |x| <= 3.8 for the package's probes over the band that is swept.
+// polynomial (of the packed instructions per pair of sources and step 17 are its own at 14 terms, 10 at 8):
+// a least-squares fit in u on [0, 16], its coefficients fixed one after the other from the lowest
+// order, each rounded to FP32 before the rest is fitted again.  Truncation 2e-9; evaluated in FP32 its
+// largest error is 1.51e-7 and its rms error 2.6e-8 on |x| <= 4 (the series: 1.55e-7 and 2.8e-8).  The
+// automatic sub-element count gives |x| <= 3.5 for the package's probes over the default -60 dB band.
 constexpr int kSincShort = 8;
 constexpr double kSincShortMax = 4.0;
 template <int T>

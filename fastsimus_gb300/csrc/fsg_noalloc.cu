@@ -12,7 +12,7 @@
 //   - The scratch is kNoAllocScratchBytes (16 MiB).  fsg_simus cuts the scatterers into chunks
 //     whose geometry cache fits the workspace it is given, so the scratch bounds only the fixed
 //     part of a request: the per-frequency tables, the partial spectra (a few slots of
-//     n_freq x n_elements complex64) and the geometry block of one tile.  That is about 12 MiB
+//     n_freq x n_elements complex64) and the geometry block of one tile.  That is about 6 MiB
 //     for the 128-element, 1,142-frequency probe of the 200,000-scatterer frame, whatever the
 //     scatterer count; a larger scatterer count only means more, smaller chunks.  Requests whose
 //     fixed part does not fit (plans with many thousands of frequencies) are rejected with

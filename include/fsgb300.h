@@ -158,7 +158,8 @@ typedef struct FsgPhantom {
  * reads freqs_per_item and chunk_scatterers only. */
 typedef struct FsgBatchTuning {
   int32_t freqs_per_item;    /* 1 or 2 frequencies per work item (Green's tile reuse) */
-  int32_t chunk_scatterers;  /* scatterers per work item (rounded up to a multiple of the tile) */
+  int32_t chunk_scatterers;  /* most scatterers per work item (rounded up to a multiple of the tile); the FP32
+                              * path cuts further, down to 2,048, until there are sixteen items per SM */
   int32_t ctas_per_sm;       /* persistent CTAs per SM (2: the shape's registers are capped for two) */
   int32_t tile_scatterers;   /* scatterers per tile: 32, 64 or 128 (0 = 64) */
   int32_t packed;            /* 1: complex MACs on the FP32x2 pipe (one frequency, 64-element tile) */
