@@ -251,6 +251,7 @@ struct DasArgs {
   double pitch, radius;
   float c, inv_c, fs, two_fc, t0;
   float aperture;      // 1 / (2 f-number), or < 0 for every element
+  int slices;          // das_kernel: threads per pixel, each taking every slices-th group of firings
 };
 
 // Element centre and frame (sin, cos of its angle): linear arrays along x, convex arrays on
@@ -361,12 +362,17 @@ __device__ __forceinline__ float das_sqrt(float d2) {
 // offsets, das_sqrt and the delays of four groups staged at a time (barriers per group were 11% of the
 // stalls).  Twelve firings 919 -> 373, one 759 -> 254.  Groups of 8 keep the kernel within 72 registers,
 // seven CTAs per SM: six took 150 us more, eight 50; groups of 16 (five CTAs) 350, of 12 (five CTAs) 530.
-template <int G, bool kLinear, bool kLong = false>
+// An image of few pixels leaves SMs idle behind a thread's chain of firings: `slices` threads share a
+// pixel's groups, and their sums are added in order.
+template <int G, bool kLinear, bool kLong = false, bool kSliced = false>
 __global__ void __launch_bounds__(kDasImgThreads, kDasImgBlocks) das_kernel(const __grid_constant__ DasArgs A) {
   __shared__ DasShared S;
   extern __shared__ __align__(16) float ctx_s[];  // [kDasStage][E][G]
   das_load_elements(A, S);
-  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int slices = kSliced ? A.slices : 1, px_cta = kDasImgThreads / slices;
+  const int slice = kSliced ? threadIdx.x / px_cta : 0;
+  const int64_t p = kSliced ? (int64_t)blockIdx.x * px_cta + threadIdx.x % px_cta
+                            : (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const bool valid = p < A.n_pix;
   const float px = valid ? (float)A.pix[2 * p] : 0.f, pz = valid ? (float)A.pix[2 * p + 1] : 0.f;
   const float k_cyc = 0.5f * A.two_fc * A.inv_c;  // cycles per metre of path, fc / c
@@ -388,6 +394,7 @@ __global__ void __launch_bounds__(kDasImgThreads, kDasImgBlocks) das_kernel(cons
       __syncthreads();
     }
     if (!valid) continue;
+    if (kSliced && stage % slices != slice) continue;
     const float* ctx_g = ctx_s + stage * G * A.E;
     float dtx[G];
 #pragma unroll
@@ -446,6 +453,18 @@ __global__ void __launch_bounds__(kDasImgThreads, kDasImgBlocks) das_kernel(cons
       if (A.iq_rot) sincospif(2.f * k_cyc * dr, &sn, &cs);
       acc.x = fmaf(ae.x, cs, fmaf(-ae.y, sn, acc.x));
       acc.y = fmaf(ae.x, sn, fmaf(ae.y, cs, acc.y));
+    }
+  }
+  if constexpr (kSliced) {  // the slices' sums, in order
+    __syncthreads();
+    float2* part = reinterpret_cast<float2*>(ctx_s);
+    part[threadIdx.x] = acc;
+    __syncthreads();
+    if (slice > 0) return;
+    for (int q = 1; q < slices; ++q) {
+      const float2 v = part[q * px_cta + threadIdx.x];
+      acc.x += v.x;
+      acc.y += v.y;
     }
   }
   if (valid) A.out[p] = acc;
@@ -606,9 +625,16 @@ static int das_args(const FsgProbe* probe, const FsgDasParams* p, int n_frames, 
   A->two_fc = (float)(2.0 * p->fc);
   A->t0 = (float)p->t0;
   A->aperture = p->fnumber > 0 ? (float)(0.5 / p->fnumber) : -1.f;
+  A->slices = 1;
   A->crow = nullptr;
   A->col = nullptr;
   return FSG_OK;
+}
+
+template <int G, bool kLong, bool kSliced>
+static void launch_das(const DasArgs& A, bool linear, unsigned grid, size_t smem, cudaStream_t s) {
+  if (linear) das_kernel<G, true, kLong, kSliced><<<grid, kDasImgThreads, smem, s>>>(A);
+  else das_kernel<G, false, kLong, kSliced><<<grid, kDasImgThreads, smem, s>>>(A);
 }
 
 extern "C" int32_t fsg_das(const FsgProbe* probe, const FsgDasParams* params, const void* iq, int32_t n_frames,
@@ -621,24 +647,35 @@ extern "C" int32_t fsg_das(const FsgProbe* probe, const FsgDasParams* params, co
   if (n_pixels == 0) return FSG_OK;
   A.iq = static_cast<const float2*>(iq);
   A.out = static_cast<float2*>(image_out);
-  const unsigned grid = (unsigned)((n_pixels + kDasImgThreads - 1) / kDasImgThreads);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   // up to four firings in one group of four: 259 us against 299 for one firing, 268 against 313 for four
   // (131,072 pixels, 64 elements); at five and more the groups of eight are as fast (311 / 312).  Records
   // or calls beyond 32-bit offsets take 64-bit ones.
-  const bool linear = A.method == FSG_DAS_LINEAR, 
+  const bool linear = A.method == FSG_DAS_LINEAR,
              lng = n_samples > kDasShort || (int64_t)n_frames * probe->n_elements * n_samples > INT32_MAX,
              few = n_frames <= 4 || lng;
-  const size_t smem = (size_t)(few ? 4 : kDasGroup) * kDasStage * A.E * sizeof(float);
-  if (lng) {
-    if (linear) das_kernel<4, true, true><<<grid, kDasImgThreads, smem, s>>>(A);
-    else das_kernel<4, false, true><<<grid, kDasImgThreads, smem, s>>>(A);
-  } else if (few) {
-    if (linear) das_kernel<4, true><<<grid, kDasImgThreads, smem, s>>>(A);
-    else das_kernel<4, false><<<grid, kDasImgThreads, smem, s>>>(A);
+  // few pixels: up to four threads per pixel, as long as the CTAs still fit the SMs at once (75 firings, call:
+  // 3,600 pixels 1,111 us with one thread each and 488 with four, 22,372 pixels 1,098 and 502, 65,536 pixels
+  // 976 and, with two, 710; 18 firings 401 and 311, 382 and 343)
+  int sms = 0;
+  if ((st = device_sm_count(&sms)) != FSG_OK) return st;
+  const int group = few ? 4 : kDasGroup, groups = (n_frames + group - 1) / group;
+  const int64_t ctas = (n_pixels + kDasImgThreads - 1) / kDasImgThreads;
+  while (A.slices < kDasStage && 2 * A.slices <= groups && 2 * A.slices * ctas <= (int64_t)sms * kDasImgBlocks)
+    A.slices *= 2;
+  const unsigned grid = (unsigned)((n_pixels * A.slices + kDasImgThreads - 1) / kDasImgThreads);
+  size_t smem = (size_t)group * kDasStage * A.E * sizeof(float);
+  if (smem < kDasImgThreads * sizeof(float2)) smem = kDasImgThreads * sizeof(float2);
+  // (their own instantiations: with the slices in every kernel the 75-firing image takes 4% more)
+  // (their own instantiations: with the slices in every kernel the image of 131,072 pixels takes 4% more)
+  if (A.slices == 1) {
+    if (lng) launch_das<4, true, false>(A, linear, grid, smem, s);
+    else if (few) launch_das<4, false, false>(A, linear, grid, smem, s);
+    else launch_das<kDasGroup, false, false>(A, linear, grid, smem, s);
   } else {
-    if (linear) das_kernel<kDasGroup, true><<<grid, kDasImgThreads, smem, s>>>(A);
-    else das_kernel<kDasGroup, false><<<grid, kDasImgThreads, smem, s>>>(A);
+    if (lng) launch_das<4, true, true>(A, linear, grid, smem, s);
+    else if (few) launch_das<4, false, true>(A, linear, grid, smem, s);
+    else launch_das<kDasGroup, false, true>(A, linear, grid, smem, s);
   }
   return check_cuda(cudaGetLastError(), "das_kernel launch");
 }

@@ -49,11 +49,11 @@ def test_rf2iq_chunks_and_segments(ns, nc, nf, bw):
 
 
 @pytest.mark.parametrize("nf,n_pix,n_s", [(1, 1, 300), (4, 127, 300), (5, 128, 300), (8, 129, 300), (9, 300, 300),
-                                          (17, 33, 300), (2, 40, (1 << 22) + 1)])
+                                          (17, 33, 300), (2, 40, (1 << 22) + 1), (40, 65, 300), (75, 31, 300)])
 @pytest.mark.parametrize("method", ["linear", "nearest"])
 def test_das_firing_groups(nf, n_pix, n_s, method):
-    """Firing groups (up to four firings, full groups of eight, tails), pixels around a CTA's 128 and a
-    record beyond the short-record floor.  FP32 phases at ~100 wavelengths of path: relative L2 <= 1e-3;
+    """Firing groups (up to four firings, full groups of eight, tails; two and four threads per pixel), pixels
+    around a CTA's 128 and a record beyond the short-record floor.  FP32 phases at ~100 wavelengths of path: relative L2 <= 1e-3;
     the signal varies slowly, so that a nearest tap that rounds the other way stays within it."""
     require_gpu()
     from fastsimus_gb300.beamform import DasParam, das
