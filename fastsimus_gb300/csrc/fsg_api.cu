@@ -349,6 +349,10 @@ SweepConfig pfield_config(int E, int U, int F, int64_t n_pts, int num_sms, int f
   const int nb = want < 1 ? 1 : (want > max_nb ? max_nb : (int)want);
   const int per = (F + nb - 1) / nb;
   c.fb = ((per + kAnchor - 1) / kAnchor) * kAnchor;
+  // a band's tables fit beside the geometry, with full-frequency directivity too (one band count for
+  // the workspace of both)
+  while (c.fb > kAnchor && pfield_layout(c.fb, E, true).total > kMaxDynSmem - 1024)
+    c.fb = ((c.fb / 2 + kAnchor - 1) / kAnchor) * kAnchor;
   c.n_bands = (F + c.fb - 1) / c.fb;
   int64_t slices = (2 * (int64_t)num_sms) / c.n_bands;
   if (slices < 1) slices = 1;

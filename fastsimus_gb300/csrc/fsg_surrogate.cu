@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(128) txfield_kernel(const __grid_constant__ Tx
   }
   // times pulse (= i * pulse_im) * probe, mean over the sub-elements
   const float s = pulse_im * probe * a.C.inv_nsub;
-  const bool out_field = zs.hi < 0.f;
+  const bool out_field = a.samples[4 * i + 1] < 0.0;
   a.out[i] = out_field ? make_float2(0.f, 0.f) : make_float2(-acc.y * s, acc.x * s);
 }
 

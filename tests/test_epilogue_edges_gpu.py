@@ -121,3 +121,22 @@ def test_surrogate_forward_of_many_tiles():
     assert sur.tc_status() == 0
     ref, _, _ = M.forward(u.double().cpu().numpy(), *sur.oracle_params())
     assert G.rel_l2(np64(got), ref) < 1e-4
+
+
+@pytest.mark.parametrize("step,ffd", [(0.05, False), (0.01, False), (0.01, True)])
+def test_pfield_long_plans(step, ffd):
+    """2,074 and 10,368 frequencies on a grid large enough for one band: the band's tables fit shared
+    memory beside the geometry, or the frequencies take more bands.  Relative L2 < 1e-5, as for the
+    plans of the golden vectors."""
+    require_gpu()
+    import fastsimus_gb300 as F
+    import oracle.fastsimus_fp64 as O
+
+    p = F.TransducerParams(freq_center=4e6, pitch=3e-4, n_elements=8, width=2.7e-4, bandwidth=0.7)
+    m, d = F.MediumParams(attenuation=0.2), np.linspace(0.0, 3e-7, 8)
+    grid = np.stack(np.meshgrid(np.linspace(-5e-3, 5e-3, 400), np.linspace(3e-3, 30e-3, 420)), axis=-1)
+    plan = F.pfield_precompute(grid, d, p, m, frequency_step=step)
+    got = np64(F.pfield_compute(grid, d, plan, p, m, full_frequency_directivity=ffd)).reshape(-1)
+    at = np.random.default_rng(1).choice(got.size, 24, replace=False)
+    ref = O.pfield_compute(grid.reshape(-1, 2)[at], d, plan, p, m, full_frequency_directivity=ffd)
+    assert G.rel_l2(got[at], np.asarray(ref).reshape(-1)) < 1e-5
