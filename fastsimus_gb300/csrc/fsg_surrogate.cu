@@ -13,8 +13,8 @@
 // fsg_mlp_tc.cu) predicts the complex amplitudes of a few analytic carriers whose phases carry
 // the fast oscillation of the field: the ideal plane wave of the firing, the waves from the
 // two ends of the aperture and the two first grating lobes of the element pitch.  fsg_surrogate_inputs normalises the samples and evaluates the
-// carriers (double-float phases) for training; fsg_surrogate_combine multiplies the predicted
-// amplitudes back onto the carriers.
+// carriers (FP64 phases) for training; fsg_surrogate_combine multiplies the predicted amplitudes back
+// onto the carriers (double-float phases).
 
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -34,9 +34,9 @@ struct TxFieldArgs {
   const float4* src_pos;  // [E*U], z = 0
   float pitch;            // element x = (e - (E-1)/2) * pitch in float32 (utils/geometry.py:33-37)
   int E, U;
-  dfl fc, inv_c, cyc_fc;  // centre frequency, 1 / c, tx_n_wavelengths / fc (cycles of the pulse per Hz)
-  float alpha_hz;         // attenuation, Np/m per Hz
-  float inv_sigma, shape; // probe response sqrt(exp(-(|f - fc| inv_sigma)^shape))
+  double fc, c, cyc_fc;   // centre frequency, speed of sound, tx_n_wavelengths / fc (cycles of the pulse per Hz)
+  double alpha_hz;        // attenuation, Np/m per Hz
+  double inv_sigma, shape; // probe response sqrt(exp(-(|f - fc| inv_sigma)^shape))
   SweepConst C;           // geometry constants (dk/dalpha unused)
 };
 
@@ -60,101 +60,68 @@ __device__ __forceinline__ dfl df_mul(dfl a, dfl b) {
 
 __device__ __forceinline__ dfl df_neg(dfl a) { return {-a.hi, -a.lo}; }
 
-// exp(2 pi i k path), k in cycles per metre, both double-float: the whole cycles drop out exactly.
-__device__ __forceinline__ float2 df_cis_cycles(dfl k, dfl path) {
-  const float p = __fmul_rn(k.hi, path.hi);
-  float e = fmaf(k.hi, path.hi, -p);
-  e = fmaf(k.hi, path.lo, e);
-  e = fmaf(k.lo, path.hi, e);
-  const float x = __fadd_rn(__fsub_rn(p, rintf(p)), e);
-  float s, c;
-  sincospif(2.0f * x, &s, &c);
-  return make_float2(c, s);
-}
-
-// sin(pi x) / (pi x), the rounding of x to FP32 corrected to first order.
-__device__ __forceinline__ float sinc_pi(dfl x) {
-  if (x.hi == 0.0f) return 1.0f;
-  const dfl px = df_mul(split_double(kPi), x);
-  float s, c;
-  sincospif(x.hi, &s, &c);
-  return __fdiv_rn(fmaf((float)kPi * x.lo, c, s), px.hi);
-}
+// sin(pi x) / (pi x) (numpy.sinc)
+__device__ __forceinline__ double sinc_pi(double x) { return x == 0.0 ? 1.0 : sinpi(x) / (kPi * x); }
 
 // One thread per sample, one loop over the sources.  The array is linear, so a source differs by its x
-// alone and sin and cos of the angle are dx / r and z / r.  Paths and phases are double-float: the
-// distance is s = r^2 y, y = rsqrt(r^2), plus the residual (r^2 - s^2) y / 2, the delay's phase
-// x_e k sin(theta) is reduced to a fraction of a cycle per element and the distance's per source (their
-// sum is exact: both are multiples of 2^-20 or so below one), and the amplitudes are FP32 from y after
-// one Newton step.  FP64 is left to sin(theta) and the splits of the sample.
+// alone and its angle's sine is dx / r.  What a training target must not lose stays as exact as FP64
+// gives it: the pulse and the probe response are FP64, once per sample, and the delay's phase,
+// x_e k sin(theta), is reduced to a fraction of a cycle in double-float and rounded to FP32 once.  The
+// distance is double-float from one y = rsqrt(r^2): s = r^2 y plus the residual (r^2 - s^2) y / 2.
 //
-// What bounds it: issue, about 90 instructions per source (a third of them sincospi).  1,048,576 samples
-// of the 64-element probe (two sources per element): 3.2 ms with delays, phases and spectra in FP64,
-// which the part runs at 1/64 of the FP32 rate; 883 us with the sweeps' double-float geometry per
-// source (two correctly rounded divisions, two square roots); 491 us now.
+// What bounds it: issue, and the FP64 pipe (1/64 of the FP32 rate) beside it.  1,048,576 samples of the
+// 64-element probe (two sources per element): 3.2 ms with the delay of every element in FP64, 678 us now.
+// With the pulse, the probe response and the angles in double-float and FP32 it took 491 us and moved 0.99 of
+// the results by an FP32 ulp, and the gradients of a training step on them by 1e-5 to 1e-4 of their norm.
 template <int kBaffle>
 __global__ void __launch_bounds__(128) txfield_kernel(const __grid_constant__ TxFieldArgs a) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.n) return;
-  const dfl xs = split_double(a.samples[4 * i]), zs = split_double(a.samples[4 * i + 1]);
-  const dfl fs = split_double(a.samples[4 * i + 2]);
-  const dfl st = split_double(sin(a.samples[4 * i + 3]));
+  const double z = a.samples[4 * i + 1], f = a.samples[4 * i + 2];
   // pulse (times -i) * probe at f (spectrum.py:24-107)
-  const dfl df = df_add(fs, df_neg(a.fc));
-  const float pulse_im = sinc_pi(df_mul(a.cyc_fc, df)) - sinc_pi(df_mul(a.cyc_fc, df_add(fs, a.fc)));
-  const float probe = expf(-0.5f * powf(fabsf(df.hi) * a.inv_sigma, a.shape));
-  const dfl kc = df_mul(fs, a.inv_c);  // cycles per metre
+  const double pulse_im = sinc_pi(a.cyc_fc * (f - a.fc)) - sinc_pi(a.cyc_fc * (f + a.fc));
+  const double probe = exp(-0.5 * pow(fabs(f - a.fc) * a.inv_sigma, a.shape));
+  const float scale = (float)(pulse_im * probe);
+  const dfl xs = split_double(a.samples[4 * i]), zs = split_double(z);
+  const dfl kf = split_double(2.0 * kPi * f / a.c);
   // cycles of the plane-wave delays, x_e k sin(theta) - min_e(...) (the minimum is at an end)
-  const dfl ks = df_mul(kc, st);
+  const dfl ks = split_double(f / a.c * sin(a.samples[4 * i + 3]));
   const dfl first = df_scale(element_x(a.E - 1, a.E, a.pitch), ks.hi < 0.f ? df_neg(ks) : ks);
   const float first_r = __fsub_rn(first.hi, rintf(first.hi));
   const dfl z2 = df_sqr(zs);
-  const float alpha = a.alpha_hz * fs.hi;
+  const float alpha = (float)(a.alpha_hz * f);
   const float half = (float)((a.E - 1) * 0.5);
   float2 acc = make_float2(0.f, 0.f);
   for (int e = 0; e < a.E; ++e) {
-    const float xe = __fmul_rn(__fsub_rn((float)e, half), a.pitch);
-    const float p = __fmul_rn(xe, ks.hi);
-    const float lead_lo = fmaf(xe, ks.lo, fmaf(xe, ks.hi, -p)) + first.lo;
-    const float lead_r = __fadd_rn(__fsub_rn(p, rintf(p)), first_r);
+    float2 es = make_float2(0.f, 0.f);
     for (int u = 0; u < a.U; ++u) {
       const float2 sp = *reinterpret_cast<const float2*>(a.src_pos + e * a.U + u);
-      dfl dx = two_sum(xs.hi, -sp.x);
-      dx.lo = __fadd_rn(dx.lo, __fsub_rn(xs.lo, sp.y));
-      const float d2 = __fmul_rn(dx.hi, dx.hi);
-      const float d2_lo = fmaf(2.0f * dx.hi, dx.lo, fmaf(dx.hi, dx.hi, -d2));
-      dfl r2 = two_sum(d2, z2.hi);
-      r2.lo = __fadd_rn(r2.lo, __fadd_rn(d2_lo, z2.lo));
-      const bool apart = r2.hi > 0.f && r2.hi <= 3.402823466e38f;
-      float y = rsqrt_normal(fmaxf(r2.hi, 1.17549435e-38f));
-      float s = __fmul_rn(r2.hi, y);
-      float lo = __fmul_rn(0.5f * y, __fadd_rn(fmaf(-s, s, r2.hi), r2.lo));
-      y = fmaf(0.5f * y, fmaf(-s, y, 1.0f), y);
-      // a point on the source (or no number) is seen under 90 degrees
-      const float sth = apart ? dx.hi * y : 1.0f, cth = apart ? zs.hi * y : 0.0f;
-      if (!(s > a.C.min_dist.x || (s == a.C.min_dist.x && lo >= a.C.min_dist.y))) {
-        s = a.C.min_dist.x;
-        lo = a.C.min_dist.y;
-      }
-      const float r = __fadd_rn(s, lo);
-      float m = kBaffle == 0 ? cth : (kBaffle == 1 ? 1.0f : __fdiv_rn(cth, cth + a.C.baffle_val));
-      if (cth <= 0.0f) m = 1e-16f;
-      m *= sinc_rad(a.C.dir_coef * sth) * rsqrt_normal(r);
-      if (alpha != 0.f) m *= expf(-alpha * r);
-      const float q = __fmul_rn(kc.hi, s);
-      const float q_lo = fmaf(kc.lo, s, fmaf(kc.hi, lo, fmaf(kc.hi, s, -q)));
-      float c = __fadd_rn(__fsub_rn(q, rintf(q)), lead_r);
-      c = __fadd_rn(__fsub_rn(c, rintf(c)), __fadd_rn(q_lo, lead_lo));
-      float sn, cs;
-      sincospif(2.0f * c, &sn, &cs);
-      acc.x = fmaf(m, cs, acc.x);
-      acc.y = fmaf(m, sn, acc.y);
+      const dfl dx = df_add(xs, dfl{-sp.x, -sp.y});
+      const dfl r2 = df_add(df_sqr(dx), z2);
+      // a point on the source (or no number) is seen under 90 degrees, from the clipped distance
+      const bool apart = r2.hi > 0.f;
+      const float y = rsqrt_normal(fmaxf(r2.hi, 1.17549435e-38f)), s = __fmul_rn(r2.hi, y);
+      dfl r = fast_two_sum(s, __fmul_rn(0.5f * y, __fadd_rn(fmaf(-s, s, r2.hi), r2.lo)));
+      const float sth = apart ? fminf(1.0f, fmaxf(-1.0f, __fdiv_rn(dx.hi, r.hi))) : 1.0f;
+      const float cth = sqrtf((1.0f - sth) * (1.0f + sth));
+      if (!apart || r.hi < a.C.min_dist.x || (r.hi == a.C.min_dist.x && r.lo < a.C.min_dist.y))
+        r = dfl{a.C.min_dist.x, a.C.min_dist.y};
+      float ob = kBaffle == 0 ? cth : (kBaffle == 1 ? 1.0f : __fdiv_rn(cth, cth + a.C.baffle_val));
+      if (cth <= 0.0f) ob = 1e-16f;
+      const float amp = ob * sinc_rad(a.C.dir_coef * sth) * rsqrt_normal(r.hi) * a.C.inv_nsub;
+      es = cadd(es, anchor_value(r.hi, r.lo, amp, make_float2(kf.hi, kf.lo), alpha));
     }
+    // the delay's phase in cycles: the whole ones drop out exactly
+    const float xe = __fmul_rn(__fsub_rn((float)e, half), a.pitch);
+    const float p = __fmul_rn(xe, ks.hi);
+    const dfl lead = two_sum(__fsub_rn(p, rintf(p)), first_r);
+    const float lead_lo = __fadd_rn(lead.lo, __fadd_rn(fmaf(xe, ks.lo, fmaf(xe, ks.hi, -p)), first.lo));
+    float sd, cd;
+    sincospif(2.0f * __fadd_rn(__fsub_rn(lead.hi, rintf(lead.hi)), lead_lo), &sd, &cd);
+    acc = cfma(es, make_float2(cd, sd), acc);
   }
-  // times pulse (= i * pulse_im) * probe, mean over the sub-elements
-  const float s = pulse_im * probe * a.C.inv_nsub;
-  const bool out_field = a.samples[4 * i + 1] < 0.0;
-  a.out[i] = out_field ? make_float2(0.f, 0.f) : make_float2(-acc.y * s, acc.x * s);
+  const bool out_field = z < 0.0;
+  a.out[i] = out_field ? make_float2(0.f, 0.f) : make_float2(-acc.y * scale, acc.x * scale);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -166,6 +133,18 @@ constexpr int kAux = 12;  // floats per training row: carriers c_0..c_4, target 
 struct Carriers {
   float2 c[kMaxCarriers];
 };
+
+// exp(2 pi i k path), k in cycles per metre, both double-float: the whole cycles drop out exactly.
+__device__ __forceinline__ float2 df_cis_cycles(dfl k, dfl path) {
+  const float p = __fmul_rn(k.hi, path.hi);
+  float e = fmaf(k.hi, path.hi, -p);
+  e = fmaf(k.hi, path.lo, e);
+  e = fmaf(k.lo, path.hi, e);
+  const float x = __fadd_rn(__fsub_rn(p, rintf(p)), e);
+  float s, c;
+  sincospif(2.0f * x, &s, &c);
+  return make_float2(c, s);
+}
 
 // What a thread needs of the domain beside its fields: reciprocals, formed in FP64 on the host.
 struct DomainArgs {
@@ -232,6 +211,38 @@ __device__ __forceinline__ Carriers surrogate_carriers(const DomainArgs& D, doub
   return out;
 }
 
+// The same in FP64, for training: the carriers are rounded to FP32 once, and their last bits count there
+// (the backward pass rounds their products with the residual to BF16).
+__device__ void training_carriers(const FsgSurrogateDomain& d, double x, double z, double f, double th, float* out) {
+  const double st = sin(th), ct = cos(th);
+  const double x0 = -0.5 * (d.n_elements - 1) * d.pitch, x1 = -x0;
+  const double xmin = fmin(x0 * st, x1 * st);
+  const double kc = f / d.speed_of_sound;  // cycles per metre
+  const double lp = d.speed_of_sound / f / d.pitch;  // lambda / pitch
+  double path[kMaxCarriers];
+  bool on[kMaxCarriers];
+  path[0] = x * st + z * ct - xmin;
+  const double xl = x0 - 0.5 * d.pitch, xr = x1 + 0.5 * d.pitch;
+  path[1] = sqrt((x - xl) * (x - xl) + z * z) + xl * st - xmin;
+  path[2] = sqrt((x - xr) * (x - xr) + z * z) + xr * st - xmin;
+  on[0] = on[1] = on[2] = true;
+#pragma unroll
+  for (int m = 0; m < 2; ++m) {
+    const double sm = st + (m ? lp : -lp);
+    on[3 + m] = fabs(sm) < 1.0;
+    path[3 + m] = x * sm + z * sqrt(fmax(0.0, 1.0 - sm * sm)) - xmin;
+  }
+#pragma unroll
+  for (int j = 0; j < kMaxCarriers; ++j) {
+    const double cyc = kc * path[j];
+    double s, c;
+    sincospi(2.0 * (cyc - rint(cyc)), &s, &c);
+    const bool use = on[j] && j < d.n_carriers;
+    out[2 * j] = use ? (float)c : 0.0f;
+    out[2 * j + 1] = use ? (float)s : 0.0f;
+  }
+}
+
 __global__ void surrogate_inputs_kernel(const __grid_constant__ DomainArgs D, const double* __restrict__ samples,
                                         int64_t n, const float2* __restrict__ field, double inv_scale,
                                         float4* __restrict__ u, float* __restrict__ aux) {
@@ -241,13 +252,8 @@ __global__ void surrogate_inputs_kernel(const __grid_constant__ DomainArgs D, co
   u[i] = make_float4((float)fma(x, D.mul[0], D.add[0]), (float)fma(z, D.mul[1], D.add[1]),
                      (float)fma(f, D.mul[2], D.add[2]), (float)fma(th, D.mul[3], D.add[3]));
   if (!aux) return;
-  const Carriers c = surrogate_carriers(D, x, z, f, th);
   float* o = aux + kAux * i;
-#pragma unroll
-  for (int j = 0; j < kMaxCarriers; ++j) {
-    o[2 * j] = c.c[j].x;
-    o[2 * j + 1] = c.c[j].y;
-  }
+  training_carriers(D.d, x, z, f, th, o);
   const float2 y = field ? field[i] : make_float2(0.f, 0.f);
   o[kAux - 2] = (float)(y.x * inv_scale);
   o[kAux - 1] = (float)(y.y * inv_scale);
@@ -335,16 +341,15 @@ extern "C" int32_t fsg_txfield(const FsgProbe* probe, const FsgMedium* medium, d
   a.pitch = (float)probe->pitch;
   a.E = E;
   a.U = U;
-  a.fc = split_double(probe->freq_center);
-  a.inv_c = split_double(1.0 / medium->speed_of_sound);
-  a.cyc_fc = split_double(tx_n_wavelengths / probe->freq_center);
-  a.alpha_hz = (float)(medium->attenuation / 8.685889638065035 / 1e6 * 1e2);
+  a.fc = probe->freq_center;
+  a.c = medium->speed_of_sound;
+  a.cyc_fc = tx_n_wavelengths / probe->freq_center;
+  a.alpha_hz = medium->attenuation / 8.685889638065035 / 1e6 * 1e2;
   {
     // spectrum.py:53-107, in Hz
-    const double shape = log(126.0) / log(2.0 / bandwidth);
-    const double sigma = bandwidth * probe->freq_center / 2.0 / pow(log(2.0), 1.0 / shape);
-    a.shape = (float)shape;
-    a.inv_sigma = (float)(1.0 / sigma);
+    const double sigma = bandwidth * probe->freq_center / 2.0;
+    a.shape = log(126.0) / log(2.0 / bandwidth);
+    a.inv_sigma = pow(log(2.0), 1.0 / a.shape) / sigma;
   }
   FsgFreqPlan dummy;
   memset(&dummy, 0, sizeof(dummy));

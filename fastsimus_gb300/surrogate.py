@@ -10,9 +10,9 @@ The field oscillates at the wavelength in space and at 1/delay in frequency, and
 plane wave of the firing it carries the waves that start at the two ends of the aperture and,
 at the pitch of these arrays (about one wavelength), the first grating lobes.  The head
 therefore predicts the complex amplitudes a_j of five analytic carriers c_j -- the ideal plane
-wave, the two edge waves and the grating lobes m = -1, +1, whose phases are computed in double-float
-arithmetic from the geometry -- and the field is  p = scale * sum_j a_j c_j.  What is left to learn
-is a set of slowly varying amplitudes.
+wave, the two edge waves and the grating lobes m = -1, +1, whose phases are computed from the
+geometry in FP64 (training) or double-float arithmetic (inference) -- and the field is
+p = scale * sum_j a_j c_j.  What is left to learn is a set of slowly varying amplitudes.
 
 Training runs entirely in libfsgb300's tcgen05 kernels (fsg_mlp_train_*): a step gathers its
 rows on the device, runs forward and backward on the tensor cores, reduces the weight
