@@ -131,19 +131,41 @@ constexpr int kMaxCarriers = 5;
 constexpr int kAux = 12;  // floats per training row: carriers c_0..c_4, target y (complex)
 
 struct Carriers {
-  float2 c[kMaxCarriers];
+  float2 c[kMaxCarriers], lo[kMaxCarriers];  // (re, im) and what FP32 leaves of them
 };
 
-// exp(2 pi i k path), k in cycles per metre, both double-float: the whole cycles drop out exactly.
-__device__ __forceinline__ float2 df_cis_cycles(dfl k, dfl path) {
+// exp(2 pi i k path), k in cycles per metre, both double-float: the whole cycles drop out exactly, and
+// the rest is taken to the nearest quarter cycle, |theta| <= pi / 4, for the Taylor series of sine and
+// cosine, whose leading terms are kept double-float; the angle's FP32 remainder tl (below 1e-4) enters to
+// first order.  Error about 1e-8.
+__device__ __forceinline__ void df_cis_cycles(dfl k, dfl path, float2* c, float2* lo) {
   const float p = __fmul_rn(k.hi, path.hi);
   float e = fmaf(k.hi, path.hi, -p);
   e = fmaf(k.hi, path.lo, e);
   e = fmaf(k.lo, path.hi, e);
-  const float x = __fadd_rn(__fsub_rn(p, rintf(p)), e);
-  float s, c;
-  sincospif(2.0f * x, &s, &c);
-  return make_float2(c, s);
+  const float x = __fsub_rn(p, rintf(p)), q = rintf(4.0f * x);
+  const float t = fmaf(-0.25f, q, x);  // exact
+  const float th = __fmul_rn(kTwoPiHi, t);
+  const float tl = fmaf(kTwoPiHi, e, fmaf(kTwoPiLo, t, fmaf(kTwoPiHi, t, -th)));
+  const float u = __fmul_rn(th, th), ul = fmaf(th, th, -u);
+  float ps = fmaf(u, -1.0f / 39916800.0f, 1.0f / 362880.0f);
+  ps = fmaf(u, ps, -1.0f / 5040.0f);
+  ps = fmaf(u, ps, 1.0f / 120.0f);
+  ps = fmaf(u, ps, -1.0f / 6.0f);
+  float pc = fmaf(u, 1.0f / 479001600.0f, -1.0f / 3628800.0f);
+  pc = fmaf(u, pc, 1.0f / 40320.0f);
+  pc = fmaf(u, pc, -1.0f / 720.0f);
+  pc = fmaf(u, pc, 1.0f / 24.0f);
+  const float ds = __fmul_rn(__fmul_rn(th, u), ps), dc = fmaf(__fmul_rn(u, u), pc, -0.5f * ul), cu = -0.5f * u;
+  const float s0 = __fadd_rn(th, ds), c0 = __fadd_rn(1.0f, __fadd_rn(cu, dc));
+  const dfl sn = two_sum(th, fmaf(c0, tl, ds));
+  dfl cs = fast_two_sum(1.0f, cu);
+  cs = fast_two_sum(cs.hi, __fadd_rn(cs.lo, fmaf(-s0, tl, dc)));
+  const int quarter = (int)q & 3;
+  const bool swap = quarter & 1;
+  const float sr = quarter == 1 || quarter == 2 ? -1.0f : 1.0f, si = quarter >= 2 ? -1.0f : 1.0f;
+  *c = make_float2(sr * (swap ? sn.hi : cs.hi), si * (swap ? cs.hi : sn.hi));
+  *lo = make_float2(sr * (swap ? sn.lo : cs.lo), si * (swap ? cs.lo : sn.lo));
 }
 
 // What a thread needs of the domain beside its fields: reciprocals, formed in FP64 on the host.
@@ -206,8 +228,10 @@ __device__ __forceinline__ Carriers surrogate_carriers(const DomainArgs& D, doub
   }
   Carriers out;
 #pragma unroll
-  for (int j = 0; j < kMaxCarriers; ++j)
-    out.c[j] = (on[j] && j < d.n_carriers) ? df_cis_cycles(kc, df_add(path[j], first)) : make_float2(0.f, 0.f);
+  for (int j = 0; j < kMaxCarriers; ++j) {
+    df_cis_cycles(kc, df_add(path[j], first), &out.c[j], &out.lo[j]);
+    if (!on[j] || j >= d.n_carriers) out.c[j] = out.lo[j] = make_float2(0.f, 0.f);
+  }
   return out;
 }
 
@@ -269,19 +293,19 @@ __global__ void surrogate_combine_kernel(const __grid_constant__ DomainArgs D, c
   const float* o = net + (size_t)i * 2 * D.d.n_carriers;
   // FP32 products with their errors carried along: the sum rounds once
   dfl re = {0.f, 0.f}, im = {0.f, 0.f};
-  auto add = [](dfl& s, float a, float b) {
+  auto add = [](dfl& s, float a, float b, float b_lo) {
     const float p = __fmul_rn(a, b);
     const dfl t = two_sum(s.hi, p);
-    s = dfl{t.hi, __fadd_rn(s.lo, __fadd_rn(t.lo, fmaf(a, b, -p)))};
+    s = dfl{t.hi, __fadd_rn(s.lo, __fadd_rn(t.lo, fmaf(a, b_lo, fmaf(a, b, -p))))};
   };
 #pragma unroll
   for (int j = 0; j < kMaxCarriers; ++j) {
     if (j < D.d.n_carriers) {
       const float ar = o[2 * j], ai = o[2 * j + 1];
-      add(re, ar, c.c[j].x);
-      add(re, -ai, c.c[j].y);
-      add(im, ar, c.c[j].y);
-      add(im, ai, c.c[j].x);
+      add(re, ar, c.c[j].x, c.lo[j].x);
+      add(re, -ai, c.c[j].y, c.lo[j].y);
+      add(im, ar, c.c[j].y, c.lo[j].y);
+      add(im, ai, c.c[j].x, c.lo[j].x);
     }
   }
   out[i] = make_float2((float)(((double)re.hi + (double)re.lo) * scale), (float)(((double)im.hi + (double)im.lo) * scale));

@@ -9,7 +9,7 @@ import numpy as np
 import pytest
 
 from tests import _golden as G
-from tests._gpu import require_gpu
+from tests._gpu import np64, require_gpu, torch
 
 pytestmark = pytest.mark.gpu
 
@@ -39,3 +39,24 @@ def test_training_step_keeps_its_bits(sur):
     for i, (w, b) in enumerate(zip(gW, gb)):
         assert G.rel_l2(w.double().cpu().numpy() @ np.cos(np.arange(w.shape[1])), ref[f"w{i}"]) < 1e-7, f"w{i}"
         assert G.rel_l2(b.cpu().numpy(), ref[f"b{i}"]) < 1e-7, f"b{i}"
+
+
+def test_carriers_of_the_prediction(sur):
+    """The field from one unit amplitude is the carrier itself: within FP32's half ulp below one (2^-25 in
+    each part) and 1e-8 for the phase and the series, and in the norm within the rounding's uniform error
+    (2.1e-8 for uniform angles) and 0.4e-8."""
+    import oracle.mlp_fp64 as M
+
+    q = sur.sample_domain(20000, seed=6)
+    ref = M.carriers(q.cpu().numpy(), sur.params.n_elements, sur.params.pitch, sur.medium.speed_of_sound)
+    for j in range(5):
+        for part in (0, 1):
+            net = torch.zeros(q.shape[0], 10, device=q.device)
+            net[:, 2 * j + part] = 1.0
+            out = torch.empty(q.shape[0], dtype=torch.complex64, device=q.device)
+            assert sur.lib.fsg_surrogate_combine(sur.domain, q.data_ptr(), q.shape[0], net.data_ptr(), 1.0,
+                                                 out.data_ptr(), sur._stream()) == 0
+            want = ref[:, j] * (1j if part else 1)
+            got = np64(out)
+            assert np.max(np.abs(got - want)) < np.sqrt(2) * (2.0**-25 + 1e-8)
+            assert G.rel_l2(got, want) < 2.5e-8
