@@ -116,7 +116,8 @@ def rf2iq(rf, fs: float, fc: float, B: float | None = None, tau: float = 0.0) ->
     initial conditions), run on the GPU as cascaded second-order sections in FP32.
 
     ``rf``: ``(n_samples, n_channels)`` or ``(n_frames, n_samples, n_channels)``, NumPy or
-    torch; returns complex64 of the same shape on the GPU."""
+    torch; returns complex64 of the same shape on the GPU.  Many short records are filtered in another
+    order of operations than few (the last bits of a record depend on how many there are)."""
     device = _device.pick_device(rf)
     x = rf if isinstance(rf, torch.Tensor) else torch.as_tensor(np.asarray(rf))
     x = x.to(device=device, dtype=torch.float32)

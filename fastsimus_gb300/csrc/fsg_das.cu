@@ -3,15 +3,16 @@
 // rf2iq / dasmtx algorithms, which the reference's validation tests call through PyMUST
 // (tests/_picmus_phantom_shared.py:407-460).
 //
-// rf2iq_kernel: one warp per (frame, channel) column, eight channels of a frame per CTA.  The IIR
+// rf2iq_kernel: one warp per (frame, channel) column, eight consecutive columns per CTA.  The IIR
 // filter (cascaded second-order sections in FP32; a single high-order recursion loses ~1e-3 in FP32
 // at narrow cut-offs, the cascade stays at ~1e-6) is linear in its state, so a segment of a column is
 // cut into 32 chunks, one per lane: every lane filters its chunk from a zero state, the chunk-end
 // states are combined by a scan over the lanes with the powers of the chunk's state transition
 // M = A^L (computed in FP64 on the host), and every lane filters its chunk again from its true state.
 // The same is done backward.  The down-mixed samples and the forward outputs stay in shared memory
-// (records longer than a segment go through the output array between the two passes).  The
-// down-mixing phasors depend on the sample only: each CTA tabulates them per segment.
+// (records longer than a segment go through the output array between the two passes).
+// The down-mixing phasors depend on the sample only: each CTA tabulates them per segment.
+// rf2iq_column_kernel: one thread per column, for many short records.
 //
 // das_kernel: one thread per pixel, looping over groups of firings and, per element, over the
 // group's firings.  The transmit delays (times c) and the element frames sit in shared memory;
@@ -41,6 +42,7 @@ constexpr int kDasImgBlocks = 7;      // das_kernel CTAs per SM the registers ar
 constexpr int kIqCh = 8;          // channels per CTA, one warp each
 constexpr int kIqMaxL = 71;       // samples per lane and segment: eight columns and the phasors fit shared memory
 constexpr int kIqScan = 5;        // scan levels: M, M^2, M^4, M^8, M^16
+constexpr int kIqColThreads = 64, kIqColMax = 320;  // rf2iq_column_kernel: threads, longest record
 
 struct Rf2IqArgs {
   const float* rf;   // [n_frames][n_samples][n_ch]
@@ -146,65 +148,71 @@ __device__ __forceinline__ void iir_segment(const Rf2IqArgs& A, float2* x, int d
   __syncwarp();
 }
 
-// What bounds it: the length of a lane's chunk, four filter passes of N / 32 samples (the former
-// kernel's one thread per column walked 2 N), and the column's bytes.  One frame of 64 channels x
-// 1,015 samples 172 -> see below us, 75 frames x 64 x 1,080 187 us -> .
+// What bounds it: the length of a lane's chunk, four filter passes of N / 32 samples, and with many columns
+// issue.  Eight columns of the call per CTA, whatever their frames: 153,600 columns of one channel and 1,000
+// samples 8,400 us with a CTA per frame, now 1,593 (2,614 with a thread per column and all its host work).
+// Calls, a thread per column -> now: 9,600 columns of 1,000 samples 514 -> 118 us (490 of it once on the host),
+// 115,200 of 2,400 6,151 -> 2,693.
 template <int NS>
 __global__ void __launch_bounds__(32 * kIqCh) rf2iq_kernel(const __grid_constant__ Rf2IqArgs A) {
   extern __shared__ __align__(16) float2 iq_sm[];
   __shared__ float2 right[kIqCh][FSG_RF2IQ_MAX_PAD];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int N = A.n_samples, P = A.pad, S = 32 * A.L, pitch = S + 4;  // pitch = 4 mod 16: staging writes conflict-free
-  const int groups = (A.n_ch + kIqCh - 1) / kIqCh;
-  const int fr = blockIdx.x / groups, ch0 = (blockIdx.x % groups) * kIqCh, ch = ch0 + warp;
-  const bool active = ch < A.n_ch;
-  const float* __restrict__ rf = A.rf + (size_t)fr * N * A.n_ch;
+  const int64_t cols = (int64_t)A.n_frames * A.n_ch, c0 = (int64_t)blockIdx.x * kIqCh, cid = c0 + warp;
+  const bool active = cid < cols;
+  auto column = [&](int64_t c) { return A.rf + (size_t)(c / A.n_ch) * N * A.n_ch + c % A.n_ch; };
   float2* ph = iq_sm + kIqCh * pitch;   // the segment's phasors
   float2* col = iq_sm + warp * pitch;   // this warp's samples of the segment
-  float2* __restrict__ y = A.iq + ((size_t)fr * A.n_ch + ch) * N;
+  float2* __restrict__ y = A.iq + cid * N;
   const int n_seg = (N + S - 1) / S;
-  auto mixed = [&](int n) {
-    const float v = rf[(size_t)n * A.n_ch + ch];
-    const float2 e = phasor(A, n);
-    return make_float2(v * e.x, v * e.y);
-  };
+  // the staging threads: channels side by side, or samples where there are fewer than eight
+  const int st_c = A.n_ch < kIqCh ? warp : threadIdx.x & (kIqCh - 1), st_j = A.n_ch < kIqCh ? lane : threadIdx.x / kIqCh;
+  const float* __restrict__ st_rf = c0 + st_c < cols ? column(c0 + st_c) : nullptr;
 
   float2 z[NS][2];
   // forward pass over [2 x0 - x[P..1], x[0..N-1], 2 x[N-1] - x[N-2..N-1-P]]
-  if (active) {
-    const float2 x0 = mixed(0);
-    // lanes hold the left extension, broadcast in turn
-    float2 e = make_float2(0.f, 0.f);
-    for (int k = 0; k < P; ++k) {
-      if ((k & 31) == 0) {
-        const float2 v = mixed(max(0, P - k - lane));
-        e = make_float2(2.f * x0.x - v.x, 2.f * x0.y - v.y);
-      }
-      const float2 v = make_float2(__shfl_sync(0xffffffffu, e.x, k & 31), __shfl_sync(0xffffffffu, e.y, k & 31));
-      if (k == 0) iir_init<NS>(A, z, v);
-      iir_step<NS>(A, z, v);
-    }
-    if (P == 0) iir_init<NS>(A, z, x0);
-  }
   for (int g = 0; g < n_seg; ++g) {
     const int n0 = g * S, n = min(S, N - n0);
     __syncthreads();
     for (int j = threadIdx.x; j < n; j += blockDim.x) ph[j] = phasor(A, n0 + j);
     __syncthreads();
-    {
-      const int c = threadIdx.x & (kIqCh - 1);
-      if (ch0 + c < A.n_ch) {
-        const float* src = rf + (size_t)n0 * A.n_ch + ch0 + c;
+    if (st_rf) {
+      const float* src = st_rf + (size_t)n0 * A.n_ch;
 #pragma unroll 4
-        for (int j = threadIdx.x / kIqCh; j < n; j += 32) {
-          const float v = src[(size_t)j * A.n_ch];
-          const float2 e = ph[j];
-          iq_sm[c * pitch + j] = make_float2(v * e.x, v * e.y);
-        }
+      for (int j = st_j; j < n; j += 32) {
+        const float v = src[(size_t)j * A.n_ch];
+        const float2 e = ph[j];
+        iq_sm[st_c * pitch + j] = make_float2(v * e.x, v * e.y);
       }
     }
     __syncthreads();
     if (active) {
+      if (g == 0) {  // (a segment that is not the last is longer than the pad)
+        const float2 x0 = col[0];
+        for (int k = 0; k < P; ++k) {
+          const float2 v = col[P - k], e = make_float2(2.f * x0.x - v.x, 2.f * x0.y - v.y);
+          if (k == 0) iir_init<NS>(A, z, e);
+          iir_step<NS>(A, z, e);
+        }
+        if (P == 0) iir_init<NS>(A, z, x0);
+      }
+      if (g == n_seg - 1) {
+        if (lane < P) {  // the right extension, of samples before they are filtered
+          const float2 xn = col[n - 1];
+          const int m = N - 2 - lane;
+          float2 v;
+          if (m >= n0) {
+            v = col[m - n0];
+          } else {  // in the segment before
+            const float r = column(cid)[(size_t)m * A.n_ch];
+            const float2 e = phasor(A, m);
+            v = make_float2(r * e.x, r * e.y);
+          }
+          right[warp][lane] = make_float2(2.f * xn.x - v.x, 2.f * xn.y - v.y);
+        }
+        __syncwarp();
+      }
       iir_segment<NS>(A, col, 1, n, z, 1.f);
       if (n_seg > 1)
         for (int j = lane; j < n; j += 32) y[n0 + j] = col[j];
@@ -212,14 +220,10 @@ __global__ void __launch_bounds__(32 * kIqCh) rf2iq_kernel(const __grid_constant
   }
   if (!active) return;
   {
-    const float2 xn = mixed(N - 1);
-    float2 e = make_float2(0.f, 0.f), o = e;
+    float2 o = make_float2(0.f, 0.f);
     for (int k = 0; k < P; ++k) {
-      if ((k & 31) == 0) {
-        const float2 v = mixed(max(0, N - 2 - k - lane));
-        e = make_float2(2.f * xn.x - v.x, 2.f * xn.y - v.y);
-      }
-      o = iir_step<NS>(A, z, make_float2(__shfl_sync(0xffffffffu, e.x, k & 31), __shfl_sync(0xffffffffu, e.y, k & 31)));
+      o = iir_step<NS>(A, z, right[warp][k]);
+      __syncwarp();
       if (lane == 0) right[warp][k] = o;
     }
     __syncwarp();
@@ -236,6 +240,63 @@ __global__ void __launch_bounds__(32 * kIqCh) rf2iq_kernel(const __grid_constant
     }
     iir_segment<NS>(A, col + n - 1, -1, n, z, 2.f);
     for (int j = lane; j < n; j += 32) y[n0 + j] = col[j];
+  }
+}
+
+// One thread per column, its recurrence from end to end; the phasors of the whole record in shared memory
+// and a chunk's samples requested before they are filtered.  What bounds it: the chain of the recurrence, 0.16 us per
+// sample, up to about 100,000 columns (all resident); beyond, the lines of A.iq that a warp's 32 columns touch.
+constexpr int kIqColChunk = 16;
+template <int NS>
+__global__ void __launch_bounds__(kIqColThreads) rf2iq_column_kernel(const __grid_constant__ Rf2IqArgs A) {
+  __shared__ float2 ph[kIqColMax];
+  const int N = A.n_samples, P = A.pad;
+  for (int j = threadIdx.x; j < N; j += blockDim.x) ph[j] = phasor(A, j);
+  __syncthreads();
+  const int64_t cid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (cid >= (int64_t)A.n_frames * A.n_ch) return;
+  const float* __restrict__ col = A.rf + (size_t)(cid / A.n_ch) * N * A.n_ch + cid % A.n_ch;
+  float2* __restrict__ y = A.iq + cid * N;
+  auto mixed = [&](int n) {
+    const float v = col[(size_t)n * A.n_ch];
+    return make_float2(v * ph[n].x, v * ph[n].y);
+  };
+  float2 z[NS][2], right[FSG_RF2IQ_MAX_PAD];
+  const float2 x0 = mixed(0), xn = mixed(N - 1);
+  iir_init<NS>(A, z, x0);
+  for (int k = 0; k < P; ++k) {
+    const float2 v = mixed(P - k), e = make_float2(2.f * x0.x - v.x, 2.f * x0.y - v.y);
+    if (k == 0) iir_init<NS>(A, z, e);
+    iir_step<NS>(A, z, e);
+  }
+  for (int m0 = 0; m0 < N; m0 += kIqColChunk) {
+    float v[kIqColChunk];
+#pragma unroll
+    for (int j = 0; j < kIqColChunk; ++j) v[j] = m0 + j < N ? col[(size_t)(m0 + j) * A.n_ch] : 0.f;
+#pragma unroll
+    for (int j = 0; j < kIqColChunk; ++j)
+      if (m0 + j < N) {
+        const float2 e = ph[m0 + j];
+        y[m0 + j] = iir_step<NS>(A, z, make_float2(v[j] * e.x, v[j] * e.y));
+      }
+  }
+  for (int k = 0; k < P; ++k) {
+    const float2 v = mixed(N - 2 - k);
+    right[k] = iir_step<NS>(A, z, make_float2(2.f * xn.x - v.x, 2.f * xn.y - v.y));
+  }
+  // backward pass, started from the last forward output
+  iir_init<NS>(A, z, P > 0 ? right[P - 1] : y[N - 1]);
+  for (int k = P - 1; k >= 0; --k) iir_step<NS>(A, z, right[k]);
+  for (int n1 = N - 1; n1 >= 0; n1 -= kIqColChunk) {
+    float2 w[kIqColChunk];
+#pragma unroll
+    for (int j = 0; j < kIqColChunk; ++j) w[j] = n1 - j >= 0 ? y[n1 - j] : make_float2(0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < kIqColChunk; ++j)
+      if (n1 - j >= 0) {
+        const float2 o = iir_step<NS>(A, z, w[j]);
+        y[n1 - j] = make_float2(2.f * o.x, 2.f * o.y);
+      }
   }
 }
 
@@ -512,6 +573,15 @@ __global__ void __launch_bounds__(kDasThreads) dasmtx_kernel(const __grid_consta
 
 using namespace fsg;
 
+// Whether the columns of a call are many and short enough for a thread each: the recurrence takes
+// 0.16 us a sample however many columns run beside it, the scan of short chunks about 0.005 us a column.
+// Calls (scan, thread each): 38,400 columns of 64 samples 164 us, 45; of 300 samples 213, 155; 9,600 of 300
+// 61, 52; 307,200 of 300 1,577, 1,408.  From 384 samples on the scan is ahead (38,400 columns 225, 261;
+// 115,200 639, 1,212).
+static bool rf2iq_by_column(int n_samples, int64_t cols) {
+  return n_samples <= kIqColMax && cols >= 28 * (int64_t)n_samples;
+}
+
 extern "C" int32_t fsg_rf2iq(const float* rf, int32_t n_frames, int32_t n_samples, int32_t n_channels, double fs,
                              double fc, double tau, int32_t n_sections, const double* sos, const double* zi,
                              int32_t pad, void* iq_out, void* stream) {
@@ -576,23 +646,26 @@ extern "C" int32_t fsg_rf2iq(const float* rf, int32_t n_frames, int32_t n_sample
       memcpy(m, sq, sizeof(m));
     }
   }
-  const int64_t grid64 = (int64_t)n_frames * ((n_channels + kIqCh - 1) / kIqCh);
+  const int64_t cols = (int64_t)n_frames * n_channels;
+  const bool by_column = rf2iq_by_column(n_samples, cols);
+  const int per_cta = by_column ? kIqColThreads : kIqCh, threads = by_column ? kIqColThreads : 32 * kIqCh;
+  const int64_t grid64 = (cols + per_cta - 1) / per_cta;
   if (grid64 > INT32_MAX) return set_error(FSG_EUNSUPPORTED, "%lld channel groups exceed the grid", (long long)grid64);
   const unsigned grid = (unsigned)grid64;
-  const size_t smem = ((size_t)kIqCh * (32 * A.L + 4) + 32 * A.L) * sizeof(float2);
+  const size_t smem = by_column ? 0 : ((size_t)kIqCh * (32 * A.L + 4) + 32 * A.L) * sizeof(float2);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   auto launch = [&](auto kernel) {
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    kernel<<<grid, 32 * kIqCh, smem, s>>>(A);
+    kernel<<<grid, threads, smem, s>>>(A);
     return cudaGetLastError();
   };
   cudaError_t e;
   switch (n_sections) {
-    case 1: e = launch(rf2iq_kernel<1>); break;
-    case 2: e = launch(rf2iq_kernel<2>); break;
-    case 3: e = launch(rf2iq_kernel<3>); break;
-    default: e = launch(rf2iq_kernel<4>); break;
+    case 1: e = by_column ? launch(rf2iq_column_kernel<1>) : launch(rf2iq_kernel<1>); break;
+    case 2: e = by_column ? launch(rf2iq_column_kernel<2>) : launch(rf2iq_kernel<2>); break;
+    case 3: e = by_column ? launch(rf2iq_column_kernel<3>) : launch(rf2iq_kernel<3>); break;
+    default: e = by_column ? launch(rf2iq_column_kernel<4>) : launch(rf2iq_kernel<4>); break;
   }
   return check_cuda(e, "rf2iq_kernel launch");
 }
