@@ -6,11 +6,11 @@
 // rf2iq_kernel: one warp per (frame, channel) column, eight consecutive columns per CTA.  The IIR
 // filter (cascaded second-order sections in FP32; a single high-order recursion loses ~1e-3 in FP32
 // at narrow cut-offs, the cascade stays at ~1e-6) is linear in its state, so a segment of a column is
-// cut into 32 chunks, one per lane: every lane filters its chunk from a zero state, the chunk-end
-// states are combined by a scan over the lanes with the powers of the chunk's state transition
-// M = A^L (computed in FP64 on the host), and every lane filters its chunk again from its true state.
-// The same is done backward.  The down-mixed samples and the forward outputs stay in shared memory
-// (records longer than a segment go through the output array between the two passes).
+// cut into 32 chunks, one per lane: every lane filters its chunk from a zero state (the first from the
+// true one), the chunk-end states are combined by a scan over the lanes with the powers of the chunk's
+// state transition M = A^L (computed in FP64 on the host), and every lane filters its chunk again from
+// its true state.  The same is done backward.  The down-mixed samples and the forward outputs stay in
+// shared memory (records longer than a segment go through the output array between the two passes).
 // The down-mixing phasors depend on the sample only: each CTA tabulates them per segment.
 // rf2iq_column_kernel: one thread per column, for many short records.
 //
@@ -53,7 +53,10 @@ struct Rf2IqArgs {
   float sos[FSG_RF2IQ_MAX_SECTIONS][5];  // b0, b1, b2, a1, a2
   float zi[FSG_RF2IQ_MAX_SECTIONS][2];   // steady state for a unit input
   int L;                                 // samples per lane and segment (odd)
-  float m[kIqScan][2 * FSG_RF2IQ_MAX_SECTIONS][2 * FSG_RF2IQ_MAX_SECTIONS];  // A^(L 2^k): state after from state before
+  int levels, compensated;               // scan levels whose power is not negligible; bit k: level k's sums compensated
+  // A^(L 2^k): state after from state before, FP32 and what it leaves
+  float m[kIqScan][2 * FSG_RF2IQ_MAX_SECTIONS][2 * FSG_RF2IQ_MAX_SECTIONS];
+  float m_lo[kIqScan][2 * FSG_RF2IQ_MAX_SECTIONS][2 * FSG_RF2IQ_MAX_SECTIONS];
 };
 
 // Down-mixing phasor of sample n: exp(-2 pi i (n fc / fs + fc tau)), the phase reduced to
@@ -88,20 +91,43 @@ __device__ __forceinline__ void iir_init(const Rf2IqArgs& A, float2 (*z)[2], flo
     for (int k = 0; k < 2; ++k) z[s][k] = make_float2(A.zi[s][k] * x0.x, A.zi[s][k] * x0.y);
 }
 
-// Adds the state that `from` becomes after A^(L 2^k).
+// Adds the state that `from` becomes after A^(L 2^k).  Where little is left of it the sum rounds once; else the
+// products and sums are compensated, since the powers of a narrow filter reach 10^6 and cancel.  Error of the
+// forward pass with one plain FP32 sum, the serial recursion, and so: 2.1e-5, 1.2e-5, 0.7e-5 at a cut-off
+// of 0.01 of Nyquist and 1,015 samples; 7.8e-8, 6.2e-8, 6.2e-8 at 0.5 and 64 samples.
+constexpr double kIqPlainMax = 1.0 / 4.0;
 template <int NS>
 __device__ __forceinline__ void iir_carry(const Rf2IqArgs& A, int k, float2 (*z)[2], const float2 (*from)[2]) {
+  if (A.compensated >> k & 1) {
 #pragma unroll
-  for (int i = 0; i < 2 * NS; ++i) {
-    float2 s = z[i >> 1][i & 1];
+    for (int i = 0; i < 2 * NS; ++i) {
+      float2 s = z[i >> 1][i & 1], lo = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int j = 0; j < 2 * NS; ++j) {
-      if ((j >> 1) > (i >> 1)) continue;  // a section is driven by the ones before it only
-      const float c = A.m[k][i][j];
-      s.x = fmaf(c, from[j >> 1][j & 1].x, s.x);
-      s.y = fmaf(c, from[j >> 1][j & 1].y, s.y);
+      for (int j = 0; j < 2 * NS; ++j) {
+        if ((j >> 1) > (i >> 1)) continue;  // a section is driven by the ones before it only
+        const float c = A.m[k][i][j], cl = A.m_lo[k][i][j];
+        const float2 f = from[j >> 1][j & 1];
+        const float2 p = make_float2(__fmul_rn(c, f.x), __fmul_rn(c, f.y));
+        const dfl x = two_sum(s.x, p.x), y = two_sum(s.y, p.y);
+        s = make_float2(x.hi, y.hi);
+        lo.x = __fadd_rn(lo.x, fmaf(cl, f.x, __fadd_rn(x.lo, fmaf(c, f.x, -p.x))));
+        lo.y = __fadd_rn(lo.y, fmaf(cl, f.y, __fadd_rn(y.lo, fmaf(c, f.y, -p.y))));
+      }
+      z[i >> 1][i & 1] = make_float2(__fadd_rn(s.x, lo.x), __fadd_rn(s.y, lo.y));
     }
-    z[i >> 1][i & 1] = s;
+  } else {
+#pragma unroll
+    for (int i = 0; i < 2 * NS; ++i) {
+      float2 t = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int j = 0; j < 2 * NS; ++j) {
+        if ((j >> 1) > (i >> 1)) continue;
+        const float c = A.m[k][i][j];
+        t.x = fmaf(c, from[j >> 1][j & 1].x, t.x);
+        t.y = fmaf(c, from[j >> 1][j & 1].y, t.y);
+      }
+      z[i >> 1][i & 1] = cadd(z[i >> 1][i & 1], t);
+    }
   }
 }
 
@@ -114,12 +140,15 @@ __device__ __forceinline__ void iir_segment(const Rf2IqArgs& A, float2* x, int d
   const int i0 = lane * L, cnt = max(0, min(L, n - i0));
   float2 s[NS][2];
 #pragma unroll
-  for (int q = 0; q < NS; ++q) s[q][0] = s[q][1] = make_float2(0.f, 0.f);
+  for (int q = 0; q < 2 * NS; ++q) s[q >> 1][q & 1] = lane == 0 ? z[q >> 1][q & 1] : make_float2(0.f, 0.f);
   for (int i = 0; i < cnt; ++i) iir_step<NS>(A, s, x[(i0 + i) * dir]);
-  // inclusive scan of the chunk-end states, the incoming state entering through lane 0
-  if (lane == 0) iir_carry<NS>(A, 0, s, z);
+  // inclusive scan of the chunk-end states; one that is not finite reaches every later chunk
+  float sum = 0.f;
 #pragma unroll
-  for (int k = 0; k < kIqScan; ++k) {
+  for (int q = 0; q < 2 * NS; ++q) sum += fabsf(s[q >> 1][q & 1].x) + fabsf(s[q >> 1][q & 1].y);
+  const int levels = __any_sync(0xffffffffu, !(sum <= 3.402823466e38f)) ? kIqScan : A.levels;
+#pragma unroll 1
+  for (int k = 0; k < levels; ++k) {
     float2 f[NS][2];
 #pragma unroll
     for (int q = 0; q < 2 * NS; ++q) {
@@ -634,9 +663,22 @@ extern "C" int32_t fsg_rf2iq(const float* rf, int32_t n_frames, int32_t n_sample
       for (int i = 0; i < ns2; ++i) m[i][j] = z[i / 2][i % 2];
     }
     memset(A.m, 0, sizeof(A.m));
+    memset(A.m_lo, 0, sizeof(A.m_lo));
+    A.levels = kIqScan;
+    A.compensated = 0;
     for (int k = 0; k < kIqScan; ++k) {
+      double top = 0.0;
       for (int i = 0; i < ns2; ++i)
-        for (int j = 0; j < ns2; ++j) A.m[k][i][j] = (float)m[i][j];
+        for (int j = 0; j < ns2; ++j) {
+          A.m[k][i][j] = (float)m[i][j];
+          A.m_lo[k][i][j] = (float)(m[i][j] - (double)A.m[k][i][j]);
+          if (!(fabs(m[i][j]) <= top)) top = fabs(m[i][j]);
+        }
+      if (top < 1e-16) {  // nothing of a state is left after the chunks of this level
+        A.levels = k;
+        break;
+      }
+      if (!(top <= kIqPlainMax)) A.compensated |= 1 << k;
       for (int i = 0; i < ns2; ++i)
         for (int j = 0; j < ns2; ++j) {
           double s = 0.0;
