@@ -84,6 +84,8 @@ __device__ __forceinline__ void store_a8(unsigned char* sm, int r, int k, const 
 constexpr int kMlpWorkers = 512, kMlpBlock = kMlpWorkers + 64;
 constexpr int kMlpPiecesPerTile = (kMlpFeat + 3 * kMlpWidth) / kMlpPieceK;
 
+// kWide: the queries start on a 16-byte boundary and are read as such words; else float by float.
+template <bool kWide>
 __global__ void __launch_bounds__(kMlpBlock, 1) mlp_tc_forward_kernel(const __grid_constant__ FsgMlpWeights W,
                                                                        const float* __restrict__ u, int64_t n,
                                                                        float* __restrict__ out, int* status) {
@@ -222,7 +224,10 @@ __global__ void __launch_bounds__(kMlpBlock, 1) mlp_tc_forward_kernel(const __gr
     auto features = [&](int64_t tile, int blk) {
       const int64_t q = tile * kMlpRows + row;
       float4 uv = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (q < n) uv = *reinterpret_cast<const float4*>(u + 4 * q);
+      if (q < n) {
+        if constexpr (kWide) uv = *reinterpret_cast<const float4*>(u + 4 * q);
+        else uv = make_float4(u[4 * q], u[4 * q + 1], u[4 * q + 2], u[4 * q + 3]);
+      }
       float sv[8], cv[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
@@ -384,11 +389,11 @@ extern "C" int32_t fsg_mlp_tc_forward(const FsgMlpWeights* weights, const float*
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return check_cuda(e, "device query");
-  e = cudaFuncSetAttribute(mlp_tc_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMlpSmem);
+  const auto kernel = (reinterpret_cast<uintptr_t>(u) & 15) == 0 ? mlp_tc_forward_kernel<true> : mlp_tc_forward_kernel<false>;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMlpSmem);
   if (e != cudaSuccess) return check_cuda(e, "cudaFuncSetAttribute(mlp_tc_forward_kernel)");
   const int64_t tiles = (n + kMlpRows - 1) / kMlpRows;
   const int grid = (int)(tiles < sms ? tiles : sms);
-  mlp_tc_forward_kernel<<<grid, kMlpBlock, kMlpSmem, reinterpret_cast<cudaStream_t>(stream_ptr)>>>(*weights, u, n, out,
-                                                                                               status);
+  kernel<<<grid, kMlpBlock, kMlpSmem, reinterpret_cast<cudaStream_t>(stream_ptr)>>>(*weights, u, n, out, status);
   return check_cuda(cudaGetLastError(), "mlp_tc_forward_kernel launch");
 }

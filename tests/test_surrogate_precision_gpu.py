@@ -60,3 +60,14 @@ def test_carriers_of_the_prediction(sur):
             got = np64(out)
             assert np.max(np.abs(got - want)) < np.sqrt(2) * (2.0**-25 + 1e-8)
             assert G.rel_l2(got, want) < 2.5e-8
+
+
+@pytest.mark.parametrize("offset", [1, 2, 3])
+def test_forward_of_queries_at_any_float(sur, offset):
+    """A contiguous view need not start on a 16-byte boundary: the same bits as from an aligned copy."""
+    u, _ = sur.inputs(sur.sample_domain(300, seed=8), with_aux=False)
+    store = torch.empty(4 * 300 + 4, device=u.device)
+    view = store[offset:offset + 4 * 300].view(300, 4)
+    view.copy_(u)
+    assert view.is_contiguous() and view.data_ptr() % 16 == 4 * offset
+    assert torch.equal(sur.forward_tc(view), sur.forward_tc(u)) and sur.tc_status() == 0
