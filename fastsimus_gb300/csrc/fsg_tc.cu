@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_kernel(const __grid_constant__
   extern __shared__ __align__(1024) unsigned char sm[];
   __shared__ uint64_t mbar_tx, mbar_rx;
   __shared__ uint32_t tmem_holder;
-  __shared__ int s_item, s_fail;
+  __shared__ int s_item, s_fail, s_late;  // s_late: the barriers (1 TX, 2 RX) whose phase thread 0 has not seen done
   __shared__ float rcs[2][kTcT];
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_kernel(const __grid_constant__
     tc::mbar_init(&mbar_tx, 1);
     tc::mbar_init(&mbar_rx, 1);
     tc::fence_mbar_init();
-    s_fail = 0;
+    s_fail = s_late = 0;
   }
   if (warp == 0) tc::tmem_alloc(&tmem_holder, kTmemCols);
   tc::fence_before_sync();
@@ -179,8 +179,13 @@ __global__ void __launch_bounds__(kThreads, 1) tc_kernel(const __grid_constant__
   const uint32_t trow = tmem + ((uint32_t)(32 * q) << 16);
 
   auto wait = [&](uint64_t* mb, uint32_t& ph) {
-    if (!tc::mbar_test(mb, ph) && !s_fail && !tc::mbar_wait_bounded(mb, ph, kWaitTries)) s_fail = 1;
-    ph ^= 1u;
+    const bool done = tc::phase_pass(ph, [&](uint32_t parity) {
+      return tc::mbar_test(mb, parity) || (!s_fail && tc::mbar_wait_bounded(mb, parity, kWaitTries));
+    });
+    if (!done) {
+      s_fail = 1;
+      if (tid == 0) s_late |= mb == &mbar_tx ? 1 : 2;
+    }
     __syncwarp();
   };
   auto meet = [&]() {
@@ -442,12 +447,12 @@ __global__ void __launch_bounds__(kThreads, 1) tc_kernel(const __grid_constant__
       }
     }
   }
-  // ---- release TMEM (after a wait that gave up: once what is still in flight has had its bounded time) ----
+  // ---- release TMEM (after a wait that gave up: once the phase it waited for is done or has had its time) ----
   tc::fence_before_sync();
   __syncthreads();
   if (s_fail && tid == 0) {
-    tc::mbar_wait_bounded(&mbar_tx, ph_tx, kWaitTries);
-    tc::mbar_wait_bounded(&mbar_rx, ph_rx, kWaitTries);
+    if (s_late & 1) tc::mbar_wait_bounded(&mbar_tx, ph_tx, kWaitTries);
+    if (s_late & 2) tc::mbar_wait_bounded(&mbar_rx, ph_rx, kWaitTries);
     atomicExch(A.status, FSG_ETIMEOUT);
   }
   __syncthreads();

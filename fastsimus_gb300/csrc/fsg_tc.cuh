@@ -102,6 +102,15 @@ __device__ __forceinline__ uint64_t global_ns() {
 
 constexpr uint64_t kMaxWaitNs = 2000000000ull;  // a wait gives up after 2 s, whatever max_tries
 
+// One wait for the phase of `parity`: done(parity) says whether it has completed.  Only then does the
+// parity move on; after a wait that gave up it still names the phase that is outstanding.
+template <class Done>
+__host__ __device__ __forceinline__ bool phase_pass(uint32_t& parity, Done done) {
+  const bool ok = done(parity);
+  if (ok) parity ^= 1u;
+  return ok;
+}
+
 // Bounded wait: returns false if the phase did not complete within `max_tries` polls or
 // kMaxWaitNs nanoseconds of the global timer, whichever comes first.
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* mbar, uint32_t parity, uint32_t max_tries) {
