@@ -168,6 +168,21 @@ def _pixels(x, z, device):
     return torch.as_tensor(np.ascontiguousarray(pix), device=device), xa.shape
 
 
+# From here on the pixels' coordinates are interleaved on the device (an upload each and a kernel, 54 to
+# 73 us for up to 131,072 pixels) instead of on the host (one upload: 19 us for 1,000 pixels, 37 for 10,000,
+# 55 for 20,000, 85 for 40,000, 295 for 131,072).
+INTERLEAVE_ON_DEVICE = 20_000
+
+
+def _interleaved(x: np.ndarray, z: np.ndarray, device) -> torch.Tensor:
+    """(n, 2) float64 pixels in the grids' own order: neighbours of a row read neighbouring samples."""
+    if x.size >= INTERLEAVE_ON_DEVICE:
+        return torch.stack([torch.as_tensor(np.ascontiguousarray(a).reshape(-1), device=device) for a in (x, z)], dim=1)
+    pix = np.empty((x.size, 2))
+    pix[:, 0], pix[:, 1] = x.reshape(-1), z.reshape(-1)
+    return torch.as_tensor(pix, device=device)
+
+
 def _from_fortran(flat: torch.Tensor, shape) -> torch.Tensor:
     if len(shape) <= 1:
         return flat.reshape(shape)
@@ -236,8 +251,7 @@ def das(iq, x, z, delays, param, method: str = "linear") -> torch.Tensor:
     xa, za = np.asarray(x, dtype=np.float64), np.asarray(z, dtype=np.float64)
     if xa.shape != za.shape:
         raise ValueError(f"x and z must have the same shape, got {xa.shape} and {za.shape}")
-    # pixels in the grids' own order: neighbours of a row read neighbouring samples
-    pix = torch.stack([torch.as_tensor(np.ascontiguousarray(a).reshape(-1), device=device) for a in (xa, za)], dim=1)
+    pix = _interleaved(xa, za, device)
     out = torch.empty(pix.shape[0], dtype=torch.complex64, device=device)
     _native.check(_native.load().fsg_das(ctypes.byref(probe), ctypes.byref(p), cm.data_ptr(), nf, ns, txd.data_ptr(),
                                          pix.data_ptr(), pix.shape[0], out.data_ptr(),
