@@ -195,36 +195,6 @@ void convex_geometry(const FsgProbe* p, int* convex, double* apex, double* radiu
   }
 }
 
-// Padding between the sub-element planes of the geometry arrays that minimises shared-memory
-// bank conflicts of the transmit accesses: lane l of a warp touches source g + GN i of tile
-// point l / GN (g = l % GN), i.e. word u * plane + e * pitch + point.  Ties go to the smaller
-// pad; the receive reads (consecutive elements, stride pitch) are conflict-free for any pad.
-static int choose_plane_pad(int E, int U, int gn, int st) {
-  const int pitch = st + 1;
-  int best_pad = 0, best_cost = 1 << 30;
-  for (int pad = 0; pad < 32; ++pad) {
-    const int plane = E * pitch + pad;
-    int cost = 0;
-    for (int i = 0; i < kSrcPerThread; ++i) {
-      int count[32] = {0};
-      int worst = 0;
-      for (int l = 0; l < 32; ++l) {
-        const int g = l % gn, pt = l / gn, src = g + gn * i;
-        if (src >= E * U) continue;
-        const int word = (src % U) * plane + (src / U) * pitch + pt;
-        const int c = ++count[word % 32];
-        if (c > worst) worst = c;
-      }
-      cost += worst;
-    }
-    if (cost < best_cost) {
-      best_cost = cost;
-      best_pad = pad;
-    }
-  }
-  return best_pad;
-}
-
 // Geometry cache per chunk: sized to stay resident in the 129 MB L2 while every band's CTAs read it
 // (200,000 scatterers x 128 elements: 26.37 ms at 48 MiB, 26.11 at 80, 26.00 at 112: fewer chunks,
 // fewer launches and tails).
@@ -248,7 +218,20 @@ static int simus_grid(int n_bands, int64_t chunk_tiles, int num_sms) {
 // (16 source slots per lane; one, two, four or eight per element for U = 1, 2, 3-4, 5-8), with
 // bands of kTxAnchor frequencies, else of kAnchor, such that the shared memory fits.
 constexpr int kBandCost = 6;
-static bool sweep_shape(int E, int U, int F, int64_t tiles_of_points, int num_sms, int ffd, SweepConfig* c) {
+
+// The plane pads found in one call, by lanes per point: they depend on neither the frequencies, the
+// workspace nor the directivity, for which a call sets up several configurations.
+struct PlanePads {
+  int found[33];
+  PlanePads() { for (int& p : found) p = -1; }
+  int operator()(int E, int U, int gn, int st) {
+    if (found[gn] < 0) found[gn] = choose_plane_pad(E, U, gn, st);
+    return found[gn];
+  }
+};
+
+static bool sweep_shape(int E, int U, int F, int64_t tiles_of_points, int num_sms, int ffd, PlanePads& pads,
+                        SweepConfig* c) {
   if (U < 1 || U > 8) return false;
   if (E > 32 && U <= 4) {
     const int nw = (E + 63) / 64, threads = lane_threads(nw, ffd != 0), groups = threads / (32 * nw);
@@ -287,7 +270,7 @@ static bool sweep_shape(int E, int U, int F, int64_t tiles_of_points, int num_sm
     for (int gn = 4; gn <= 32; gn *= 2) {
       if (gn * epl < E) continue;
       const int st = kThreads / gn;
-      const int pad = choose_plane_pad(E, U, gn, st);
+      const int pad = pads(E, U, gn, st);
       const StashLayout L = stash_layout(st, fb, E, U, pad, ffd != 0);
       if (L.total > kMaxDynSmem - 1024) continue;
       c->kind = 1;
@@ -313,11 +296,11 @@ static bool sweep_shape(int E, int U, int F, int64_t tiles_of_points, int num_sm
 // chunk size: a band's ct units hold fewer than ceil(grid / n_bands) CTA starts besides its
 // first unit's CTA.
 // short_bands: the lane kernel's bands of kAnchor frequencies, whose slots take the least memory.
-SweepConfig simus_config(int E, int U, int F, int64_t n_scat, int num_sms, size_t cache_budget, int ffd,
+SweepConfig simus_config(int E, int U, int F, int64_t n_scat, int num_sms, size_t cache_budget, int ffd, PlanePads& pads,
                          bool short_bands = false) {
   SweepConfig c;
   memset(&c, 0, sizeof(c));
-  if (!sweep_shape(E, U, F, n_scat, num_sms, ffd, &c)) return c;  // kind 0
+  if (!sweep_shape(E, U, F, n_scat, num_sms, ffd, pads, &c)) return c;  // kind 0
   if (short_bands && c.kind == 2 && c.fb > kAnchor) {
     c.fb = kAnchor;
     c.smem = lane_layout(c.nw, c.fb, lane_threads(c.nw, ffd != 0), ffd != 0).total;
@@ -384,9 +367,10 @@ static size_t simus_ws_size(const SweepConfig& c, int E, int U, int F) {
 static size_t simus_ws_size(const FsgProbe* probe, const FsgFreqPlan* plan, int64_t n_scat, int num_sms) {
   size_t need = 0;
   const int E = probe->n_elements, U = probe->n_sub, F = plan->n_freq;
+  PlanePads pads;
   for (int ffd = 0; ffd < 2; ++ffd) {
-    SweepConfig c = simus_config(E, U, F, n_scat, num_sms, kGeoCacheBudget, ffd);
-    const int slots = simus_config(E, U, F, 0, num_sms, 0, ffd).n_slices;
+    SweepConfig c = simus_config(E, U, F, n_scat, num_sms, kGeoCacheBudget, ffd, pads);
+    const int slots = simus_config(E, U, F, 0, num_sms, 0, ffd, pads).n_slices;
     if (slots > c.n_slices) c.n_slices = slots;
     const size_t n = simus_ws_size(c, E, U, F);
     if (n > need) need = n;
@@ -400,14 +384,15 @@ static size_t simus_ws_size(const FsgProbe* probe, const FsgFreqPlan* plan, int6
 // smallest.  *grid_cap: the CTAs that the slots allow.
 static bool simus_fit(int E, int U, int F, int64_t n_scat, int num_sms, int ffd, size_t bytes, SweepConfig* c,
                       int* grid_cap) {
+  PlanePads pads;
   *grid_cap = num_sms;
-  *c = simus_config(E, U, F, n_scat, num_sms, kGeoCacheBudget, ffd);
+  *c = simus_config(E, U, F, n_scat, num_sms, kGeoCacheBudget, ffd, pads);
   if (c->kind == 0 || simus_ws_size(*c, E, U, F) <= bytes) return true;
   for (int cut = 0; cut < 2; ++cut) {
-    *c = simus_config(E, U, F, n_scat, num_sms, 0, ffd, cut != 0);
+    *c = simus_config(E, U, F, n_scat, num_sms, 0, ffd, pads, cut != 0);
     const size_t fixed = simus_ws_size(*c, E, U, F) - align256(c->geo_bytes);
     if (bytes >= fixed + align256(c->geo_bytes)) {
-      *c = simus_config(E, U, F, n_scat, num_sms, (bytes - fixed) & ~size_t(255), ffd, cut != 0);
+      *c = simus_config(E, U, F, n_scat, num_sms, (bytes - fixed) & ~size_t(255), ffd, pads, cut != 0);
       return true;
     }
   }
@@ -436,7 +421,9 @@ extern "C" int32_t fsg_simus_launches(const FsgProbe* probe, const FsgFreqPlan* 
   if (!probe || !plan || probe->n_elements < 1 || probe->n_sub < 1 || plan->n_freq < 1 || n_scat < 0) return -1;
   int sms = 0;
   if (device_sm_count(&sms) != FSG_OK) return -1;
-  const SweepConfig c = simus_config(probe->n_elements, probe->n_sub, plan->n_freq, n_scat, sms, kGeoCacheBudget, ffd);
+  PlanePads pads;
+  const SweepConfig c =
+      simus_config(probe->n_elements, probe->n_sub, plan->n_freq, n_scat, sms, kGeoCacheBudget, ffd, pads);
   return 2 + (n_scat > 0 ? (int32_t)(2 * c.n_chunks) : 0);  // setup_tables, per chunk geometry + band, simus_reduce
 }
 
