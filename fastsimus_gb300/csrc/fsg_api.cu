@@ -118,9 +118,17 @@ SweepConst make_sweep_const(const FsgProbe* p, const FsgMedium* m, const FsgFreq
 
 static size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 
-// The shortest band of a sweep: the anchor tables hold a row per band.  simus_lane_kernel's largest
-// band is 24 to 52 frequencies, whatever the probe (lane_layout).
+// The shortest band of a sweep: the anchor tables hold a row per band.  It fits simus_lane_kernel's shared
+// memory for every probe, and so does no band longer than 28 (384 threads) or 44 (256) frequencies.
 constexpr int kMinBand = 24;
+constexpr bool lane_band_fits(int fb) {
+  for (int nw = 1; nw <= kThreads / 64; ++nw)
+    for (int ffd = 0; ffd < 2; ++ffd)
+      if (lane_layout(nw, fb, lane_threads(nw, ffd != 0), ffd != 0).total > kMaxDynSmem - 1024) return false;
+  return true;
+}
+static_assert(lane_band_fits(kMinBand), "every probe's sweep takes bands of kMinBand frequencies");
+static_assert(kMinBand % 8 == 0, "whole sub-blocks of 4 and 8 frequencies");
 
 size_t tables_bytes(int E, int U, int F) {
   const int n_src = E * U;
@@ -232,7 +240,7 @@ struct PlanePads {
 
 static bool sweep_shape(int E, int U, int F, int64_t tiles_of_points, int num_sms, int ffd, PlanePads& pads,
                         SweepConfig* c) {
-  if (U < 1 || U > 8) return false;
+  if (U < 1 || U > 8 || E > kThreads) return false;
   if (E > 32 && U <= 4) {
     const int nw = (E + 63) / 64, threads = lane_threads(nw, ffd != 0), groups = threads / (32 * nw);
     const int fs = 16 / lane_points(U);
@@ -295,14 +303,14 @@ static bool sweep_shape(int E, int U, int F, int64_t tiles_of_points, int num_sm
 // bounds the number of CTAs that share a band (the partial-spectrum slots per band) for any
 // chunk size: a band's ct units hold fewer than ceil(grid / n_bands) CTA starts besides its
 // first unit's CTA.
-// short_bands: the lane kernel's bands of kAnchor frequencies, whose slots take the least memory.
+// short_bands: the lane kernel's bands of kMinBand frequencies at most, whose slots take the least memory.
 SweepConfig simus_config(int E, int U, int F, int64_t n_scat, int num_sms, size_t cache_budget, int ffd, PlanePads& pads,
                          bool short_bands = false) {
   SweepConfig c;
   memset(&c, 0, sizeof(c));
   if (!sweep_shape(E, U, F, n_scat, num_sms, ffd, pads, &c)) return c;  // kind 0
-  if (short_bands && c.kind == 2 && c.fb > kAnchor) {
-    c.fb = kAnchor;
+  if (short_bands && c.kind == 2 && c.fb > kMinBand) {
+    c.fb = kMinBand;
     c.smem = lane_layout(c.nw, c.fb, lane_threads(c.nw, ffd != 0), ffd != 0).total;
   }
   c.n_bands = (F + c.fb - 1) / c.fb;
@@ -379,7 +387,7 @@ static size_t simus_ws_size(const FsgProbe* probe, const FsgFreqPlan* plan, int6
 }
 
 // The sweep of a request within a workspace of `bytes`: the default shape, in smaller chunks of
-// scatterers if its geometry cache does not fit; else bands of kAnchor frequencies; else also
+// scatterers if its geometry cache does not fit; else bands of kMinBand frequencies; else also
 // fewer CTAs, down to one slot per band beyond the first.  False when nothing fits; c is then the
 // smallest.  *grid_cap: the CTAs that the slots allow.
 static bool simus_fit(int E, int U, int F, int64_t n_scat, int num_sms, int ffd, size_t bytes, SweepConfig* c,

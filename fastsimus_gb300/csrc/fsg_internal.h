@@ -85,7 +85,7 @@ struct SmemLayout {
   size_t geo_bytes;    // the geometry arrays, contiguous from offset 0
 };
 
-__host__ __device__ inline size_t align16(size_t v) { return (v + 15) & ~size_t(15); }
+__host__ __device__ constexpr size_t align16(size_t v) { return (v + 15) & ~size_t(15); }
 
 // With ffd, a fifth geometry array holds half_seg * sin(theta) per (source, point).
 __host__ __device__ inline SmemLayout smem_layout(int st, int E, int U, int plane_pad, bool ffd) {
@@ -203,8 +203,8 @@ constexpr int kLaneTrPitch = 18;  // complex per lane row of the transpose buffe
 struct LaneLayout {
   size_t off_pp, off_kb, off_part, off_w, off_tr, total;
 };
-__host__ __device__ inline LaneLayout lane_layout(int nw, int fb, int threads, bool ffd) {
-  LaneLayout S;
+__host__ __device__ constexpr LaneLayout lane_layout(int nw, int fb, int threads, bool ffd) {
+  LaneLayout S{};
   size_t o = (size_t)fb * threads * 16;
   S.off_pp = o; o = align16(o + (size_t)fb * 8);
   S.off_kb = o; o = align16(o + (ffd ? (size_t)fb * 4 : 0));

@@ -11,7 +11,7 @@ cudaError_t launch_simus_lane(int U, const SweepConfig& c, const BandArgs& A, cu
 // lane_block order: a block's threads take consecutive (group, pair, thread) slots of one tile, two
 // elements each, so every store of a warp is contiguous.  gridDim.y CTAs share a tile's slots.
 __global__ void __launch_bounds__(kThreads) lane_geometry_kernel(const BandArgs A, int64_t chunk_tiles) {
-  __shared__ float4 xz[kThreads];  // st <= 32 points of the tile
+  __shared__ float4 xz[kThreads];  // st <= 48 points of the tile
   const int T = 32 * A.nw, PPT = lane_points(A.U), NP = A.U * PPT;
   const int n_grp = A.st / PPT, slots = n_grp * NP * T;
   for (int64_t tile = blockIdx.x; tile < chunk_tiles; tile += gridDim.x) {
