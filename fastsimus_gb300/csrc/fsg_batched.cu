@@ -390,9 +390,6 @@ __global__ void __launch_bounds__(kThreads) batched_geometry_kernel(const __grid
   const BatchPhantom& P = A.ph[blockIdx.y];
   const int n_src = A.E * A.U;
   const int spb = n_src >= kThreads ? 1 : kThreads / n_src;
-  SweepConst C = A.C;
-  C.dkc = P.dkc;
-  C.dalpha = P.dalpha;
   for (int64_t s0 = (int64_t)blockIdx.x * spb; s0 < P.n_scat; s0 += (int64_t)gridDim.x * spb) {
     __syncthreads();
     if (threadIdx.x < spb && s0 + threadIdx.x < P.n_scat) {
@@ -406,9 +403,9 @@ __global__ void __launch_bounds__(kThreads) batched_geometry_kernel(const __grid
       const int64_t s = s0 + sl;
       if (s >= P.n_scat) continue;
       const float4 c = xz[sl];
-      const SrcGeo g = source_geometry(dfl{c.x, c.y}, dfl{c.z, c.w}, A.src_pos[src], A.rot_e[src / A.U], C);
+      const SrcGeo g = source_geometry(dfl{c.x, c.y}, dfl{c.z, c.w}, A.src_pos[src], A.rot_e[src / A.U], A.C);
       const int64_t rec = (P.geo0 + s) * (int64_t)n_src + src;
-      A.geo[rec] = make_float4(g.r_hi, g.r_lo, g.amp, C.half_seg * g.sth);
+      A.geo[rec] = make_float4(g.r_hi, g.r_lo, g.amp, A.C.half_seg * g.sth);
     }
   }
 }
@@ -492,7 +489,7 @@ int plan_layout(const FsgProbe* probe, const FsgPhantom* ph, int n_ph, int n_tx,
   int64_t chunk = (tu && tu->chunk_scatterers > 0) ? tu->chunk_scatterers : 32768;
   // at most that many scatterers per item, and as many items as keep the SMs evenly loaded to the end:
   // sixteen per SM, of not less than kMinChunk scatterers (an item sets up its transmit matrices and
-  // writes a partial spectrum of 80 x 64 complex per frequency)
+  // writes a partial spectrum of 40 or 80 x 64 or 128 complex per frequency)
   {
     int64_t work = 0;
     for (int p = 0; p < n_ph; ++p) work += (int64_t)((ph[p].plan.n_freq + L->fb - 1) / L->fb) * ph[p].n_scat;
@@ -652,11 +649,6 @@ static int32_t simus_batched_impl(const FsgProbe* probe, const FsgMedium* medium
     b.f0 = q.plan.freq_start;
     b.df = q.plan.freq_step;
     b.corr = (float)q.plan.correction_factor;
-    {
-      const SweepConst cp = make_sweep_const(probe, medium, &q.plan, 0);
-      b.dkc = cp.dkc;
-      b.dalpha = cp.dalpha;
-    }
     b.pulse_src = q.plan.pulse_spectrum;
     b.probe_src = q.plan.probe_spectrum;
     unsigned char* tb = ws + L.off_tab[p];

@@ -21,9 +21,8 @@ struct BatchPhantom {
   int n_freq, n_freq_full, freq_idx_start, n_bands, n_chunks, item0;
   double f0, df;
   float corr;
-  float dalpha;             // per-step attenuation of this phantom's plan (Np/m)
-  float2 dk;                // per-step wavenumber of this phantom's plan (double-float)
-  float2 dkc;               // the same in cycles per metre
+  float dalpha;             // tensor-core path: per-step attenuation of this phantom's plan (Np/m)
+  float2 dk;                // tensor-core path: per-step wavenumber of this phantom's plan (double-float)
   const double* pulse_src;  // plan pulse spectrum, complex128 [n_freq]
   const double* probe_src;  // plan probe spectrum, float64 [n_freq]
   float2* kf;               // workspace: k_f double-float

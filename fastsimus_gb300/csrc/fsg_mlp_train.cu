@@ -53,9 +53,9 @@ constexpr int kPart = kHO + 1;                        // per-tile partials: head
 // contiguous.  The kernels stream pieces of kPieceK columns through kBufs buffers.
 constexpr int kChunkK = 64;                           // K columns per packed chunk
 constexpr uint32_t kChunkBytes = kW * kChunkK * 2;    // 32 KB
-constexpr int kPieceK = 64;                           // K columns per streamed piece (32 or 64)
+constexpr int kPieceK = 64;                           // K columns per streamed piece: a whole chunk
 constexpr uint32_t kPieceBytes = kW * kPieceK * 2;    // 32 KB
-constexpr int kBufs = kPieceK == 32 ? 5 : 2;          // streamed pieces in shared memory
+constexpr int kBufs = 2;                              // streamed pieces in shared memory
 constexpr uint32_t kABytes = kRows * kW * 2;          // one BF16 copy of a 128 x 256 operand
 constexpr uint32_t kOffAHi = 0, kOffALo = kABytes, kOffB = 2 * kABytes;
 constexpr uint32_t kFbSmem = kOffB + kBufs * kPieceBytes;
@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(256, 1) mlp_train_fb_kernel(const __grid_const
     ph_mma ^= 1u;
     return true;
   };
-  // One GEMM of the tile on the tensor cores (warp 0): np pieces of 2 K-steps of 16.
+  // One GEMM of the tile on the tensor cores (warp 0): np pieces of four K-steps of 16.
   // Forward: D = A_hi W^T + A_lo W^T; backward: D = dZ W (dZ in the A_hi region).
   auto gemm = [&](int64_t piece0, int np, bool bwd) -> bool {
     for (int c = 0; c < np; ++c) {

@@ -74,8 +74,8 @@ __device__ __forceinline__ void stash_receive(const float2* __restrict__ stash, 
 // The sums are then reduced over the GN lanes: halving exchanges while a lane holds more than
 // one frequency, all-reduce over the lanes left sharing one.  On return v[r] (r < R) holds
 // the full sum of sub-block frequency R (g / SH) + r, SH = max(1, GN / FS) lanes holding each.
-// GUARD: the lanes' element slots may run past E (no stash write for those).
-template <int U, int GN, bool FFD, bool GUARD>
+// The lanes' element slots may run past E (no stash write for those).
+template <int U, int GN, bool FFD>
 __device__ __forceinline__ void stash_transmit(float2 (&Gr)[kSrcPerThread / 2], float2 (&Gi)[kSrcPerThread / 2],
                                                const float2 (&Sr)[kSrcPerThread / 2],
                                                const float2 (&Si)[kSrcPerThread / 2],
@@ -142,7 +142,7 @@ __device__ __forceinline__ void stash_transmit(float2 (&Gr)[kSrcPerThread / 2], 
         m = make_float2(tr.x + tr.y, ti.x + ti.y);
       }
       const int e = g + GN * k;
-      if (!GUARD || e < E) stash_row[j * ep + e] = m;
+      if (e < E) stash_row[j * ep + e] = m;
       v[j] = __ffma2_rn(m, make_float2(wk[k], wk[k]), v[j]);
     }
 #pragma unroll
@@ -293,8 +293,8 @@ __global__ void __launch_bounds__(kThreads, 1) simus_stash_kernel(const BandArgs
       for (int sb = 0; sb < fb / FS; ++sb) {
         // ---------------- transmit: FS recurrence steps, stash writes, source sums ----------------
         float2 v[FS];
-        stash_transmit<U, GN, FFD, true>(Gr, Gi, Sr, Si, Sn, Dh, wk, stash + sl * FS * ep, ep, g, E,
-                                         FFD ? kb + sb * FS : nullptr, v);
+        stash_transmit<U, GN, FFD>(Gr, Gi, Sr, Si, Sn, Dh, wk, stash + sl * FS * ep, ep, g, E,
+                                   FFD ? kb + sb * FS : nullptr, v);
         if (g % (GN >= FS ? GN / FS : 1) == 0) {
 #pragma unroll
           for (int r = 0; r < R; ++r) {
@@ -305,9 +305,7 @@ __global__ void __launch_bounds__(kThreads, 1) simus_stash_kernel(const BandArgs
         }
         __syncthreads();
         // ---------------- receive from the stash ----------------
-        if (E >= 128) {
-          stash_receive<ST, 4>(stash, W, Ys, E, ep, sb);
-        } else if (E >= 64) {
+        if (E >= 64) {
           stash_receive<ST, 2>(stash, W, Ys, E, ep, sb);
         } else {
           stash_receive<ST, 1>(stash, W, Ys, E, ep, sb);
