@@ -56,20 +56,8 @@ constexpr uint32_t kMlpWaitTries = 1u << 26;
 constexpr uint64_t kMlpDrainNs = 1000000;  // a copy or a layer's products take microseconds
 constexpr int kMlpMaxOut = 10;
 
-// SiLU z / (1 + 2^(-z log2 e)) of two values: the fast exponential and reciprocal, products and sums on the
-// packed FP32x2 pipe.  A few FP32 ulps from the training kernels' tc::sigmoid2, whose calls would cost
-// an eighth of this kernel (1,048,576 queries and the exact field 1,624 -> 1,758 us).
-__device__ __forceinline__ float2 mlp_silu2(float2 z) {
-  const float kMinusLog2e = -1.4426950408889634f;
-  const float2 t = __fmul2_rn(z, make_float2(kMinusLog2e, kMinusLog2e));
-  float2 e, r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.x) : "f"(t.x));
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.y) : "f"(t.y));
-  e = __fadd2_rn(e, make_float2(1.0f, 1.0f));
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(e.x));
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(e.y));
-  return __fmul2_rn(z, r);
-}
+// SiLU z * sigmoid(z) of two values, evaluated exactly as the training kernels evaluate it.
+__device__ __forceinline__ float2 mlp_silu2(float2 z) { return __fmul2_rn(z, tc::sigmoid2(z)); }
 
 // Writes 8 consecutive activations (row r, columns k..k+7) as hi and lo BF16 into the K-major
 // A operand.
