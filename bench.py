@@ -45,11 +45,11 @@ WORKLOAD = ("cfg2: 128-element linear array (pitch 0.30 mm, width 0.27 mm, fc 5.
             "c 1540 m/s, 0.5 dB/cm/MHz, 0-degree plane wave, 200,000 scatterers x in [-19,19] mm, "
             "z in [5,50] mm, rc N(0,1) with three 2 mm anechoic disks; + pfield on 256x512 grid")
 L2_FLUSH_BYTES = 512 << 20
-# DRAM bytes (read + write) of one simus_lane_kernel launch measured by ncu on a 9,000-scatterer
-# chunk of the benchmark frame's probe: the tile geometry blocks read once from HBM (then from L2
-# by the other bands' CTAs) plus the partial spectra.  The bench cannot run ncu;
-# the figure is refreshed from a capture whenever the kernel changes.
-BAND_KERNEL_DRAM_BYTES = 55_388_160 + 741_120
+# DRAM bytes (read + write) of one simus_lane_kernel launch measured by ncu on 22,896 scatterers, a whole
+# chunk of the benchmark frame: the chunk's 117 MB of tile geometry, which the bands' CTAs read about six
+# times from HBM and otherwise from L2, plus the partial spectra.  The bench cannot run ncu;
+# the figure is refreshed from a capture whenever the kernel or its chunks change.
+BAND_KERNEL_DRAM_BYTES = 702_517_760 + 3_962_624
 
 
 def _env_int(name, default):
@@ -458,7 +458,7 @@ def run_gpu_arm(args, rank, world):
                      "unit": "TFLOP/s", "frac": achieved / peak if peak else None,
                      "traffic": BAND_KERNEL_DRAM_BYTES, "traffic_unit": "bytes per sweep-kernel launch",
                      "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one simus_lane_kernel "
-                                       "launch on a 9,000-scatterer chunk of this frame's probe and plan",
+                                       "launch on a whole 22,896-scatterer chunk of this frame's probe and plan",
                      "peak_source": "measured in-run by fsg_fp32_fma_probe (FP32 FMA chains); MEASURED_PEAKS.json "
                                     "holds only HBM and bf16 tensor peaks",
                      "peak_theoretical": fp32_theoretical_tflops(device),
