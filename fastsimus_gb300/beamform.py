@@ -231,7 +231,8 @@ def das(iq, x, z, delays, param, method: str = "linear") -> torch.Tensor:
     TXdelay = delays[f]) @ iq_f.flatten(order="F")``, computed in one kernel without the
     matrices.  ``iq``: ``(n_samples, n_channels)`` or ``(n_frames, n_samples, n_channels)``
     (complex I/Q or real RF); ``delays``: ``(n_channels,)`` or ``(n_frames, n_channels)``.
-    Returns complex64 of x's shape."""
+    Returns complex64 of x's shape.  Images of few pixels and many firings sum the firings in another
+    order (the last bits of a pixel depend on the size of its image)."""
     device = _device.pick_device(iq)
     t = iq if isinstance(iq, torch.Tensor) else torch.as_tensor(np.asarray(iq))
     t = t.to(device)

@@ -203,9 +203,10 @@ void convex_geometry(const FsgProbe* p, int* convex, double* apex, double* radiu
   }
 }
 
-// Geometry cache per chunk: sized to stay resident in the 129 MB L2 while every band's CTAs read it
-// (200,000 scatterers x 128 elements: 26.37 ms at 48 MiB, 26.11 at 80, 26.00 at 112: fewer chunks,
-// fewer launches and tails).
+// Geometry cache per chunk: about the 129 MB of L2.  Not all of it stays there while every band's CTAs read
+// it (a chunk of 22,896 scatterers x 128 elements reads its 117 MB six times from DRAM, 0.26 TB/s, which the
+// sweep does not notice), and larger chunks have fewer launches and tails (200,000 scatterers x 128 elements:
+// 26.37 ms at 48 MiB, 26.11 at 80, 26.00 at 112).
 constexpr size_t kGeoCacheBudget = size_t(112) << 20;
 
 // Grid of one simus chunk: every (band, tile) unit is one CTA's work at most.

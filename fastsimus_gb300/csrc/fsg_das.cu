@@ -430,8 +430,8 @@ __device__ __forceinline__ float das_floor(float s, int* i) {
   return r - (float)down;
 }
 
-// sqrt(d2) from one reciprocal root: s = d2 y plus the residual (d2 - s^2) y / 2, within an ulp (the
-// correctly rounded root takes three times the instructions).
+// sqrt(d2) from one reciprocal root: s = d2 y plus the residual (d2 - s^2) y / 2, within an ulp.  Images of
+// 1 to 25 firings are as far from 64 bits as with correctly rounded roots (2.5e-5 to 1.3e-3, within 0.5%).
 __device__ __forceinline__ float das_sqrt(float d2) {
   const float y = rsqrt_normal(fmaxf(d2, 1.17549435e-38f)), s = d2 * y;
   return fmaf(0.5f * y, fmaf(-s, s, d2), s);
@@ -781,8 +781,7 @@ extern "C" int32_t fsg_das(const FsgProbe* probe, const FsgDasParams* params, co
   const unsigned grid = (unsigned)((n_pixels * A.slices + kDasImgThreads - 1) / kDasImgThreads);
   size_t smem = (size_t)group * kDasStage * A.E * sizeof(float);
   if (smem < kDasImgThreads * sizeof(float2)) smem = kDasImgThreads * sizeof(float2);
-  // (their own instantiations: with the slices in every kernel the 75-firing image takes 4% more)
-  // (their own instantiations: with the slices in every kernel the image of 131,072 pixels takes 4% more)
+  // (their own instantiations: with the slices in every kernel 75 firings of 131,072 pixels take 4% more)
   if (A.slices == 1) {
     if (lng) launch_das<4, true, false>(A, linear, grid, smem, s);
     else if (few) launch_das<4, false, false>(A, linear, grid, smem, s);

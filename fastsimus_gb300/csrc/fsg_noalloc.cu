@@ -27,7 +27,7 @@
 //     the device, the cached address is not valid.
 //   - All calls share the array and it keeps the last call's contents.  Every byte the sweep
 //     reads is written earlier in the same call (tables by the set-up kernel; the partial
-//     spectra are zeroed by the call, then accumulated by the band kernels; each tile's
+//     spectra are zeroed by the call, then accumulated by the sweep kernel; each tile's
 //     geometry block is written before it is read), so nothing has to start at zero.
 //   - Calls whose work overlaps on the GPU (different streams, or different host threads on
 //     one device) race on the shared scratch and corrupt each other's results; serialise them.

@@ -201,7 +201,7 @@ __device__ __forceinline__ dfl df_div(dfl a, dfl b) {
 // m = -1, +1 of the pitch, exp(i k (x sin th_m + z cos th_m - xmin)) with
 // sin th_m = sin th + m lambda / pitch, zero where |sin th_m| >= 1 (evanescent).  Everything but sin and
 // cos of theta is double-float: 1,048,576 samples of the combine kernel took 628 us with all of it in
-// FP64, 225 us with the edges, lambda / pitch and sin th_m in FP64, 108 us now.
+// FP64, 225 us with the edges, lambda / pitch and sin th_m in FP64, 110 us now.
 __device__ __forceinline__ Carriers surrogate_carriers(const DomainArgs& D, double x, double z, double f, double th) {
   const FsgSurrogateDomain& d = D.d;
   double st, ct;

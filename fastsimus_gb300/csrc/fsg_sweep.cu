@@ -1,6 +1,6 @@
 // Plain fused FP32 simus and pfield sweeps for GB300 (sm_103a): set-up tables, the geometry
-// pre-pass, the reductions and the launch dispatch.  The band kernels themselves are templates
-// in fsg_sweep_kernels.cuh.
+// pre-pass, the reductions and the launch dispatch.  The sweep kernels themselves are templates
+// in fsg_sweep_lane.cuh, fsg_sweep_stash.cuh and fsg_sweep_kernels.cuh (pfield).
 //
 // simus, per chunk of scatterers:
 //   geometry           once per (scatterer, source): double-float distance, amplitude
@@ -101,7 +101,7 @@ __global__ void setup_tables(SetupArgs a) {
 // takes one tile at a time: its scatterers' coordinates are split into double-float pairs
 // once, then thread i handles (source, point) items i, i + 256, ...; consecutive threads take
 // consecutive points, so the writes of a warp are contiguous.  Points past the end of the
-// scatterer list repeat the tile's first point (their rc is 0 in the band kernel).
+// scatterer list repeat the tile's first point (their rc is 0 in the sweep).
 __global__ void __launch_bounds__(kThreads) geometry_kernel(const BandArgs A, int64_t chunk_tiles) {
   __shared__ float4 xz[kThreads];  // st <= 64 points of the tile
   const SmemLayout L = smem_layout(A.st, A.E, A.U, A.plane_pad, A.C.ffd != 0);

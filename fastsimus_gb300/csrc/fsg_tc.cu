@@ -137,7 +137,7 @@ __device__ __forceinline__ uint32_t a_off(int s, int c, int e) {
 // pass's P is formed, behind one more barrier.
 //
 // What bounds it: the CUDA cores' part of a step (32 recurrences, the split and its stores and the
-// epilogue per thread, about 1,000 issue cycles), with the tensor pipe (768 cycles of MMAs at N = 64)
+// epilogue per thread, about 1,000 issue cycles), with the tensor pipe (24 MMAs of 50 cycles at N = 64)
 // under it.  The kernel before this one kept the Green's tile twice (once per product), exchanged P
 // through shared memory and met at seven barriers per step: 5,800 cycles a step at 31 firings.
 template <int U, int NC>

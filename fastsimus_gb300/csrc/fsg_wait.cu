@@ -1,5 +1,5 @@
-// Self-test of the bounded mbarrier wait that every sweep kernel relies on (simus band kernel,
-// tensor-core sweep, MLP forward): a wait whose phase never completes must give up, report
+// Self-test of the bounded mbarrier wait that the kernels with asynchronous copies and products rely on
+// (stash sweep, tensor-core sweep, MLP forward and training): a wait whose phase never completes must give up, report
 // FSG_ETIMEOUT through a status word and leave the context usable.  The kernel waits on a
 // barrier that nothing arrives on (or, as the control, on one it arrived on itself).
 

@@ -97,7 +97,7 @@ const char* fsg_last_error_string(void);
 size_t fsg_simus_workspace_size(const FsgProbe* probe, const FsgFreqPlan* plan, int64_t n_scat);
 
 /* Kernel launches one fsg_simus call makes with the default workspace (set-up, a geometry and a
- * band kernel per scatterer chunk, the reduction), or -1 for invalid arguments.  No counterpart
+ * sweep kernel per scatterer chunk, the reduction), or -1 for invalid arguments.  No counterpart
  * in the reference: a measurement aid. */
 int32_t fsg_simus_launches(const FsgProbe* probe, const FsgFreqPlan* plan, int64_t n_scat, int32_t ffd);
 
