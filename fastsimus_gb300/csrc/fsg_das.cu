@@ -3,7 +3,7 @@
 // rf2iq / dasmtx algorithms, which the reference's validation tests call through PyMUST
 // (tests/_picmus_phantom_shared.py:407-460).
 //
-// rf2iq_kernel: one warp per (frame, channel) column, eight consecutive columns per CTA.  The IIR
+// rf2iq_kernel: one warp per (frame, channel) column, up to eight consecutive columns per CTA.  The IIR
 // filter (cascaded second-order sections in FP32; a single high-order recursion loses ~1e-3 in FP32
 // at narrow cut-offs, the cascade stays at ~1e-6) is linear in its state, so a segment of a column is
 // cut into 32 chunks, one per lane: every lane filters its chunk from a zero state (the first from the
@@ -53,6 +53,7 @@ struct Rf2IqArgs {
   float sos[FSG_RF2IQ_MAX_SECTIONS][5];  // b0, b1, b2, a1, a2
   float zi[FSG_RF2IQ_MAX_SECTIONS][2];   // steady state for a unit input
   int L;                                 // samples per lane and segment (odd)
+  int per_cta;                           // columns per CTA: 1, 2, 4 or 8
   int levels, compensated;               // scan levels whose power is not negligible; bit k: level k's sums compensated
   // A^(L 2^k): state after from state before, FP32 and what it leaves
   float m[kIqScan][2 * FSG_RF2IQ_MAX_SECTIONS][2 * FSG_RF2IQ_MAX_SECTIONS];
@@ -188,15 +189,18 @@ __global__ void __launch_bounds__(32 * kIqCh) rf2iq_kernel(const __grid_constant
   __shared__ float2 right[kIqCh][FSG_RF2IQ_MAX_PAD];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int N = A.n_samples, P = A.pad, S = 32 * A.L, pitch = S + 4;  // pitch = 4 mod 16: staging writes conflict-free
-  const int64_t cols = (int64_t)A.n_frames * A.n_ch, c0 = (int64_t)blockIdx.x * kIqCh, cid = c0 + warp;
-  const bool active = cid < cols;
+  const int64_t cols = (int64_t)A.n_frames * A.n_ch, c0 = (int64_t)blockIdx.x * A.per_cta, cid = c0 + warp;
+  const bool active = warp < A.per_cta && cid < cols;
   auto column = [&](int64_t c) { return A.rf + (size_t)(c / A.n_ch) * N * A.n_ch + c % A.n_ch; };
-  float2* ph = iq_sm + kIqCh * pitch;   // the segment's phasors
-  float2* col = iq_sm + warp * pitch;   // this warp's samples of the segment
+  float2* ph = iq_sm + A.per_cta * pitch;  // the segment's phasors
+  float2* col = iq_sm + warp * pitch;      // this warp's samples of the segment
   float2* __restrict__ y = A.iq + cid * N;
   const int n_seg = (N + S - 1) / S;
   // the staging threads: channels side by side, or samples where there are fewer than eight
-  const int st_c = A.n_ch < kIqCh ? warp : threadIdx.x & (kIqCh - 1), st_j = A.n_ch < kIqCh ? lane : threadIdx.x / kIqCh;
+  const bool by_sample = A.n_ch < kIqCh;
+  const int st_c = (by_sample ? warp : threadIdx.x) & (A.per_cta - 1);
+  const int st_j = by_sample ? lane + 32 * (warp / A.per_cta) : threadIdx.x / kIqCh;
+  const int st_step = 32 * kIqCh / A.per_cta;
   const float* __restrict__ st_rf = c0 + st_c < cols ? column(c0 + st_c) : nullptr;
 
   float2 z[NS][2];
@@ -209,7 +213,7 @@ __global__ void __launch_bounds__(32 * kIqCh) rf2iq_kernel(const __grid_constant
     if (st_rf) {
       const float* src = st_rf + (size_t)n0 * A.n_ch;
 #pragma unroll 4
-      for (int j = st_j; j < n; j += 32) {
+      for (int j = st_j; j < n; j += st_step) {
         const float v = src[(size_t)j * A.n_ch];
         const float2 e = ph[j];
         iq_sm[st_c * pitch + j] = make_float2(v * e.x, v * e.y);
@@ -690,11 +694,18 @@ extern "C" int32_t fsg_rf2iq(const float* rf, int32_t n_frames, int32_t n_sample
   }
   const int64_t cols = (int64_t)n_frames * n_channels;
   const bool by_column = rf2iq_by_column(n_samples, cols);
-  const int per_cta = by_column ? kIqColThreads : kIqCh, threads = by_column ? kIqColThreads : 32 * kIqCh;
+  // few columns of fewer than eight channels are spread over the SMs (20 columns of 30,000 samples: on three
+  // SMs 390 us, on twenty 244; 200 of 5,000: on 25 73, on 100 49)
+  int sms = 0;
+  const int st = device_sm_count(&sms);
+  if (st != FSG_OK) return st;
+  A.per_cta = kIqCh;
+  while (n_channels < kIqCh && A.per_cta > 1 && cols <= (int64_t)sms * (A.per_cta / 2)) A.per_cta /= 2;
+  const int per_cta = by_column ? kIqColThreads : A.per_cta, threads = by_column ? kIqColThreads : 32 * kIqCh;
   const int64_t grid64 = (cols + per_cta - 1) / per_cta;
   if (grid64 > INT32_MAX) return set_error(FSG_EUNSUPPORTED, "%lld channel groups exceed the grid", (long long)grid64);
   const unsigned grid = (unsigned)grid64;
-  const size_t smem = by_column ? 0 : ((size_t)kIqCh * (32 * A.L + 4) + 32 * A.L) * sizeof(float2);
+  const size_t smem = by_column ? 0 : ((size_t)A.per_cta * (32 * A.L + 4) + 32 * A.L) * sizeof(float2);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   auto launch = [&](auto kernel) {
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -20,7 +20,8 @@ def _iq(rf, bw=None):
     return np64(rf2iq(torch.as_tensor(rf, device="cuda"), FS, FC, bw))
 
 
-@pytest.mark.parametrize("ns,nc,nf", [(1000, 1, 9), (33, 3, 5), (40, 5, 13), (2273, 2, 7), (5000, 1, 3),  # a warp per column
+@pytest.mark.parametrize("ns,nc,nf", [(1000, 1, 9), (33, 3, 5), (40, 5, 13), (2273, 2, 7), (5000, 1, 3),  # a warp per column,
+                                      (1000, 3, 50), (400, 3, 101), (700, 1, 609), (330, 7, 180),  # 1 to 8 per CTA
                                       (19, 64, 9), (64, 7, 300), (200, 1, 5700), (320, 8, 1121)])  # a thread per column
 def test_columns_of_several_frames(ns, nc, nf):
     """Every frame and channel ends up in its own place; FP32 cascade: relative L2 <= 2e-5, as for the
