@@ -1029,6 +1029,8 @@ int validate_train(const FsgMlpTrain* t) {
   if (t->n_out < 2 || t->n_out > kMaxOut || t->n_out % 2)
     return set_error(FSG_EUNSUPPORTED, "n_out must be even and in [2, %d] (got %d)", kMaxOut, t->n_out);
   if (t->n_data < 1 || !t->u || !t->aux) return set_error(FSG_EINVAL, "empty training set");
+  if ((reinterpret_cast<uintptr_t>(t->u) | reinterpret_cast<uintptr_t>(t->aux)) & 15)
+    return set_error(FSG_EINVAL, "u and aux must start on a 16-byte boundary (their rows are read as such words)");
   if (t->n_split < 1 || t->n_split > 64) return set_error(FSG_EINVAL, "n_split must be in [1, 64]");
   for (int l = 0; l < 4; ++l)
     if (!t->w[l] || !t->m_w[l] || !t->v_w[l] || !t->packed_fwd[l] || !t->b[l] || !t->m_b[l] || !t->v_b[l] ||

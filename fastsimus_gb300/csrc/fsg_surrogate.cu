@@ -400,6 +400,7 @@ extern "C" int32_t fsg_surrogate_inputs(const FsgSurrogateDomain* dom, const dou
   int st = validate_domain(dom);
   if (st != FSG_OK) return st;
   if (n < 0 || (n > 0 && (!samples || !u))) return set_error(FSG_EINVAL, "bad surrogate input arguments");
+  if (reinterpret_cast<uintptr_t>(u) & 15) return set_error(FSG_EINVAL, "u must start on a 16-byte boundary");
   if (n == 0) return FSG_OK;
   surrogate_inputs_kernel<<<(unsigned)((n + 255) / 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       domain_args(*dom), samples, n, static_cast<const float2*>(field), inv_scale, reinterpret_cast<float4*>(u), aux);

@@ -262,8 +262,8 @@ typedef struct FsgSurrogateDomain {
   int32_t n_carriers;             /* 1..5, in the order above */
 } FsgSurrogateDomain;
 
-/* samples: device [n][4] float64 (x, z, f, theta).  Writes u: [n][4] float32 (normalised) and,
- * if aux != NULL, aux: [n][12] float32 = c_0 .. c_4 (complex; zero beyond n_carriers),
+/* samples: device [n][4] float64 (x, z, f, theta).  Writes u: [n][4] float32 (normalised, 16-byte
+ * aligned) and, if aux != NULL, aux: [n][12] float32 = c_0 .. c_4 (complex; zero beyond n_carriers),
  * field * inv_scale (complex),
  * with field: device complex64 [n] (the exact transmit field, or NULL for zeros). */
 int32_t fsg_surrogate_inputs(const FsgSurrogateDomain* dom, const double* samples, int64_t n, const void* field,
@@ -287,8 +287,8 @@ int32_t fsg_surrogate_combine(const FsgSurrogateDomain* dom, const double* sampl
  * writes the packed copies from the FP32 weights and clears the workspace counters.
  */
 typedef struct FsgMlpTrain {
-  const float* u;                 /* [n_data][4] */
-  const float* aux;               /* [n_data][12] (fsg_surrogate_inputs) */
+  const float* u;                 /* [n_data][4], 16-byte aligned */
+  const float* aux;               /* [n_data][12] (fsg_surrogate_inputs), 16-byte aligned */
   int64_t n_data;
   uint64_t seed;
   const float* bmat;              /* [64][4] */
